@@ -110,6 +110,24 @@ int wkv7_fwd(const void* r, const void* w, const void* k, const void* v, const v
              int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* stream);
 
 /*
+ * Scratch for spreading the chains evenly over the SMs.  One CTA walks one (batch, head) chain; when B*H exceeds the
+ * number of resident CTAs the last round of chains is rarely full.  The *_ws calls below take wkv7_workspace_bytes()
+ * bytes of device scratch (16-byte aligned, contents overwritten, used by one call at a time) and cut chains at the
+ * boundaries of equal shares of work: results are bit for bit those of the plain calls, which leave every chain whole.
+ * A cut needs somewhere to keep the state in between: it is kept in sT, so sT must be given for it (otherwise, and with
+ * workspace null, the call is the plain one).
+ */
+size_t wkv7_workspace_bytes(void);
+int wkv7_fwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                const float* s0, void* y, float* sT, float* ckpt,
+                int64_t B, int64_t T, int64_t H, int64_t N,
+                int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
+int wkv7_attn_ln_fwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                        const void* g, const float* params, const float* s0, void* y, float* sT, float* ckpt,
+                        float eps, int64_t B, int64_t T, int64_t H, int64_t N,
+                        int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
+
+/*
  * WKV7 decode step(s): the recurrence itself, time step by time step, for generation after a prefill.
  * Restates the loop body of the reference's naive recurrence (wind_rwkv/rwkv7/time_mixer.py:13-15); the
  * reference has no kernel for it (its chunked kernels require T % 16 == 0, rwkv7_attn.py:22).  Same

@@ -80,6 +80,34 @@ int check_common(int64_t B, int64_t T, int64_t H, int64_t N, int64_t sb, int64_t
 
 }  // namespace
 
+namespace wkv7 {
+static int sm_count() {
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> cache[kMaxDevices];
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+    int n = cache[dev].load(std::memory_order_relaxed);
+    if (!n) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+        cache[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+WorkSplit plan_work(long long chains, long long per_chain, int per_sm, unsigned* flags) {
+    long long ctas = chains, per_cta = per_chain;
+    const long long slots = (long long)sm_count() * per_sm;
+    if (flags && slots > 0 && slots * sizeof(unsigned) <= WORK_FLAG_BYTES && chains > slots) {
+        ctas = slots;
+        per_cta = (chains * per_chain + slots - 1) / slots;
+        ctas = (chains * per_chain + per_cta - 1) / per_cta;  // no empty ranges
+    } else {
+        flags = nullptr;
+    }
+    return WorkSplit{(int)ctas, (int)per_cta, (int)per_chain, (int)(chains * per_chain), flags};
+}
+}  // namespace wkv7
+
 extern "C" {
 
 const char* wkv7_status_string(int status) {
@@ -146,7 +174,7 @@ int wkv7_peek_status(void) {
 static int fwd_common(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                       const void* g, const float* params, bool ln, float eps, const float* s0, void* y, float* sT,
                       float* ckpt, int64_t B, int64_t T, int64_t H, int64_t N, int64_t sb, int64_t st, int64_t sh,
-                      int io_dtype, void* stream) {
+                      int io_dtype, void* workspace, void* stream) {
     int rc = check_common(B, T, H, N, sb, st, sh, io_dtype);
     if (rc) return rc;
     if (B == 0 || H == 0) return WKV7_OK;
@@ -160,7 +188,7 @@ static int fwd_common(const void* r, const void* w, const void* k, const void* v
         return WKV7_OK;
     }
     if (!r || !w || !k || !v || !a || !b || !y || (ln && (!g || !params))) return WKV7_ERR_NULL;
-    const void* ptrs[] = {r, w, k, v, a, b, y, g, s0, sT, ckpt, params};
+    const void* ptrs[] = {r, w, k, v, a, b, y, g, s0, sT, ckpt, params, workspace};
     for (const void* p : ptrs)
         if (p && !aligned16(p)) return WKV7_ERR_ALIGN;
     wkv7::FwdParams p{};
@@ -169,6 +197,7 @@ static int fwd_common(const void* r, const void* w, const void* k, const void* v
     p.B = B; p.T = T; p.H = H;
     p.st = wkv7::Strides{sb, st, sh};
     p.eps = eps;
+    p.flags = (unsigned*)workspace;
     p.status = status_ptr();
     if (!p.status) return WKV7_ERR_LAUNCH;
     if (io_dtype == WKV7_BF16) {
@@ -182,7 +211,16 @@ int wkv7_fwd(const void* r, const void* w, const void* k, const void* v, const v
              const float* s0, void* y, float* sT, float* ckpt, int64_t B, int64_t T, int64_t H, int64_t N,
              int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* stream) {
     return fwd_common(r, w, k, v, a, b, nullptr, nullptr, false, 0.f, s0, y, sT, ckpt, B, T, H, N, stride_b, stride_t,
-                      stride_h, io_dtype, stream);
+                      stride_h, io_dtype, nullptr, stream);
+}
+
+size_t wkv7_workspace_bytes(void) { return wkv7::WORK_FLAG_BYTES; }
+
+int wkv7_fwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                const float* s0, void* y, float* sT, float* ckpt, int64_t B, int64_t T, int64_t H, int64_t N,
+                int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream) {
+    return fwd_common(r, w, k, v, a, b, nullptr, nullptr, false, 0.f, s0, y, sT, ckpt, B, T, H, N, stride_b, stride_t,
+                      stride_h, io_dtype, workspace, stream);
 }
 
 int wkv7_step(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* s0,
@@ -216,7 +254,15 @@ int wkv7_attn_ln_fwd(const void* r, const void* w, const void* k, const void* v,
                      int64_t B, int64_t T, int64_t H, int64_t N, int64_t stride_b, int64_t stride_t, int64_t stride_h,
                      int io_dtype, void* stream) {
     return fwd_common(r, w, k, v, a, b, g, params, true, eps, s0, y, sT, ckpt, B, T, H, N, stride_b, stride_t,
-                      stride_h, io_dtype, stream);
+                      stride_h, io_dtype, nullptr, stream);
+}
+
+int wkv7_attn_ln_fwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                        const void* g, const float* params, const float* s0, void* y, float* sT, float* ckpt, float eps,
+                        int64_t B, int64_t T, int64_t H, int64_t N, int64_t stride_b, int64_t stride_t, int64_t stride_h,
+                        int io_dtype, void* workspace, void* stream) {
+    return fwd_common(r, w, k, v, a, b, g, params, true, eps, s0, y, sT, ckpt, B, T, H, N, stride_b, stride_t,
+                      stride_h, io_dtype, workspace, stream);
 }
 
 static int bwd_common(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,

@@ -72,7 +72,7 @@ template <typename IoT, int PREC, bool LN> struct BwdSmem {
     alignas(16) float wq[L * OPS], wa[L * OPS], kwi[L * OPS], bwi[L * OPS];
     alignas(16) float cum[L * OPS];
     alignas(16) float lw[PREC == 3 ? L * OPS : 4];   // single-TF32 path derives it from cum
-    // The chunk's four 16x16 matrices AK, QK, AI, QB (matrix m, row r: row group 2m + r/8 of the record's 64-row operand
+    // The chunk's four 16x16 matrices AK, QK, AI^T, QB (matrix m, row r: row group 2m + r/8 of the record's 64-row operand
     // tile), filled by two bulk tensor loads: rows with (r & 4) == 0 form a dense block of [8 row groups][4 rows][24 floats]
     // (16 values, 8 floats of fill), the other rows a second block whose rows start with the fill.  See mat_at().
     alignas(128) float mats[2 * MAT_BLK];
@@ -188,7 +188,7 @@ __device__ __forceinline__ void store_quad(float* row, float a0, float a1, float
 // 4..7 of one block with 8-byte loads, and lanes over rows 0,2,4,6 (or 1,3,5,7) x 8 columns, where the second block's
 // shift by 8 floats separates rows r and r + 4.
 constexpr int S0_BLK = 32 * SS;
-// Offset of element (row, col) of matrix m (0 AK, 1 QK, 2 AI, 3 QB) in the matrices buffer; the same split by row bit 2
+// Offset of element (row, col) of matrix m (0 AK, 1 QK, 2 AI^T, 3 QB) in the matrices buffer; the same split by row bit 2
 // and the same shift of the second block by 8 floats as for the state, here with the 24-float row pitch.
 __device__ __forceinline__ int mat_at(int m, int row, int col) {
     return ((row >> 2) & 1) * (MAT_BLK + 8) + ((2 * m + (row >> 3)) * 4 + (row & 3)) * SCS + col;
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int kk = 0; kk <= nt; ++kk) mma<PREC>(U[nt], xa[kk], mat_nk(2, nt, kk));
+                for (int kk = 0; kk <= nt; ++kk) mma<PREC>(U[nt], xa[kk], mat_kn(2, nt, kk));
             if (LN) {
                 // ---- rebuild Y, then GroupNorm / bonus / gate backward in the [value][time] layout ----
                 FragA<PREC> ua0[2] = {fragA_from_acc<PREC>(U[0]), fragA_from_acc<PREC>(U[1])};
@@ -630,7 +630,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
             for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
-                for (int kb = nb; kb < 2; ++kb) mma<PREC>(dabu[nb], da2[kb], mat_kn(2, nb, kb));
+                for (int kb = nb; kb < 2; ++kb) mma<PREC>(dabu[nb], da2[kb], mat_nk(2, nb, kb));
         }
         FragA<PREC> dbf[2] = {fragA_from_acc<PREC>(dabu[0]), fragA_from_acc<PREC>(dabu[1])};
 #pragma unroll
@@ -975,7 +975,7 @@ static bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long re
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float*>(ckpt), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-static bool encode_bthn_map(CUtensorMap* m, void* base, long long B, long long T, long long H, const Strides& st) {
+bool encode_bthn_map(CUtensorMap* m, void* base, long long B, long long T, long long H, const Strides& st) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[4] = {(cuuint64_t)N, (cuuint64_t)H, (cuuint64_t)T, (cuuint64_t)B};

@@ -16,11 +16,11 @@ constexpr int OPS = N + 8;   // row stride (floats) of the [time][key] operand b
 constexpr int SCS = L + 8;   // row stride (floats) of the [time][time] score buffers
 // One checkpoint record per 16-step chunk, written by the forward for the backward: the fp32 state at
 // the start of the chunk [N][N], then the chunk's four state-independent 16x16 matrices QK, QB (lower
-// triangular), AK (strictly lower), AI = (I - AB)^-1.  The backward loads them instead of rebuilding
+// triangular), AK (strictly lower), AI = (I - AB)^-1 (stored transposed: it is an operand in that form).  The backward loads them instead of rebuilding
 // them (two score products per warp and the 16-step inverse).  The matrices are kept in the layout of
 // the tcgen05 forward's operand tiles, so that that kernel can copy them out with one bulk copy:
 // three K-major tiles of 16-byte chunks, element (row, col) at float (row/8)*128 + (col/4)*32 + (row%8)*4
-// + col%4; the first tile has 32 rows (AK in rows 0-15, QK in rows 16-31), then AI, then QB.
+// + col%4; the first tile has 32 rows (AK in rows 0-15, QK in rows 16-31), then AI^T, then QB.
 constexpr int CK_STATE = 0, CK_MATS = N * N;
 constexpr int CK_SC = CK_MATS, CK_AI = CK_SC + 2 * L * L, CK_QB = CK_AI + L * L;
 __host__ __device__ constexpr int ck_tile_at(int row, int chunk) { return (row >> 3) * 128 + chunk * 32 + (row & 7) * 4; }
@@ -368,10 +368,13 @@ constexpr long long MBAR_WAIT_LIMIT = 1LL << 28;  // clocks (~0.15 s): far beyon
 template <bool SLEEP>
 __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort, int* status, long long limit = MBAR_WAIT_LIMIT) {
     const uint32_t addr = smem_u32(bar);
-    long long start = 0;
-    // (Polling variant: the abort flag is read after every failed probe.  A tighter loop that looked at it only every
-    // 32nd probe made the tcgen05 forward 1.3 % slower: the chain's polls take issue slots from the working warps.)
-    for (int spin = 0;; ++spin) {
+    const uint32_t start = clock(), most = (uint32_t)limit;
+    uint32_t spin = 0;
+    // Polling variant: the abort flag is read after every failed probe.  A tighter loop that looked at it only every
+    // 32nd probe made the tcgen05 forward 1.3 % slower: the chain's polls take issue slots from the working warps.
+    // The loop is kept as small as it can be: it is inlined at some fifteen places, and the tcgen05 forward's warps run
+    // different code at the same time out of one instruction cache (the clock64 form of this loop was 1 KB a place).
+    for (;;) {
         uint32_t ok;
         if (SLEEP)
             asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\nselp.u32 %0, 1, 0, P;\n}\n"
@@ -381,14 +384,11 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
                          : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
         if (ok) return;
         if (*abort) return;
-        if (spin == 0) start = clock64();
-        else if ((SLEEP || (spin & 63) == 0) && clock64() - start > limit) {
-            *abort = 1;
-            *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;  // the launchers always pass the status word (host-visible)
-            __threadfence_system();
-            return;
-        }
+        if ((SLEEP || (++spin & 63) == 0) && (uint32_t)clock() - start > most) break;
     }
+    *abort = 1;
+    *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;  // the launchers always pass the status word (host-visible)
+    __threadfence_system();
 }
 
 // 16-byte asynchronous copy global -> shared through the load/store unit (no TMA request)
@@ -403,6 +403,57 @@ __device__ __forceinline__ void cp_async16_zfill(void* smem, const void* gmem, b
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N_> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_) : "memory"); }
 
+
+// ---- how chains are spread over the CTAs ---------------------------------------------------------
+// A chain is serial in time, but nothing ties a whole chain to one CTA.  With one chain per CTA, B*H chains on S resident
+// CTAs take ceil(B*H / S) rounds, and the last round is rarely full (768 chains on 148 SMs: 6 rounds for 5.19 rounds' worth
+// of work).  So the chunks of all chains, chain after chain, are cut into S equal ranges, one per CTA (the wrap-around
+// rule of preemptive scheduling).  A range is [the end of a chain | whole chains | the start of a chain]; the CTA works the
+// START piece first and the END piece last.  The two pieces of a cut chain belong to neighbouring CTAs: CTA i works the
+// start at the beginning of its time and leaves the state in the chain's final-state buffer, CTA i + 1 takes it up at
+// the end of its time.  A chain is no longer than a range, so the start is finished by the time the end is due (equal
+// speeds assumed; otherwise the wait is short, and bounded).  Results are bit for bit those of the uncut chain.
+// CTA i only ever waits for CTA i - 1, which was dispatched before it, and which waits for nothing before it publishes.
+struct WorkSplit {
+    int ctas, per_cta, per_chain, total;  // CTAs; chunks per range (the last may be shorter); chunks per chain; chunks in all
+    unsigned* flags;                      // one word per CTA, zero at launch: the state of its start piece is ready; null: no chain is cut
+};
+struct WorkRange {
+    int first, n, h, t;  // first chunk (chain-major), chunks, chunks in the start piece (worked first), in the end piece (worked last)
+    __device__ __forceinline__ WorkRange(const WorkSplit& s, int cta) {
+        first = cta * s.per_cta;
+        n = min(s.per_cta, s.total - first);
+        h = (first + n) % s.per_chain;
+        t = (s.per_chain - first % s.per_chain) % s.per_chain;
+    }
+    // chain and chunk (in processing order) of position v of the CTA's work
+    __device__ __forceinline__ void locate(int v, int per_chain, int& chain, int& chunk) const {
+        const int x = v < h ? first + n - h + v : v < n - t ? first + t + v - h : first + v - (n - t);
+        chain = (int)((unsigned)x / (unsigned)per_chain);
+        chunk = x - chain * per_chain;
+    }
+    // whether position v, whose chunk is `chunk`, does not continue the chain of position v - 1
+    __device__ __forceinline__ bool starts_segment(int v, int chunk) const { return v == 0 || chunk == 0 || (t > 0 && v == n - t); }
+};
+__device__ __forceinline__ void publish_handoff(unsigned* flag) {
+    asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(flag) : "memory");
+}
+// Bounded like every wait of this library (see mbar_wait_bounded).
+__device__ __forceinline__ void wait_handoff(const unsigned* flag, volatile int* abort, int* status) {
+    const long long start = clock64();
+    for (;;) {
+        unsigned ready;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(ready) : "l"(flag) : "memory");
+        if (ready || *abort) return;
+        if (clock64() - start > 16 * MBAR_WAIT_LIMIT) {  // a whole range of work may lie in between when the GPU is shared
+            *abort = 1;
+            *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;
+            __threadfence_system();
+            return;
+        }
+        __nanosleep(200);
+    }
+}
 
 // Tensor addressing shared by all launchers: element (b,t,h,0) of a [B,T,H,N] tensor.
 struct Strides {

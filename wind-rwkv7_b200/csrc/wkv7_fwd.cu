@@ -202,11 +202,19 @@ __global__ void __launch_bounds__(THREADS) wkv7_fwd_kernel(FwdParams p) {
         if (p.ckpt) {  // the chunk's four 16x16 matrices go into the checkpoint record: 8 floats per thread
             float* ck = p.ckpt + (bh * nchunks + c) * (long long)CK_FLOATS;
             const int m = tid >> 5, r = (tid & 31) >> 1, hf = tid & 1;
-            const float* src = (m == 0 ? sm.QK : m == 1 ? sm.QB : m == 2 ? sm.AK : sm.AI) + r * SCS + 8 * hf;
+            float x[8];
+            if (m == 3) {  // AI goes out transposed
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[i] = sm.AI[(8 * hf + i) * SCS + r];
+            } else {
+                const float* src = (m == 0 ? sm.QK : m == 1 ? sm.QB : sm.AK) + r * SCS + 8 * hf;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[i] = src[i];
+            }
             float* dst = ck + (m == 0 ? CK_SC + ck_tile_at(16 + r, 2 * hf) : m == 1 ? CK_QB + ck_tile_at(r, 2 * hf)
                                                                             : m == 2 ? CK_SC + ck_tile_at(r, 2 * hf) : CK_AI + ck_tile_at(r, 2 * hf));
-            *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(src);
-            *reinterpret_cast<float4*>(dst + 32) = *reinterpret_cast<const float4*>(src + 4);
+            *reinterpret_cast<float4*>(dst) = make_float4(x[0], x[1], x[2], x[3]);
+            *reinterpret_cast<float4*>(dst + 32) = make_float4(x[4], x[5], x[6], x[7]);
         }
 
         // ---------------- chain, part 2 ----------------------------------------------------------

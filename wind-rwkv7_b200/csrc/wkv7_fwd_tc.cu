@@ -65,34 +65,48 @@ constexpr int G_V = 16384;     // V   [time][value]  MN-major                409
 constexpr int G_KWF = 20480;   // kwf [time][key]    MN-major                4096
 constexpr int G_BWF = 24576;   // bwf [time][key]    MN-major                4096
 constexpr int G_SC = 28672;    // [AK;QK]  32 rows x 16, K-major             2048
-constexpr int G_AI = 30720;    // AI       16 x 16, K-major                  1024
+constexpr int G_AI = 30720;    // AI^T     16 x 16, K-major                  1024
 constexpr int G_QB = 31744;    // QB       16 x 16, K-major                  1024
-static_assert(G_AI == G_SC + 2048 && G_QB == G_AI + 1024, "[AK;QK], AI, QB must be contiguous: they leave as one bulk copy");
+static_assert(G_AI == G_SC + 2048 && G_QB == G_AI + 1024, "[AK;QK], AI^T, QB must be contiguous: they leave as one bulk copy");
 constexpr int G_DF = 32768;    // eight 8x8 diagonal blocks of fw, K-major   2048
 constexpr int G_ABT = 34816;   // AB transposed, fp32 [16][SCS]              1536
+constexpr int G_QBU = 34816;   // QB AI, 16 x 16, K-major (AB is dead by then) 1024
 constexpr int G_RAW = 36352;   // q, w, k, a, b, v staging                   6 * 2048
-constexpr int G_GRAW = 48640;  // attn_ln only: the gate tile, double buffered (read one iteration later)  2 * 2048
-constexpr int G_BYTES_PLAIN = 49152;  // 48 KB (48640 rounded up to 1 KB)
-constexpr int G_BYTES_LN = 53248;     // 52 KB
+constexpr int G_Y = 48128 + 1024;     // the chunk's output as [time][value], bf16, 128-byte swizzle             2048
+constexpr int G_GRAW = G_Y + 2048;    // attn_ln only: the gate tile, double buffered (read one iteration later)  2 * 2048
+constexpr int G_BYTES_PLAIN = G_GRAW;  // 50 KB
+constexpr int G_BYTES_LN = G_GRAW + 2 * RAW_TILE;  // 54 KB
+static_assert(G_RAW + 6 * RAW_TILE <= G_Y && G_Y % 1024 == 0 && G_BYTES_PLAIN % 1024 == 0 && G_BYTES_LN % 1024 == 0, "tile alignment");
 // attn_ln epilogue scratch inside the kwf / bwf tiles, which are dead once the chain step has completed
 constexpr int LN_YS = 68;                  // row stride (floats) of the fp32 [time][value] staging of Y
 constexpr int LN_PART = L * LN_YS * 4;     // byte offset of the per-warp partial sums [4][16][2] behind it
 
 // tensor-memory columns (32-bit each, 128 lanes; the M = 64 products use lanes 0-15 of each 32-lane quarter)
-constexpr int C_S = 0;      // two 64-column state buffers
-constexpr int C_XY = 128;   // two buffers of X (16) | Y (16)
-constexpr int C_U = 192;    // U (16)
-constexpr int C_SCORE = 208;  // + 32 * group: [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47
+constexpr int C_S = 0;       // four 64-column state buffers: chunk c reads c % 4 and writes (c + 1) % 4
+constexpr int C_INIT = 256;  // start state of the next segment (written by the group that prepares its first chunk)
+constexpr int C_XY = 320;    // + 32 * group: X (16) | Y (16) of the group's chunk; before that its score products,
+                             // [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47, and then the products (AI^T bwf)^T | QB AI
 
 constexpr long long WAIT_LIMIT = MBAR_WAIT_LIMIT;
 
+// One chunk of the CTA's work list, as its preparation group (and the chain thread) need it.
+struct ChunkDesc {
+    long long off;   // element offset of (batch, time 0, head) in the inputs
+    int bh, c;       // chain and chunk within it
+    int c_end;       // end of the segment (the chunks of this chain that follow one another in the list)
+    int flags;
+    int bi, hi;      // batch entry, head
+    int prev_first;  // SEG_FIRST: list position of the previous segment's first chunk if that lies less than G back, else -1
+};
+enum : int { SEG_FIRST = 1, SEG_LAST = 2 };  // first / last chunk of a segment
+
 struct Ctrl {
-    uint64_t full[4], done[4], rdone[4], score[4], hop;
+    uint64_t full[4], done[4], score[4], hop;
     uint64_t drain;            // abort path only: completion of the chain thread's outstanding tensor-core work
     uint32_t tmem_base;
     volatile int abort;
     volatile int zero;         // stays 0: the abort-path drain waits with this in place of the abort flag
-    float lnp[3 * N];          // attn_ln: GroupNorm weight, bias, bonus of this head
+    ChunkDesc desc[4][4];      // [group][own-chunk number mod 4]: where the chunk lies (written one iteration ahead by the group)
     float bdot[4][2][4][L];    // attn_ln: per-warp partial bonus dots [group][iteration parity][warp][time]
 };
 
@@ -127,16 +141,8 @@ __device__ __forceinline__ void drain_tensor_work(uint64_t* bar, volatile int* n
     tc_commit(bar);
     mbar_wait_bounded<false>(bar, 0, never_set, status);
 }
-// named barrier of one preparation group; immediate ids, so that ptxas counts G + 1 barriers for the CTA
-// and not all sixteen
-__device__ __forceinline__ void group_bar(int grp) {
-    switch (grp) {
-        case 0: asm volatile("bar.sync 1, 128;" ::: "memory"); break;
-        case 1: asm volatile("bar.sync 2, 128;" ::: "memory"); break;
-        case 2: asm volatile("bar.sync 3, 128;" ::: "memory"); break;
-        default: asm volatile("bar.sync 4, 128;" ::: "memory"); break;
-    }
-}
+// named barrier of one preparation group (the id in a register: a switch over immediate ids costs instruction-cache space)
+__device__ __forceinline__ void group_bar(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); }
 
 // shared-memory matrix descriptor (sm_100 version field set); byte offsets are added to the low word
 __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr, uint32_t sbo) {
@@ -162,6 +168,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t ta, uint32_t* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(v[0]),"=r"(v[1]),"=r"(v[2]),"=r"(v[3]),"=r"(v[4]),"=r"(v[5]),"=r"(v[6]),"=r"(v[7]),"=r"(v[8]),"=r"(v[9]),"=r"(v[10]),"=r"(v[11]),"=r"(v[12]),"=r"(v[13]),"=r"(v[14]),"=r"(v[15]) : "r"(ta));
 }
+// the 16 lanes of an M = 64 product's quarter x 16 columns in the mma.sync accumulator layout: registers 4j..4j+3 = rows
+// lane/4, lane/4 + 8 x columns 8j + 2(lane%4), +1
+__device__ __forceinline__ void tmem_ld_frag(uint32_t ta, uint32_t* v) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(v[0]),"=r"(v[1]),"=r"(v[2]),"=r"(v[3]),"=r"(v[4]),"=r"(v[5]),"=r"(v[6]),"=r"(v[7]) : "r"(ta));
+}
 __device__ __forceinline__ void tmem_st16(uint32_t ta, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
         :: "r"(v[0]),"r"(v[1]),"r"(v[2]),"r"(v[3]),"r"(v[4]),"r"(v[5]),"r"(v[6]),"r"(v[7]),"r"(v[8]),"r"(v[9]),"r"(v[10]),"r"(v[11]),"r"(v[12]),"r"(v[13]),"r"(v[14]),"r"(v[15]), "r"(ta) : "memory");
@@ -169,59 +181,80 @@ __device__ __forceinline__ void tmem_st16(uint32_t ta, const uint32_t* v) {
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// (The conversion instruction cvt.rna.tf32 is one instead of two, but slow: the operand tiles took 1750 cycles with it, 750
+// without.)
 __device__ __forceinline__ float rnd(float x) { return __uint_as_float(tf32_rna(x)); }
+
+// Two fp32 operations in one instruction (sm_100 packed arithmetic).
+struct F2 { float x, y; };
+__device__ __forceinline__ unsigned long long f2_bits(F2 a) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y)); return r; }
+__device__ __forceinline__ F2 f2_from(unsigned long long r) { F2 a; asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r)); return a; }
+__device__ __forceinline__ F2 f2(float x, float y) { return F2{x, y}; }
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b))); return f2_from(r); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { unsigned long long r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b))); return f2_from(r); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { unsigned long long r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c))); return f2_from(r); }
 
 // byte offset of the 16-byte chunk holding (row, k..k+3) in a K-major tile; sbo = bytes per 8-row group
 __device__ __forceinline__ int kchunk(int row, int kc, int sbo) { return (row >> 3) * sbo + kc * 128 + (row & 7) * 16; }
 
-// Column `col` of AI = (I - AB)^-1 (AB strictly lower triangular), written into the K-major AI tile
-// as element (row S_, k = col).  Right-looking substitution as in tri_inverse_column().
-template <int S_> __device__ __forceinline__ void tri_step_tc(float (&r)[L], const float (&c)[L], float (&cn)[L], const float* ABt, unsigned char* AI, int col) {
-    if (S_ + 1 < L) tri_fetch_row<(S_ + 1 < L ? S_ + 1 : 0)>(cn, ABt);
-    const float ms = r[S_], msr = rnd(ms);
-    *reinterpret_cast<float*>(AI + kchunk(S_, col >> 2, 512) + (col & 3) * 4) = msr;
+// Column `col` of AI = (I - AB)^-1 (AB strictly lower triangular), written as row `col` of the K-major tile of AI^T.
+// Right-looking substitution as in tri_inverse_column().
+template <int S_> __device__ __forceinline__ void tri_fetch_tc(F2 (&dst)[L / 2], const float* ABt) {  // row S_ of ABt, entries > S_
 #pragma unroll
-    for (int tq = S_ + 1; tq < L; ++tq) r[tq] = fmaf(c[tq], ms, r[tq]);
+    for (int v = (S_ + 1) / 4; v < L / 4; ++v) {
+        const float4 x = *reinterpret_cast<const float4*>(ABt + S_ * SCS + 4 * v);
+        dst[2 * v] = f2(x.x, x.y); dst[2 * v + 1] = f2(x.z, x.w);
+    }
 }
-__device__ __forceinline__ void tri_inverse_tc(const float* ABt, unsigned char* AI, int col) {
-    float r[L], ca[L], cb[L];
+template <int S_> __device__ __forceinline__ void tri_step_tc(F2 (&r)[L / 2], const F2 (&c)[L / 2], F2 (&cn)[L / 2], const float* ABt) {
+    if (S_ + 1 < L - 1) tri_fetch_tc<(S_ + 1 < L - 1 ? S_ + 1 : 0)>(cn, ABt);
+    const float ms = S_ & 1 ? r[S_ / 2].y : r[S_ / 2].x;
+    if (!(S_ & 1)) r[S_ / 2].y = fmaf(c[S_ / 2].y, ms, r[S_ / 2].y);
 #pragma unroll
-    for (int tq = 0; tq < L; ++tq) r[tq] = (tq == col) ? 1.f : 0.f;
-    tri_fetch_row<0>(ca, ABt);
-    tri_step_tc<0>(r, ca, cb, ABt, AI, col);   tri_step_tc<1>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<2>(r, ca, cb, ABt, AI, col);   tri_step_tc<3>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<4>(r, ca, cb, ABt, AI, col);   tri_step_tc<5>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<6>(r, ca, cb, ABt, AI, col);   tri_step_tc<7>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<8>(r, ca, cb, ABt, AI, col);   tri_step_tc<9>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<10>(r, ca, cb, ABt, AI, col);  tri_step_tc<11>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<12>(r, ca, cb, ABt, AI, col);  tri_step_tc<13>(r, cb, ca, ABt, AI, col);
-    tri_step_tc<14>(r, ca, cb, ABt, AI, col);  tri_step_tc<15>(r, cb, ca, ABt, AI, col);
+    for (int h = S_ / 2 + 1; h < L / 2; ++h) r[h] = fma2(c[h], f2(ms, ms), r[h]);
+}
+__device__ __forceinline__ void tri_inverse_tc(const float* ABt, unsigned char* AIt, int col) {
+    F2 r[L / 2], ca[L / 2], cb[L / 2];
+#pragma unroll
+    for (int h = 0; h < L / 2; ++h) r[h] = f2(2 * h == col ? 1.f : 0.f, 2 * h + 1 == col ? 1.f : 0.f);
+    tri_fetch_tc<0>(ca, ABt);
+    tri_step_tc<0>(r, ca, cb, ABt);   tri_step_tc<1>(r, cb, ca, ABt);
+    tri_step_tc<2>(r, ca, cb, ABt);   tri_step_tc<3>(r, cb, ca, ABt);
+    tri_step_tc<4>(r, ca, cb, ABt);   tri_step_tc<5>(r, cb, ca, ABt);
+    tri_step_tc<6>(r, ca, cb, ABt);   tri_step_tc<7>(r, cb, ca, ABt);
+    tri_step_tc<8>(r, ca, cb, ABt);   tri_step_tc<9>(r, cb, ca, ABt);
+    tri_step_tc<10>(r, ca, cb, ABt);  tri_step_tc<11>(r, cb, ca, ABt);
+    tri_step_tc<12>(r, ca, cb, ABt);  tri_step_tc<13>(r, cb, ca, ABt);
+    tri_step_tc<14>(r, ca, cb, ABt);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4*>(AIt + kchunk(col, q, 512)) = make_float4(rnd(r[2 * q].x), rnd(r[2 * q].y), rnd(r[2 * q + 1].x), rnd(r[2 * q + 1].y));
 }
 
 // two 16-byte chunks of an operand tile; R: round to TF32 (nearest) first, otherwise the tensor core
 // truncates the low 13 mantissa bits when it reads the operand
-template <bool R> __device__ __forceinline__ void store8t(unsigned char* p0, unsigned char* p1, const float (&f)[8]) {
-    if (R) {
-        *reinterpret_cast<float4*>(p0) = make_float4(rnd(f[0]), rnd(f[1]), rnd(f[2]), rnd(f[3]));
-        *reinterpret_cast<float4*>(p1) = make_float4(rnd(f[4]), rnd(f[5]), rnd(f[6]), rnd(f[7]));
-    } else {
-        *reinterpret_cast<float4*>(p0) = make_float4(f[0], f[1], f[2], f[3]);
-        *reinterpret_cast<float4*>(p1) = make_float4(f[4], f[5], f[6], f[7]);
-    }
+template <bool R> __device__ __forceinline__ float4 quad(F2 a, F2 b) {
+    return R ? make_float4(rnd(a.x), rnd(a.y), rnd(b.x), rnd(b.y)) : make_float4(a.x, a.y, b.x, b.y);
+}
+template <bool R> __device__ __forceinline__ void store8t(unsigned char* p0, unsigned char* p1, const F2 (&f)[4]) {
+    *reinterpret_cast<float4*>(p0) = quad<R>(f[0], f[1]);
+    *reinterpret_cast<float4*>(p1) = quad<R>(f[2], f[3]);
 }
 // 32 bytes of an MN-major tile in two 16-byte stores; `flip` swaps the order of the two halves so that the
 // eight lanes of a quarter-warp (rows r..r+7, where r and r+4 share a 32-byte unit) never hit the same bank
-template <bool R> __device__ __forceinline__ void store8mn(unsigned char* p, const float (&f)[8], bool flip) {
-    float x[4], y[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float lo = R ? rnd(f[i]) : f[i], hi = R ? rnd(f[4 + i]) : f[4 + i];
-        x[i] = flip ? hi : lo;  // goes out first
-        y[i] = flip ? lo : hi;
-    }
+template <bool R> __device__ __forceinline__ void store8mn(unsigned char* p, const F2 (&f)[4], bool flip) {
+    const float4 lo = quad<R>(f[0], f[1]), hi = quad<R>(f[2], f[3]);
     const int off = flip ? 16 : 0;
-    *reinterpret_cast<float4*>(p + off) = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float4*>(p + (16 - off)) = make_float4(y[0], y[1], y[2], y[3]);
+    // selected float by float: a whole-struct select is turned back into unswapped stores (and 16-way bank conflicts)
+    *reinterpret_cast<float4*>(p + off) = make_float4(flip ? hi.x : lo.x, flip ? hi.y : lo.y, flip ? hi.z : lo.z, flip ? hi.w : lo.w);
+    *reinterpret_cast<float4*>(p + (16 - off)) = make_float4(flip ? lo.x : hi.x, flip ? lo.y : hi.y, flip ? lo.z : hi.z, flip ? lo.w : hi.w);
+}
+// 8 bf16 values of a staging tile as four pairs
+__device__ __forceinline__ void load8f2(const unsigned char* p, F2 (&f)[4]) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = f2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
 __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
@@ -235,12 +268,14 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 // TAIL: the sequence length is not a multiple of 16 (a build of its own, so that whole-chunk sequences carry none of
 // the row tests in their register budget).
+struct alignas(64) FwdMaps { CUtensorMap ck, y; };  // checkpoint states; the output
+
 template <int G, bool RND, bool LN, bool TAIL>
-__global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams p, const __grid_constant__ CUtensorMap ckmap) {
+__global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams p, WorkSplit ws, const __grid_constant__ FwdMaps maps) {
     using IoT = __nv_bfloat16;
     constexpr int G_BYTES = LN ? G_BYTES_LN : G_BYTES_PLAIN;
     constexpr int NCOLS = 512;
-    static_assert(C_SCORE + 32 * G <= NCOLS, "tensor memory columns");
+    static_assert(C_XY + 32 * G <= NCOLS, "tensor memory columns");
     // Register reallocation (G == 4 only).  setmaxnreg.inc blocks, without a bound, until the CTA's
     // register pool can satisfy it, and the pool is what the CTA was launched with: 640 threads x 96
     // registers (65536 / 640 rounded down to a multiple of 8; build.py checks that ptxas reports 96).
@@ -253,17 +288,14 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // provably warp-uniform
-    const long long bh = blockIdx.x;
-    const long long bi = bh / p.H, hi = bh % p.H;
-    const long long base = bi * p.st.b + hi * p.st.h;
-    const int nchunks = (int)((p.T + L - 1) / L);  // the last chunk may be partial: its missing rows read as zeros
+    const int nchunks = ws.per_chain;  // the last chunk may be partial: its missing rows read as zeros
+    const WorkRange work(ws, blockIdx.x);
     const int tail = TAIL ? (int)(p.T - (long long)(nchunks - 1) * L) : L;  // time steps of the last chunk (1..16)
 
     if (tid == 0) {
         for (int g = 0; g < G; ++g) {
             mbar_init(&ctrl->full[g], 128);
             mbar_init(&ctrl->done[g], 1);
-            mbar_init(&ctrl->rdone[g], 128);
             mbar_init(&ctrl->score[g], 1);
         }
         mbar_init(&ctrl->hop, 1);
@@ -272,9 +304,27 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         ctrl->zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (LN) {
-        for (int i = tid; i < 3 * N; i += blockDim.x) ctrl->lnp[i] = p.params[(long long)(i / N) * p.H * N + hi * N + (i % N)];
-    }
+    // descriptors of every group's first two chunks
+    auto describe = [&](int g, int k) {
+        const int v = g + k * G;
+        if (v >= work.n) return;
+        ChunkDesc d;
+        work.locate(v, nchunks, d.bh, d.c);
+        d.bi = (int)((unsigned)d.bh / (unsigned)p.H);
+        d.hi = d.bh - d.bi * (int)p.H;
+        d.off = d.bi * p.st.b + d.hi * p.st.h;
+        d.c_end = v < work.h ? work.h : nchunks;  // the start piece is chunks 0 .. h - 1 of its chain
+        d.flags = (work.starts_segment(v, d.c) ? SEG_FIRST : 0) | (d.c + 1 == d.c_end ? SEG_LAST : 0);
+        d.prev_first = -1;
+        if (d.flags & SEG_FIRST)
+            for (int u = v - 1; u >= 0 && u > v - G; --u) {
+                int ub, uc;
+                work.locate(u, nchunks, ub, uc);
+                if (work.starts_segment(u, uc)) { d.prev_first = u; break; }
+            }
+        ctrl->desc[g][k & 3] = d;
+    };
+    if (tid < 2 * G) describe(tid >> 1, tid & 1);
     // the off-diagonal zeros of the decay blocks are written once
     for (int i = tid; i < G * (2048 / 16); i += blockDim.x)
         *reinterpret_cast<uint4*>(sm + (i / 128) * G_BYTES + G_DF + (i % 128) * 16) = make_uint4(0, 0, 0, 0);
@@ -287,29 +337,32 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
     tc_fence_after();
     const uint32_t tmem = ctrl->tmem_base;
 
-    // initial state -> tensor memory buffer 0 (and checkpoint 0): warp w of group 0 owns lanes 32w..32w+31,
-    // of which lanes 0-15 hold value rows 16w..16w+15
-    if (warp < 4) {
-        const int i = 16 * warp + (lane & 15);
-        const float* s0 = p.s0 ? p.s0 + bh * N * N + i * N : nullptr;
-        float* ck = (p.ckpt && lane < 16) ? p.ckpt + bh * nchunks * (long long)CK_FLOATS + i * N : nullptr;
-#pragma unroll
+    // Start state of a segment -> tensor memory and its checkpoint: warp wq of the group owns lanes 32 wq .. 32 wq + 31, of
+    // which lanes 0-15 hold value rows 16 wq .. 16 wq + 15.  A chain's first chunk starts from s0 (or zeros); a chain that
+    // the list cuts starts from the state that the CTA before this one left in sT (see WorkSplit).
+    auto load_state = [&](const ChunkDesc& d, int wq) {
+        const int sbh = d.bh, sc = d.c;
+        const uint32_t ta = tmem + C_INIT;
+        if (d.prev_first >= 0) mbar_wait<true>(&ctrl->done[d.prev_first % G], (d.prev_first / G) & 1, ctrl, p.status);  // its start state has been used
+        const int i = 16 * wq + (lane & 15);
+        if (sc > 0) wait_handoff(ws.flags + blockIdx.x - 1, &ctrl->abort, p.status);
+        const float* src = sc > 0 ? p.sT : p.s0;
+        if (src) src += (long long)sbh * N * N + i * N;
+        float* ck = (p.ckpt && lane < 16) ? p.ckpt + ((long long)sbh * nchunks + sc) * CK_FLOATS + i * N : nullptr;
+#pragma unroll 1
         for (int cb = 0; cb < N; cb += 16) {
             uint32_t v[16];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                float4 x = s0 ? *reinterpret_cast<const float4*>(s0 + cb + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 x = src ? __ldcg(reinterpret_cast<const float4*>(src + cb + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 x.x *= STATE_SCALE; x.y *= STATE_SCALE; x.z *= STATE_SCALE; x.w *= STATE_SCALE;  // the state is carried as S~ = 2^-64 S (see ANCHOR_LN)
                 v[4 * q] = __float_as_uint(x.x); v[4 * q + 1] = __float_as_uint(x.y); v[4 * q + 2] = __float_as_uint(x.z); v[4 * q + 3] = __float_as_uint(x.w);
                 if (ck) *reinterpret_cast<float4*>(ck + cb + 4 * q) = x;
             }
-            tmem_st16(tmem + ((uint32_t)(32 * warp) << 16) + C_S + cb, v);
+            tmem_st16(ta + ((uint32_t)(32 * wq) << 16) + cb, v);
         }
         tmem_st_wait();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
+    };
 
     if (warp >= 4 * G) {
         // ------------------------------ chain warp group -----------------------------------------
@@ -319,17 +372,22 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         // scheduler of the groups' warps 0 the chain's instructions waited longer for issue slots (forward +5 %).
         if (warp == 4 * G + 3 && elect_one()) {
             const uint32_t sb = smem_u32(sm);
-            uint32_t hop_phase = 0;
-            for (int c = 0; c < nchunks; ++c) {
+            int seg_first = 0;  // list position at which the next segment begins
+            for (int c = 0; c < work.n; ++c) {  // position in the CTA's list
                 const int g = c % G, k = c / G;
                 const uint32_t gb = sb + g * G_BYTES;
-                const uint64_t dWAQ = desc_kmajor(gb + G_WAQ, 2048), dSC = desc_kmajor(gb + G_SC, 512), dAI = desc_kmajor(gb + G_AI, 512),
-                               dQB = desc_kmajor(gb + G_QB, 512), dDF = desc_kmajor(gb + G_DF, 256);
-                const uint64_t dV = desc_mnmajor(gb + G_V), dKWF = desc_mnmajor(gb + G_KWF), dBWF = desc_mnmajor(gb + G_BWF);
-                const uint32_t Sa = tmem + C_S + 64 * (c & 1), Sn = tmem + C_S + 64 * ((c + 1) & 1), XY = tmem + C_XY + 32 * (c & 1), U = tmem + C_U;
-                mbar_wait<true>(&ctrl->full[g], k & 1, ctrl, p.status);
-                // the Y buffer and the state buffer about to be overwritten were last read for chunk c-2
-                if (c > 1) mbar_wait<true>(&ctrl->rdone[(c - 2) % G], ((c - 2) / G) & 1, ctrl, p.status);
+                const uint64_t dWAQ = desc_kmajor(gb + G_WAQ, 2048), dSC = desc_kmajor(gb + G_SC, 512),
+                               dQBU = desc_kmajor(gb + G_QBU, 512), dDF = desc_kmajor(gb + G_DF, 256);
+                const uint64_t dV = desc_mnmajor(gb + G_V), dKWF = desc_mnmajor(gb + G_KWF), dBWU = desc_mnmajor(gb + G_BWF);
+                const uint32_t Sn = tmem + C_S + 64 * ((c + 1) & 3), XY = tmem + C_XY + 32 * g;
+                uint32_t Sa = tmem + C_S + 64 * (c & 3);
+                if (c == seg_first) {
+                    Sa = tmem + C_INIT;
+                    seg_first = c < work.h ? work.h : c < work.n - work.t ? min(c + nchunks, work.n - work.t) : work.n;
+                }
+                // The group has also read the results of its previous chunk by then, so the buffers about to be written
+                // (X | Y of this group, and the state buffer, last read for chunk c - 4) are free.
+                mbar_wait<false>(&ctrl->full[g], k & 1, ctrl, p.status);
                 tc_fence_after();
                 // hop 1
 #pragma unroll
@@ -337,27 +395,20 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) mma_ss(XY, dV + (uint64_t)(ks * 64), dSC + (uint64_t)(ks * 16), idesc(32, true, false), 1);
                 tc_commit(&ctrl->hop);
-                // the decay of the old state goes into the other buffer while hop 1 drains
+                // the decay of the old state and the V part of the update go into the other buffer while hop 1 drains
 #pragma unroll
                 for (int s = 0; s < 8; ++s) mma_ts(Sn + 8 * s, Sa + 8 * s, dDF + (uint64_t)(s * 16), idesc(8, false, false), 0);
-                mbar_wait<false>(&ctrl->hop, hop_phase++ & 1, ctrl, p.status);
-                tc_fence_after();
-                // hop 2
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(U, XY + 8 * ks, dAI + (uint64_t)(ks * 16), idesc(16, false, false), ks > 0);
-                tc_commit(&ctrl->hop);
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) mma_ss(Sn, dV + (uint64_t)(ks * 64), dKWF + (uint64_t)(ks * 64), idesc(64, true, true), 1);
-                mbar_wait<false>(&ctrl->hop, hop_phase++ & 1, ctrl, p.status);
+                mbar_wait<false>(&ctrl->hop, c & 1, ctrl, p.status);
                 tc_fence_after();
-                // hop 3 and the U part of the state update
+                // hop 2: the X part of the state update and of Y
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(XY + 16, U + 8 * ks, dQB + (uint64_t)(ks * 16), idesc(16, false, false), 1);
+                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, XY + 8 * ks, dBWU + (uint64_t)(ks * 64), idesc(64, false, true), 1);
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, U + 8 * ks, dBWF + (uint64_t)(ks * 64), idesc(64, false, true), 1);
+                for (int ks = 0; ks < 2; ++ks) mma_ts(XY + 16, XY + 8 * ks, dQBU + (uint64_t)(ks * 16), idesc(16, false, false), 1);
                 tc_commit(&ctrl->done[g]);
-                tc_commit(&ctrl->hop);
-                mbar_wait<false>(&ctrl->hop, hop_phase++ & 1, ctrl, p.status);  // S' is the next chunk's A operand
+                mbar_wait<false>(&ctrl->done[g], k & 1, ctrl, p.status);  // S' is the next chunk's A operand
                 tc_fence_after();
             }
             if (ctrl->abort) drain_tensor_work(&ctrl->drain, &ctrl->zero, p.status);
@@ -369,14 +420,15 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         const int grp = warp >> 2, wg = warp & 3, gt = tid & 127;
         unsigned char* gs = sm + grp * G_BYTES;
         const uint32_t tlane = tmem + ((uint32_t)(32 * wg) << 16);
-        const IoT* gin[6] = {(const IoT*)p.r + base, (const IoT*)p.w + base, (const IoT*)p.k + base,
-                             (const IoT*)p.a + base, (const IoT*)p.b + base, (const IoT*)p.v + base};
-        IoT* gy = (IoT*)p.y + base;
-        const IoT* gg = LN ? (const IoT*)p.g + base : nullptr;
-        auto issue_raw = [&](int c, int gbuf) {  // gbuf: parity of the iteration that will process chunk c
+        const IoT* const gin[6] = {(const IoT*)p.r, (const IoT*)p.w, (const IoT*)p.k, (const IoT*)p.a, (const IoT*)p.b, (const IoT*)p.v};
+        const IoT* const gg = LN ? (const IoT*)p.g : nullptr;
+        auto issue_raw = [&](int ko) {  // own chunk number ko
+            const int gbuf = ko & 1;
+            const ChunkDesc& d = ctrl->desc[grp][ko & 3];
+            const int c = d.c;
             const int r = gt >> 3, seg = gt & 7;
             const bool live = !TAIL || c + 1 < nchunks || r < tail;  // rows beyond the end of the sequence are filled with zeros, nothing is read
-            const long long goff = ((long long)c * L + (live ? r : 0)) * p.st.t;
+            const long long goff = d.off + ((long long)c * L + (live ? r : 0)) * p.st.t;
             const int at = r * ROWB + ((seg ^ (r & 7)) << 4);
 #pragma unroll
             for (int ten = 0; ten < 6; ++ten) {
@@ -389,34 +441,30 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             }
             cp_async_commit();
         };
-        // Results of own chunk number kk (chunk cc): Y^T into registers, the chunk-end state straight to the
-        // checkpoint (or the final state) in two halves, then "results read" for the chain.
-        auto read_results = [&](int cc, int kk) {
+        // Results of own chunk number kk (list position vv): Y^T into registers, the chunk-end state straight to the
+        // checkpoint (or the final state).  All of it is read before the group announces its next chunk.
+        auto read_results = [&](int kk) {
             mbar_wait<true>(&ctrl->done[grp], kk & 1, ctrl, p.status);
             tc_fence_after();
-            const bool last = cc + 1 == nchunks;
-            float* sdst = last ? (p.sT ? p.sT + bh * N * N : nullptr)
-                               : (p.ckpt ? p.ckpt + (bh * nchunks + cc + 1) * (long long)CK_FLOATS : nullptr);
-#ifdef WKV7_TC_NOCKPT
-            sdst = nullptr;
-#endif
+            const ChunkDesc& d = ctrl->desc[grp][kk & 3];
+            const int vv = grp + kk * G, cc = d.c;
+            const bool seg_last = d.flags & SEG_LAST;
+            float* sdst = seg_last ? (p.sT ? p.sT + (long long)d.bh * N * N : nullptr)
+                                   : (p.ckpt ? p.ckpt + ((long long)d.bh * nchunks + cc + 1) * CK_FLOATS : nullptr);
             if (!LN) {
-                // Y^T sits one value row per thread.  Lanes i and i^1 swap half of their 16 time steps, so that
-                // every lane holds (row i&~1, row i|1) pairs for 8 time steps and stores them as bf16x2.
-                uint32_t yv[16];
-                tmem_ld16(tlane + C_XY + 32 * (cc & 1) + 16, yv);
+                // Y^T [value][time], read as accumulator fragments, goes as bf16 through a transposing matrix store into the
+                // [time][value] tile (128-byte rows, 16-byte units XOR-ed with the row as the tensor map's swizzle wants), which
+                // leaves by one bulk tensor store; the map clips rows beyond the end of the sequence.
+                uint32_t yv[8];
+                tmem_ld_frag(tlane + C_XY + 32 * grp + 16, yv);
                 tmem_ld_wait();
-                const int odd = lane & 1;
-                IoT* yo = gy + ((long long)cc * L + odd) * p.st.t + 16 * wg + (lane & 14);
+                uint32_t h[4];  // 8x8 blocks: values 0-7 | 8-15 of time steps 0-7, then of time steps 8-15
 #pragma unroll
-                for (int m = 0; m < 8; ++m) {
-                    const float mine = __uint_as_float(odd ? yv[2 * m + 1] : yv[2 * m]);
-                    const float give = __uint_as_float(odd ? yv[2 * m] : yv[2 * m + 1]);
-                    const float got = __shfl_xor_sync(0xffffffffu, give, 1);
-                    const __nv_bfloat162 pr = odd ? __floats2bfloat162_rn(got, mine) : __floats2bfloat162_rn(mine, got);
-                    if (lane < 16 && (!TAIL || !last || 2 * m + odd < tail)) *reinterpret_cast<__nv_bfloat162*>(yo + (long long)(2 * m) * p.st.t) = pr;
-                }
-            } else {
+                for (int j = 0; j < 4; ++j) h[j] = pack_bf16x2_rn(__uint_as_float(yv[2 * j]), __uint_as_float(yv[2 * j + 1]));
+                const int t = (lane & 7) + 8 * (lane >> 4), unit = 2 * wg + ((lane >> 3) & 1);  // row address of block lane / 8
+                asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
+                             ::"r"(smem_u32(gs + G_Y + t * 128 + ((unit ^ (t & 7)) << 4))), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
+                        } else {
                 // attn_ln epilogue (reference: wind_rwkv/rwkv7/attn_ln.cu:176-205): GroupNorm over the head's 64
                 // value channels of each time step, + bonus dot * v, * gate.  Y^T goes to shared memory as
                 // fp32 [time][value] (in the dead kwf / bwf tiles); then one thread = one time step x 8 value channels, the mapping of the scan.
@@ -424,7 +472,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 float* part = reinterpret_cast<float*>(gs + G_KWF + LN_PART);
                 {
                     uint32_t yv[16];
-                    tmem_ld16(tlane + C_XY + 32 * (cc & 1) + 16, yv);
+                    tmem_ld16(tlane + C_XY + 32 * grp + 16, yv);
                     tmem_ld_wait();
                     if (lane < 16) {
 #pragma unroll
@@ -461,21 +509,31 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     // v of this chunk is still in the fp32 MN-major tile, the gate in its own double buffer
                     const int mo = (i0 >> 5) * 2048 + t * 128 + ((((i0 & 31) >> 3) ^ (t & 3)) << 5);
                     const float4 v0 = *reinterpret_cast<const float4*>(gs + G_V + mo), v1 = *reinterpret_cast<const float4*>(gs + G_V + mo + 16);
-                    const float vv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                    const float vval[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
                     float gv[8];
                     load8<IoT>(gs + G_GRAW + (kk & 1) * RAW_TILE + t * ROWB + (((i0 >> 3) ^ (t & 7)) << 4), gv);
                     float o8[8];
+                    const float* lnp = p.params + d.hi * N + i0;  // GroupNorm weight, then bias: 32 bytes each per thread, in L1
+                    const float4 w0 = __ldg(reinterpret_cast<const float4*>(lnp)), w1 = __ldg(reinterpret_cast<const float4*>(lnp) + 1);
+                    const float4 b0 = __ldg(reinterpret_cast<const float4*>(lnp + p.H * N)), b1 = __ldg(reinterpret_cast<const float4*>(lnp + p.H * N) + 1);
+                    const float lw8[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w}, lb8[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        o8[i] = ((yv8[i] - mu) * rstd * ctrl->lnp[i0 + i] + ctrl->lnp[N + i0 + i] + bd * vv[i]) * gv[i];
+                    for (int i = 0; i < 8; ++i) o8[i] = ((yv8[i] - mu) * rstd * lw8[i] + lb8[i] + bd * vval[i]) * gv[i];
                     uint4 pk;
                     pk.x = pack_bf16x2_rn(o8[0], o8[1]); pk.y = pack_bf16x2_rn(o8[2], o8[3]);
                     pk.z = pack_bf16x2_rn(o8[4], o8[5]); pk.w = pack_bf16x2_rn(o8[6], o8[7]);
-                    if (!TAIL || !last || t < tail) *reinterpret_cast<uint4*>(gy + ((long long)cc * L + t) * p.st.t + i0) = pk;
+                    *reinterpret_cast<uint4*>(gs + G_Y + t * 128 + (((i0 >> 3) ^ (t & 7)) << 4)) = pk;
                 }
-                group_bar(grp);  // the scratch lies in an operand tile that is rewritten next
             }
-            if (sdst && !last) {
+            fence_async_smem();
+            group_bar(grp);
+            if (wg == 0 && elect_one()) {
+                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                             ::"l"(&maps.y), "r"(0), "r"(d.hi), "r"(cc * L), "r"(d.bi), "r"(smem_u32(gs + G_Y)) : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            __syncwarp();
+            if (sdst && !seg_last) {
                 // checkpoint state: exact fp32 (the backward's tensor-core products read its upper 19 bits, its carried
                 // decay term all of them), staged in the 128-byte-swizzled layout the tensor-map store expects: half h = columns 32h..32h+31,
                 // row i at i*128 bytes, its 16-byte unit u at (u ^ (i & 7))
@@ -484,12 +542,8 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
                 for (int qt = 0; qt < 4; ++qt) {
                     uint32_t sv[16];
-                    tmem_ld16(tlane + C_S + 64 * ((cc + 1) & 1) + 16 * qt, sv);
+                    tmem_ld16(tlane + C_S + 64 * ((vv + 1) & 3) + 16 * qt, sv);
                     tmem_ld_wait();
-                    if (qt == 3) {
-                        tc_fence_before();
-                        mbar_arrive(&ctrl->rdone[grp]);
-                    }
                     if (lane < 16) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
@@ -502,11 +556,11 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 fence_async_smem();
                 group_bar(grp);
                 if (wg == 0 && elect_one()) {
-                    const int rec_row = (int)((bh * nchunks + cc + 1) * (CK_FLOATS / N));  // a record is 80 rows of 64 floats
+                    const int rec_row = (int)(((long long)d.bh * nchunks + cc + 1) * (CK_FLOATS / N));  // a record is 80 rows of 64 floats
                     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                                 ::"l"(&ckmap), "r"(0), "r"(rec_row), "r"(smem_u32(stage)) : "memory");
+                                 ::"l"(&maps.ck), "r"(0), "r"(rec_row), "r"(smem_u32(stage)) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];"
-                                 ::"l"(&ckmap), "r"(32), "r"(rec_row), "r"(smem_u32(stage + 8192)) : "memory");
+                                 ::"l"(&maps.ck), "r"(32), "r"(rec_row), "r"(smem_u32(stage + 8192)) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
                 __syncwarp();
@@ -516,12 +570,8 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
                 for (int qt = 0; qt < 4; ++qt) {
                     uint32_t sv[16];
-                    tmem_ld16(tlane + C_S + 64 * ((cc + 1) & 1) + 16 * qt, sv);
+                    tmem_ld16(tlane + C_S + 64 * ((vv + 1) & 3) + 16 * qt, sv);
                     tmem_ld_wait();
-                    if (qt == 3) {
-                        tc_fence_before();
-                        mbar_arrive(&ctrl->rdone[grp]);
-                    }
 #pragma unroll
                     for (int e = 0; e < 16; ++e) sv[e] = __float_as_uint(__uint_as_float(sv[e]) * STATE_UNSCALE);  // S = 2^64 S~
                     if (lane < 16) {
@@ -531,15 +581,18 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                                          "r"(sv[8 * q8 + 2]), "r"(sv[8 * q8 + 3]), "r"(sv[8 * q8 + 4]), "r"(sv[8 * q8 + 5]), "r"(sv[8 * q8 + 6]), "r"(sv[8 * q8 + 7]) : "memory");
                     }
                 }
-            } else {
-                tc_fence_before();
-                mbar_arrive(&ctrl->rdone[grp]);
+                if (cc + 1 < nchunks) {  // the rest of this chain is another CTA's: hand the state over
+                    __threadfence();
+                    group_bar(grp);
+                    if (gt == 0) publish_handoff(ws.flags + blockIdx.x);
+                }
             }
         };
         const int row = lane & 15, j0 = 16 * wg + 8 * (lane >> 4);
-        if (grp < nchunks) issue_raw(grp, 0);
-        int k = 0, cprev = -1;
-        for (int c = grp; c < nchunks; c += G, ++k) {
+        if (grp < work.n) issue_raw(0);
+        // One more iteration than there are own chunks: the last one only reads the last results (one copy of that code).
+        for (int k = 0, v0 = grp; ; v0 += G, ++k) {
+            const bool have = v0 < work.n;
             cp_async_wait<0>();
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the matrix copy of the previous own chunk (its issuer only)
             group_bar(grp);
@@ -547,105 +600,130 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             // One thread = one time step x 8 adjacent key channels.  The three transcendentals per
             // element go to the special-function unit: with the matrix products on tcgen05 the FMA
             // pipe and the issue slots are what this kernel runs out of, not MUFU throughput.
-            float o[4][8], v[8], fwv[8];  // kwf, bwf are formed from kwi, bwi and fw when the tiles are written
-            {
+            F2 o[4][4], v[4], fwv[4];  // kwf, bwf are formed from kwi, bwi and fw when the tiles are written
+            if (have) {
                 const unsigned char* raw = gs + G_RAW + row * ROWB + (((j0 >> 3) ^ (row & 7)) << 4);
-                float cum[8], q[8], kk[8], a[8], b[8];
-                load8<IoT>(raw + 1 * RAW_TILE, cum);
-                load8<IoT>(raw + 0 * RAW_TILE, q);
-                load8<IoT>(raw + 2 * RAW_TILE, kk);
-                load8<IoT>(raw + 3 * RAW_TILE, a);
-                load8<IoT>(raw + 4 * RAW_TILE, b);
-                load8<IoT>(raw + 5 * RAW_TILE, v);
+                F2 cum[4], q[4], kk[4], a[4], b[4];
+                load8f2(raw + 1 * RAW_TILE, cum);
+                load8f2(raw + 0 * RAW_TILE, q);
+                load8f2(raw + 2 * RAW_TILE, kk);
+                load8f2(raw + 3 * RAW_TILE, a);
+                load8f2(raw + 4 * RAW_TILE, b);
+                load8f2(raw + 5 * RAW_TILE, v);
                 if (LN) {  // bonus dot sum_j r_j k_j bonus_j of this time step: 8 channels here, the rest by shuffle and in the epilogue
-                    float acc = 0.f;
+                    F2 acc = f2(0.f, 0.f);
+                    const float4* bp = reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][k & 3].hi) * N + j0);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc = fmaf(q[i] * kk[i], ctrl->lnp[2 * N + j0 + i], acc);
-                    acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-                    if (lane < 16) ctrl->bdot[grp][k & 1][wg][row] = acc;
+                    for (int i = 0; i < 2; ++i) {
+                        const float4 bo = __ldg(bp + i);
+                        acc = fma2(mul2(q[2 * i], kk[2 * i]), f2(bo.x, bo.y), acc);
+                        acc = fma2(mul2(q[2 * i + 1], kk[2 * i + 1]), f2(bo.z, bo.w), acc);
+                    }
+                    float dot = acc.x + acc.y;
+                    dot += __shfl_xor_sync(0xffffffffu, dot, 16);
+                    if (lane < 16) ctrl->bdot[grp][k & 1][wg][row] = dot;
                 }
                 // log2 of the per-step decay: -exp(w) * log2(e); running sum along the 16 time rows
+                constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // the per-step floor in log2 units
 #pragma unroll
-                for (int i = 0; i < 8; ++i)  // with the per-step floor (see MIN_STEP_LOG_DECAY)
-                    cum[i] = fmaxf(ex2_approx(cum[i] * 1.4426950408889634f) * -1.4426950408889634f, MIN_STEP_LOG_DECAY * 1.4426950408889634f);  // log2 units
-                if (TAIL && c + 1 == nchunks && row >= tail) {  // a row beyond the end of the sequence: no decay, the state passes through
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) cum[i] = 0.f;
+                for (int i = 0; i < 4; ++i) {
+                    cum[i] = mul2(cum[i], f2(LOG2E, LOG2E));
+                    cum[i] = mul2(f2(ex2_approx(cum[i].x), ex2_approx(cum[i].y)), f2(-LOG2E, -LOG2E));
+                    cum[i] = f2(fmaxf(cum[i].x, FLOOR), fmaxf(cum[i].y, FLOOR));
                 }
-                float step[8];  // this row's own log2 decay: P_{t-1} = 2^(cum_t - step_t), cheaper than a shuffle for the row above
+                if (TAIL && ctrl->desc[grp][k & 3].c + 1 == nchunks && row >= tail) {  // a row beyond the end of the sequence: no decay, the state passes through
 #pragma unroll
-                for (int i = 0; i < 8; ++i) step[i] = cum[i];
+                    for (int i = 0; i < 4; ++i) cum[i] = f2(0.f, 0.f);
+                }
+                F2 step[4];  // this row's own log2 decay: P_{t-1} = 2^(cum_t - step_t), cheaper than a shuffle for the row above
+#pragma unroll
+                for (int i = 0; i < 4; ++i) step[i] = cum[i];
 #pragma unroll
                 for (int d = 1; d < 16; d <<= 1)
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float up = __shfl_up_sync(0xffffffffu, cum[i], d, 16);
-                        if (row >= d) cum[i] += up;
+                    for (int i = 0; i < 4; ++i) {
+                        const F2 up = f2(__shfl_up_sync(0xffffffffu, cum[i].x, d, 16), __shfl_up_sync(0xffffffffu, cum[i].y, d, 16));
+                        if (row >= d) cum[i] = add2(cum[i], up);
                     }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     // P~_t = 2^64 P_t and its reciprocal (see ANCHOR_LN): both finite for cum >= -179 (2^-115 ~ e^-80)
-                    const float ca = cum[i] + ANCHOR_LOG2;
-                    const float cc = fmaxf(ca, -115.f);
-                    const float incl = ex2_approx(cc);
-                    const float inv = ex2_approx(-cc);
-                    const float non = ex2_approx(fmaxf(ca - step[i], -115.f));
-                    const float fw = __shfl_sync(0xffffffffu, incl, 15, 16);  // P~_L = 2^64 P_L (P_L itself may lie below fp32's normal range)
-                    o[0][i] = q[i] * incl;   // wq
-                    o[1][i] = a[i] * non;    // wa
-                    o[2][i] = kk[i] * inv;   // kwi
-                    o[3][i] = b[i] * inv;    // bwi
-                    fwv[i] = fw;
+                    const F2 ca = add2(cum[i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = fma2(step[i], f2(-1.f, -1.f), ca);
+                    const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
+                    const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
+                    const F2 inv = f2(ex2_approx(-cx), ex2_approx(-cy));
+                    const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
+                    o[0][i] = mul2(q[i], incl);   // wq
+                    o[1][i] = mul2(a[i], non);    // wa
+                    o[2][i] = mul2(kk[i], inv);   // kwi
+                    o[3][i] = mul2(b[i], inv);    // bwi
+                    // P~_L = 2^64 P_L (P_L itself may lie below fp32's normal range)
+                    fwv[i] = f2(__shfl_sync(0xffffffffu, incl.x, 15, 16), __shfl_sync(0xffffffffu, incl.y, 15, 16));
                 }
             }
             // ---------------- results of the previous own chunk (its operand tiles are free afterwards) --
-            if (cprev >= 0) {
-                read_results(cprev, k - 1);
-                if (p.ckpt) {  // the staging tiles are operand tiles: wait until the bulk stores have read them
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    group_bar(grp);
-                }
-            }
+            if (k > 0) read_results(k - 1);
+            if (!have) break;
             // ---------------- operand tiles -----------------------------------------------------------
             {
                 const int jc = j0 >> 2;
-                store8t<RND>(gs + G_WAQ + kchunk(row, jc, 2048), gs + G_WAQ + kchunk(row, jc + 1, 2048), o[1]);
-                store8t<RND>(gs + G_WAQ + kchunk(16 + row, jc, 2048), gs + G_WAQ + kchunk(16 + row, jc + 1, 2048), o[0]);
-                store8t<RND>(gs + G_KB + kchunk(row, jc, 2048), gs + G_KB + kchunk(row, jc + 1, 2048), o[2]);
-                store8t<RND>(gs + G_KB + kchunk(16 + row, jc, 2048), gs + G_KB + kchunk(16 + row, jc + 1, 2048), o[3]);
                 const int mo = (j0 >> 5) * 2048 + row * 128 + ((((j0 & 31) >> 3) ^ (row & 3)) << 5);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) { o[2][i] = o[2][i] * fwv[i] * STATE_SCALE; o[3][i] = o[3][i] * fwv[i] * STATE_SCALE; }  // k P_L / P_t first, then 2^-64
                 const bool flip = (row >> 2) & 1;
-                store8mn<RND>(gs + G_KWF + mo, o[2], flip);
-                store8mn<RND>(gs + G_BWF + mo, o[3], flip);
+                F2 kf[4], bf[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {  // k P_L / P_t first, then 2^-64
+                    kf[i] = mul2(mul2(o[2][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                    bf[i] = mul2(mul2(o[3][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                }
+                store8mn<RND>(gs + G_KWF + mo, kf, flip);
+                store8mn<RND>(gs + G_BWF + mo, bf, flip);
                 store8mn<false>(gs + G_V + mo, v, flip);  // bf16 values are exact in TF32
                 if (row == 15) {
                     unsigned char* df = gs + G_DF + (j0 >> 3) * 256;
 #pragma unroll
                     for (int n = 0; n < 8; ++n) {
-                        const float pl = fwv[n] * STATE_SCALE;  // P_L; where it underflows, so does S~ P_L
+                        const float pl = (n & 1 ? fwv[n / 2].y : fwv[n / 2].x) * STATE_SCALE;  // P_L; where it underflows, so does S~ P_L
                         *reinterpret_cast<float*>(df + (n >> 2) * 128 + n * 16 + (n & 3) * 4) = RND ? rnd(pl) : pl;
                     }
                 }
+                if (k > 0 && p.ckpt) {  // the state's staging tiles are the next two operand tiles: wait until the bulk stores have read them
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    group_bar(grp);
+                }
+                store8t<RND>(gs + G_WAQ + kchunk(row, jc, 2048), gs + G_WAQ + kchunk(row, jc + 1, 2048), o[1]);
+                store8t<RND>(gs + G_WAQ + kchunk(16 + row, jc, 2048), gs + G_WAQ + kchunk(16 + row, jc + 1, 2048), o[0]);
+                store8t<RND>(gs + G_KB + kchunk(row, jc, 2048), gs + G_KB + kchunk(row, jc + 1, 2048), o[2]);
+                store8t<RND>(gs + G_KB + kchunk(16 + row, jc, 2048), gs + G_KB + kchunk(16 + row, jc + 1, 2048), o[3]);
             }
             fence_async_smem();
             group_bar(grp);
-            if (c + G < nchunks) issue_raw(c + G, (k + 1) & 1);
+            if (v0 + G < work.n) issue_raw(k + 1);
+            if (gt == 127 && v0 + 2 * G < work.n) {  // read after this group's next barrier
+                ChunkDesc d = ctrl->desc[grp][(k + 1) & 3];
+                d.c += G;
+                if (d.c < d.c_end) {
+                    d.flags = d.c + 1 == d.c_end ? SEG_LAST : 0;
+                    ctrl->desc[grp][(k + 2) & 3] = d;
+                } else {
+                    describe(grp, k + 2);
+                }
+            }
+            __syncwarp();
+            if (ctrl->desc[grp][k & 3].flags & SEG_FIRST) load_state(ctrl->desc[grp][k & 3], wg);
             // ---------------- the four score matrices as one product ---------------------------------
             if (wg == 0 && elect_one()) {
                 const uint64_t dA = desc_kmajor(smem_u32(gs + G_WAQ), 2048), dB = desc_kmajor(smem_u32(gs + G_KB), 2048);
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) mma_ss(tmem + C_SCORE + 32 * grp, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
+                for (int ks = 0; ks < 8; ++ks) mma_ss(tmem + C_XY + 32 * grp, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
                 tc_commit(&ctrl->score[grp]);
             }
             __syncwarp();
             if (wg < 2) {
-                mbar_wait<true>(&ctrl->score[grp], k & 1, ctrl, p.status);
+                mbar_wait<true>(&ctrl->score[grp], 0, ctrl, p.status);
                 tc_fence_after();
                 uint32_t sv[32];
-                tmem_ld16(tlane + C_SCORE + 32 * grp, sv);
-                tmem_ld16(tlane + C_SCORE + 32 * grp + 16, sv + 16);
+                tmem_ld16(tlane + C_XY + 32 * grp, sv);
+                tmem_ld16(tlane + C_XY + 32 * grp + 16, sv + 16);
                 tmem_ld_wait();
                 const int t = lane;
                 if (wg == 0) {
@@ -686,30 +764,59 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             }
             fence_async_smem();
             tc_fence_before();
+            group_bar(grp);
+            tc_fence_after();
+            // ---------------- U folded into the operands: U = X AI^T, so U bwf = X (AI^T bwf) and U QB^T = X (QB AI)^T --------
+            // (one dependent tensor-core round trip per chunk less for the chain, which is what this kernel waits for)
+            if (wg == 0 && elect_one()) {
+                const uint64_t dB = desc_mnmajor(smem_u32(gs + G_BWF)), dQ = desc_kmajor(smem_u32(gs + G_QB), 512), dI = desc_kmajor(smem_u32(gs + G_AI), 512);
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_XY + 32 * grp, dB + (uint64_t)(ks * 64), dI + (uint64_t)(ks * 16), idesc(16, true, false), ks > 0);
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_XY + 32 * grp + 16, dQ + (uint64_t)(ks * 16), dI + (uint64_t)(ks * 16), idesc(16, false, false), ks > 0);
+                tc_commit(&ctrl->score[grp]);
+            }
+            __syncwarp();
+            mbar_wait<true>(&ctrl->score[grp], 1, ctrl, p.status);
+            tc_fence_after();
+            {
+                uint32_t bv[16], qv[16];
+                tmem_ld16(tlane + C_XY + 32 * grp, bv);             // lane: key 16 wg + lane, 16 time steps
+                if (wg == 0) tmem_ld16(tlane + C_XY + 32 * grp + 16, qv);  // lane: row of QB AI
+                tmem_ld_wait();
+                if (lane < 16) {
+                    const int key = 16 * wg + lane;
+                    unsigned char* bw = gs + G_BWF + (key >> 5) * 2048 + (key & 7) * 4;
+#pragma unroll
+                    for (int t = 0; t < 16; ++t)
+                        *reinterpret_cast<float*>(bw + t * 128 + ((((key & 31) >> 3) ^ (t & 3)) << 5)) = rnd(__uint_as_float(bv[t]));
+                    if (wg == 0) {
+#pragma unroll
+                        for (int qd = 0; qd < 4; ++qd)
+                            *reinterpret_cast<float4*>(gs + G_QBU + kchunk(lane, qd, 512)) =
+                                make_float4(rnd(__uint_as_float(qv[4 * qd])), rnd(__uint_as_float(qv[4 * qd + 1])),
+                                            rnd(__uint_as_float(qv[4 * qd + 2])), rnd(__uint_as_float(qv[4 * qd + 3])));
+                    }
+                }
+            }
+            fence_async_smem();
+            tc_fence_before();
             mbar_arrive(&ctrl->full[grp]);
             // The chunk's four 16x16 matrices go into its checkpoint record: the three tiles [AK;QK], AI, QB are
             // contiguous in shared memory and are stored as they are, by one bulk copy issued after the chain
-            // has been given the go-ahead.  The issuing thread waits on the same barrier as the chain (all 128
-            // threads have written and fenced their part of the tiles by then).
-#ifndef WKV7_TC_NOCKPT
+            // has been given the go-ahead (their writers have fenced and passed the group's barrier by then).
             if (p.ckpt && wg == 0) {
                 if (elect_one()) {
-                    mbar_wait<true>(&ctrl->full[grp], k & 1, ctrl, p.status);
-                    float* ckm = p.ckpt + (bh * nchunks + c) * (long long)CK_FLOATS + CK_MATS;
+                    const ChunkDesc& d = ctrl->desc[grp][k & 3];
+                    float* ckm = p.ckpt + ((long long)d.bh * nchunks + d.c) * CK_FLOATS + CK_MATS;
                     asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
                                  ::"l"(__cvta_generic_to_global(ckm)), "r"(smem_u32(gs + G_SC)), "n"(4 * L * L * 4) : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
                 __syncwarp();
             }
-#endif
-            cprev = c;
         }
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last matrix copy
-        if (cprev >= 0) {
-            read_results(cprev, k - 1);
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // ... and the last state copy
-        }
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last copies
     }
 
     tc_fence_before();
@@ -745,10 +852,13 @@ template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdPar
     auto kern = wkv7_fwd_tc_kernel<G, RND, LN, TAIL>;
     const int smem = G * (LN ? G_BYTES_LN : G_BYTES_PLAIN) + (int)sizeof(Ctrl) + 1024;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
-    alignas(64) CUtensorMap ckmap;
-    memset(&ckmap, 0, sizeof(ckmap));
-    if (p.ckpt && !encode_checkpoint_map(&ckmap, p.ckpt, p.B * p.H * ((p.T + L - 1) / L))) return kLaunchFailed;
-    kern<<<(unsigned)(p.B * p.H), 128 * (G + 1), smem, stream>>>(p, ckmap);
+    FwdMaps maps;
+    memset(&maps, 0, sizeof(maps));
+    if (p.ckpt && !encode_checkpoint_map(&maps.ck, p.ckpt, p.B * p.H * ((p.T + L - 1) / L))) return kLaunchFailed;
+    if (!encode_bthn_map(&maps.y, p.y, p.B, p.T, p.H, p.st)) return kLaunchFailed;
+    const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 1, p.sT ? p.flags : nullptr);
+    if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
+    kern<<<(unsigned)ws.ctas, 128 * (G + 1), smem, stream>>>(p, ws, maps);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 

@@ -1,5 +1,6 @@
 // Internal launcher interface between the C ABI (capi.cu) and the kernel translation units.
 #pragma once
+#include <cuda.h>
 #include "wkv7_common.cuh"
 
 namespace wkv7 {
@@ -16,6 +17,7 @@ struct FwdParams {
     Strides st;
     float eps;
     int* status;                        // device status word
+    unsigned* flags;                    // scratch for cut chains (WorkSplit), or null: every chain is worked by one CTA
 };
 
 struct BwdParams {
@@ -44,6 +46,14 @@ struct StepParams {
     long long B, T, H;
     Strides st;
 };
+
+// Work split for `chains` chains of `per_chain` chunks with `per_sm` resident CTAs per SM.  Chains are cut only when there are
+// more of them than resident CTAs (below that every chain has a CTA to itself and cutting gains nothing).
+WorkSplit plan_work(long long chains, long long per_chain, int per_sm, unsigned* flags);
+constexpr size_t WORK_FLAG_BYTES = 4096;  // room for the flags of 1024 CTAs
+
+// tensor map of a bf16 [B,T,H,N] tensor, box = 16 time steps of one head, 128-byte swizzle
+bool encode_bthn_map(CUtensorMap* m, void* base, long long B, long long T, long long H, const Strides& st);
 
 int launch_fwd(const FwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
 // the recurrence step by step on fp32 FMAs (decode); io_dtype 0 = bf16, otherwise fp32 tensors

@@ -39,6 +39,9 @@ _SIGNATURES = {
     'wkv7_set_fwd_impl': (_int, [_int]),
     'wkv7_get_fwd_impl': (_int, []),
     'wkv7_fwd': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp]),
+    'wkv7_workspace_bytes': (ctypes.c_size_t, []),
+    'wkv7_fwd_ws': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp, _vp]),
+    'wkv7_attn_ln_fwd_ws': (_int, [_vp] * 12 + [_f32] + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_step': (_int, [_vp] * 9 + [_i64] * 7 + [_int, _vp]),
     'wkv7_bwd': (_int, [_vp] * 17 + [_i64] * 7 + [_int, _vp]),
     'wkv7_attn_ln_fwd': (_int, [_vp] * 12 + [_f32] + [_i64] * 7 + [_int, _vp]),
@@ -108,6 +111,17 @@ def io_dtype(t):
     if t.dtype == th.float32:
         return WKV7_F32
     raise TypeError(f'wkv7 ops take bfloat16 or float32 tensors, got {t.dtype}')
+
+
+_SCRATCH_BYTES = None
+
+
+def scratch(device):
+    """Device scratch of one call of a *_ws entry point (spreads the chains over the SMs)."""
+    global _SCRATCH_BYTES
+    if _SCRATCH_BYTES is None:
+        _SCRATCH_BYTES = lib().wkv7_workspace_bytes()
+    return th.empty(_SCRATCH_BYTES, dtype=th.uint8, device=device)
 
 
 def ptr(t):

@@ -29,12 +29,13 @@ def fw_attn(w, q, k, v, a, b, s0, save_checkpoints=True):
         y = th.empty_strided(v.shape, v.stride(), dtype=v.dtype, device=v.device)
     sT = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
     s = th.empty(B, H, _lib.chunks(T) if save_checkpoints else 0, _lib.CKPT_FLOATS, dtype=th.float32, device=w.device)
+    ws = _lib.scratch(w.device)
     sb, st, sh = _lib.strides4(w)
     with _lib.on_device(w, q, k, v, a, b, s0):
-        rc = _lib.lib().wkv7_fwd(q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(),
-                                 _lib.ptr(s0), y.data_ptr(), sT.data_ptr(), s.data_ptr() if save_checkpoints else None,
-                                 B, T, H, C, sb, st, sh, _lib.io_dtype(w), _lib.stream_of(w))
-    _lib.check(rc, 'wkv7_fwd')
+        rc = _lib.lib().wkv7_fwd_ws(q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(),
+                                    _lib.ptr(s0), y.data_ptr(), sT.data_ptr(), s.data_ptr() if save_checkpoints else None,
+                                    B, T, H, C, sb, st, sh, _lib.io_dtype(w), ws.data_ptr(), _lib.stream_of(w))
+    _lib.check(rc, 'wkv7_fwd_ws')
     return y, sT, s
 
 
@@ -176,12 +177,13 @@ def _fw_into(w, q, k, v, a, b, s0, y):
     B, T, H, C = w.shape
     assert _same_layout([w, q, k, v, a, b, y]), 'inputs and output must share one layout'
     sT = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
+    ws = _lib.scratch(w.device)
     sb, st, sh = _lib.strides4(w)
     with _lib.on_device(w, q, k, v, a, b, s0):
-        rc = _lib.lib().wkv7_fwd(q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(),
-                                 _lib.ptr(s0), y.data_ptr(), sT.data_ptr(), None, B, T, H, C, sb, st, sh,
-                                 _lib.io_dtype(w), _lib.stream_of(w))
-    _lib.check(rc, 'wkv7_fwd')
+        rc = _lib.lib().wkv7_fwd_ws(q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(),
+                                    _lib.ptr(s0), y.data_ptr(), sT.data_ptr(), None, B, T, H, C, sb, st, sh,
+                                    _lib.io_dtype(w), ws.data_ptr(), _lib.stream_of(w))
+    _lib.check(rc, 'wkv7_fwd_ws')
     return sT
 
 
