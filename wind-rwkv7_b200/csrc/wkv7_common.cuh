@@ -365,6 +365,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // returns: a lost copy or a missing arrival ends with an error code, never with a hung GPU.
 // SLEEP: the thread is suspended by the hardware (try_wait with a time hint) instead of polling.
 constexpr long long MBAR_WAIT_LIMIT = 1LL << 28;  // clocks (~0.15 s): far beyond any legitimate wait
+__device__ __forceinline__ void give_up(volatile int* abort, int* status) {
+    *abort = 1;
+    *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;  // the launchers always pass the status word (host-visible)
+    __threadfence_system();
+}
 template <bool SLEEP>
 __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort, int* status, long long limit = MBAR_WAIT_LIMIT) {
     const uint32_t addr = smem_u32(bar);
@@ -386,9 +391,7 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
         if (*abort) return;
         if ((SLEEP || (++spin & 63) == 0) && (uint32_t)clock() - start > most) break;
     }
-    *abort = 1;
-    *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;  // the launchers always pass the status word (host-visible)
-    __threadfence_system();
+    give_up(abort, status);
 }
 
 // 16-byte asynchronous copy global -> shared through the load/store unit (no TMA request)
@@ -446,9 +449,7 @@ __device__ __forceinline__ void wait_handoff(const unsigned* flag, volatile int*
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(ready) : "l"(flag) : "memory");
         if (ready || *abort) return;
         if (clock64() - start > 16 * MBAR_WAIT_LIMIT) {  // a whole range of work may lie in between when the GPU is shared
-            *abort = 1;
-            *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;
-            __threadfence_system();
+            give_up(abort, status);
             return;
         }
         __nanosleep(200);

@@ -2,36 +2,32 @@
 //
 // Same mathematics as wkv7_fwd.cu (the reference's forward_kernel, wind_rwkv/rwkv7/attn.cu:11-106, and
 // with LN = true its fused GroupNorm + bonus + gate variant, wind_rwkv/rwkv7/attn_ln.cu:106-212),
-// different machine mapping.  One CTA walks one (batch, head) chain.  The 64x64 state S[value][key]
-// lives in tensor memory for the whole sequence and is never held in registers: per 16-step chunk
-// one elected thread issues 26 tcgen05.mma instructions (M = 64 value rows, TF32 operands, fp32
-// accumulate)
+// different machine mapping.  One CTA per SM walks its share of the chunks (WorkSplit: whole chains and at most two pieces of
+// cut ones).  The 64x64 state S[value][key] lives in tensor memory and is never held in registers: per 16-step chunk one
+// elected thread issues 24 tcgen05.mma instructions (M = 64 value rows, TF32 operands, fp32 accumulate)
 //     hop 1   [X | Yp] = S [wa;wq]^T + V^T [AK;QK]^T        A = S straight from tensor memory
-//     hop 2   U  = X AI^T                                    A = X from tensor memory
-//     hop 3   Y  = Yp + U QB^T                               A = U from tensor memory
-//     hop 4   S' = S diag(fw) + V^T kwf + U bwf              eight N = 8 products apply the decay
-// with kwf = kwi*fw, bwf = bwi*fw, so the column scaling of the state never touches a CUDA core.
-// An accumulator that the next product reads as its A operand needs an explicit completion wait
-// (tcgen05.commit -> mbarrier); only same-accumulator chains are ordered by the tensor pipe, so the
-// decay product and the V^T kwf product are issued inside those waits.
+//             S' = S diag(fw) + V^T kwf                      into the next of four state buffers; eight N = 8 products
+//                                                            apply the decay; issued while hop 1 drains
+//     hop 2   S' += X (AI^T bwf),  Y = Yp + X (QB AI)^T      A = X from tensor memory
+// with kwf = kwi*fw, bwf = bwi*fw, so the column scaling of the state never touches a CUDA core.  U = X AI^T itself is never
+// formed: AI^T bwf and QB AI come from two small products off the chain.  An accumulator that the next product reads as its A
+// operand needs an explicit completion wait (tcgen05.commit -> mbarrier); only same-accumulator products are ordered by the
+// tensor pipe.  With three hops (U explicit) and a wait for "results of chunk c-2 read" a chunk took the chain 2000 cycles,
+// most of them waits; what bounds it now is the latency from a chunk's operand tiles to its completion over the four chunks
+// in flight (shared memory has room for four sets of tiles): 1820 cycles per chunk without checkpoints (2070 before), 2500 with (2780).
 //
-// Everything state-independent is done by G "preparation groups" of four warps, each working on
-// its own chunk (c, c+G, ...): cp.async of the six input tiles, the decay scan, the operand tiles
-// in the shared-memory layouts the tensor core reads directly, the four 16x16 score matrices as
-// ONE tcgen05 product ([wa;wq] x [kwi;bwi]^T, M = 64 of which 32 rows are used), masking, the
-// triangular inverse, and afterwards the read-back of Y (and of the chunk-end state for the
-// checkpoints) from tensor memory.  A group's loop is software-pipelined: the decay scan of its next
-// chunk is computed into registers while the chain works on its previous chunk, and the read-back of
-// that chunk's results happens just before the operand tiles are overwritten.
+// Warp roles (128 (G+1) threads).  Warps 0..4G-1 are G preparation groups of four warps, each working on its own chunk
+// (position g, g+G, ... of the CTA's list): the decay scan of the six input tiles (bulk tensor loads, one chunk ahead), the
+// operand tiles in the shared-memory layouts the tensor core reads, the four 16x16 score matrices as ONE tcgen05 product
+// ([wa;wq] x [kwi;bwi]^T, M = 64 of which 32 rows are used), and afterwards the read-back of Y (and of the chunk-end state for
+// the checkpoints).  The scan of a group's next chunk is computed into registers while its current one goes through the rest.
+// Warps 4G, 4G+1 read the scores back from their quarter of tensor memory, mask them and write AK, AB, QK, QB; warp 4G+2
+// inverts (I - AB) and issues the two fold products, whose results warps 4G, 4G+1 write as operand tiles; warp 4G+3 issues
+// the chain.  (With the scores, the inverse and the fold done by the preparation groups, three of a group's four warps
+// waited through half of its time.)  The kernel's hot code has to stay small: its warps run different parts of it at the same
+// time out of one instruction cache, and 10 KB more of it cost 30 % once all SMs missed at the same time.
 //
-// Warp roles (128 (G+1) threads): warps 0..4G-1 are the preparation groups, warp 4G+3 issues the chain,
-// the other three warps of its warp group only exist so that setmaxnreg can be used: the chain
-// warp group shrinks to 32 registers per thread and the preparation warps grow to 112 (a kernel-wide
-// 96, which is all that 20 warps leave, makes the decay scan spill, and the spills cost more than
-// the whole scan).  The chain thread waits for "operands of chunk c ready" and "results of chunk c-2
-// read", so the 16-step dependency is ~1100 cycles per chunk.
-//
-// Shared-memory operand layouts (no TMA: the tiles are produced by threads, not copied):
+// Shared-memory operand layouts (the tiles are produced by threads, not copied):
 //   K-major (contraction index contiguous): 16-byte chunks [row/8][k/4][row%8][k%4], descriptor
 //     LBO = 128 B (next k-chunk), SBO = bytes per 8-row group, no swizzle.
 //   MN-major TF32 (V, kwf, bwf: contraction index = time): only the 128-byte swizzle with 32-byte
@@ -71,12 +67,12 @@ static_assert(G_AI == G_SC + 2048 && G_QB == G_AI + 1024, "[AK;QK], AI^T, QB mus
 constexpr int G_DF = 32768;    // eight 8x8 diagonal blocks of fw, K-major   2048
 constexpr int G_ABT = 34816;   // AB transposed, fp32 [16][SCS]              1536
 constexpr int G_QBU = 34816;   // QB AI, 16 x 16, K-major (AB is dead by then) 1024
-constexpr int G_RAW = 36352;   // q, w, k, a, b, v staging                   6 * 2048
-constexpr int G_Y = 48128 + 1024;     // the chunk's output as [time][value], bf16, 128-byte swizzle             2048
-constexpr int G_GRAW = G_Y + 2048;    // attn_ln only: the gate tile, double buffered (read one iteration later)  2 * 2048
+constexpr int G_RAW = 36864;   // q, w, k, a, b, v staging                   6 * 2048
+constexpr int G_Y = 49152;            // the chunk's output as [time][value], bf16, 128-byte swizzle             2048
+constexpr int G_GRAW = G_Y + 2048;    // attn_ln only: the gate tile                                            2048
 constexpr int G_BYTES_PLAIN = G_GRAW;  // 50 KB
-constexpr int G_BYTES_LN = G_GRAW + 2 * RAW_TILE;  // 54 KB
-static_assert(G_RAW + 6 * RAW_TILE <= G_Y && G_Y % 1024 == 0 && G_BYTES_PLAIN % 1024 == 0 && G_BYTES_LN % 1024 == 0, "tile alignment");
+constexpr int G_BYTES_LN = G_GRAW + RAW_TILE;  // 52 KB
+static_assert(G_RAW % 1024 == 0 && G_RAW + 6 * RAW_TILE <= G_Y && G_Y % 1024 == 0 && G_BYTES_PLAIN % 1024 == 0 && G_BYTES_LN % 1024 == 0, "tile alignment");
 // attn_ln epilogue scratch inside the kwf / bwf tiles, which are dead once the chain step has completed
 constexpr int LN_YS = 68;                  // row stride (floats) of the fp32 [time][value] staging of Y
 constexpr int LN_PART = L * LN_YS * 4;     // byte offset of the per-warp partial sums [4][16][2] behind it
@@ -85,7 +81,8 @@ constexpr int LN_PART = L * LN_YS * 4;     // byte offset of the per-warp partia
 constexpr int C_S = 0;       // four 64-column state buffers: chunk c reads c % 4 and writes (c + 1) % 4
 constexpr int C_INIT = 256;  // start state of the next segment (written by the group that prepares its first chunk)
 constexpr int C_XY = 320;    // + 32 * group: X (16) | Y (16) of the group's chunk; before that its score products,
-                             // [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47, and then the products (AI^T bwf)^T | QB AI
+                             // [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47, and then QB AI in lanes 32-47 of columns 16-31
+constexpr int C_FOLD = 448;  // AI^T bwf (64) in lanes 0-15
 
 constexpr long long WAIT_LIMIT = MBAR_WAIT_LIMIT;
 
@@ -101,7 +98,7 @@ struct ChunkDesc {
 enum : int { SEG_FIRST = 1, SEG_LAST = 2 };  // first / last chunk of a segment
 
 struct Ctrl {
-    uint64_t full[4], done[4], score[4], hop;
+    uint64_t full[4], done[4], score[4], raw[4], gate[4], mats[4], fold[4], rec[4], fread, hop;
     uint64_t drain;            // abort path only: completion of the chain thread's outstanding tensor-core work
     uint32_t tmem_base;
     volatile int abort;
@@ -141,6 +138,12 @@ __device__ __forceinline__ void drain_tensor_work(uint64_t* bar, volatile int* n
     tc_commit(bar);
     mbar_wait_bounded<false>(bar, 0, never_set, status);
 }
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {  // has the phase completed? (whole warp)
+    uint32_t ok;
+    asm volatile("{\n.reg .pred P;\nmbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return __all_sync(0xffffffffu, ok);
+}
 // named barrier of one preparation group (the id in a register: a switch over immediate ids costs instruction-cache space)
 __device__ __forceinline__ void group_bar(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); }
 
@@ -173,6 +176,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t ta, uint32_t* v) {
 __device__ __forceinline__ void tmem_ld_frag(uint32_t ta, uint32_t* v) {
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
         : "=r"(v[0]),"=r"(v[1]),"=r"(v[2]),"=r"(v[3]),"=r"(v[4]),"=r"(v[5]),"=r"(v[6]),"=r"(v[7]) : "r"(ta));
+}
+__device__ __forceinline__ void tmem_ld_frag4(uint32_t ta, uint32_t* v) {  // 32 columns
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]),"=r"(v[1]),"=r"(v[2]),"=r"(v[3]),"=r"(v[4]),"=r"(v[5]),"=r"(v[6]),"=r"(v[7]),"=r"(v[8]),"=r"(v[9]),"=r"(v[10]),"=r"(v[11]),"=r"(v[12]),"=r"(v[13]),"=r"(v[14]),"=r"(v[15]) : "r"(ta));
 }
 __device__ __forceinline__ void tmem_st16(uint32_t ta, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
@@ -256,6 +263,18 @@ __device__ __forceinline__ void load8f2(const unsigned char* p, F2 (&f)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) f[i] = f2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
+// A 16x16 matrix from its accumulator fragment into a K-major operand tile, rounded to TF32; entries with
+// column > row + keep are written as zero (keep = 16: all kept).
+__device__ __forceinline__ void store_frag16(unsigned char* tile, const uint32_t* x, int r0, int c0, int keep) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = r0 + 8 * h, col = 8 * j + c0;
+            *reinterpret_cast<float2*>(tile + kchunk(row, col >> 2, 512) + (col & 3) * 4) =
+                make_float2(col <= row + keep ? rnd(__uint_as_float(x[4 * j + 2 * h])) : 0.f, col + 1 <= row + keep ? rnd(__uint_as_float(x[4 * j + 2 * h + 1])) : 0.f);
+        }
+}
 __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -268,19 +287,19 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 // TAIL: the sequence length is not a multiple of 16 (a build of its own, so that whole-chunk sequences carry none of
 // the row tests in their register budget).
-struct alignas(64) FwdMaps { CUtensorMap ck, y; };  // checkpoint states; the output
+struct alignas(64) FwdMaps { CUtensorMap ck, y, in[6], g; };  // checkpoint states; output; q, w, k, a, b, v; gate
 
 template <int G, bool RND, bool LN, bool TAIL>
 __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams p, WorkSplit ws, const __grid_constant__ FwdMaps maps) {
     using IoT = __nv_bfloat16;
     constexpr int G_BYTES = LN ? G_BYTES_LN : G_BYTES_PLAIN;
     constexpr int NCOLS = 512;
-    static_assert(C_XY + 32 * G <= NCOLS, "tensor memory columns");
+    static_assert(C_XY + 32 * G <= C_FOLD && C_FOLD + 64 <= NCOLS, "tensor memory columns");
     // Register reallocation (G == 4 only).  setmaxnreg.inc blocks, without a bound, until the CTA's
     // register pool can satisfy it, and the pool is what the CTA was launched with: 640 threads x 96
     // registers (65536 / 640 rounded down to a multiple of 8; build.py checks that ptxas reports 96).
     // The raised and lowered counts must therefore fit into that pool exactly or with room to spare.
-    constexpr int LAUNCH_REGS = 96, PREP_REGS = 112, CHAIN_REGS = 32;
+    constexpr int LAUNCH_REGS = 96, PREP_REGS = 104, CHAIN_REGS = 64;
     static_assert(G != 4 || 128 * G * PREP_REGS + 128 * CHAIN_REGS <= 128 * (G + 1) * LAUNCH_REGS, "setmaxnreg would never be satisfied");
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* sm = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
@@ -294,11 +313,17 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 
     if (tid == 0) {
         for (int g = 0; g < G; ++g) {
-            mbar_init(&ctrl->full[g], 128);
+            mbar_init(&ctrl->full[g], 2);
+            mbar_init(&ctrl->mats[g], 2);
+            mbar_init(&ctrl->fold[g], 1);
+            mbar_init(&ctrl->rec[g], 1);
             mbar_init(&ctrl->done[g], 1);
             mbar_init(&ctrl->score[g], 1);
+            mbar_init(&ctrl->raw[g], 1);
+            mbar_init(&ctrl->gate[g], 1);
         }
         mbar_init(&ctrl->hop, 1);
+        mbar_init(&ctrl->fread, 1);
         mbar_init(&ctrl->drain, 1);
         ctrl->abort = 0;
         ctrl->zero = 0;
@@ -367,10 +392,8 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
     if (warp >= 4 * G) {
         // ------------------------------ chain warp group -----------------------------------------
         if (G == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CHAIN_REGS));
-        // The chain is issued by the LAST warp of its warp group: warp 4G + 3 shares its scheduler (warp index mod 4) with
-        // warp 3 of every preparation group, which has the least to do (no score read-back, no inverse); on the
-        // scheduler of the groups' warps 0 the chain's instructions waited longer for issue slots (forward +5 %).
-        if (warp == 4 * G + 3 && elect_one()) {
+        if (warp == 4 * G + 3) {
+          if (elect_one()) {
             const uint32_t sb = smem_u32(sm);
             int seg_first = 0;  // list position at which the next segment begins
             for (int c = 0; c < work.n; ++c) {  // position in the CTA's list
@@ -412,6 +435,117 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 tc_fence_after();
             }
             if (ctrl->abort) drain_tensor_work(&ctrl->drain, &ctrl->zero, p.status);
+          }
+        } else if (warp < 4 * G + 2) {
+            // ---- score warps: warp 4G reads [AK|AB] and later AI^T bwf (tensor-memory lanes 0-15), warp 4G + 1 reads [QK|QB]
+            // and later QB AI (lanes 32-47).  Both take whatever is ready: the fold products of the older chunk first.
+            const int q = warp - 4 * G;
+            const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);
+            const int r0 = lane >> 2, c0 = 2 * (lane & 3);  // this lane's fragment: rows r0, r0 + 8, columns c0, c0 + 1 of every 8
+            int r = 0, f = 0;
+            uint32_t since = clock();
+            while (f < work.n) {
+                const int gf = f % G, gr = r % G;
+                if (f < r && mbar_test(&ctrl->fold[gf], (f / G) & 1)) {
+                    unsigned char* gs = sm + gf * G_BYTES;
+                    tc_fence_after();
+                    if (q == 0) {
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            uint32_t x[16];
+                            tmem_ld_frag4(tq + C_FOLD + 32 * half, x);
+                            tmem_ld_wait();
+                            if (half == 1) {
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(&ctrl->fread);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h)  // time step r0 + 8h, keys 32 half + 8j + c0, +1
+                                    *reinterpret_cast<float2*>(gs + G_BWF + half * 2048 + (r0 + 8 * h) * 128 + ((j ^ (r0 & 3)) << 5) + c0 * 4) =
+                                        make_float2(rnd(__uint_as_float(x[4 * j + 2 * h])), rnd(__uint_as_float(x[4 * j + 2 * h + 1])));
+                        }
+                    } else {
+                        uint32_t x[8];
+                        tmem_ld_frag(tq + C_XY + 32 * gf + 16, x);
+                        tmem_ld_wait();
+                        tc_fence_before();
+                        store_frag16(gs + G_QBU, x, r0, c0, 16);
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctrl->full[gf]);
+                    ++f;
+                } else if (r < work.n && mbar_test(&ctrl->score[gr], (r / G) & 1)) {
+                    unsigned char* gs = sm + gr * G_BYTES;
+                    tc_fence_after();
+                    uint32_t x[16];
+                    tmem_ld_frag4(tq + C_XY + 32 * gr, x);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    // the previous chunk's matrices have left for its checkpoint record
+                    if (p.ckpt && r >= G) mbar_wait<true>(&ctrl->rec[gr], (r / G - 1) & 1, ctrl, p.status);
+                    store_frag16(gs + G_SC + 1024 * q, x, r0, c0, q ? 0 : -1);          // AK (strictly lower) or QK (lower triangular)
+                    if (q == 0) {  // AB, strictly lower, kept transposed for the inverse
+                        float* ABt = reinterpret_cast<float*>(gs + G_ABT);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int row = r0 + 8 * ((i >> 1) & 1), col = 8 * (i >> 2) + c0 + (i & 1);
+                            ABt[col * SCS + row] = col < row ? __uint_as_float(x[8 + i]) : 0.f;
+                        }
+                    } else {
+                        store_frag16(gs + G_QB, x + 8, r0, c0, 0);
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctrl->mats[gr]);
+                    ++r;
+                } else {
+                    if (ctrl->abort) break;
+                    if ((uint32_t)clock() - since > (uint32_t)WAIT_LIMIT) give_up(&ctrl->abort, p.status);
+                    continue;
+                }
+                since = clock();
+            }
+        } else if (warp == 4 * G + 2) {
+            // ---- inverse warp: AI^T, then the two products that fold U into its consumers: U = X AI^T, so U bwf = X (AI^T bwf)
+            // and U QB^T = X (QB AI)^T (one dependent tensor-core round trip per chunk less for the chain).  A = [AI^T; QB] for both.
+            for (int c = 0; c < work.n; ++c) {
+                const int g = c % G, k = c / G;
+                unsigned char* gs = sm + g * G_BYTES;
+                mbar_wait<false>(&ctrl->mats[g], k & 1, ctrl, p.status);
+                if (p.ckpt && c > 0) {  // the previous chunk's record copy has read its tiles
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctrl->rec[(c - 1) % G]);
+                }
+                if (lane < 16) tri_inverse_tc(reinterpret_cast<const float*>(gs + G_ABT), gs + G_AI, lane);
+                fence_async_smem();
+                if (c > 0) mbar_wait<false>(&ctrl->fread, (c - 1) & 1, ctrl, p.status);
+                tc_fence_after();
+                __syncwarp();
+                if (elect_one()) {
+                    const uint64_t dA = desc_kmajor(smem_u32(gs + G_AI), 512), dB = desc_mnmajor(smem_u32(gs + G_BWF));
+#pragma unroll
+                    for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_FOLD, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 64), idesc(64, false, true), ks > 0);
+#pragma unroll
+                    for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_XY + 32 * g + 16, dA + (uint64_t)(ks * 16), dA + (uint64_t)(ks * 16), idesc(16, false, false), ks > 0);
+                    tc_commit(&ctrl->fold[g]);
+                    // The chunk's four 16x16 matrices go into its checkpoint record: the three tiles [AK;QK], AI^T, QB are
+                    // contiguous in shared memory and are stored as they are, by one bulk copy.
+                    if (p.ckpt) {
+                        const ChunkDesc& d = ctrl->desc[g][k & 3];
+                        float* ckm = p.ckpt + ((long long)d.bh * nchunks + d.c) * CK_FLOATS + CK_MATS;
+                        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                                     ::"l"(__cvta_generic_to_global(ckm)), "r"(smem_u32(gs + G_SC)), "n"(4 * L * L * 4) : "memory");
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                }
+                __syncwarp();
+            }
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last copy
         }
         __syncwarp();
     } else {
@@ -420,31 +554,26 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         const int grp = warp >> 2, wg = warp & 3, gt = tid & 127;
         unsigned char* gs = sm + grp * G_BYTES;
         const uint32_t tlane = tmem + ((uint32_t)(32 * wg) << 16);
-        const IoT* const gin[6] = {(const IoT*)p.r, (const IoT*)p.w, (const IoT*)p.k, (const IoT*)p.a, (const IoT*)p.b, (const IoT*)p.v};
-        const IoT* const gg = LN ? (const IoT*)p.g : nullptr;
-        auto issue_raw = [&](int ko) {  // own chunk number ko
-            const int gbuf = ko & 1;
+        // The raw tiles of own chunk number ko by bulk tensor loads (16 rows of 128 bytes, 16-byte units XOR-ed with the row;
+        // rows beyond the end of the sequence arrive as zeros).  One thread of the group.
+        auto load_tile = [&](const CUtensorMap& m, int at, const ChunkDesc& d, uint64_t* bar) {
+            asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                         ::"r"(smem_u32(gs + at)), "l"(&m), "r"(smem_u32(bar)), "r"(0), "r"(d.hi), "r"(d.c * L), "r"(d.bi) : "memory");
+        };
+        auto expect_bytes = [&](uint64_t* bar, int bytes) {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+        };
+        auto load_raw = [&](int ko) {
             const ChunkDesc& d = ctrl->desc[grp][ko & 3];
-            const int c = d.c;
-            const int r = gt >> 3, seg = gt & 7;
-            const bool live = !TAIL || c + 1 < nchunks || r < tail;  // rows beyond the end of the sequence are filled with zeros, nothing is read
-            const long long goff = d.off + ((long long)c * L + (live ? r : 0)) * p.st.t;
-            const int at = r * ROWB + ((seg ^ (r & 7)) << 4);
+            expect_bytes(&ctrl->raw[grp], 6 * RAW_TILE);
 #pragma unroll
-            for (int ten = 0; ten < 6; ++ten) {
-                if (TAIL) cp_async16_zfill(gs + G_RAW + ten * RAW_TILE + at, reinterpret_cast<const unsigned char*>(gin[ten] + goff) + seg * 16, live);
-                else cp_async16(gs + G_RAW + ten * RAW_TILE + at, reinterpret_cast<const unsigned char*>(gin[ten] + goff) + seg * 16);
-            }
-            if (LN) {
-                if (TAIL) cp_async16_zfill(gs + G_GRAW + gbuf * RAW_TILE + at, reinterpret_cast<const unsigned char*>(gg + goff) + seg * 16, live);
-                else cp_async16(gs + G_GRAW + gbuf * RAW_TILE + at, reinterpret_cast<const unsigned char*>(gg + goff) + seg * 16);
-            }
-            cp_async_commit();
+            for (int ten = 0; ten < 6; ++ten) load_tile(maps.in[ten], G_RAW + ten * RAW_TILE, d, &ctrl->raw[grp]);
         };
         // Results of own chunk number kk (list position vv): Y^T into registers, the chunk-end state straight to the
         // checkpoint (or the final state).  All of it is read before the group announces its next chunk.
         auto read_results = [&](int kk) {
             mbar_wait<true>(&ctrl->done[grp], kk & 1, ctrl, p.status);
+            if (LN) mbar_wait<true>(&ctrl->gate[grp], kk & 1, ctrl, p.status);
             tc_fence_after();
             const ChunkDesc& d = ctrl->desc[grp][kk & 3];
             const int vv = grp + kk * G, cc = d.c;
@@ -471,13 +600,12 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 float* ysf = reinterpret_cast<float*>(gs + G_KWF);
                 float* part = reinterpret_cast<float*>(gs + G_KWF + LN_PART);
                 {
-                    uint32_t yv[16];
-                    tmem_ld16(tlane + C_XY + 32 * grp + 16, yv);
+                    uint32_t yv[8];
+                    tmem_ld_frag(tlane + C_XY + 32 * grp + 16, yv);
                     tmem_ld_wait();
-                    if (lane < 16) {
 #pragma unroll
-                        for (int t = 0; t < 16; ++t) ysf[t * LN_YS + 16 * wg + lane] = __uint_as_float(yv[t]);
-                    }
+                    for (int i = 0; i < 8; ++i)
+                        ysf[(8 * (i >> 2) + 2 * (lane & 3) + (i & 1)) * LN_YS + 16 * wg + (lane >> 2) + 8 * ((i >> 1) & 1)] = __uint_as_float(yv[i]);
                 }
                 group_bar(grp);
                 const int t = lane & 15, i0 = 16 * wg + 8 * (lane >> 4);
@@ -511,7 +639,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     const float4 v0 = *reinterpret_cast<const float4*>(gs + G_V + mo), v1 = *reinterpret_cast<const float4*>(gs + G_V + mo + 16);
                     const float vval[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
                     float gv[8];
-                    load8<IoT>(gs + G_GRAW + (kk & 1) * RAW_TILE + t * ROWB + (((i0 >> 3) ^ (t & 7)) << 4), gv);
+                    load8<IoT>(gs + G_GRAW + t * ROWB + (((i0 >> 3) ^ (t & 7)) << 4), gv);
                     float o8[8];
                     const float* lnp = p.params + d.hi * N + i0;  // GroupNorm weight, then bias: 32 bytes each per thread, in L1
                     const float4 w0 = __ldg(reinterpret_cast<const float4*>(lnp)), w1 = __ldg(reinterpret_cast<const float4*>(lnp) + 1);
@@ -538,20 +666,18 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 // decay term all of them), staged in the 128-byte-swizzled layout the tensor-map store expects: half h = columns 32h..32h+31,
                 // row i at i*128 bytes, its 16-byte unit u at (u ^ (i & 7))
                 unsigned char* stage = gs + G_WAQ;
-                const int i = 16 * wg + (lane & 15);
+                const int i = 16 * wg + (lane >> 2);  // rows i, i + 8
 #pragma unroll
-                for (int qt = 0; qt < 4; ++qt) {
-                    uint32_t sv[16];
-                    tmem_ld16(tlane + C_S + 64 * ((vv + 1) & 3) + 16 * qt, sv);
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t x[16];
+                    tmem_ld_frag4(tlane + C_S + 64 * ((vv + 1) & 3) + 32 * half, x);
                     tmem_ld_wait();
-                    if (lane < 16) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int u = 4 * qt + j;
-                            *reinterpret_cast<uint4*>(stage + (u >> 3) * 8192 + i * 128 + (((u & 7) ^ (i & 7)) << 4)) =
-                                make_uint4(sv[4 * j], sv[4 * j + 1], sv[4 * j + 2], sv[4 * j + 3]);
-                        }
-                    }
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            *reinterpret_cast<uint2*>(stage + half * 8192 + (i + 8 * h) * 128 + (((2 * j + ((lane & 3) >> 1)) ^ (i & 7)) << 4) + (lane & 1) * 8) =
+                                make_uint2(x[4 * j + 2 * h], x[4 * j + 2 * h + 1]);
                 }
                 fence_async_smem();
                 group_bar(grp);
@@ -589,19 +715,84 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             }
         };
         const int row = lane & 15, j0 = 16 * wg + 8 * (lane >> 4);
-        if (grp < work.n) issue_raw(0);
-        // One more iteration than there are own chunks: the last one only reads the last results (one copy of that code).
-        for (int k = 0, v0 = grp; ; v0 += G, ++k) {
-            const bool have = v0 < work.n;
-            cp_async_wait<0>();
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the matrix copy of the previous own chunk (its issuer only)
-            group_bar(grp);
-            // ---------------- decay scan, into registers ---------------------------------------------
+        if (wg == 2 && grp < work.n && elect_one()) load_raw(0);
+        __syncwarp();
+        // Iteration k: read the results of own chunk k - 1, write the operand tiles of chunk k (whose scan is in registers),
+        // start its score product; then scan chunk k + 1 while the score, inverse and chain warps finish chunk k.  (k = -1 only
+        // scans, the last one only reads results: one copy of each piece of code.)
+        F2 o[4][4], v[4], fwv[4];  // wq, wa, kwi, bwi; kwf, bwf are formed from kwi, bwi and fw when the tiles are written
+        for (int k = -1, v0 = grp - G; ; v0 += G, ++k) {
+            if (k >= 0) {
+                // ---------------- results of the previous own chunk (its operand tiles are free afterwards) --
+                if (k > 0) read_results(k - 1);
+                if (v0 >= work.n) break;
+                // ---------------- operand tiles -----------------------------------------------------------
+                {
+                    const int jc = j0 >> 2;
+                    const int mo = (j0 >> 5) * 2048 + row * 128 + ((((j0 & 31) >> 3) ^ (row & 3)) << 5);
+                    const bool flip = (row >> 2) & 1;
+                    F2 kf[4], bf[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {  // k P_L / P_t first, then 2^-64
+                        kf[i] = mul2(mul2(o[2][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                        bf[i] = mul2(mul2(o[3][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                    }
+                    store8mn<RND>(gs + G_KWF + mo, kf, flip);
+                    store8mn<RND>(gs + G_BWF + mo, bf, flip);
+                    store8mn<false>(gs + G_V + mo, v, flip);  // bf16 values are exact in TF32
+                    if (row == 15) {
+                        unsigned char* df = gs + G_DF + (j0 >> 3) * 256;
+#pragma unroll
+                        for (int n = 0; n < 8; ++n) {
+                            const float pl = (n & 1 ? fwv[n / 2].y : fwv[n / 2].x) * STATE_SCALE;  // P_L; where it underflows, so does S~ P_L
+                            *reinterpret_cast<float*>(df + (n >> 2) * 128 + n * 16 + (n & 3) * 4) = RND ? rnd(pl) : pl;
+                        }
+                    }
+                    if (k > 0 && p.ckpt) {  // the state's staging tiles are the next two operand tiles: wait until the bulk stores have read them
+                        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                        group_bar(grp);
+                    }
+                    store8t<RND>(gs + G_WAQ + kchunk(row, jc, 2048), gs + G_WAQ + kchunk(row, jc + 1, 2048), o[1]);
+                    store8t<RND>(gs + G_WAQ + kchunk(16 + row, jc, 2048), gs + G_WAQ + kchunk(16 + row, jc + 1, 2048), o[0]);
+                    store8t<RND>(gs + G_KB + kchunk(row, jc, 2048), gs + G_KB + kchunk(row, jc + 1, 2048), o[2]);
+                    store8t<RND>(gs + G_KB + kchunk(16 + row, jc, 2048), gs + G_KB + kchunk(16 + row, jc + 1, 2048), o[3]);
+                }
+                if (ctrl->desc[grp][k & 3].flags & SEG_FIRST) load_state(ctrl->desc[grp][k & 3], wg);
+                fence_async_smem();
+                tc_fence_before();
+                group_bar(grp);
+                tc_fence_after();
+                if (LN && wg == 2 && elect_one()) {
+                    expect_bytes(&ctrl->gate[grp], RAW_TILE);
+                    load_tile(maps.g, G_GRAW, ctrl->desc[grp][k & 3], &ctrl->gate[grp]);
+                }
+                __syncwarp();
+                if (gt == 127 && v0 + 2 * G < work.n) {  // read after this group's next barrier
+                    ChunkDesc d = ctrl->desc[grp][(k + 1) & 3];
+                    d.c += G;
+                    if (d.c < d.c_end) {
+                        d.flags = d.c + 1 == d.c_end ? SEG_LAST : 0;
+                        ctrl->desc[grp][(k + 2) & 3] = d;
+                    } else {
+                        describe(grp, k + 2);
+                    }
+                }
+                __syncwarp();
+                // ---------------- the four score matrices as one product ---------------------------------
+                if (wg == 0 && elect_one()) {
+                    const uint64_t dA = desc_kmajor(smem_u32(gs + G_WAQ), 2048), dB = desc_kmajor(smem_u32(gs + G_KB), 2048);
+#pragma unroll
+                    for (int ks = 0; ks < 8; ++ks) mma_ss(tmem + C_XY + 32 * grp, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
+                    tc_commit(&ctrl->score[grp]);
+                }
+                __syncwarp();
+            }
+            // ---------------- decay scan of the next own chunk, into registers -----------------------
             // One thread = one time step x 8 adjacent key channels.  The three transcendentals per
             // element go to the special-function unit: with the matrix products on tcgen05 the FMA
             // pipe and the issue slots are what this kernel runs out of, not MUFU throughput.
-            F2 o[4][4], v[4], fwv[4];  // kwf, bwf are formed from kwi, bwi and fw when the tiles are written
-            if (have) {
+            if (v0 + G < work.n) {
+                mbar_wait<true>(&ctrl->raw[grp], (k + 1) & 1, ctrl, p.status);
                 const unsigned char* raw = gs + G_RAW + row * ROWB + (((j0 >> 3) ^ (row & 7)) << 4);
                 F2 cum[4], q[4], kk[4], a[4], b[4];
                 load8f2(raw + 1 * RAW_TILE, cum);
@@ -612,7 +803,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 load8f2(raw + 5 * RAW_TILE, v);
                 if (LN) {  // bonus dot sum_j r_j k_j bonus_j of this time step: 8 channels here, the rest by shuffle and in the epilogue
                     F2 acc = f2(0.f, 0.f);
-                    const float4* bp = reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][k & 3].hi) * N + j0);
+                    const float4* bp = reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][(k + 1) & 3].hi) * N + j0);
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         const float4 bo = __ldg(bp + i);
@@ -621,7 +812,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     }
                     float dot = acc.x + acc.y;
                     dot += __shfl_xor_sync(0xffffffffu, dot, 16);
-                    if (lane < 16) ctrl->bdot[grp][k & 1][wg][row] = dot;
+                    if (lane < 16) ctrl->bdot[grp][(k + 1) & 1][wg][row] = dot;
                 }
                 // log2 of the per-step decay: -exp(w) * log2(e); running sum along the 16 time rows
                 constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // the per-step floor in log2 units
@@ -631,7 +822,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     cum[i] = mul2(f2(ex2_approx(cum[i].x), ex2_approx(cum[i].y)), f2(-LOG2E, -LOG2E));
                     cum[i] = f2(fmaxf(cum[i].x, FLOOR), fmaxf(cum[i].y, FLOOR));
                 }
-                if (TAIL && ctrl->desc[grp][k & 3].c + 1 == nchunks && row >= tail) {  // a row beyond the end of the sequence: no decay, the state passes through
+                if (TAIL && ctrl->desc[grp][(k + 1) & 3].c + 1 == nchunks && row >= tail) {  // a row beyond the end of the sequence: no decay, the state passes through
 #pragma unroll
                     for (int i = 0; i < 4; ++i) cum[i] = f2(0.f, 0.f);
                 }
@@ -661,160 +852,10 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     fwv[i] = f2(__shfl_sync(0xffffffffu, incl.x, 15, 16), __shfl_sync(0xffffffffu, incl.y, 15, 16));
                 }
             }
-            // ---------------- results of the previous own chunk (its operand tiles are free afterwards) --
-            if (k > 0) read_results(k - 1);
-            if (!have) break;
-            // ---------------- operand tiles -----------------------------------------------------------
-            {
-                const int jc = j0 >> 2;
-                const int mo = (j0 >> 5) * 2048 + row * 128 + ((((j0 & 31) >> 3) ^ (row & 3)) << 5);
-                const bool flip = (row >> 2) & 1;
-                F2 kf[4], bf[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {  // k P_L / P_t first, then 2^-64
-                    kf[i] = mul2(mul2(o[2][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
-                    bf[i] = mul2(mul2(o[3][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
-                }
-                store8mn<RND>(gs + G_KWF + mo, kf, flip);
-                store8mn<RND>(gs + G_BWF + mo, bf, flip);
-                store8mn<false>(gs + G_V + mo, v, flip);  // bf16 values are exact in TF32
-                if (row == 15) {
-                    unsigned char* df = gs + G_DF + (j0 >> 3) * 256;
-#pragma unroll
-                    for (int n = 0; n < 8; ++n) {
-                        const float pl = (n & 1 ? fwv[n / 2].y : fwv[n / 2].x) * STATE_SCALE;  // P_L; where it underflows, so does S~ P_L
-                        *reinterpret_cast<float*>(df + (n >> 2) * 128 + n * 16 + (n & 3) * 4) = RND ? rnd(pl) : pl;
-                    }
-                }
-                if (k > 0 && p.ckpt) {  // the state's staging tiles are the next two operand tiles: wait until the bulk stores have read them
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    group_bar(grp);
-                }
-                store8t<RND>(gs + G_WAQ + kchunk(row, jc, 2048), gs + G_WAQ + kchunk(row, jc + 1, 2048), o[1]);
-                store8t<RND>(gs + G_WAQ + kchunk(16 + row, jc, 2048), gs + G_WAQ + kchunk(16 + row, jc + 1, 2048), o[0]);
-                store8t<RND>(gs + G_KB + kchunk(row, jc, 2048), gs + G_KB + kchunk(row, jc + 1, 2048), o[2]);
-                store8t<RND>(gs + G_KB + kchunk(16 + row, jc, 2048), gs + G_KB + kchunk(16 + row, jc + 1, 2048), o[3]);
-            }
-            fence_async_smem();
-            group_bar(grp);
-            if (v0 + G < work.n) issue_raw(k + 1);
-            if (gt == 127 && v0 + 2 * G < work.n) {  // read after this group's next barrier
-                ChunkDesc d = ctrl->desc[grp][(k + 1) & 3];
-                d.c += G;
-                if (d.c < d.c_end) {
-                    d.flags = d.c + 1 == d.c_end ? SEG_LAST : 0;
-                    ctrl->desc[grp][(k + 2) & 3] = d;
-                } else {
-                    describe(grp, k + 2);
-                }
-            }
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // y's tile has been read (its issuer only)
+            group_bar(grp);  // the raw tiles have been read
+            if (wg == 2 && v0 + 2 * G < work.n && elect_one()) load_raw(k + 2);
             __syncwarp();
-            if (ctrl->desc[grp][k & 3].flags & SEG_FIRST) load_state(ctrl->desc[grp][k & 3], wg);
-            // ---------------- the four score matrices as one product ---------------------------------
-            if (wg == 0 && elect_one()) {
-                const uint64_t dA = desc_kmajor(smem_u32(gs + G_WAQ), 2048), dB = desc_kmajor(smem_u32(gs + G_KB), 2048);
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks) mma_ss(tmem + C_XY + 32 * grp, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
-                tc_commit(&ctrl->score[grp]);
-            }
-            __syncwarp();
-            if (wg < 2) {
-                mbar_wait<true>(&ctrl->score[grp], 0, ctrl, p.status);
-                tc_fence_after();
-                uint32_t sv[32];
-                tmem_ld16(tlane + C_XY + 32 * grp, sv);
-                tmem_ld16(tlane + C_XY + 32 * grp + 16, sv + 16);
-                tmem_ld_wait();
-                const int t = lane;
-                if (wg == 0) {
-                    // lane t: row t of AK (strictly lower) and of AB (strictly lower, kept transposed for the inverse)
-                    if (lane < 16) {
-                        float* ABt = reinterpret_cast<float*>(gs + G_ABT);
-#pragma unroll
-                        for (int qd = 0; qd < 4; ++qd) {
-                            float4 x;
-                            x.x = (4 * qd + 0 < t) ? rnd(__uint_as_float(sv[4 * qd + 0])) : 0.f;
-                            x.y = (4 * qd + 1 < t) ? rnd(__uint_as_float(sv[4 * qd + 1])) : 0.f;
-                            x.z = (4 * qd + 2 < t) ? rnd(__uint_as_float(sv[4 * qd + 2])) : 0.f;
-                            x.w = (4 * qd + 3 < t) ? rnd(__uint_as_float(sv[4 * qd + 3])) : 0.f;
-                            *reinterpret_cast<float4*>(gs + G_SC + kchunk(t, qd, 512)) = x;
-                        }
-#pragma unroll
-                        for (int s = 0; s < 16; ++s) ABt[s * SCS + t] = (s < t) ? __uint_as_float(sv[16 + s]) : 0.f;
-                    }
-                    __syncwarp();
-                    if (lane < 16) tri_inverse_tc(reinterpret_cast<const float*>(gs + G_ABT), gs + G_AI, lane);
-                } else if (lane < 16) {
-                    // lane t: row t of QK and QB (lower triangular including the diagonal)
-#pragma unroll
-                    for (int qd = 0; qd < 4; ++qd) {
-                        float4 x, x2;
-                        x.x = (4 * qd + 0 <= t) ? rnd(__uint_as_float(sv[4 * qd + 0])) : 0.f;
-                        x.y = (4 * qd + 1 <= t) ? rnd(__uint_as_float(sv[4 * qd + 1])) : 0.f;
-                        x.z = (4 * qd + 2 <= t) ? rnd(__uint_as_float(sv[4 * qd + 2])) : 0.f;
-                        x.w = (4 * qd + 3 <= t) ? rnd(__uint_as_float(sv[4 * qd + 3])) : 0.f;
-                        x2.x = (4 * qd + 0 <= t) ? rnd(__uint_as_float(sv[16 + 4 * qd + 0])) : 0.f;
-                        x2.y = (4 * qd + 1 <= t) ? rnd(__uint_as_float(sv[16 + 4 * qd + 1])) : 0.f;
-                        x2.z = (4 * qd + 2 <= t) ? rnd(__uint_as_float(sv[16 + 4 * qd + 2])) : 0.f;
-                        x2.w = (4 * qd + 3 <= t) ? rnd(__uint_as_float(sv[16 + 4 * qd + 3])) : 0.f;
-                        *reinterpret_cast<float4*>(gs + G_SC + kchunk(16 + t, qd, 512)) = x;
-                        *reinterpret_cast<float4*>(gs + G_QB + kchunk(t, qd, 512)) = x2;
-                    }
-                }
-            }
-            fence_async_smem();
-            tc_fence_before();
-            group_bar(grp);
-            tc_fence_after();
-            // ---------------- U folded into the operands: U = X AI^T, so U bwf = X (AI^T bwf) and U QB^T = X (QB AI)^T --------
-            // (one dependent tensor-core round trip per chunk less for the chain, which is what this kernel waits for)
-            if (wg == 0 && elect_one()) {
-                const uint64_t dB = desc_mnmajor(smem_u32(gs + G_BWF)), dQ = desc_kmajor(smem_u32(gs + G_QB), 512), dI = desc_kmajor(smem_u32(gs + G_AI), 512);
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_XY + 32 * grp, dB + (uint64_t)(ks * 64), dI + (uint64_t)(ks * 16), idesc(16, true, false), ks > 0);
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_XY + 32 * grp + 16, dQ + (uint64_t)(ks * 16), dI + (uint64_t)(ks * 16), idesc(16, false, false), ks > 0);
-                tc_commit(&ctrl->score[grp]);
-            }
-            __syncwarp();
-            mbar_wait<true>(&ctrl->score[grp], 1, ctrl, p.status);
-            tc_fence_after();
-            {
-                uint32_t bv[16], qv[16];
-                tmem_ld16(tlane + C_XY + 32 * grp, bv);             // lane: key 16 wg + lane, 16 time steps
-                if (wg == 0) tmem_ld16(tlane + C_XY + 32 * grp + 16, qv);  // lane: row of QB AI
-                tmem_ld_wait();
-                if (lane < 16) {
-                    const int key = 16 * wg + lane;
-                    unsigned char* bw = gs + G_BWF + (key >> 5) * 2048 + (key & 7) * 4;
-#pragma unroll
-                    for (int t = 0; t < 16; ++t)
-                        *reinterpret_cast<float*>(bw + t * 128 + ((((key & 31) >> 3) ^ (t & 3)) << 5)) = rnd(__uint_as_float(bv[t]));
-                    if (wg == 0) {
-#pragma unroll
-                        for (int qd = 0; qd < 4; ++qd)
-                            *reinterpret_cast<float4*>(gs + G_QBU + kchunk(lane, qd, 512)) =
-                                make_float4(rnd(__uint_as_float(qv[4 * qd])), rnd(__uint_as_float(qv[4 * qd + 1])),
-                                            rnd(__uint_as_float(qv[4 * qd + 2])), rnd(__uint_as_float(qv[4 * qd + 3])));
-                    }
-                }
-            }
-            fence_async_smem();
-            tc_fence_before();
-            mbar_arrive(&ctrl->full[grp]);
-            // The chunk's four 16x16 matrices go into its checkpoint record: the three tiles [AK;QK], AI, QB are
-            // contiguous in shared memory and are stored as they are, by one bulk copy issued after the chain
-            // has been given the go-ahead (their writers have fenced and passed the group's barrier by then).
-            if (p.ckpt && wg == 0) {
-                if (elect_one()) {
-                    const ChunkDesc& d = ctrl->desc[grp][k & 3];
-                    float* ckm = p.ckpt + ((long long)d.bh * nchunks + d.c) * CK_FLOATS + CK_MATS;
-                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                                 ::"l"(__cvta_generic_to_global(ckm)), "r"(smem_u32(gs + G_SC)), "n"(4 * L * L * 4) : "memory");
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                }
-                __syncwarp();
-            }
         }
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last copies
     }
@@ -855,7 +896,10 @@ template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdPar
     FwdMaps maps;
     memset(&maps, 0, sizeof(maps));
     if (p.ckpt && !encode_checkpoint_map(&maps.ck, p.ckpt, p.B * p.H * ((p.T + L - 1) / L))) return kLaunchFailed;
-    if (!encode_bthn_map(&maps.y, p.y, p.B, p.T, p.H, p.st)) return kLaunchFailed;
+    const void* ins[8] = {p.y, p.r, p.w, p.k, p.a, p.b, p.v, p.g};
+    CUtensorMap* const ms[8] = {&maps.y, &maps.in[0], &maps.in[1], &maps.in[2], &maps.in[3], &maps.in[4], &maps.in[5], &maps.g};
+    for (int i = 0; i < (LN ? 8 : 7); ++i)
+        if (!encode_bthn_map(ms[i], const_cast<void*>(ins[i]), p.B, p.T, p.H, p.st)) return kLaunchFailed;
     const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 1, p.sT ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
     kern<<<(unsigned)ws.ctas, 128 * (G + 1), smem, stream>>>(p, ws, maps);
