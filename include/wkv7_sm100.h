@@ -126,6 +126,20 @@ int wkv7_attn_ln_fwd_ws(const void* r, const void* w, const void* k, const void*
                         const void* g, const float* params, const float* s0, void* y, float* sT, float* ckpt,
                         float eps, int64_t B, int64_t T, int64_t H, int64_t N,
                         int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
+/* The backward keeps a cut chain's state gradient in ds0, which must be given for a cut. */
+int wkv7_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                const void* dy, const float* ckpt, const float* dsT, const float* sT,
+                void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* ds0,
+                int64_t B, int64_t T, int64_t H, int64_t N,
+                int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
+/* As wkv7_attn_ln_bwd; dparams_workspace is that call's workspace.  Where a chain is cut, its part of dparams is summed in two
+ * pieces: dparams then agrees with the plain call's up to fp32 rounding (and is still deterministic). */
+int wkv7_attn_ln_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                        const void* g, const float* params, const void* dy, const float* ckpt, const float* dsT,
+                        const float* sT, void* dr, void* dw, void* dk, void* dv, void* da, void* db, void* dg,
+                        float* dparams, float* dparams_workspace, float* ds0, float eps,
+                        int64_t B, int64_t T, int64_t H, int64_t N,
+                        int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
 
 /*
  * WKV7 decode step(s): the recurrence itself, time step by time step, for generation after a prefill.

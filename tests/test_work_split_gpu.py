@@ -37,3 +37,40 @@ def test_forward(extra, T, ckpt, ln):
     for a, b in zip(call(False), call(True)):
         assert bool(th.isfinite(a.float()).all()) and th.equal(a, b)
     assert L.wkv7_device_status() == 0
+
+
+@pytest.mark.parametrize('ln', [False, True])
+@pytest.mark.parametrize('extra,T,dsT', [(1, 16, False), (-1, 48, True), (70, 7, True), (200, 33, False), (149, 500, True), (400, 65, True)])
+def test_backward(extra, T, dsT, ln):
+    from wind_rwkv.rwkv7 import _lib, synthetic
+    from wind_rwkv.rwkv7.rwkv7_attn import fw_attn
+    L = _lib.lib()
+    B, H = 1, sms() + extra
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=T, dtype=th.bfloat16, device='cuda', s0_std=0.1)
+    g, params = synthetic.attn_ln_extras(B, T, H, N, seed=T, dtype=th.bfloat16, device='cuda')
+    _, sT, ck = fw_attn(*[d[n].view(B, T, H, N) for n in 'wrkvab'], d['s0'])
+    gs = th.randn(B, H, N, N, device='cuda') if dsT else None
+    ws = th.full((L.wkv7_workspace_bytes(),), 255, dtype=th.uint8, device='cuda')
+    part = th.empty(B, 3, H * N, device='cuda')
+
+    def call(split):
+        outs = [th.full_like(d['r'], float('nan')) for _ in range(7 if ln else 6)]
+        outs += [th.full((B, H, N, N), float('nan'), device='cuda')] + ([th.full_like(params, float('nan'))] if ln else [])
+        a = [d[n].data_ptr() for n in 'rwkvab'] + ([g.data_ptr(), params.data_ptr()] if ln else [])
+        a += [d['dy'].data_ptr(), ck.data_ptr(), _lib.ptr(gs), _lib.ptr(sT if dsT else None)]
+        if ln:
+            a += [o.data_ptr() for o in outs[:7]] + [outs[8].data_ptr(), part.data_ptr(), outs[7].data_ptr(), 64e-5]
+        else:
+            a += [o.data_ptr() for o in outs]
+        a += [B, T, H, N, T * H * N, H * N, N, 0] + ([ws.data_ptr()] if split else []) + [None]
+        assert getattr(L, ('wkv7_attn_ln_bwd' if ln else 'wkv7_bwd') + ('_ws' if split else ''))(*a) == 0
+        th.cuda.synchronize()
+        return outs
+
+    for i, (a, b) in enumerate(zip(call(False), call(True))):
+        assert bool(th.isfinite(a.float()).all())
+        if i == 8:  # parameter gradients of a cut chain are summed in two pieces
+            assert (a - b).norm() <= 1e-5 * a.norm()
+        else:
+            assert th.equal(a, b)
+    assert L.wkv7_device_status() == 0

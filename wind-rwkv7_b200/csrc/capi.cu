@@ -269,7 +269,7 @@ static int bwd_common(const void* r, const void* w, const void* k, const void* v
                       const void* g, const float* params, bool ln, float eps, const void* dy, const float* ckpt,
                       const float* dsT, const float* sT, void* dr, void* dw, void* dk, void* dv, void* da, void* db,
                       void* dg, float* dparams, float* dparams_ws, float* ds0, int64_t B, int64_t T, int64_t H, int64_t N,
-                      int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* stream) {
+                      int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream) {
     int rc = check_common(B, T, H, N, stride_b, stride_t, stride_h, io_dtype);
     if (rc) return rc;
     if (B == 0 || H == 0) return WKV7_OK;
@@ -289,7 +289,7 @@ static int bwd_common(const void* r, const void* w, const void* k, const void* v
     if (!r || !w || !k || !v || !a || !b || !dy || !ckpt || !dr || !dw || !dk || !dv || !da || !db) return WKV7_ERR_NULL;
     if (dsT && !sT) return WKV7_ERR_NULL;
     if (ln && (!g || !params || !dg || !dparams || !dparams_ws)) return WKV7_ERR_NULL;
-    const void* ptrs[] = {r, w, k, v, a, b, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, ds0, g, params, dg, dparams, dparams_ws};
+    const void* ptrs[] = {r, w, k, v, a, b, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, ds0, g, params, dg, dparams, dparams_ws, workspace};
     for (const void* p : ptrs)
         if (p && !aligned16(p)) return WKV7_ERR_ALIGN;
     wkv7::BwdParams p{};
@@ -299,6 +299,7 @@ static int bwd_common(const void* r, const void* w, const void* k, const void* v
     p.dr = dr; p.dw = dw; p.dk = dk; p.dv = dv; p.da = da; p.db = db; p.ds0 = ds0;
     p.B = B; p.T = T; p.H = H;
     p.st = wkv7::Strides{stride_b, stride_t, stride_h};
+    p.flags = (unsigned*)workspace;
     p.status = status_ptr();
     if (!p.status) return WKV7_ERR_LAUNCH;
     return wkv7::launch_bwd(p, io_dtype, ln, (cudaStream_t)stream);
@@ -309,7 +310,15 @@ int wkv7_bwd(const void* r, const void* w, const void* k, const void* v, const v
              void* dv, void* da, void* db, float* ds0, int64_t B, int64_t T, int64_t H, int64_t N, int64_t stride_b,
              int64_t stride_t, int64_t stride_h, int io_dtype, void* stream) {
     return bwd_common(r, w, k, v, a, b, nullptr, nullptr, false, 0.f, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, nullptr,
-                      nullptr, nullptr, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, stream);
+                      nullptr, nullptr, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, nullptr, stream);
+}
+
+int wkv7_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                const void* dy, const float* ckpt, const float* dsT, const float* sT, void* dr, void* dw, void* dk,
+                void* dv, void* da, void* db, float* ds0, int64_t B, int64_t T, int64_t H, int64_t N, int64_t stride_b,
+                int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream) {
+    return bwd_common(r, w, k, v, a, b, nullptr, nullptr, false, 0.f, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, nullptr,
+                      nullptr, nullptr, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, workspace, stream);
 }
 
 int64_t wkv7_attn_ln_bwd_workspace_bytes(int64_t B, int64_t H, int64_t N) {
@@ -323,7 +332,16 @@ int wkv7_attn_ln_bwd(const void* r, const void* w, const void* k, const void* v,
                      float* dparams, float* workspace, float* ds0, float eps, int64_t B, int64_t T, int64_t H,
                      int64_t N, int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* stream) {
     return bwd_common(r, w, k, v, a, b, g, params, true, eps, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, dg, dparams,
-                      workspace, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, stream);
+                      workspace, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, nullptr, stream);
+}
+
+int wkv7_attn_ln_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                        const void* g, const float* params, const void* dy, const float* ckpt, const float* dsT,
+                        const float* sT, void* dr, void* dw, void* dk, void* dv, void* da, void* db, void* dg,
+                        float* dparams, float* dparams_workspace, float* ds0, float eps, int64_t B, int64_t T, int64_t H,
+                        int64_t N, int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream) {
+    return bwd_common(r, w, k, v, a, b, g, params, true, eps, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, dg, dparams,
+                      dparams_workspace, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, workspace, stream);
 }
 
 int wkv7_attn_ln_bwd_static(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
@@ -336,7 +354,7 @@ int wkv7_attn_ln_bwd_static(const void* r, const void* w, const void* k, const v
     float* scratch = static_scratch();
     if (!scratch) return WKV7_ERR_LAUNCH;
     return bwd_common(r, w, k, v, a, b, g, params, true, eps, dy, ckpt, dsT, sT, dr, dw, dk, dv, da, db, dg, dparams,
-                      scratch, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, stream);
+                      scratch, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, nullptr, stream);
 }
 
 int wkv7_proj_gemm(const void* A, const void* W, void* C, int64_t M, int64_t N, int64_t K, int64_t tanh_from,

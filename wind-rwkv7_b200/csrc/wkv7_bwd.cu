@@ -1,5 +1,5 @@
-// WKV7 backward for sm_100a: one CTA per (batch, head) chain, 4 warps, chunks of 16 time steps
-// walked in reverse; the gradient dS of the state stays in registers across chunks.
+// WKV7 backward for sm_100a, fp32 tensors (single or triple TF32 products; bf16 tensors: wkv7_bwd_bf16.cu): one CTA per
+// (batch, head) chain, 4 warps, chunks of 16 time steps walked in reverse; the gradient dS of the state stays in registers.
 //
 // Replaces the reference's backward_kernel (wind_rwkv/rwkv7/attn.cu:131-326).  The forward
 // intermediates of a chunk are rebuilt from the fp32 chunk-start state S0 the forward wrote (exact fp32; in the
@@ -37,9 +37,7 @@
 
 namespace wkv7 {
 
-// Tensor maps of the five [time x key] outputs (dq, dw, dk, da, db) for the bulk-store epilogue.
-// ck: the checkpoint states, for the bulk tensor loads of the chunk-start state.
-struct alignas(64) OutMaps { CUtensorMap m[7]; CUtensorMap ck, ckm; };  // m[5]: dv, m[6]: dg (attn_ln); ck, ckm: checkpoint states, matrices
+struct alignas(64) CkptMaps { CUtensorMap ck, ckm; };  // checkpoint states, matrices
 
 constexpr int SS = N + 8;  // row stride (floats) of the [value][key] state buffers
 constexpr int MAT_BLK = 8 * 4 * SCS;  // floats per block of the matrices buffer
@@ -80,7 +78,7 @@ template <typename IoT, int PREC, bool LN> struct BwdSmem {
     // the per-warp transposition scratch for dv / dg and as the GroupNorm reduction buffers.
     static constexpr int SCRATCH_FLOATS = WARPS * L * Lay::YS * (int)sizeof(IoT) / 4 + WARPS * L * 5;
     static constexpr int SGRAD_FLOATS = 4 * L * SCS > SCRATCH_FLOATS ? 4 * L * SCS : SCRATCH_FLOATS;
-    alignas(LN && sizeof(IoT) == 2 ? 1024 : 16) float sgrad[SGRAD_FLOATS];  // score gradient i at sgrad + i * L * SCS
+    alignas(16) float sgrad[SGRAD_FLOATS];  // score gradient i at sgrad + i * L * SCS
     // attn_ln: Ut, Dt, Yt are dead between stage C and the next chunk's stage B and double as the output staging tiles
     alignas(LN ? 1024 : 16) float Ut[L * OPS];  // U and dabu as [time][value]
     alignas(16) float Dt[L * OPS];
@@ -96,21 +94,7 @@ template <typename IoT, int PREC, bool LN> struct BwdSmem {
     alignas(16) float Gp[2][WARPS][N];
     alignas(16) float lnp[LN ? 3 * N : 4];
     float bdot[L], sbon[L];
-    // bf16: the five [16 x 64] output tiles of a chunk, 128-byte rows with the 16-byte unit index XOR-ed
-    // with (row % 8) (what a 128-byte-swizzle tensor map expects), stored by five bulk tensor copies per chunk
-    static constexpr bool TMA_OUT = sizeof(IoT) == 2;
-    // (attn: a sixth tile carries dv, which is formed one stage earlier)
-    // (attn_ln: the five tiles alias Ut, Dt, Yt; only dv's tile lives here)
-    alignas(TMA_OUT ? 1024 : 16) unsigned char ostage[TMA_OUT ? (LN ? 1 : 6) * 2048 : 16];
-    __device__ __forceinline__ unsigned char* out_tiles() { return LN ? reinterpret_cast<unsigned char*>(Ut) : ostage; }
-    __device__ __forceinline__ unsigned char* dv_tile() { return ostage + (TMA_OUT && !LN ? 5 * 2048 : 0); }
 };
-static_assert(sizeof(BwdSmem<__nv_bfloat16, 1, false>) <= 115712, "bf16 backward must fit two CTAs per SM");
-static_assert(sizeof(BwdSmem<__nv_bfloat16, 1, true>) <= 115712, "bf16 attn_ln backward must fit two CTAs per SM");
-using BwdSmemLnBf16 = BwdSmem<__nv_bfloat16, 1, true>;
-static_assert(offsetof(BwdSmemLnBf16, Yt) - offsetof(BwdSmemLnBf16, Ut) == 2 * L * OPS * 4 && 3 * L * OPS * 4 >= 5 * 2048 &&
-                  offsetof(BwdSmemLnBf16, Ut) % 1024 == 0,
-              "attn_ln output staging tiles alias Ut, Dt, Yt");
 
 template <typename IoT> __device__ __forceinline__ float bst_elem(const unsigned char* tile, int row, int col) {
     return to_f32<IoT>(*reinterpret_cast<const IoT*>(tile + BwdLayout<IoT>::at(row, col)));
@@ -119,9 +103,6 @@ template <typename IoT> __device__ __forceinline__ float bst_elem(const unsigned
 template <typename IoT> __device__ __forceinline__ float2 bst_pair(const unsigned char* tile, int row, int col);
 template <> __device__ __forceinline__ float2 bst_pair<float>(const unsigned char* tile, int row, int col) {
     return *reinterpret_cast<const float2*>(tile + BwdLayout<float>::at(row, col));
-}
-template <> __device__ __forceinline__ float2 bst_pair<__nv_bfloat16>(const unsigned char* tile, int row, int col) {
-    return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(tile + BwdLayout<__nv_bfloat16>::at(row, col)));
 }
 // A operand [m = time][k = value] straight from a staging tile laid out [time][value]
 template <typename IoT, int PREC>
@@ -158,24 +139,12 @@ template <typename IoT> __device__ __forceinline__ void store_pair(IoT* p, float
 template <> __device__ __forceinline__ void store_pair<float>(float* p, float x, float y) {
     *reinterpret_cast<float2*>(p) = make_float2(x, y);
 }
-template <> __device__ __forceinline__ void store_pair<__nv_bfloat16>(__nv_bfloat16* p, float x, float y) {
-    *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);
-}
-
 // Epilogue stores.  A thread holds columns (2*t4, 2*t4+1) of two adjacent 8-column tiles; stored as they
 // are, a warp-wide store writes 16 bytes per row (half a 32-byte sector).  Lanes t4 and t4^1 swap one
 // pair, after which the even lane holds columns 4m..4m+3 of the first tile and the odd lane the same
 // columns of the second tile (m = t4 / 2): 8-byte stores (bf16), whole sectors per row.
 // `row` points at column 16*warp of the output row; live = false (rows beyond the end of the sequence) keeps the
 // exchange but skips the store.
-__device__ __forceinline__ void store_quad(__nv_bfloat16* row, float a0, float a1, float b0, float b1, int t4, bool live) {
-    const __nv_bfloat162 p0 = __floats2bfloat162_rn(a0, a1), p1 = __floats2bfloat162_rn(b0, b1);  // tile 0, tile 1
-    const uint32_t u0 = *reinterpret_cast<const uint32_t*>(&p0), u1 = *reinterpret_cast<const uint32_t*>(&p1);
-    const bool odd = t4 & 1;
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? u0 : u1, 1);
-    const uint2 v = odd ? make_uint2(got, u1) : make_uint2(u0, got);
-    if (live) *reinterpret_cast<uint2*>(row + 8 * (t4 & 1) + 4 * (t4 >> 1)) = v;
-}
 __device__ __forceinline__ void store_quad(float* row, float a0, float a1, float b0, float b1, int t4, bool live) {
     const bool odd = t4 & 1;
     const float g0 = __shfl_xor_sync(0xffffffffu, odd ? a0 : b0, 1), g1 = __shfl_xor_sync(0xffffffffu, odd ? a1 : b1, 1);
@@ -207,12 +176,11 @@ __device__ __forceinline__ void s0_wait(uint64_t* bar, uint32_t parity, volatile
 // TAIL: the sequence length is not a multiple of 16 (an instantiation of its own, so that whole-chunk sequences carry
 // none of the row tests).
 template <typename IoT, int PREC, bool LN, bool TAIL>
-__global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __grid_constant__ OutMaps omaps) {
+__global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __grid_constant__ CkptMaps cmaps) {
     using Lay = BwdLayout<IoT>;
     using Smem = BwdSmem<IoT, PREC, LN>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
-    constexpr bool TMA_OUT = Smem::TMA_OUT;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const long long bh = blockIdx.x;
@@ -289,14 +257,14 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
             for (int blk = 0; blk < 2; ++blk)
                 asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-                             ::"r"(smem_u32(sm.S0s + blk * S0_BLK)), "l"(&omaps.ck), "r"(bar), "r"(-8 * blk), "r"(0), "r"(blk), "r"(0), "r"(record) : "memory");
+                             ::"r"(smem_u32(sm.S0s + blk * S0_BLK)), "l"(&cmaps.ck), "r"(bar), "r"(-8 * blk), "r"(0), "r"(blk), "r"(0), "r"(record) : "memory");
             // the matrices: the record keeps them as the forward's operand tiles, 16-byte pieces [row / 8][column / 4][row % 8];
             // seen as [row group][row bit 2][row % 4][piece][4 floats], a box of 6 pieces per row (2 of them beyond the
             // row: zero fill) lands as rows of 24 floats; the second block starts at piece -2
 #pragma unroll
             for (int blk = 0; blk < 2; ++blk)
                 asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-                             ::"r"(smem_u32(sm.mats + blk * MAT_BLK)), "l"(&omaps.ckm), "r"(bar), "r"(0), "r"(-2 * blk), "r"(0), "r"(blk), "r"(record * (CK_FLOATS / 128) + CK_MATS / 128) : "memory");
+                             ::"r"(smem_u32(sm.mats + blk * MAT_BLK)), "l"(&cmaps.ckm), "r"(bar), "r"(0), "r"(-2 * blk), "r"(0), "r"(blk), "r"(record * (CK_FLOATS / 128) + CK_MATS / 128) : "memory");
         }
     };
     if (nchunks > 0) {
@@ -366,7 +334,6 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 if (part == 0) sm.bdot[row] = acc;
             }
         }
-        if (TMA_OUT && !LN) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // previous chunk's output tiles have been read
         __syncthreads();  // (A)
         if (c > 0) {
             issue_in(c - 1);
@@ -555,20 +522,8 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                         red2[(warp * L + tq + 1) * 3 + which] = asum[1];
                     }
                 }
-                // dg out.  bf16: as a 128-byte-swizzled [time][value] tile at the start of the score-gradient buffer (dead
-                // until the end of stage C's first part), stored by a bulk tensor copy issued after the barrier below and
-                // waited for before barrier (C1); otherwise through the per-warp scratch tile
-                if constexpr (TMA_OUT) {
-                    unsigned char* dgt = reinterpret_cast<unsigned char*>(sm.sgrad);
-#pragma unroll
-                    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int tq = 8 * nt + 2 * t4 + (i & 1), vc = 16 * warp + g + 8 * (i >> 1);
-                            *reinterpret_cast<__nv_bfloat16*>(dgt + tq * 128 + (((vc >> 3) ^ (tq & 7)) << 4) + (vc & 7) * 2) = __float2bfloat16_rn(Y[nt][i]);
-                        }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                } else {
+                // dg out, through the per-warp scratch tile for 16-byte stores
+                {
                     IoT* sc = dvsc;
 #pragma unroll
                     for (int nt = 0; nt < 2; ++nt) {
@@ -588,13 +543,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                     }
                     __syncwarp();
                 }
-                if (TMA_OUT) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // previous chunk's output tiles (in Ut, Dt, Yt) have been read
                 __syncthreads();  // (D2)
-                if (TMA_OUT && tid == 0) {
-                    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
-                                 ::"l"(&omaps.m[6]), "r"(0), "r"((int)hi), "r"(c * L), "r"((int)bi), "r"(smem_u32(sm.sgrad)) : "memory");
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                }
 #pragma unroll
                 for (int i4 = 0; i4 < 4; ++i4) {
                     const int nt = i4 >> 1, e = i4 & 1, tq = 8 * nt + 2 * t4 + e;
@@ -638,17 +587,8 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
             for (int tb = sb; tb < 2; ++tb) mma<PREC>(dV[sb], dbf[tb], mat_kn(0, sb, tb));
 
-        // dv out: the bf16 kernels write it into its staging tile; otherwise transposed through a per-warp scratch tile
-        // for 16-byte stores
-        if constexpr (TMA_OUT) {
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int tq = 8 * nt + 2 * t4 + (i & 1), vc = 16 * warp + g + 8 * (i >> 1);
-                    *reinterpret_cast<__nv_bfloat16*>(sm.dv_tile() + tq * 128 + (((vc >> 3) ^ (tq & 7)) << 4) + (vc & 7) * 2) = __float2bfloat16_rn(dV[nt][i] + dvx[nt][i]);
-                }
-        } else {
+        // dv out, transposed through a per-warp scratch tile for 16-byte stores
+        {
             IoT* sc = dvsc;
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
@@ -718,7 +658,6 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             const int nt_own = (b2 ? 1 : 0) + (b1 ? 2 : 0) + (b0 ? 4 : 0);
             *reinterpret_cast<float2*>(&sm.Gp[it & 1][warp][8 * nt_own + 2 * t4]) = make_float2(gp[0], gp[1]);
         }
-        if (TMA_OUT && LN) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // dg's tile lies where stage C writes the score gradients
         __syncthreads();  // (C1)
         // ---------------- stage C: contractions over the value index --------------------------
         float DA[2][4] = {}, DQ[2][4] = {}, DB[2][4] = {}, DK[2][4] = {};
@@ -856,21 +795,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 outv[1][nt][hrow][0] = d0; outv[1][nt][hrow][1] = d1;
             }
         }
-        if (TMA_OUT) {
-            // into the swizzled staging tiles: 4-byte stores, a warp-wide store covers 8 rows x 16 bytes in 8 different
-            // 16-byte units (conflict-free); the tiles leave by bulk tensor stores after the barrier below
-#pragma unroll
-            for (int ten = 0; ten < 5; ++ten)
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                    for (int hrow = 0; hrow < 2; ++hrow) {
-                        const int tq = g + 8 * hrow;
-                        const __nv_bfloat162 v2 = __floats2bfloat162_rn(outv[ten][nt][hrow][0], outv[ten][nt][hrow][1]);
-                        *reinterpret_cast<__nv_bfloat162*>(sm.out_tiles() + ten * 2048 + tq * 128 + ((((2 * warp + nt) ^ (tq & 7))) << 4) + 4 * t4) = v2;
-                    }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        } else {
+        {
 #pragma unroll
             for (int hrow = 0; hrow < 2; ++hrow) {
                 const long long off = ((long long)c * L + g + 8 * hrow) * p.st.t + 16 * warp;
@@ -882,15 +807,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         }
         cp_async_wait<0>();
         __syncthreads();  // (E)
-        if (TMA_OUT && tid == 0) {
-#pragma unroll
-            for (int ten = 0; ten < 6; ++ten)
-                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
-                             ::"l"(&omaps.m[ten]), "r"(0), "r"((int)hi), "r"(c * L), "r"((int)bi), "r"(smem_u32(ten < 5 ? sm.out_tiles() + ten * 2048 : sm.dv_tile())) : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
     }
-    if (TMA_OUT) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last stores
 
     if (LN) {
         // per-(batch, head) partial parameter gradients: ws[b][0..2][h*N + channel]
@@ -950,7 +867,7 @@ static EncodeTiledFn encode_tiled_fn() {
 // Tensor map over the states of `records` checkpoint records (fp32 [64][64] at the start of each record of CK_FLOATS
 // floats), seen as [record][a = row / 8][row bit 2][b = row % 4][column]; a box is the 32 rows of one value of bit 2,
 // N + 8 floats wide (the part outside the 64 columns reads as zero).
-static bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long records) {
+bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long records) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     const cuuint64_t dims[5] = {(cuuint64_t)N, 4, 2, 8, (cuuint64_t)records};
@@ -964,7 +881,7 @@ static bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long r
 // 8 of matrices: [AK;QK], AI, QB as operand tiles, a row group = [4 pieces][8 rows][4 floats]); the map sees the whole
 // buffer as [row group][row bit 2][row % 4][piece][4 floats]; a box is the rows of one value of bit 2 in 8 row groups,
 // 6 pieces wide (pieces 4, 5 do not exist and read as zero).
-static bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long records) {
+bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long records) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
     static_assert(CK_FLOATS % 128 == 0 && CK_MATS % 128 == 0, "records and their matrices part are whole row groups");
@@ -994,28 +911,24 @@ template <typename IoT, int PREC, bool LN> static int launch_bwd_t(const BwdPara
     const int smem = (int)sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return kLaunchFailed;
-    OutMaps omaps;
-    memset(&omaps, 0, sizeof(omaps));
-    if (Smem::TMA_OUT) {
-        void* outs[7] = {p.dr, p.dw, p.dk, p.da, p.db, p.dv, p.dg};
-        for (int i = 0; i < (LN ? 7 : 6); ++i)
-            if (!encode_bthn_map(&omaps.m[i], outs[i], p.B, p.T, p.H, p.st)) return kLaunchFailed;
-    }
+    CkptMaps cmaps;
+    memset(&cmaps, 0, sizeof(cmaps));
     const long long records = p.B * p.H * ((p.T + L - 1) / L);
-    if (!(encode_ckpt_state_map(&omaps.ck, p.ckpt, records) && encode_ckpt_mats_map(&omaps.ckm, p.ckpt, records)))
+    if (!(encode_ckpt_state_map(&cmaps.ck, p.ckpt, records) && encode_ckpt_mats_map(&cmaps.ckm, p.ckpt, records)))
         return kLaunchFailed;
-    kern<<<(unsigned)(p.B * p.H), THREADS, smem, stream>>>(p, omaps);
+    kern<<<(unsigned)(p.B * p.H), THREADS, smem, stream>>>(p, cmaps);
     if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
-    if (LN) {
-        const long long n3 = 3 * p.H * N;
-        reduce_dparams_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, stream>>>(p.dparams_ws, p.dparams, p.B, n3);
-        if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
-    }
-    return kOk;
+    return LN ? launch_reduce_dparams(p, stream) : kOk;
+}
+
+int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream) {
+    const long long n3 = 3 * p.H * N;
+    reduce_dparams_kernel<<<(unsigned)((n3 + 255) / 256), 256, 0, stream>>>(p.dparams_ws, p.dparams, p.B, n3);
+    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream) {
-    if (io_dtype == 0) return ln ? launch_bwd_t<__nv_bfloat16, 1, true>(p, stream) : launch_bwd_t<__nv_bfloat16, 1, false>(p, stream);
+    if (io_dtype == 0) return launch_bwd_bf16(p, ln, stream);
     if (io_dtype == 2) return ln ? launch_bwd_t<float, 1, true>(p, stream) : launch_bwd_t<float, 1, false>(p, stream);
     return ln ? launch_bwd_t<float, 3, true>(p, stream) : launch_bwd_t<float, 3, false>(p, stream);
 }

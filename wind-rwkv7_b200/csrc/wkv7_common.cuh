@@ -322,6 +322,27 @@ __device__ __forceinline__ void decay_scan(const unsigned char* tq, const unsign
     if (lw_out) store8(lw_out + at, lw, flip);
 }
 
+// Two fp32 operations in one instruction (sm_100 packed arithmetic).
+struct F2 { float x, y; };
+__device__ __forceinline__ unsigned long long f2_bits(F2 a) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y)); return r; }
+__device__ __forceinline__ F2 f2_from(unsigned long long r) { F2 a; asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r)); return a; }
+__device__ __forceinline__ F2 f2(float x, float y) { return F2{x, y}; }
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b))); return f2_from(r); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { unsigned long long r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b))); return f2_from(r); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { unsigned long long r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c))); return f2_from(r); }
+// 8 bf16 values of a staging tile as four pairs
+__device__ __forceinline__ void load8f2(const unsigned char* p, F2 (&f)[4]) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f[i] = f2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+}
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Column `col` of AI = (I - AB)^-1 for a strictly lower-triangular 16x16 AB, one lane per column.
 // ABt holds AB TRANSPOSED (ABt[s][tq] = AB[tq][s], row stride SCS), so that everything step s needs
 // is one contiguous row.  Right-looking substitution: as soon as entry s is final it is pushed
@@ -381,18 +402,28 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
     // different code at the same time out of one instruction cache (the clock64 form of this loop was 1 KB a place).
     for (;;) {
         uint32_t ok;
-        if (SLEEP)
-            asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2, %3;\nselp.u32 %0, 1, 0, P;\n}\n"
-                         : "=r"(ok) : "r"(addr), "r"(parity), "r"(4000u) : "memory");
-        else
-            asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
-                         : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+        asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
+                     : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
         if (ok) return;
         if (*abort) return;
+        if (SLEEP) __nanosleep(100);
         if ((SLEEP || (++spin & 63) == 0) && (uint32_t)clock() - start > most) break;
     }
     give_up(abort, status);
 }
+
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+    return p;
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // 16-byte asynchronous copy global -> shared through the load/store unit (no TMA request)
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {

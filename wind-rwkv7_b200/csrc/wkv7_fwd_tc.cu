@@ -107,17 +107,6 @@ struct Ctrl {
     float bdot[4][2][4][L];    // attn_ln: per-warp partial bonus dots [group][iteration parity][warp][time]
 };
 
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t p;
-    asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
-    return p;
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 // Bounded wait for the phase with the given parity.  Returns at once when the CTA has aborted.
 // SLEEP: the thread is suspended by the hardware (try_wait with a time hint) instead of polling, so
 // that the many warps that wait for the chain do not take issue slots from the warps that work; the
@@ -126,7 +115,6 @@ template <bool SLEEP>
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, Ctrl* ctrl, int* status, long long limit = WAIT_LIMIT) {
     mbar_wait_bounded<SLEEP>(bar, parity, &ctrl->abort, status, limit);
 }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
@@ -192,15 +180,6 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // without.)
 __device__ __forceinline__ float rnd(float x) { return __uint_as_float(tf32_rna(x)); }
 
-// Two fp32 operations in one instruction (sm_100 packed arithmetic).
-struct F2 { float x, y; };
-__device__ __forceinline__ unsigned long long f2_bits(F2 a) { unsigned long long r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y)); return r; }
-__device__ __forceinline__ F2 f2_from(unsigned long long r) { F2 a; asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r)); return a; }
-__device__ __forceinline__ F2 f2(float x, float y) { return F2{x, y}; }
-__device__ __forceinline__ F2 mul2(F2 a, F2 b) { unsigned long long r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b))); return f2_from(r); }
-__device__ __forceinline__ F2 add2(F2 a, F2 b) { unsigned long long r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b))); return f2_from(r); }
-__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { unsigned long long r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c))); return f2_from(r); }
-
 // byte offset of the 16-byte chunk holding (row, k..k+3) in a K-major tile; sbo = bytes per 8-row group
 __device__ __forceinline__ int kchunk(int row, int kc, int sbo) { return (row >> 3) * sbo + kc * 128 + (row & 7) * 16; }
 
@@ -256,13 +235,6 @@ template <bool R> __device__ __forceinline__ void store8mn(unsigned char* p, con
     *reinterpret_cast<float4*>(p + off) = make_float4(flip ? hi.x : lo.x, flip ? hi.y : lo.y, flip ? hi.z : lo.z, flip ? hi.w : lo.w);
     *reinterpret_cast<float4*>(p + (16 - off)) = make_float4(flip ? lo.x : hi.x, flip ? lo.y : hi.y, flip ? lo.z : hi.z, flip ? lo.w : hi.w);
 }
-// 8 bf16 values of a staging tile as four pairs
-__device__ __forceinline__ void load8f2(const unsigned char* p, F2 (&f)[4]) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = f2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-}
 // A 16x16 matrix from its accumulator fragment into a K-major operand tile, rounded to TF32; entries with
 // column > row + keep are written as zero (keep = 16: all kept).
 __device__ __forceinline__ void store_frag16(unsigned char* tile, const uint32_t* x, int r0, int c0, int keep) {
@@ -278,11 +250,6 @@ __device__ __forceinline__ void store_frag16(unsigned char* tile, const uint32_t
 __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&h);
-}
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
 }
 
 // TAIL: the sequence length is not a multiple of 16 (a build of its own, so that whole-chunk sequences carry none of

@@ -36,6 +36,7 @@ struct BwdParams {
     long long B, T, H;
     Strides st;
     int* status;
+    unsigned* flags;     // scratch for cut chains (WorkSplit), or null
 };
 
 struct StepParams {
@@ -58,6 +59,11 @@ bool encode_bthn_map(CUtensorMap* m, void* base, long long B, long long T, long 
 int launch_fwd(const FwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
 // the recurrence step by step on fp32 FMAs (decode); io_dtype 0 = bf16, otherwise fp32 tensors
 int launch_step(const StepParams& p, int io_dtype, cudaStream_t stream);
+// tensor maps over the checkpoint records' states and matrices, for the backward kernels' loads (see wkv7_bwd.cu)
+bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long records);
+bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long records);
+int launch_bwd_bf16(const BwdParams& p, bool ln, cudaStream_t stream);
+int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
 // tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
 // not rounded to TF32 by their producer (the tensor core truncates them)

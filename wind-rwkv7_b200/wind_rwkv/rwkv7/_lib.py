@@ -41,6 +41,8 @@ _SIGNATURES = {
     'wkv7_fwd': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp]),
     'wkv7_workspace_bytes': (ctypes.c_size_t, []),
     'wkv7_fwd_ws': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp, _vp]),
+    'wkv7_bwd_ws': (_int, [_vp] * 17 + [_i64] * 7 + [_int, _vp, _vp]),
+    'wkv7_attn_ln_bwd_ws': (_int, [_vp] * 22 + [_f32] + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_attn_ln_fwd_ws': (_int, [_vp] * 12 + [_f32] + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_step': (_int, [_vp] * 9 + [_i64] * 7 + [_int, _vp]),
     'wkv7_bwd': (_int, [_vp] * 17 + [_i64] * 7 + [_int, _vp]),

@@ -41,15 +41,16 @@ def bw_attn_ln(w, q, k, v, a, b, g, params, s, dy, dsT, sT):
     dparams = th.empty(3, H * C, dtype=th.float32, device=w.device)
     ws = th.empty(B, 3, H * C, dtype=th.float32, device=w.device)
     ds0 = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
+    sched = _lib.scratch(w.device)
     sb, st, sh = _lib.strides4(w)
     with _lib.on_device(w, q, k, v, a, b, g, params, s, dy, dsT):
-        rc = _lib.lib().wkv7_attn_ln_bwd(
+        rc = _lib.lib().wkv7_attn_ln_bwd_ws(
             q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), g.data_ptr(),
             params.data_ptr(), dy.data_ptr(), s.data_ptr(), _lib.ptr(dsT), _lib.ptr(sT if dsT is not None else None),
             dq.data_ptr(), dw.data_ptr(), dk.data_ptr(), dv.data_ptr(), da.data_ptr(), db.data_ptr(), dg.data_ptr(),
             dparams.data_ptr(), ws.data_ptr(), ds0.data_ptr(), EPS, B, T, H, C, sb, st, sh,
-            _lib.io_dtype(w), _lib.stream_of(w))
-    _lib.check(rc, 'wkv7_attn_ln_bwd')
+            _lib.io_dtype(w), sched.data_ptr(), _lib.stream_of(w))
+    _lib.check(rc, 'wkv7_attn_ln_bwd_ws')
     return dw, dq, dk, dv, da, db, dg, dparams, ds0
 
 
