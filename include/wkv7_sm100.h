@@ -39,7 +39,7 @@ extern "C" {
 #define WKV7_OK 0
 #define WKV7_ERR_SHAPE (-1)          /* negative or inconsistent dimensions */
 #define WKV7_ERR_HEAD_SIZE (-2)      /* only N == 64 is built */
-#define WKV7_ERR_CHUNK (-3)          /* expand_loras: T not a multiple of 16; ddlerp, expand_loras: C not a multiple of 64 */
+#define WKV7_ERR_CHUNK (-3)          /* ddlerp, expand_loras: C not a multiple of 64 */
 #define WKV7_ERR_ALIGN (-4)          /* a pointer or stride breaks 16-byte row alignment */
 #define WKV7_ERR_DTYPE (-5)
 #define WKV7_ERR_NULL (-6)           /* a required pointer is null */
@@ -258,7 +258,7 @@ int wkv7_proj_gemm(const void* A, const void* W, void* C, int64_t M, int64_t N, 
  * expand_loras: second-stage LoRA expansion producing (w, k, kk, b) for the mixer.  Replaces
  * fw_triton_ (wind_rwkv/rwkv7/rwkv7_expand_loras.py:32-89) behind ExpandLoras.forward (:215-231).
  * All tensors bf16, contiguous: w_in,k_in [B,T,C]; z_in,a_in,ma_in,mk_in [B,T,D]; W* [C,D];
- * biases [C]; outputs [B,T,C].  Head size 64 (C % 64 == 0), T % 16 == 0, D in {16,32,64,128}.
+ * biases [C]; outputs [B,T,C].  Head size 64 (C % 64 == 0), D in {16,32,64,128}; any T.
  *   w = -softplus(-(w_bias+w_in)) - 0.5 ;  z = tanh(z_in)@Wz^T + k_in ;  kk = z/||z||_head
  *   a, ma, mk = sigmoid(x_in@W^T + bias) ;  k = k_in*(ma+a-ma*a)*exp(w*mk) ;  b = -kk*a
  */
@@ -267,6 +267,14 @@ int wkv7_expand_loras_fwd(const void* w_in, const void* k_in, const void* z_in, 
                           const void* w_bias, const void* a_bias, const void* ma_bias, const void* mk_bias,
                           void* w_out, void* k_out, void* kk_out, void* b_out,
                           int64_t B, int64_t T, int64_t C, int64_t D, void* stream);
+
+/* The same with the rank-D inputs as columns of wider tensors: ld[i] is the row pitch in elements (a multiple of 8) of z_in,
+ * a_in, ma_in, mk_in in this order; null: D each. */
+int wkv7_expand_loras_fwd_ld(const void* w_in, const void* k_in, const void* z_in, const void* a_in, const void* ma_in,
+                             const void* mk_in, const int64_t* ld, const void* Wz, const void* Wa, const void* Wma, const void* Wmk,
+                             const void* w_bias, const void* a_bias, const void* ma_bias, const void* mk_bias,
+                             void* w_out, void* k_out, void* kk_out, void* b_out,
+                             int64_t B, int64_t T, int64_t C, int64_t D, void* stream);
 
 /* Bytes of workspace wkv7_expand_loras_bwd needs: 4*B*T*(C/64)*D*2 (per-head partials of the
  * rank-D input gradients, bf16, as the reference keeps them, rwkv7_expand_loras.py:201,207-210). */
@@ -285,6 +293,20 @@ int wkv7_expand_loras_bwd(const void* w_in, const void* k_in, const void* z_in, 
                           float* dWz, float* dWa, float* dWma, float* dWmk,
                           float* dw_bias, float* da_bias, float* dma_bias, float* dmk_bias,
                           void* workspace, int64_t B, int64_t T, int64_t C, int64_t D, void* stream);
+/* As wkv7_expand_loras_fwd_ld; ld_grad: the same for dz_in, da_in, dma_in, dmk_in. */
+int wkv7_expand_loras_bwd_ld(const void* w_in, const void* k_in, const void* z_in, const void* a_in, const void* ma_in,
+                             const void* mk_in, const int64_t* ld, const void* Wz, const void* Wa, const void* Wma, const void* Wmk,
+                             const void* w_bias, const void* a_bias, const void* ma_bias, const void* mk_bias,
+                             const void* dw_out, const void* dk_out, const void* dkk_out, const void* db_out, void* dw_in,
+                             void* dk_in, void* dz_in, void* da_in, void* dma_in, void* dmk_in, const int64_t* ld_grad,
+                             float* dWz, float* dWa, float* dWma, float* dWmk, float* dw_bias, float* da_bias, float* dma_bias,
+                             float* dmk_bias, void* workspace, int64_t B, int64_t T, int64_t C, int64_t D, void* stream);
+
+/* Converts up to WKV7_CAST_MAX contiguous tensors in one launch: numel[i] elements (a multiple of 8, 16-byte aligned) from
+ * src[i] to dst[i]; kind[i] 0: fp32 -> bf16, 1: bf16 -> fp32, 2: fp32 -> fp32.  The arrays are host memory. */
+#define WKV7_CAST_MAX 32
+int wkv7_cast(const void* const* src, void* const* dst, const int64_t* numel, const int* kind, int count, void* stream);
+
 
 /*
  * wkv7_attn_ln_bwd for callers that cannot hand over a workspace.  No counterpart in the

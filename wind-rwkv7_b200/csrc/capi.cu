@@ -115,7 +115,7 @@ const char* wkv7_status_string(int status) {
         case WKV7_OK: return "ok";
         case WKV7_ERR_SHAPE: return "bad shape: negative or inconsistent dimensions";
         case WKV7_ERR_HEAD_SIZE: return "unsupported head size: only N == 64 is built";
-        case WKV7_ERR_CHUNK: return "expand_loras: T must be a multiple of 16; ddlerp, expand_loras: C must be a multiple of 64";
+        case WKV7_ERR_CHUNK: return "ddlerp, expand_loras: C must be a multiple of 64";
         case WKV7_ERR_ALIGN: return "pointer or stride breaks 16-byte row alignment";
         case WKV7_ERR_DTYPE: return "unknown io_dtype";
         case WKV7_ERR_NULL: return "a required pointer is null";
@@ -463,15 +463,32 @@ int wkv7_ddlerp_bwd_tc(const void* x, const void* alpha, const void* L, const vo
 
 static int loras_check(int64_t B, int64_t T, int64_t C, int64_t D) {
     if (B < 0 || T < 0 || C <= 0 || D <= 0) return WKV7_ERR_SHAPE;
-    if (T % 16 != 0 || C % 64 != 0) return WKV7_ERR_CHUNK;
+    if (C % 64 != 0) return WKV7_ERR_CHUNK;
     if (D != 16 && D != 32 && D != 64 && D != 128) return WKV7_ERR_SHAPE;
     return WKV7_OK;
+}
+
+// row pitches of the rank-D tensors: null = D each
+static bool loras_pitches(const int64_t* ld, int64_t D, long long (&out)[4]) {
+    for (int i = 0; i < 4; ++i) {
+        out[i] = ld ? ld[i] : D;
+        if (out[i] < D || out[i] % 8 != 0) return false;
+    }
+    return true;
 }
 
 int wkv7_expand_loras_fwd(const void* w_in, const void* k_in, const void* z_in, const void* a_in, const void* ma_in,
                           const void* mk_in, const void* Wz, const void* Wa, const void* Wma, const void* Wmk,
                           const void* w_bias, const void* a_bias, const void* ma_bias, const void* mk_bias, void* w_out,
                           void* k_out, void* kk_out, void* b_out, int64_t B, int64_t T, int64_t C, int64_t D, void* stream) {
+    return wkv7_expand_loras_fwd_ld(w_in, k_in, z_in, a_in, ma_in, mk_in, nullptr, Wz, Wa, Wma, Wmk, w_bias, a_bias, ma_bias, mk_bias,
+                                    w_out, k_out, kk_out, b_out, B, T, C, D, stream);
+}
+
+int wkv7_expand_loras_fwd_ld(const void* w_in, const void* k_in, const void* z_in, const void* a_in, const void* ma_in,
+                             const void* mk_in, const int64_t* ld, const void* Wz, const void* Wa, const void* Wma, const void* Wmk,
+                             const void* w_bias, const void* a_bias, const void* ma_bias, const void* mk_bias, void* w_out,
+                             void* k_out, void* kk_out, void* b_out, int64_t B, int64_t T, int64_t C, int64_t D, void* stream) {
     int rc = loras_check(B, T, C, D);
     if (rc) return rc;
     if (B == 0 || T == 0) return WKV7_OK;
@@ -485,7 +502,8 @@ int wkv7_expand_loras_fwd(const void* w_in, const void* k_in, const void* z_in, 
     p.W[0] = Wz; p.W[1] = Wa; p.W[2] = Wma; p.W[3] = Wmk;
     p.w_bias = w_bias; p.bias[0] = a_bias; p.bias[1] = ma_bias; p.bias[2] = mk_bias;
     p.w_out = w_out; p.k_out = k_out; p.kk_out = kk_out; p.b_out = b_out;
-    p.rows = B * T; p.T = T; p.C = C; p.D = (int)D;
+    p.rows = B * T; p.C = C; p.D = (int)D;
+    if (!loras_pitches(ld, D, p.ld)) return WKV7_ERR_ALIGN;
     return wkv7::launch_loras_fwd(p, (cudaStream_t)stream);
 }
 
@@ -501,6 +519,18 @@ int wkv7_expand_loras_bwd(const void* w_in, const void* k_in, const void* z_in, 
                           void* dk_in, void* dz_in, void* da_in, void* dma_in, void* dmk_in, float* dWz, float* dWa,
                           float* dWma, float* dWmk, float* dw_bias, float* da_bias, float* dma_bias, float* dmk_bias,
                           void* workspace, int64_t B, int64_t T, int64_t C, int64_t D, void* stream) {
+    return wkv7_expand_loras_bwd_ld(w_in, k_in, z_in, a_in, ma_in, mk_in, nullptr, Wz, Wa, Wma, Wmk, w_bias, a_bias, ma_bias, mk_bias,
+                                    dw_out, dk_out, dkk_out, db_out, dw_in, dk_in, dz_in, da_in, dma_in, dmk_in, nullptr,
+                                    dWz, dWa, dWma, dWmk, dw_bias, da_bias, dma_bias, dmk_bias, workspace, B, T, C, D, stream);
+}
+
+int wkv7_expand_loras_bwd_ld(const void* w_in, const void* k_in, const void* z_in, const void* a_in, const void* ma_in,
+                             const void* mk_in, const int64_t* ld, const void* Wz, const void* Wa, const void* Wma, const void* Wmk,
+                             const void* w_bias, const void* a_bias, const void* ma_bias, const void* mk_bias,
+                             const void* dw_out, const void* dk_out, const void* dkk_out, const void* db_out, void* dw_in,
+                             void* dk_in, void* dz_in, void* da_in, void* dma_in, void* dmk_in, const int64_t* ld_grad,
+                             float* dWz, float* dWa, float* dWma, float* dWmk, float* dw_bias, float* da_bias, float* dma_bias,
+                             float* dmk_bias, void* workspace, int64_t B, int64_t T, int64_t C, int64_t D, void* stream) {
     int rc = loras_check(B, T, C, D);
     if (rc) return rc;
     const void* ptrs[] = {w_in, k_in, z_in, a_in, ma_in, mk_in, Wz, Wa, Wma, Wmk, w_bias, a_bias, ma_bias, mk_bias,
@@ -519,17 +549,23 @@ int wkv7_expand_loras_bwd(const void* w_in, const void* k_in, const void* z_in, 
     p.dW[0] = dWz; p.dW[1] = dWa; p.dW[2] = dWma; p.dW[3] = dWmk;
     p.dw_bias = dw_bias; p.dbias[0] = da_bias; p.dbias[1] = dma_bias; p.dbias[2] = dmk_bias;
     p.partial = workspace;
-    p.rows = B * T; p.T = T; p.C = C; p.D = (int)D;
-    if (B == 0 || T == 0) {
-        cudaStream_t s = (cudaStream_t)stream;
-        float* w4[] = {dWz, dWa, dWma, dWmk};
-        float* b4[] = {dw_bias, da_bias, dma_bias, dmk_bias};
-        for (int i = 0; i < 4; ++i)
-            if (cudaMemsetAsync(w4[i], 0, sizeof(float) * C * D, s) != cudaSuccess || cudaMemsetAsync(b4[i], 0, sizeof(float) * C, s) != cudaSuccess)
-                return WKV7_ERR_LAUNCH;
-        return WKV7_OK;
-    }
+    p.rows = B * T; p.C = C; p.D = (int)D;
+    if (!loras_pitches(ld, D, p.ld) || !loras_pitches(ld_grad, D, p.ldg)) return WKV7_ERR_ALIGN;
     return wkv7::launch_loras_bwd(p, (cudaStream_t)stream);
+}
+
+int wkv7_cast(const void* const* src, void* const* dst, const int64_t* numel, const int* kind, int count, void* stream) {
+    if (count < 0 || count > WKV7_CAST_MAX) return WKV7_ERR_SHAPE;
+    wkv7::CastParams p{};
+    for (int i = 0; i < count; ++i) {
+        if (numel[i] < 0 || kind[i] < 0 || kind[i] > 2) return WKV7_ERR_SHAPE;
+        if (numel[i] == 0) continue;
+        if (!src[i] || !dst[i]) return WKV7_ERR_NULL;
+        if (numel[i] % 8 != 0 || !aligned16(src[i]) || !aligned16(dst[i])) return WKV7_ERR_ALIGN;
+        p.src[p.count] = src[i]; p.dst[p.count] = dst[i]; p.numel[p.count] = numel[i]; p.kind[p.count] = kind[i];
+        ++p.count;
+    }
+    return p.count ? wkv7::launch_cast(p, (cudaStream_t)stream) : WKV7_OK;
 }
 
 }  // extern "C"

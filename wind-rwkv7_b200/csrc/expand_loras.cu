@@ -6,7 +6,7 @@
 //     k  = k_in * (ma + a - ma*a) * exp(w * mk) ;   b = -kk * a
 // One warp handles 16 tokens x one head (64 channels): the rank-D products are bf16 m16n8k16 MMAs
 // with the head's weight slices staged in shared memory, the per-head L2 norm is a 4-lane shuffle.
-// Forward: grid (H, rows/64).  Backward: grid (H, B), walking the sequence in 64-token tiles so the
+// Forward: grid (H, rows/64).  Backward: grid (H, segments), each walking its rows in 64-token tiles so the
 // weight gradients stay in registers (one LoRA per warp; bias gradients ride along as an extra
 // all-ones input column) and are flushed once with fp32 atomics; the input gradients, which
 // contract over all heads, are written as per-head partials and summed by a small kernel.
@@ -45,9 +45,9 @@ template <int D> struct LorasFwdSmem {
 
 // A fragments of a [16, D] input block straight from global memory (rows r0+g, r0+g+8).
 template <int D, bool TANH>
-__device__ __forceinline__ void load_in_frags(uint32_t (&a)[D / 16][4], const bf16* base, long long r0, int g, int t4) {
-    const bf16* p0 = base + (r0 + g) * D + 2 * t4;
-    const bf16* p1 = p0 + 8 * D;
+__device__ __forceinline__ void load_in_frags(uint32_t (&a)[D / 16][4], const bf16* base, long long ld, long long r0, long long rows, int g, int t4) {
+    const bf16* p0 = base + min(r0 + g, rows - 1) * ld + 2 * t4;      // (rows past the end: any values, nothing of them is stored)
+    const bf16* p1 = base + min(r0 + g + 8, rows - 1) * ld + 2 * t4;
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
         uint32_t v[4] = {*reinterpret_cast<const uint32_t*>(p0 + 16 * ks), *reinterpret_cast<const uint32_t*>(p1 + 16 * ks),
@@ -69,13 +69,12 @@ __global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
     auto& sm = *reinterpret_cast<LorasFwdSmem<D>*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int h = blockIdx.x, C = (int)p.C;
-    const long long r0 = (long long)blockIdx.y * 64 + 16 * warp;
+    const long long t0 = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * 64, r0 = t0 + 16 * warp;
     for (int i = tid; i < 4 * HC * (D / 8); i += 128) {
         const int l = i / (HC * (D / 8)), r = (i / (D / 8)) % HC, ch = i % (D / 8);
         cp_async16(&sm.W[l][r][ch * 8], (const bf16*)p.W[l] + (long long)(h * HC + r) * D + ch * 8);
     }
     {   // this CTA's 64 tokens of w_in and k_in; rows past the end are filled with zeros
-        const long long t0 = (long long)blockIdx.y * 64;
         for (int i = tid; i < 2 * 64 * 8; i += 128) {
             const int ten = i / 512, r = (i / 8) % 64, ch = i % 8;
             const bool live = t0 + r < p.rows;
@@ -88,10 +87,10 @@ __global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
     // copies, so that the two latencies overlap
     uint32_t az[D / 16][4], aa[D / 16][4], am[D / 16][4], ak[D / 16][4];
     if (r0 < p.rows) {
-        load_in_frags<D, true>(az, (const bf16*)p.lin[0], r0, g, t4);
-        load_in_frags<D, false>(aa, (const bf16*)p.lin[1], r0, g, t4);
-        load_in_frags<D, false>(am, (const bf16*)p.lin[2], r0, g, t4);
-        load_in_frags<D, false>(ak, (const bf16*)p.lin[3], r0, g, t4);
+        load_in_frags<D, true>(az, (const bf16*)p.lin[0], p.ld[0], r0, p.rows, g, t4);
+        load_in_frags<D, false>(aa, (const bf16*)p.lin[1], p.ld[1], r0, p.rows, g, t4);
+        load_in_frags<D, false>(am, (const bf16*)p.lin[2], p.ld[2], r0, p.rows, g, t4);
+        load_in_frags<D, false>(ak, (const bf16*)p.lin[3], p.ld[3], r0, p.rows, g, t4);
     }
     cp_async_wait<0>();
     __syncthreads();
@@ -167,7 +166,7 @@ __global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
 #pragma unroll
             for (int it = 0; it < 4; ++it) {
                 const int r = lr + 4 * it + (lane >> 3), ch = lane & 7;
-                const long long row = (long long)blockIdx.y * 64 + r;
+                const long long row = t0 + r;
                 if (row < p.rows) *reinterpret_cast<uint4*>(outs[ten] + row * C + h * HC + ch * 8) = *reinterpret_cast<const uint4*>(&sm.io[ten][r][ch * 8]);
             }
     }
@@ -189,8 +188,8 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<LorasBwdSmem<D>*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const int h = blockIdx.x, C = (int)p.C, T = (int)p.T, H = C / HC;
-    const long long b0 = (long long)blockIdx.y * T;
+    const int h = blockIdx.x, C = (int)p.C, H = C / HC;
+    const long long T = p.rows;
 
     for (int i = tid; i < 4 * HC * (D / 8); i += 128) {
         const int l = i / (HC * (D / 8)), r = (i / (D / 8)) % HC, ch = i % (D / 8);
@@ -208,12 +207,12 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
     float dWacc[4][NT][4] = {};
     float dwb[4] = {};
 
-    // gridDim.z CTAs share a sequence: each walks a contiguous range of 64-token tiles (more resident
+    // gridDim.y CTAs share a head's rows: each walks a contiguous range of 64-token tiles (more resident
     // CTAs per SM; the price is one more flush of the weight-gradient accumulators per extra CTA)
-    const int tiles = (T + 63) / 64, per = (tiles + (int)gridDim.z - 1) / (int)gridDim.z;
-    const int tbeg = (int)blockIdx.z * per * 64, tend = min(T, tbeg + per * 64);
-    for (int t0 = tbeg; t0 < tend; t0 += 64) {
-        const long long r0 = b0 + t0 + 16 * warp;
+    const long long tiles = (T + 63) / 64, per = (tiles + gridDim.y - 1) / gridDim.y;
+    const long long tbeg = blockIdx.y * per * 64, tend = min(T, tbeg + per * 64);
+    for (long long t0 = tbeg; t0 < tend; t0 += 64) {
+        const long long r0 = t0 + 16 * warp;
         const bool valid = t0 + 16 * warp < T;
         // ---- the six [token][channel] tiles first (asynchronous copies), then this tile's LoRA inputs under them ------------
         {
@@ -222,7 +221,7 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
             for (int i = tid; i < 6 * 64 * 8; i += 128) {
                 const int ten = i / 512, r = (i / 8) % 64, ch = i % 8;
                 const bool live = t0 + r < T;
-                cp_async16_zfill(&sm.gr[ten][r][ch * 8], src6[ten] + (b0 + (live ? t0 + r : 0)) * C + h * HC + ch * 8, live);
+                cp_async16_zfill(&sm.gr[ten][r][ch * 8], src6[ten] + (live ? t0 + r : 0) * C + h * HC + ch * 8, live);
             }
             cp_async_commit();
         }
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
                     const int i = tid + 128 * (i0 + u);
                     const int l = i / (64 * (D / 8)), r = (i / (D / 8)) % 64, ch = i % (D / 8);
                     v[u] = make_uint4(0, 0, 0, 0);
-                    if (t0 + r < T) v[u] = *reinterpret_cast<const uint4*>((const bf16*)p.lin[l] + (b0 + t0 + r) * D + ch * 8);
+                    if (t0 + r < T) v[u] = *reinterpret_cast<const uint4*>((const bf16*)p.lin[l] + (t0 + r) * p.ld[l] + ch * 8);
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
@@ -370,7 +369,7 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
                     for (int it = 0; it < 4; ++it) {
                         const int r = lr + 4 * it + (lane >> 3), ch = lane & 7;
                         if (t0 + r < T)
-                            *reinterpret_cast<uint4*>((bf16*)(ten == 4 ? p.dw_in : p.dk_in) + (b0 + t0 + r) * C + h * HC + ch * 8) =
+                            *reinterpret_cast<uint4*>((bf16*)(ten == 4 ? p.dw_in : p.dk_in) + (t0 + r) * C + h * HC + ch * 8) =
                                 *reinterpret_cast<const uint4*>(&sm.gr[ten][r][ch * 8]);
                     }
             }
@@ -399,8 +398,8 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
                         v0 *= 1.f - t0v.x * t0v.x; v1 *= 1.f - t0v.y * t0v.y;
                         v2 *= 1.f - t1v.x * t1v.x; v3 *= 1.f - t1v.y * t1v.y;
                     }
-                    *reinterpret_cast<uint32_t*>(po + 8 * j) = pack_bf16x2(v0, v1);
-                    *reinterpret_cast<uint32_t*>(po + 8LL * H * D + 8 * j) = pack_bf16x2(v2, v3);
+                    if (r0 + g < T) *reinterpret_cast<uint32_t*>(po + 8 * j) = pack_bf16x2(v0, v1);
+                    if (r0 + g + 8 < T) *reinterpret_cast<uint32_t*>(po + 8LL * H * D + 8 * j) = pack_bf16x2(v2, v3);
                 }
             }
         } else {
@@ -452,47 +451,59 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
     }
 }
 
-// sums the per-head partials: out[l][row][d] = sum_h partial[l][row][h][d]
+// sums the per-head partials: out[l][row][d] = sum_h partial[l][row][h][d]; 8 values (16 bytes) per thread
 __global__ void loras_reduce_heads_kernel(LorasParams p, int H, int D) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;  // index over [4, rows, D]
-    const long long per = p.rows * D;
-    if (i >= 4 * per) return;
-    const int l = (int)(i / per);
-    const long long rd = i % per, row = rd / D;
-    const int d = (int)(rd % D);
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;  // index over [rows, D / 8]
+    const int l = blockIdx.y, per = D / 8;
+    const long long row = i / per;
+    if (row >= p.rows) return;
+    const int d = (int)(i - row * per) * 8;
     const bf16* src = (const bf16*)p.partial + ((long long)l * p.rows + row) * H * D + d;
-    float acc = 0.f;
-    for (int hh = 0; hh < H; ++hh) acc += __bfloat162float(src[(long long)hh * D]);
-    ((bf16*)p.dlin[l])[rd] = __float2bfloat16_rn(acc);
+    float acc[8] = {};
+#pragma unroll 4
+    for (int hh = 0; hh < H; ++hh) {
+        float f[8];
+        unpack8(*reinterpret_cast<const uint4*>(src + (long long)hh * D), f);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[q] += f[q];
+    }
+    *reinterpret_cast<uint4*>((bf16*)p.dlin[l] + row * p.ldg[l] + d) = pack8(acc);
 }
 
 template <int D> static int launch_loras_fwd_t(const LorasParams& p, cudaStream_t stream) {
     auto kern = loras_fwd_kernel<D>;
     const int smem = (int)sizeof(LorasFwdSmem<D>);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
-    kern<<<dim3((unsigned)(p.C / HC), (unsigned)((p.rows + 63) / 64)), 128, smem, stream>>>(p);
+    const long long tiles = (p.rows + 63) / 64, ny = tiles < 32768 ? tiles : 32768;  // y and z end at 65535
+    kern<<<dim3((unsigned)(p.C / HC), (unsigned)ny, (unsigned)((tiles + ny - 1) / ny)), 128, smem, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 
 template <int D> static int launch_loras_bwd_t(const LorasParams& p, cudaStream_t stream) {
     const int C = (int)p.C, H = C / HC;
-    for (int l = 0; l < 4; ++l)
-        if (cudaMemsetAsync(p.dW[l], 0, sizeof(float) * C * D, stream) != cudaSuccess) return kLaunchFailed;
-    if (cudaMemsetAsync(p.dw_bias, 0, sizeof(float) * C, stream) != cudaSuccess) return kLaunchFailed;
-    for (int l = 0; l < 3; ++l)
-        if (cudaMemsetAsync(p.dbias[l], 0, sizeof(float) * C, stream) != cudaSuccess) return kLaunchFailed;
+    // the accumulated outputs start from zero; one call where they lie back to back
+    struct { float* p; size_t n; } z[8] = {{p.dW[0], (size_t)C * D}, {p.dW[1], (size_t)C * D}, {p.dW[2], (size_t)C * D}, {p.dW[3], (size_t)C * D},
+                                           {p.dw_bias, (size_t)C}, {p.dbias[0], (size_t)C}, {p.dbias[1], (size_t)C}, {p.dbias[2], (size_t)C}};
+    for (int i = 0; i < 8;) {
+        size_t n = z[i].n;
+        int j = i + 1;
+        while (j < 8 && z[j].p == z[i].p + n) n += z[j++].n;
+        if (cudaMemsetAsync(z[i].p, 0, sizeof(float) * n, stream) != cudaSuccess) return kLaunchFailed;
+        i = j;
+    }
+    if (p.rows == 0) return kOk;
     auto kern = loras_bwd_kernel<D>;
     const int smem = (int)sizeof(LorasBwdSmem<D>);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
     // enough CTAs for about eight per SM (three are resident at a time), at most one per 64-token tile
-    const long long seqs = (long long)H * (p.rows / p.T), tiles = (p.T + 63) / 64;
-    long long nseg = (8 * 148 + seqs - 1) / seqs;
+    const long long tiles = (p.rows + 63) / 64;
+    long long nseg = (8 * 148 + H - 1) / H;
     if (nseg > tiles) nseg = tiles;
     if (nseg < 1) nseg = 1;
-    kern<<<dim3((unsigned)H, (unsigned)(p.rows / p.T), (unsigned)nseg), 128, smem, stream>>>(p);
+    kern<<<dim3((unsigned)H, (unsigned)nseg), 128, smem, stream>>>(p);
     if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
-    const long long n = 4 * p.rows * D;
-    loras_reduce_heads_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(p, H, D);
+    const long long n = p.rows * (D / 8);
+    loras_reduce_heads_kernel<<<dim3((unsigned)((n + 255) / 256), 4), 256, 0, stream>>>(p, H, D);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 

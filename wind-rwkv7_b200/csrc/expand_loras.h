@@ -15,12 +15,23 @@ struct LorasParams {
     const void *dw_out, *dk_out, *dkk_out, *db_out;
     void *dw_in, *dk_in;                // bf16 [rows,C]
     void* dlin[4];                      // bf16 [rows,D]: dz_in, da_in, dma_in, dmk_in
+    long long ld[4], ldg[4];            // row pitches (elements, multiples of 8) of lin, dlin: D, or that of the tensor they are columns of
     void* partial;                      // bf16 [4, rows, H, D] per-head partials of dlin
     float* dW[4];                       // fp32 [C,D]
     float *dw_bias, *dbias[3];          // fp32 [C]
-    long long rows, T, C;               // rows = B*T
+    long long rows, C;                  // rows = B*T: tokens are independent, sequences need not be told apart
     int D;
 };
+
+// Several tensors converted in one launch; kind: 0 = fp32 -> bf16, 1 = bf16 -> fp32, 2 = fp32 -> fp32
+constexpr int CAST_MAX = 32;
+struct CastParams {
+    const void* src[CAST_MAX];
+    void* dst[CAST_MAX];
+    long long numel[CAST_MAX];
+    int kind[CAST_MAX], count;
+};
+int launch_cast(const CastParams& p, cudaStream_t stream);
 
 int launch_loras_fwd(const LorasParams& p, cudaStream_t stream);
 int launch_loras_bwd(const LorasParams& p, cudaStream_t stream);

@@ -4,11 +4,13 @@ There is no fallback: if the library cannot be loaded, or a call returns a non-z
 status, a RuntimeError is raised.
 """
 import ctypes
+import importlib.util
 import os
 
 import torch as th
 
 _PKG_ROOT = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+EXT_PATH = os.path.join(_PKG_ROOT, 'lib', '_wkv7_torch.so')
 LIB_PATH = os.path.join(_PKG_ROOT, 'lib', 'libwkv7_sm100.so')
 
 WKV7_BF16, WKV7_F32 = 0, 1
@@ -57,6 +59,9 @@ _SIGNATURES = {
     'wkv7_ddlerp_bwd_tc': (_int, [_vp] * 17 + [_i64] * 4 + [_vp]),
     'wkv7_ddlerp_bwd_tc_workspace_bytes': (ctypes.c_size_t, [_i64] * 2),
     'wkv7_expand_loras_fwd': (_int, [_vp] * 18 + [_i64] * 4 + [_vp]),
+    'wkv7_expand_loras_fwd_ld': (_int, [_vp] * 19 + [_i64] * 4 + [_vp]),
+    'wkv7_expand_loras_bwd_ld': (_int, [_vp] * 35 + [_i64] * 4 + [_vp]),
+    'wkv7_cast': (_int, [_vp] * 4 + [_int, _vp]),
     'wkv7_expand_loras_bwd_workspace_bytes': (_i64, [_i64] * 4),
     'wkv7_expand_loras_bwd': (_int, [_vp] * 33 + [_i64] * 4 + [_vp]),
     'wkv7_attn_ln_bwd_static': (_int, [_vp] * 21 + [_f32] + [_i64] * 7 + [_int, _vp]),
@@ -81,6 +86,24 @@ def lib():
             f.restype, f.argtypes = res, args
         _lib = L
     return _lib
+
+
+_ext = None
+
+
+def ext():
+    """The eager host path (csrc/torch_ops.cpp): each function does a whole entry point in C++, or returns None for
+    arguments that it leaves to the Python form."""
+    global _ext
+    if _ext is None:
+        lib()
+        if not os.path.exists(EXT_PATH):
+            raise RuntimeError(f'{EXT_PATH} is missing: build it with `python wind-rwkv7_b200/build.py`')
+        spec = importlib.util.spec_from_file_location('_wkv7_torch', EXT_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        _ext = mod
+    return _ext
 
 
 def check(status, what):
