@@ -1,0 +1,114 @@
+"""The eager host path in C++ (csrc/torch_ops.cpp) against the Python form of the same entry points, which torch.compile traces and which
+takes what the C++ one leaves: whole layer, ragged lengths, rows of wider tensors, frozen parameters."""
+import types
+
+import pytest
+import torch as th
+
+pytestmark = pytest.mark.gpu
+N = 64
+
+
+class _Nothing:
+    """Stands for the extension and leaves every call to the Python form."""
+
+    def __getattr__(self, name):
+        return lambda *a: None
+
+
+def _python_form(monkeypatch, f):
+    from wind_rwkv.rwkv7 import _lib
+    with monkeypatch.context() as m:
+        m.setattr(_lib, '_ext', _Nothing())
+        return f()
+
+
+def _close(got, want, rel):
+    assert (got is None) == (want is None)
+    if want is not None:
+        assert got.dtype == want.dtype and got.shape == want.shape
+        d, s = (got.double() - want.double()).norm().item(), want.double().norm().item()
+        assert d <= rel * s + 1e-12, (d, s)
+
+
+def _grads(outs, ins, seed):
+    gen = th.Generator('cuda').manual_seed(seed)
+    dys = [th.randn(o.shape, generator=gen, device='cuda').to(o.dtype) for o in outs]
+    return th.autograd.grad(outs, [i for i in ins if i.requires_grad], dys)
+
+
+@pytest.mark.parametrize('B,T,C,frozen', [(1, 1, 64, ()), (2, 17, 128, ('Wr', 'time_aaa_w1', 'gate_w1')), (3, 80, 192, ())])
+def test_mixer(B, T, C, frozen, monkeypatch):
+    from wind_rwkv.rwkv7 import TimeMixer
+    th.manual_seed(5)
+    mixer = TimeMixer(types.SimpleNamespace(n_layer=4, n_head=C // N, n_embd=C), 1).cuda()
+    for name, p in mixer.named_parameters():
+        p.data += 0.05 * th.randn_like(p)
+        p.requires_grad_(name not in frozen)
+    x = th.randn(B, T, C, device='cuda').bfloat16().requires_grad_()
+    ins = [x] + list(mixer.parameters())
+
+    def run():
+        y = mixer(x)
+        return [y] + list(_grads([y], ins, 6))
+
+    got, want = run(), _python_form(monkeypatch, run)
+    for g, w in zip(got, want, strict=True):
+        _close(g, w, 2e-2)
+    with th.no_grad():
+        assert th.equal(mixer(x), got[0])
+
+
+@pytest.mark.parametrize('T', [1, 15, 16, 65])
+def test_expand_loras_rows_of_wider_tensors(T, monkeypatch):
+    from wind_rwkv.rwkv7 import expand_loras
+    B, C, D = 3, 128, 16
+    th.manual_seed(T)
+    big = [th.randn(B, T, C, device='cuda').bfloat16().requires_grad_() for _ in range(2)]
+    wide = th.randn(B, T, 4 * D, device='cuda').bfloat16().requires_grad_()
+    par = [0.3 * th.randn(C, D, device='cuda') for _ in range(4)] + [th.randn(C, device='cuda') for _ in range(4)]
+    par = [p.requires_grad_() for p in par]
+
+    def run():
+        outs = expand_loras(*big, *wide.split(D, dim=2), *par, N)
+        return list(outs) + list(_grads(outs, big + [wide] + par, 7))
+
+    got, want = run(), _python_form(monkeypatch, run)
+    for g, w in zip(got[:7], want[:7]):
+        assert th.equal(g, w)
+    for g, w in zip(got[7:], want[7:], strict=True):  # sums over rows by atomics
+        _close(g, w, 1e-5)
+
+
+@pytest.mark.parametrize('dtype', [th.bfloat16, th.float32])
+def test_attn_state_and_slices(dtype, monkeypatch):
+    from wind_rwkv.rwkv7 import attn, synthetic
+    B, T, H = 2, 19, 2
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=3, dtype=dtype)
+    ins = [d[n].cuda().requires_grad_() for n in 'rwkvab']
+    s0 = th.randn(B, H, N, N, device='cuda').requires_grad_()
+
+    def run():
+        y, sT = attn(*ins, N, s0=s0, return_state=True)
+        first, = _grads([y[:, :, ::2]], ins[:1], 8),   # gradient of y alone, from a strided view
+        return [y, sT] + list(first) + list(_grads(list(attn(*ins, N, s0=s0, return_state=True)), ins + [s0], 9))
+
+    for g, w in zip(run(), _python_form(monkeypatch, run), strict=True):
+        assert th.equal(g, w)
+
+
+def test_cast():
+    from wind_rwkv.rwkv7 import _lib
+    import ctypes
+    sizes = [8, 24, 2048, 100000, 8]
+    src = [th.randn(n, device='cuda') for n in sizes[:3]] + [th.randn(n, device='cuda').bfloat16() for n in sizes[3:]]
+    kind = [0, 2, 0, 1, 1]
+    dst = [th.empty(n, device='cuda', dtype=th.bfloat16 if k == 0 else th.float32) for n, k in zip(sizes, kind)]
+    arr = lambda t, v: (t * len(v))(*v)
+    n = len(sizes)
+    rc = _lib.lib().wkv7_cast(arr(ctypes.c_void_p, [t.data_ptr() for t in src]), arr(ctypes.c_void_p, [t.data_ptr() for t in dst]), arr(ctypes.c_int64, sizes),
+                              arr(ctypes.c_int, kind), n, th.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    for s, d in zip(src, dst):
+        assert th.equal(s.to(d.dtype), d)
+    assert _lib.lib().wkv7_cast(None, None, None, None, 33, None) != 0

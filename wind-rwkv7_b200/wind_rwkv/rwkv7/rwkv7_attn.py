@@ -287,6 +287,10 @@ def attn(r, w, k, v, a, b, HEAD_SIZE, *, s0=None, return_state=False, time_split
     time_split=n (no upstream counterpart; inference only, no autograd): the sequence runs as n segments in
     parallel, see _attn_time_split.  Pays when B*H is far below the number of SMs.
     time_split='tail': only the chains of the last, partly filled round of SMs are cut in time, see _attn_tail_split."""
+    if time_split is None and HEAD_SIZE == _lib.HEAD_SIZE and not th.compiler.is_compiling():
+        out = _lib.ext().attn(r, w, k, v, a, b, s0, return_state)
+        if out is not None:
+            return out
     B, T, HC = w.shape
     C = HEAD_SIZE
     H = HC // C
@@ -310,6 +314,10 @@ def attn_step(r, w, k, v, a, b, HEAD_SIZE, state=None, *, inplace=False):
     Returns (y, new_state).  `state` is the fp32 [B,H,HEAD_SIZE,HEAD_SIZE] state `attn(..., return_state=True)`
     returns (None = zeros); with inplace=True it is overwritten and returned.  No autograd, no checkpoints.
     Upstream has no counterpart; this is the loop body of its naive recurrence (time_mixer.py:13-15) as a kernel."""
+    if HEAD_SIZE == _lib.HEAD_SIZE and not th.compiler.is_compiling():
+        out = _lib.ext().attn_step(r, w, k, v, a, b, state, inplace)
+        if out is not None:
+            return out
     B, T, HC = w.shape
     C = HEAD_SIZE
     H = HC // C

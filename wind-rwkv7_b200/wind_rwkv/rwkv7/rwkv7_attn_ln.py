@@ -118,6 +118,10 @@ def load_attn_ln(HEAD_SIZE):
 
 def attn_ln(r, w, k, v, a, b, g, params, HEAD_SIZE, *, s0=None, return_state=False):
     """Fused WKV7 + GroupNorm + bonus + gate for [B,T,H*HEAD_SIZE] tensors (upstream: rwkv7_attn_ln.py:56-62)."""
+    if HEAD_SIZE == _lib.HEAD_SIZE and not th.compiler.is_compiling():
+        out = _lib.ext().attn_ln(r, w, k, v, a, b, g, params, s0, return_state)
+        if out is not None:
+            return out
     B, T, HC = w.shape
     C = HEAD_SIZE
     H = HC // C

@@ -89,4 +89,10 @@ class DDLerp(th.autograd.Function):
         return dx, dalpha.to(ta), dL.to(tL), dR.to(tR), dbeta.to(tb)
 
 
-ddlerp = DDLerp.apply
+def ddlerp(x, alpha, L, R, beta):
+    """(xrg, xwa, xk, xv) for x [B,T,C] bf16, alpha [C], L [4D,C], R [4,C,D], beta [4,1,1,C]."""
+    if not th.compiler.is_compiling():
+        out = _lib.ext().ddlerp(x, alpha, L, R, beta)
+        if out is not None:
+            return out
+    return DDLerp.apply(x, alpha, L, R, beta)

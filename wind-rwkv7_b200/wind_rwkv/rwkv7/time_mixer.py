@@ -10,6 +10,7 @@ accepted for signature compatibility and ignored; `attn_impl` must be 'cuda'.
 import torch
 import torch.nn as nn
 
+from . import _lib
 from .rwkv7_attn_ln import attn_ln, load_attn_ln
 from .rwkv7_ddlerp import ddlerp
 from .rwkv7_expand_loras import expand_loras
@@ -124,7 +125,23 @@ class TimeMixer(nn.Module):
     _BF16_PARAMS = ('Wr', 'Wk', 'Wv', 'Wo', 'gate_w1', 'gate_w2', 'time_kkk_w1', 'mk_w1', 'time_decay_w1', 'time_aaa_w1', 'ma_w1',
                     'time_decay_w2')
 
+    # what the eager host path takes, in its order: weights that it multiplies with one input are neighbours
+    _PARAMS = ('Wr', 'Wk', 'Wv', 'Wo', 'gate_w1', 'gate_w2', 'time_kkk_w1', 'mk_w1', 'time_decay_w1', 'time_aaa_w1', 'ma_w1', 'time_decay_w2',
+               'time_maa_x', 'time_maa_w1', 'time_maa_w2', 'time_maa', 'time_kkk_w2', 'time_aaa_w2', 'ma_w2', 'mk_w2',
+               'time_decay', 'time_aaaaa', 'time_misc_a', 'time_misc_k')
+
+    def _eager_params(self):
+        own, ln = self._parameters, self.ln_x._parameters
+        try:
+            return [own[n] for n in self._PARAMS] + [ln['weight'], ln['bias'], own['time_faaaa']]
+        except KeyError:  # parametrised: computed on access
+            return [getattr(self, n) for n in self._PARAMS] + [self.ln_x.weight, self.ln_x.bias, self.time_faaaa]
+
     def forward(self, x):
+        if self.head_size == _lib.HEAD_SIZE and not torch.compiler.is_compiling():
+            out = _lib.ext().mixer(x, self._eager_params())
+            if out is not None:
+                return out
         r16 = self.SMALL_RANK
         bf = torch.bfloat16
         P = dict(zip(self._BF16_PARAMS, _CastAll.apply(*[getattr(self, n) for n in self._BF16_PARAMS])))  # bf16, one launch
