@@ -113,7 +113,7 @@ int wkv7_fwd(const void* r, const void* w, const void* k, const void* v, const v
  * Scratch for spreading the chains evenly over the SMs.  One CTA walks one (batch, head) chain; when B*H exceeds the
  * number of resident CTAs the last round of chains is rarely full.  The *_ws calls below take wkv7_workspace_bytes()
  * bytes of device scratch (16-byte aligned, contents overwritten, used by one call at a time) and cut chains at the
- * boundaries of equal shares of work: results are bit for bit those of the plain calls, which leave every chain whole.
+ * boundaries of equal shares of work: the forward's results are bit for bit those of the plain calls, which leave every chain whole.
  * A cut needs somewhere to keep the state in between: it is kept in sT, so sT must be given for it (otherwise, and with
  * workspace null, the call is the plain one).
  */
@@ -126,13 +126,16 @@ int wkv7_attn_ln_fwd_ws(const void* r, const void* w, const void* k, const void*
                         const void* g, const float* params, const float* s0, void* y, float* sT, float* ckpt,
                         float eps, int64_t B, int64_t T, int64_t H, int64_t N,
                         int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
-/* The backward keeps a cut chain's state gradient in ds0, which must be given for a cut. */
+/* The backward's scratch is wkv7_bwd_ws_bytes() bytes.  It keeps a cut chain's state gradient in ds0, which must be given for a
+ * cut.  Where there are few chains (bf16), the scratch also passes each chunk's state gradient from the CTA that walks the chain
+ * to the CTAs that do the rest of the chunk's work. */
+int64_t wkv7_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype);
 int wkv7_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                 const void* dy, const float* ckpt, const float* dsT, const float* sT,
                 void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* ds0,
                 int64_t B, int64_t T, int64_t H, int64_t N,
                 int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
-/* As wkv7_attn_ln_bwd; dparams_workspace is that call's workspace.  Where a chain is cut, its part of dparams is summed in two
+/* As wkv7_attn_ln_bwd; dparams_workspace is that call's workspace.  Where a chain is cut or shared, its part of dparams is summed in
  * pieces: dparams then agrees with the plain call's up to fp32 rounding (and is still deterministic). */
 int wkv7_attn_ln_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                         const void* g, const float* params, const void* dy, const float* ckpt, const float* dsT,

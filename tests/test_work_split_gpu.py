@@ -1,5 +1,6 @@
 """Chains cut at the boundaries of equal shares of work (the *_ws entry points) against the same kernels with whole chains:
-bit for bit the same, at chain counts around the number of resident CTAs and at the shortest and ragged lengths."""
+bit for bit the same, at chain counts around the number of resident CTAs and at the shortest and ragged lengths.  Few chains: the
+backward's state gradient (attn) walked ahead of the rest by a kernel that groups its products differently, from 4 chunks on."""
 import pytest
 import torch as th
 
@@ -40,7 +41,8 @@ def test_forward(extra, T, ckpt, ln):
 
 
 @pytest.mark.parametrize('ln', [False, True])
-@pytest.mark.parametrize('extra,T,dsT', [(1, 16, False), (-1, 48, True), (70, 7, True), (200, 33, False), (149, 500, True), (400, 65, True)])
+@pytest.mark.parametrize('extra,T,dsT', [(1, 16, False), (-1, 48, True), (70, 7, True), (200, 33, False), (149, 500, True), (400, 65, True),
+                                         (-50, 64, True), (-49, 64, True), (-147, 48, True), (-147, 49, True), (-147, 2000, False), (-100, 1003, True), (-75, 333, True)])
 def test_backward(extra, T, dsT, ln):
     from wind_rwkv.rwkv7 import _lib, synthetic
     from wind_rwkv.rwkv7.rwkv7_attn import fw_attn
@@ -50,7 +52,7 @@ def test_backward(extra, T, dsT, ln):
     g, params = synthetic.attn_ln_extras(B, T, H, N, seed=T, dtype=th.bfloat16, device='cuda')
     _, sT, ck = fw_attn(*[d[n].view(B, T, H, N) for n in 'wrkvab'], d['s0'])
     gs = th.randn(B, H, N, N, device='cuda') if dsT else None
-    ws = th.full((L.wkv7_workspace_bytes(),), 255, dtype=th.uint8, device='cuda')
+    ws = th.full((L.wkv7_bwd_ws_bytes(B, T, H, N, 0),), 255, dtype=th.uint8, device='cuda')
     part = th.empty(B, 3, H * N, device='cuda')
 
     def call(split):
@@ -69,8 +71,10 @@ def test_backward(extra, T, dsT, ln):
 
     for i, (a, b) in enumerate(zip(call(False), call(True))):
         assert bool(th.isfinite(a.float()).all())
-        if i == 8:  # parameter gradients of a cut chain are summed in two pieces
+        if i == 8:  # parameter gradients of a cut or shared chain are summed in pieces
             assert (a - b).norm() <= 1e-5 * a.norm()
+        elif extra <= 0 and T > 48 and not ln:
+            assert (a.float() - b.float()).norm() <= 4e-3 * a.float().norm(), i
         else:
             assert th.equal(a, b)
     assert L.wkv7_device_status() == 0

@@ -81,7 +81,7 @@ int check_common(int64_t B, int64_t T, int64_t H, int64_t N, int64_t sb, int64_t
 }  // namespace
 
 namespace wkv7 {
-static int sm_count() {
+int sm_count() {
     constexpr int kMaxDevices = 64;
     static std::atomic<int> cache[kMaxDevices];
     int dev = -1;
@@ -215,6 +215,11 @@ int wkv7_fwd(const void* r, const void* w, const void* k, const void* v, const v
 }
 
 size_t wkv7_workspace_bytes(void) { return wkv7::WORK_FLAG_BYTES; }
+
+int64_t wkv7_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype) {
+    if (B < 0 || T < 0 || H < 0 || N != wkv7::N) return 0;
+    return (int64_t)(io_dtype == WKV7_BF16 ? wkv7::bwd_workspace_bytes(B, T, H) : wkv7::WORK_FLAG_BYTES);
+}
 
 int wkv7_fwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                 const float* s0, void* y, float* sT, float* ckpt, int64_t B, int64_t T, int64_t H, int64_t N,

@@ -22,6 +22,7 @@
 // code does not fit the instruction cache, and rolled up to fit it a single warp per scheduler and group runs at 5.5 cycles an
 // instruction.)
 #include <cuda.h>
+#include <algorithm>
 #include <cstddef>
 #include <cstring>
 
@@ -116,19 +117,36 @@ __device__ __forceinline__ FragB<1> as_b(const FragA<1>& f, int nt) {
     return b;
 }
 
-template <bool TAIL, bool LN>
-__global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p, WorkSplit ws, const __grid_constant__ BwdMaps maps) {
+// PAR: the state gradients at the chunks' ends are given (wkv7_bwd_walk_kernel), so that chunks are worked in any order and none is
+// carried here; the tiles of steps it0 .. it0 + ws.per_chain - 1 of each chain are in `tiles`.
+struct Tiles { const float* base; int it0; };
+constexpr int TILE_FLOATS = N * SS;  // layout of s0_at()
+
+template <bool TAIL, bool LN, bool PAR>
+__global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p, WorkSplit ws, Tiles tiles, const __grid_constant__ BwdMaps maps) {
     extern __shared__ unsigned char smem_dyn[];
     using Smem = bf16bwd::Smem<LN>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const int nchunks = ws.per_chain;
+    const int nchunks = PAR ? (int)((p.T + L - 1) / L) : ws.per_chain;
     const WorkRange work(ws, blockIdx.x);
 
     auto describe = [&](int n) {
         if (n >= work.n) return;
         Desc d;
         int it;
+        if (PAR) {
+            const int x = work.first + n;
+            d.bh = (int)((unsigned)x / (unsigned)ws.per_chain);
+            it = x - d.bh * ws.per_chain;
+            d.bi = (int)((unsigned)d.bh / (unsigned)p.H);
+            d.hi = d.bh - d.bi * (int)p.H;
+            d.c = nchunks - 1 - tiles.it0 - it;
+            d.left = min(ws.per_chain - 1 - it, work.n - 1 - n);
+            d.flags = 0;
+            sm.desc[n & 3] = d;
+            return;
+        }
         work.locate(n, nchunks, d.bh, it);
         d.bi = (int)((unsigned)d.bh / (unsigned)p.H);
         d.hi = d.bh - d.bi * (int)p.H;
@@ -150,7 +168,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
     auto load_record = [&](int n) {
         const Desc& d = sm.desc[n & 3];
         const int record = d.bh * nchunks + d.c;
-        expect(&sm.rec_full, (N * SS + 2 * MAT_BLK) * 4);
+        expect(&sm.rec_full, ((PAR ? 2 : 1) * N * SS + 2 * MAT_BLK) * 4);
+        if (PAR) {
+            const float* src = tiles.base + ((long long)d.bh * ws.per_chain + (nchunks - 1 - d.c - tiles.it0)) * TILE_FLOATS;
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(sm.dS)), "l"(src), "r"(TILE_FLOATS * 4), "r"(smem_u32(&sm.rec_full)) : "memory");
+        }
 #pragma unroll 1
         for (int blk = 0; blk < 2; ++blk) {
             load5(sm.S0 + blk * S0_BLK, &maps.ck, &sm.rec_full, -8 * blk, 0, blk, 0, record);
@@ -180,7 +203,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
             if (lane == 0) {
                 if (!LN && n + 1 < work.n) load_inputs(n + 1);
                 Desc e = sm.desc[(n + 1) & 3];
-                if (e.left > 1) {  // (not the last but one: the last has flags)
+                if (e.left > (PAR ? 0 : 1)) {  // (not the last but one: the last has flags)
                     --e.c; --e.left;
                     e.flags = 0;
                     sm.desc[(n + 2) & 3] = e;
@@ -335,7 +358,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
             store8(sm.cum + dst, oc, flip);
         }
         __syncthreads();  // (A)
-        if (d.flags & FIRST) {
+        if (!PAR && (d.flags & FIRST)) {
 #pragma unroll
             for (int i = 0; i < (LN ? 8 : 0); ++i) dlnw[i] = dlnb[i] = 0.f;
             if (LN) dbon[0][0] = dbon[0][1] = dbon[LN ? 1 : 0][0] = dbon[LN ? 1 : 0][1] = 0.f;
@@ -357,6 +380,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
         }
         // ---------------- stage B: rows = value index ------------------------------------------------------------------
         mbar_wait_bounded<false>(&sm.rec_full, n & 1, &sm.abort, p.status);
+        if (PAR) {
+            const float* q = sm.dS + s0_mk;
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt) {
+                const float2 lo = *reinterpret_cast<const float2*>(q + 8 * nt), hi = *reinterpret_cast<const float2*>(q + 4 * SS + 8 * nt);
+                dS[nt][0] = lo.x; dS[nt][1] = lo.y; dS[nt][2] = hi.x; dS[nt][3] = hi.y;
+            }
+        }
         const unsigned char *vt = sm.vdy[LN ? 0 : n & 1][0], *dyt = sm.vdy[LN ? 0 : n & 1][1];
         FragA<1> dyf[2], vf[2];
         frags_value_time(vf, vt, warp, lane);
@@ -537,7 +568,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
         }
         // dS0 = dSf + dY^T wq + dabu^T wa
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+        for (int nt = 0; nt < (PAR ? 0 : 8); ++nt)
 #pragma unroll
             for (int kk = 0; kk < 2; ++kk) {
                 mma<1>(dS[nt], dyf[kk], B_kn(sm.wq, nt, kk));
@@ -595,6 +626,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
                 *reinterpret_cast<float2*>(q + 8 * SCS + at) = make_float2(c <= g + 8 ? pre<1>(sc[nt][2]) : 0.f, c < g + 8 ? pre<1>(sc[nt][3]) : 0.f);
             }
         }
+        if (PAR) fence_async_smem();  // dS was written here and comes by bulk copy next
         __syncthreads();  // (C2) score gradients visible; the record's tiles are free
         // the carried part of the decay gradient (see the head of this file)
         float kw[2][2][2], bw[2][2][2], G[2][2];  // kwi, bwi: [tile][row half][column]; [tile][column]
@@ -701,6 +733,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
         }
         fence_async_smem();
         __syncthreads();  // (E)
+        if (PAR) continue;
         if (LN && (d.flags & LAST)) {
             // per-(batch, head) partial parameter gradients ws[b][0..2][h*N + channel]; of a cut chain, the later piece adds to
             // what the earlier one (whose state gradient it has taken up) left there
@@ -747,11 +780,266 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
     }
 }
 
+// ---- the state gradient alone ----------------------------------------------------------------------------------------------------
+// With dSf = dS fw, Z = AI^T bwi, M = QB (AI^T)^T and wq' = wq + M wa a chunk takes dS to
+//     dSf + dY^T wq' + (dSf Z^T) wa:
+// two products one after the other are all that a chunk waits for, everything else is formed ahead of the chain.  One CTA per chain:
+// 4 chain warps (16 value rows of dS each, no exchange between them), three groups of 4 preparing warps (16 key columns each: scan, Z,
+// wq', within a warp) that take every third chunk, two warps that issue the loads; SLOTS chunks in flight.  Leaves dS at the end of
+// every chunk in `tiles`, for chunks it0 .. it0 + n - 1 (counted from the end of the sequence).
+// Bound by the chain, about 1400 cycles a chunk (the one-kernel form: 6200).  Backward of 48 chains of 63 chunks 203 -> 117 us, of 8
+// chains of 256 chunks 745 -> 246 us, of 148 chains of 63 chunks 236 -> 210 us.
+constexpr int SLOTS = 6, PREP = 3, WALK_THREADS = 32 * (WARPS * (1 + PREP) + 2);
+struct WalkSlot {
+    alignas(1024) unsigned char raw[5][TILE];  // q, w, a, b, dy
+    alignas(128) float mats[2 * L * L];        // AI^T, QB as the record holds them
+    alignas(16) float wq[L * OPS], wa[L * OPS], z[L * OPS], fw[N];
+};
+struct WalkSmem {
+    WalkSlot slot[SLOTS];
+    uint64_t raw_full[SLOTS], ready[SLOTS], free[SLOTS];
+    volatile int abort, drain;
+};
+static_assert(sizeof(WalkSmem) + 1024 <= 232448, "one CTA per SM");
+
+template <bool TAIL>
+__global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParams p, float* tiles, int it0, int count, const __grid_constant__ BwdMaps maps) {
+    extern __shared__ unsigned char smem_dyn[];
+    WalkSmem& sm = *reinterpret_cast<WalkSmem*>(smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u));
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t4 = lane & 3, w = warp & 3;
+    const int bh = blockIdx.x, bi = bh / (int)p.H, hi = bh - bi * (int)p.H, nchunks = (int)((p.T + L - 1) / L), c0 = nchunks - 1 - it0;
+    if (tid == 0) {
+        for (int i = 0; i < SLOTS; ++i) {
+            mbar_init(&sm.raw_full[i], 1);
+            mbar_init(&sm.ready[i], WARPS);
+            mbar_init(&sm.free[i], WARPS);
+        }
+        sm.abort = sm.drain = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    const int bg = (g >> 2) & 1, bt = (t4 >> 1) & 1;  // element offsets as in wkv7_bwd_bf16_kernel
+    const int mkE = g * OPS + 2 * t4 + 8 * bg, mkO = mkE - 16 * bg, knE = 2 * t4 * OPS + g + 8 * bt, knO = knE - 16 * bt;
+    auto mk = [&](int kk) { return (kk & 1 ? mkO : mkE) + 8 * kk; };
+    auto kn = [&](int nb) { return (nb & 1 ? knO : knE) + 8 * nb; };
+    auto B_kn = [&](const float* tile, int nb, int kk) {
+        FragB<1> f;
+        const float* q = tile + 8 * kk * OPS + kn(nb);
+        f.x[0].setr(q[0]); f.x[1].setr(q[OPS]);
+        return f;
+    };
+
+    if (warp >= WARPS * (1 + PREP)) {
+        // ---- loads
+        if (lane != 0) return;
+        const int map_of[5] = {0, 1, 3, 4, 6};
+        for (int n = warp & 1; n < count; n += 2) {
+            const int s = n % SLOTS, c = c0 - n;
+            if (n >= SLOTS) mbar_wait_bounded<true>(&sm.free[s], (n / SLOTS - 1) & 1, &sm.abort, p.status);
+            WalkSlot& t = sm.slot[s];
+            expect(&sm.raw_full[s], 5 * TILE + sizeof(t.mats));
+#pragma unroll
+            for (int i = 0; i < 5; ++i) load4(t.raw[i], &maps.in[map_of[i]], &sm.raw_full[s], hi, c * L, bi);
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(smem_u32(t.mats)), "l"(p.ckpt + ((long long)bh * nchunks + c) * CK_FLOATS + CK_AI), "r"((int)sizeof(t.mats)), "r"(smem_u32(&sm.raw_full[s]))
+                         : "memory");
+        }
+        // shared memory must outlive the loads, also where a wait has given up
+        for (int n = max(0, count - SLOTS); n < count; ++n)
+            if ((n & 1) == (warp & 1)) mbar_wait_bounded<true>(&sm.raw_full[n % SLOTS], (n / SLOTS) & 1, &sm.drain, p.status);
+        return;
+    }
+    if (warp >= WARPS) {
+        // ---- preparation: this warp's 16 key columns of every PREP-th chunk
+        const int row = lane & 15, j0 = 16 * w + 8 * (lane >> 4), at = row * ROWB + (((j0 >> 3) ^ (row & 7)) << 4);
+        const int dst = row * OPS + xcol<1>(row, j0);
+        const bool flip = (row >> 2) & 1;
+        for (int n = warp / WARPS - 1; n < count; n += PREP) {
+            const int s = n % SLOTS;
+            WalkSlot& t = sm.slot[s];
+            mbar_wait_bounded<true>(&sm.raw_full[s], (n / SLOTS) & 1, &sm.abort, p.status);
+            F2 cum[4], x[4], step[4];
+            load8f2(t.raw[1] + at, cum);
+            constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // the scan of wkv7_bwd_bf16_kernel
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                cum[i] = mul2(cum[i], f2(LOG2E, LOG2E));
+                cum[i] = mul2(f2(ex2_approx(cum[i].x), ex2_approx(cum[i].y)), f2(-LOG2E, -LOG2E));
+                cum[i] = f2(fmaxf(cum[i].x, FLOOR), fmaxf(cum[i].y, FLOOR));
+            }
+            if (TAIL && (long long)(c0 - n) * L + row >= p.T) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) cum[i] = f2(0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) step[i] = cum[i];
+#pragma unroll
+            for (int d = 1; d < 16; d <<= 1)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const F2 up = f2(__shfl_up_sync(0xffffffffu, cum[i].x, d, 16), __shfl_up_sync(0xffffffffu, cum[i].y, d, 16));
+                    if (row >= d) cum[i] = add2(cum[i], up);
+                }
+            float o[8], inv[8], non[8];
+            load8f2(t.raw[0] + at, x);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const F2 ca = add2(cum[i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = fma2(step[i], f2(-1.f, -1.f), ca);
+                const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
+                const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
+                inv[2 * i] = ex2_approx(-cx); inv[2 * i + 1] = ex2_approx(-cy);
+                non[2 * i] = ex2_approx(fmaxf(cp.x, -115.f)); non[2 * i + 1] = ex2_approx(fmaxf(cp.y, -115.f));
+                const F2 wq = mul2(x[i], incl);
+                o[2 * i] = wq.x; o[2 * i + 1] = wq.y;
+                if (row == 15) *reinterpret_cast<float2*>(t.fw + j0 + 2 * i) = make_float2(incl.x * STATE_SCALE, incl.y * STATE_SCALE);
+            }
+            store8(t.wq + dst, o, flip);
+            load8f2(t.raw[2] + at, x);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const F2 v = mul2(x[i], f2(non[2 * i], non[2 * i + 1]));
+                o[2 * i] = pre<1>(v.x); o[2 * i + 1] = pre<1>(v.y);
+            }
+            store8(t.wa + dst, o, flip);
+            load8f2(t.raw[3] + at, x);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const F2 v = mul2(x[i], f2(inv[2 * i], inv[2 * i + 1]));
+                o[2 * i] = pre<1>(v.x); o[2 * i + 1] = pre<1>(v.y);
+            }
+            store8(t.z + dst, o, flip);  // bwi, until Z takes its place
+            __syncwarp();
+            // matrix m (0 AI^T, 1 QB): element (row, col) of the record's operand tiles; columns 8 kk + 2 t4, +1 of row 8 rb + g
+            auto mat = [&](int m, int rb, int kk) {
+                return *reinterpret_cast<const float2*>(t.mats + m * L * L + rb * 128 + (2 * kk + (t4 >> 1)) * 32 + g * 4 + 2 * (t4 & 1));
+            };
+            float zz[2][4] = {}, M[2][4] = {}, q[2][4];
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+                const float2 zero = make_float2(0.f, 0.f);
+                // AI^T is upper, QB lower triangular: the blocks beyond are left out
+                const float2 ulo = mat(0, 0, kk), uhi = kk ? mat(0, 1, kk) : zero, blo = kk ? zero : mat(1, 0, kk), bhi = mat(1, 1, kk);
+                FragA<1> fu, fb;
+                fu.x[0].setr(ulo.x); fu.x[1].setr(uhi.x); fu.x[2].setr(ulo.y); fu.x[3].setr(uhi.y);
+                fb.x[0].setr(blo.x); fb.x[1].setr(bhi.x); fb.x[2].setr(blo.y); fb.x[3].setr(bhi.y);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) {
+                    mma<1>(zz[nb], fu, B_kn(t.z + 16 * w, nb, kk));
+                    if (nb <= kk) mma<1>(M[nb], fb, as_b(fu, nb));
+                }
+            }
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float2 v = *reinterpret_cast<const float2*>(t.wq + 8 * h * OPS + 16 * w + mk(nb));
+                    q[nb][2 * h] = v.x; q[nb][2 * h + 1] = v.y;
+                }
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+                const FragA<1> fm = fragA_from_acc<1>(M[kk]);
+#pragma unroll
+                for (int nb = 0; nb < 2; ++nb) mma<1>(q[nb], fm, B_kn(t.wa + 16 * w, nb, kk));
+            }
+            __syncwarp();  // bwi has been read
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int e = 8 * h * OPS + 16 * w + mk(nb);
+                    *reinterpret_cast<float2*>(t.z + e) = make_float2(pre<1>(zz[nb][2 * h]), pre<1>(zz[nb][2 * h + 1]));
+                    *reinterpret_cast<float2*>(t.wq + e) = make_float2(pre<1>(q[nb][2 * h]), pre<1>(q[nb][2 * h + 1]));
+                }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.ready[s]);
+        }
+        return;
+    }
+    // ---- the chain: value rows 16 w + {g, g + 8} of dS, carried as in wkv7_bwd_bf16_kernel
+    float dS[8][4];
+    const long long st = (long long)bh * N * N + (16 * w + g) * N + 2 * t4;
+    {
+        const float* src = it0 ? p.ds0 : p.dsT;  // a later pass goes on from where the earlier one left it
+        const float scale = it0 ? 1.f : STATE_UNSCALE;
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            const float2 lo = src ? *reinterpret_cast<const float2*>(src + st + 8 * nt) : make_float2(0.f, 0.f);
+            const float2 hi = src ? *reinterpret_cast<const float2*>(src + st + 8 * N + 8 * nt) : make_float2(0.f, 0.f);
+            dS[nt][0] = lo.x * scale; dS[nt][1] = lo.y * scale; dS[nt][2] = hi.x * scale; dS[nt][3] = hi.y * scale;
+        }
+    }
+    float* out = tiles + (long long)bh * count * TILE_FLOATS + s0_at(16 * w + g, 2 * t4);
+    for (int n = 0; n < count; ++n, out += TILE_FLOATS) {
+        const int s = n % SLOTS;
+        const WalkSlot& t = sm.slot[s];
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            *reinterpret_cast<float2*>(out + 8 * nt) = make_float2(dS[nt][0], dS[nt][1]);
+            *reinterpret_cast<float2*>(out + 4 * SS + 8 * nt) = make_float2(dS[nt][2], dS[nt][3]);
+        }
+        mbar_wait_bounded<false>(&sm.ready[s], (n / SLOTS) & 1, &sm.abort, p.status);
+        FragA<1> dyf[2];
+        frags_value_time(dyf, t.raw[4], w, lane);
+        float D[4][4] = {};
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+            const float2 f = *reinterpret_cast<const float2*>(t.fw + 8 * kk + 2 * t4);
+            dS[kk][0] *= f.x; dS[kk][1] *= f.y; dS[kk][2] *= f.x; dS[kk][3] *= f.y;
+            const FragA<1> a = fragA_from_acc<1>(dS[kk]);
+#pragma unroll
+            for (int sb = 0; sb < 2; ++sb) {
+                FragB<1> b;
+                const float2 v = *reinterpret_cast<const float2*>(t.z + 8 * sb * OPS + mk(kk));
+                b.x[0].setr(v.x); b.x[1].setr(v.y);
+                mma<1>(D[2 * sb + (kk & 1)], a, b);  // (two sums: half the chain of dependent products)
+            }
+        }
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) mma<1>(dS[nt], dyf[kk], B_kn(t.wq, nt, kk));
+        FragA<1> d[2];
+#pragma unroll
+        for (int sb = 0; sb < 2; ++sb) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) D[2 * sb][e] += D[2 * sb + 1][e];
+            d[sb] = fragA_from_acc<1>(D[2 * sb]);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) mma<1>(dS[nt], d[kk], B_kn(t.wa, nt, kk));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.free[s]);
+    }
+    const float scale = it0 + count < nchunks ? 1.f : STATE_SCALE;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+        *reinterpret_cast<float2*>(p.ds0 + st + 8 * nt) = make_float2(dS[nt][0] * scale, dS[nt][1] * scale);
+        *reinterpret_cast<float2*>(p.ds0 + st + 8 * N + 8 * nt) = make_float2(dS[nt][2] * scale, dS[nt][3] * scale);
+    }
+}
+
 }  // namespace bf16bwd
+
+// When the state gradients are walked ahead of the rest, and how many chunks of each chain at a time (0: not).  One CTA per chain and
+// all of a chunk's work in it is bound by the latency of a chunk (6200 cycles) while SMs are idle; the walk takes 1/5 of that and
+// the rest spreads over the machine.  With as many chains as SMs it still pays; beyond, a walk has its second round.
+// The tiles of a pass are kept below 512 MB; longer sequences take several passes, the walk going on from ds0.
+static int walk_chunks(long long chains, long long chunks) {
+    if (chains == 0 || chains > sm_count() || chunks < 4) return 0;
+    return (int)std::min(chunks, std::max(1LL, (512LL << 20) / (chains * bf16bwd::TILE_FLOATS * 4)));
+}
+size_t bwd_workspace_bytes(long long B, long long T, long long H) {
+    return WORK_FLAG_BYTES + (size_t)(B * H * walk_chunks(B * H, (T + L - 1) / L)) * bf16bwd::TILE_FLOATS * sizeof(float);
+}
 
 template <bool LN> static int launch_bwd_bf16_t(const BwdParams& p, cudaStream_t stream) {
     using namespace bf16bwd;
-    auto kern = p.T % L ? wkv7_bwd_bf16_kernel<true, LN> : wkv7_bwd_bf16_kernel<false, LN>;
+    const long long chains = p.B * p.H, chunks = (p.T + L - 1) / L;
+    const int walked = !LN && p.flags && p.ds0 ? walk_chunks(chains, chunks) : 0;
+    auto kern = p.T % L ? wkv7_bwd_bf16_kernel<true, LN, false> : wkv7_bwd_bf16_kernel<false, LN, false>;
+    if (walked) kern = p.T % L ? wkv7_bwd_bf16_kernel<true, LN, !LN> : wkv7_bwd_bf16_kernel<false, LN, !LN>;
     const int smem = (int)sizeof(Smem<LN>) + 1024;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
     BwdMaps maps;
@@ -764,9 +1052,23 @@ template <bool LN> static int launch_bwd_bf16_t(const BwdParams& p, cudaStream_t
         if (!encode_bthn_map(&maps.out[i], out[i], p.B, p.T, p.H, p.st)) return kLaunchFailed;
     const long long records = p.B * p.H * ((p.T + L - 1) / L);
     if (!(encode_ckpt_state_map(&maps.ck, p.ckpt, records) && encode_ckpt_mats_map(&maps.ckm, p.ckpt, records))) return kLaunchFailed;
-    const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 2, p.ds0 ? p.flags : nullptr);
+    if (walked) {
+        auto walk = p.T % L ? wkv7_bwd_walk_kernel<true> : wkv7_bwd_walk_kernel<false>;
+        const int wsmem = (int)sizeof(WalkSmem) + 1024, slots = 2 * sm_count();
+        if (cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, wsmem) != cudaSuccess) return kLaunchFailed;
+        float* tiles = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.flags) + WORK_FLAG_BYTES);
+        for (long long it0 = 0; it0 < chunks; it0 += walked) {
+            const int n = (int)std::min<long long>(walked, chunks - it0), total = (int)chains * n, per = (total + slots - 1) / slots;
+            walk<<<(unsigned)chains, WALK_THREADS, wsmem, stream>>>(p, tiles, (int)it0, n, maps);
+            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+            kern<<<(unsigned)((total + per - 1) / per), NTHREADS, smem, stream>>>(p, WorkSplit{0, per, n, total, nullptr}, Tiles{tiles, (int)it0}, maps);
+            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+        }
+        return kOk;
+    }
+    const WorkSplit ws = plan_work(chains, chunks, 2, p.ds0 ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
-    kern<<<(unsigned)ws.ctas, NTHREADS, smem, stream>>>(p, ws, maps);
+    kern<<<(unsigned)ws.ctas, NTHREADS, smem, stream>>>(p, ws, Tiles{}, maps);
     if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
     return LN ? launch_reduce_dparams(p, stream) : kOk;
 }

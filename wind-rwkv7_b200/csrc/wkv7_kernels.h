@@ -51,6 +51,7 @@ struct StepParams {
 // Work split for `chains` chains of `per_chain` chunks with `per_sm` resident CTAs per SM.  Chains are cut only when there are
 // more of them than resident CTAs (below that every chain has a CTA to itself and cutting gains nothing).
 WorkSplit plan_work(long long chains, long long per_chain, int per_sm, unsigned* flags);
+int sm_count();
 constexpr size_t WORK_FLAG_BYTES = 4096;  // room for the flags of 1024 CTAs
 
 // tensor map of a bf16 [B,T,H,N] tensor, box = 16 time steps of one head, 128-byte swizzle
@@ -63,6 +64,7 @@ int launch_step(const StepParams& p, int io_dtype, cudaStream_t stream);
 bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long records);
 bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long records);
 int launch_bwd_bf16(const BwdParams& p, bool ln, cudaStream_t stream);
+size_t bwd_workspace_bytes(long long B, long long T, long long H);  // what launch_bwd wants at p.flags for bf16 tensors (attn)
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
 // tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are

@@ -42,6 +42,7 @@ _SIGNATURES = {
     'wkv7_get_fwd_impl': (_int, []),
     'wkv7_fwd': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp]),
     'wkv7_workspace_bytes': (ctypes.c_size_t, []),
+    'wkv7_bwd_ws_bytes': (_i64, [_i64] * 4 + [_int]),
     'wkv7_fwd_ws': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_bwd_ws': (_int, [_vp] * 17 + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_attn_ln_bwd_ws': (_int, [_vp] * 22 + [_f32] + [_i64] * 7 + [_int, _vp, _vp]),
@@ -141,8 +142,13 @@ def io_dtype(t):
 _SCRATCH_BYTES = None
 
 
+def bwd_scratch(w):
+    """Device scratch of one backward *_ws call for [B,T,H,N] tensors like w."""
+    return th.empty(lib().wkv7_bwd_ws_bytes(*w.shape, io_dtype(w)), dtype=th.uint8, device=w.device)
+
+
 def scratch(device):
-    """Device scratch of one call of a *_ws entry point (spreads the chains over the SMs)."""
+    """Device scratch of one forward *_ws call (spreads the chains over the SMs)."""
     global _SCRATCH_BYTES
     if _SCRATCH_BYTES is None:
         _SCRATCH_BYTES = lib().wkv7_workspace_bytes()

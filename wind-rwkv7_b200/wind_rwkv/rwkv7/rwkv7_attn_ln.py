@@ -41,7 +41,7 @@ def bw_attn_ln(w, q, k, v, a, b, g, params, s, dy, dsT, sT):
     dparams = th.empty(3, H * C, dtype=th.float32, device=w.device)
     ws = th.empty(B, 3, H * C, dtype=th.float32, device=w.device)
     ds0 = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
-    sched = _lib.scratch(w.device)
+    sched = _lib.bwd_scratch(w)
     sb, st, sh = _lib.strides4(w)
     with _lib.on_device(w, q, k, v, a, b, g, params, s, dy, dsT):
         rc = _lib.lib().wkv7_attn_ln_bwd_ws(
