@@ -113,17 +113,21 @@ __global__ void ddlerp_prep_kernel(const __nv_bfloat16* __restrict__ L, const __
 
 // ---- gemm1: m = tanh([x_t | x_{t-1}] W12^T) -----------------------------------------------------------------------------
 namespace g1 {
-constexpr int BN = 128, STAGES = 3;
+constexpr int BN = 128;
+// Operand stages: three leave room for two CTAs an SM; with no more tiles than SMs a CTA has its SM to itself and its K loop waits for
+// the latency of its loads alone: seven then (513 tokens, C = 2048: 30 -> 17.8 us).
+constexpr int FEW = 3, MANY = 7;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 192;  // warps 0-3: epilogue (tensor-memory lane quarters 0-3), warp 4: TMA, warp 5: MMA
 struct Ctrl {
-    uint64_t full[STAGES], empty[STAGES], accum, drain;
+    uint64_t full[MANY], empty[MANY], accum, drain;
     uint32_t tmem_base;
     volatile int abort, zero;
 };
 }  // namespace g1
 
 // mapX: x as (channel, time, batch), box 64 x 128 x 1;  mapW: W12 as (k, row), box 64 x 128;  mapM: m as (column, time, batch), box 64 x 32 x 1
+template <int STAGES>
 __global__ void __launch_bounds__(g1::THREADS) ddlerp_gemm1_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW,
                                                                   const __grid_constant__ CUtensorMap mapM, int C, int n4, int T, int* status) {
     using namespace g1;
@@ -1322,10 +1326,12 @@ int launch_ddlerp_fwd_tc(const DdlerpFwdParams& p, void* ws, int* status, cudaSt
             return kLaunchFailed;
     }
     {
-        const int smem = g1::STAGES * g1::STAGE_BYTES + (int)sizeof(g1::Ctrl) + 1024;
-        if (cudaFuncSetAttribute(ddlerp_gemm1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
         dim3 grid((unsigned)((n4 + g1::BN - 1) / g1::BN), (unsigned)((T + BM - 1) / BM), (unsigned)B);
-        ddlerp_gemm1_kernel<<<grid, g1::THREADS, smem, stream>>>(mX, mW, mMs, (int)C, n4, (int)T, status);
+        const bool alone = (long long)grid.x * grid.y * grid.z <= sm_count();
+        auto kern = alone ? ddlerp_gemm1_kernel<g1::MANY> : ddlerp_gemm1_kernel<g1::FEW>;
+        const int smem = (alone ? g1::MANY : g1::FEW) * g1::STAGE_BYTES + (int)sizeof(g1::Ctrl) + 1024;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
+        kern<<<grid, g1::THREADS, smem, stream>>>(mX, mW, mMs, (int)C, n4, (int)T, status);
         if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
     }
     return D == 16 ? launch_lerp<16>(mMl, mR, mXl, mY, p, B, status, stream) : launch_lerp<32>(mMl, mR, mXl, mY, p, B, status, stream);

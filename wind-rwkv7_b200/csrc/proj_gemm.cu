@@ -21,12 +21,15 @@
 namespace wkv7 {
 namespace gemm {
 
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3;
+constexpr int BM = 128, BN = 128, BK = 64;
+// Operand stages.  Three leave room for two CTAs an SM, whose loads and epilogues overlap; with no more tiles than SMs a CTA has its SM
+// to itself and the K loop waits for the latency of its loads alone: seven then (513 rows, K = 2048: 17.5 -> 11.4 us).
+constexpr int FEW = 3, MANY = 7;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int THREADS = 192;  // warps 0-3: epilogue (tensor-memory lane quarters 0-3), warp 4: TMA, warp 5: MMA
 
 struct Ctrl {
-    uint64_t full[STAGES], empty[STAGES], accum, drain;
+    uint64_t full[MANY], empty[MANY], accum, drain;
     uint32_t tmem_base;
     volatile int abort, zero;
 };
@@ -52,6 +55,7 @@ __device__ __forceinline__ float tanh_approx(float x) {
     return y;
 }
 
+template <int STAGES>
 __global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                                                            const __grid_constant__ CUtensorMap mapC, long long M, long long N, long long K,
                                                            int tanh_from, int tanh_to, int* status) {
@@ -206,10 +210,12 @@ int launch_proj_gemm(const void* A, const void* W, void* C, long long M, long lo
     alignas(64) CUtensorMap ma, mb, mc;
     // C [M, N]: the same kind of map (64 columns x 32 rows per store, one per warp and half tile)
     if (!encode_kmajor(&ma, A, M, K) || !encode_kmajor(&mb, W, N, K) || !encode_kmajor(&mc, C, M, N, 32)) return kLaunchFailed;
-    const int smem = STAGES * STAGE_BYTES + (int)sizeof(Ctrl) + 1024;
-    if (cudaFuncSetAttribute(proj_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
     dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM));
-    proj_gemm_kernel<<<grid, gemm::THREADS, smem, stream>>>(ma, mb, mc, M, N, K, tanh_from, tanh_to, status);
+    const bool alone = (long long)grid.x * grid.y <= sm_count();
+    auto kern = alone ? proj_gemm_kernel<MANY> : proj_gemm_kernel<FEW>;
+    const int smem = (alone ? MANY : FEW) * STAGE_BYTES + (int)sizeof(Ctrl) + 1024;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
+    kern<<<grid, gemm::THREADS, smem, stream>>>(ma, mb, mc, M, N, K, tanh_from, tanh_to, status);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 
