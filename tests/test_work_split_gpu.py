@@ -1,6 +1,6 @@
 """Chains cut at the boundaries of equal shares of work (the *_ws entry points) against the same kernels with whole chains:
 bit for bit the same, at chain counts around the number of resident CTAs and at the shortest and ragged lengths.  Few chains: the
-backward's state gradient (attn) walked ahead of the rest by a kernel that groups its products differently, from 4 chunks on."""
+backward's state gradient (attn) walked ahead of the rest by a kernel of its own, from 4 chunks on."""
 import pytest
 import torch as th
 
@@ -71,10 +71,8 @@ def test_backward(extra, T, dsT, ln):
 
     for i, (a, b) in enumerate(zip(call(False), call(True))):
         assert bool(th.isfinite(a.float()).all())
-        if i == 8:  # parameter gradients of a cut or shared chain are summed in pieces
+        if i == 8:  # parameter gradients of a cut chain are summed in two pieces
             assert (a - b).norm() <= 1e-5 * a.norm()
-        elif extra <= 0 and T > 48 and not ln:
-            assert (a.float() - b.float()).norm() <= 4e-3 * a.float().norm(), i
         else:
             assert th.equal(a, b)
     assert L.wkv7_device_status() == 0

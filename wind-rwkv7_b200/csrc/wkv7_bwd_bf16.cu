@@ -781,19 +781,18 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
 }
 
 // ---- the state gradient alone ----------------------------------------------------------------------------------------------------
-// With dSf = dS fw, Z = AI^T bwi, M = QB (AI^T)^T and wq' = wq + M wa a chunk takes dS to
-//     dSf + dY^T wq' + (dSf Z^T) wa:
-// two products one after the other are all that a chunk waits for, everything else is formed ahead of the chain.  One CTA per chain:
-// 4 chain warps (16 value rows of dS each, no exchange between them), three groups of 4 preparing warps (16 key columns each: scan, Z,
-// wq', within a warp) that take every third chunk, two warps that issue the loads; SLOTS chunks in flight.  Leaves dS at the end of
-// every chunk in `tiles`, for chunks it0 .. it0 + n - 1 (counted from the end of the sequence).
-// Bound by the chain, about 1400 cycles a chunk (the one-kernel form: 6200).  Backward of 48 chains of 63 chunks 203 -> 117 us, of 8
-// chains of 256 chunks 745 -> 246 us, of 148 chains of 63 chunks 236 -> 210 us.
-constexpr int SLOTS = 6, PREP = 3, WALK_THREADS = 32 * (WARPS * (1 + PREP) + 2);
+// The products that carry dS from chunk to chunk, as the chunk kernel forms them, in its order and with its rounding (so that results do
+// not depend on the number of chains): du = QB^T dY + bwi dSf^T, dabu = AI^T.. du, dS' = dSf + dY^T wq + dabu^T wa.  One CTA per
+// chain: 4 chain warps (16 value rows of dS each, no exchange between them), PREP groups of 4 preparing warps (the scan, 16 key columns
+// each) that take every PREP-th chunk, two warps that issue the loads; SLOTS chunks in flight.  Leaves dS at the end of every chunk in
+// `tiles`, for chunks it0 .. it0 + n - 1 (counted from the end of the sequence).
+// Bound by the chain of dependent products, some 1300 cycles a chunk (the one-kernel form: 6200).  Backward of 48 chains of 63 chunks
+// 203 -> 115 us, of 8 chains of 256 chunks 745 -> 230 us, of 148 chains of 63 chunks 236 -> 205 us.
+constexpr int SLOTS = 6, PREP = 2, WALK_THREADS = 32 * (WARPS * (1 + PREP) + 2);
 struct WalkSlot {
     alignas(1024) unsigned char raw[5][TILE];  // q, w, a, b, dy
     alignas(128) float mats[2 * L * L];        // AI^T, QB as the record holds them
-    alignas(16) float wq[L * OPS], wa[L * OPS], z[L * OPS], fw[N];
+    alignas(16) float wq[L * OPS], wa[L * OPS], bwi[L * OPS], fw[N];
 };
 struct WalkSmem {
     WalkSlot slot[SLOTS];
@@ -890,7 +889,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
                 inv[2 * i] = ex2_approx(-cx); inv[2 * i + 1] = ex2_approx(-cy);
                 non[2 * i] = ex2_approx(fmaxf(cp.x, -115.f)); non[2 * i + 1] = ex2_approx(fmaxf(cp.y, -115.f));
                 const F2 wq = mul2(x[i], incl);
-                o[2 * i] = wq.x; o[2 * i + 1] = wq.y;
+                o[2 * i] = pre<1>(wq.x); o[2 * i + 1] = pre<1>(wq.y);
                 if (row == 15) *reinterpret_cast<float2*>(t.fw + j0 + 2 * i) = make_float2(incl.x * STATE_SCALE, incl.y * STATE_SCALE);
             }
             store8(t.wq + dst, o, flip);
@@ -907,49 +906,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
                 const F2 v = mul2(x[i], f2(inv[2 * i], inv[2 * i + 1]));
                 o[2 * i] = pre<1>(v.x); o[2 * i + 1] = pre<1>(v.y);
             }
-            store8(t.z + dst, o, flip);  // bwi, until Z takes its place
-            __syncwarp();
-            // matrix m (0 AI^T, 1 QB): element (row, col) of the record's operand tiles; columns 8 kk + 2 t4, +1 of row 8 rb + g
-            auto mat = [&](int m, int rb, int kk) {
-                return *reinterpret_cast<const float2*>(t.mats + m * L * L + rb * 128 + (2 * kk + (t4 >> 1)) * 32 + g * 4 + 2 * (t4 & 1));
-            };
-            float zz[2][4] = {}, M[2][4] = {}, q[2][4];
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-                const float2 zero = make_float2(0.f, 0.f);
-                // AI^T is upper, QB lower triangular: the blocks beyond are left out
-                const float2 ulo = mat(0, 0, kk), uhi = kk ? mat(0, 1, kk) : zero, blo = kk ? zero : mat(1, 0, kk), bhi = mat(1, 1, kk);
-                FragA<1> fu, fb;
-                fu.x[0].setr(ulo.x); fu.x[1].setr(uhi.x); fu.x[2].setr(ulo.y); fu.x[3].setr(uhi.y);
-                fb.x[0].setr(blo.x); fb.x[1].setr(bhi.x); fb.x[2].setr(blo.y); fb.x[3].setr(bhi.y);
-#pragma unroll
-                for (int nb = 0; nb < 2; ++nb) {
-                    mma<1>(zz[nb], fu, B_kn(t.z + 16 * w, nb, kk));
-                    if (nb <= kk) mma<1>(M[nb], fb, as_b(fu, nb));
-                }
-            }
-#pragma unroll
-            for (int nb = 0; nb < 2; ++nb)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float2 v = *reinterpret_cast<const float2*>(t.wq + 8 * h * OPS + 16 * w + mk(nb));
-                    q[nb][2 * h] = v.x; q[nb][2 * h + 1] = v.y;
-                }
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-                const FragA<1> fm = fragA_from_acc<1>(M[kk]);
-#pragma unroll
-                for (int nb = 0; nb < 2; ++nb) mma<1>(q[nb], fm, B_kn(t.wa + 16 * w, nb, kk));
-            }
-            __syncwarp();  // bwi has been read
-#pragma unroll
-            for (int nb = 0; nb < 2; ++nb)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int e = 8 * h * OPS + 16 * w + mk(nb);
-                    *reinterpret_cast<float2*>(t.z + e) = make_float2(pre<1>(zz[nb][2 * h]), pre<1>(zz[nb][2 * h + 1]));
-                    *reinterpret_cast<float2*>(t.wq + e) = make_float2(pre<1>(q[nb][2 * h]), pre<1>(q[nb][2 * h + 1]));
-                }
+            store8(t.bwi + dst, o, flip);
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.ready[s]);
         }
@@ -980,7 +937,17 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
         mbar_wait_bounded<false>(&sm.ready[s], (n / SLOTS) & 1, &sm.abort, p.status);
         FragA<1> dyf[2];
         frags_value_time(dyf, t.raw[4], w, lane);
-        float D[4][4] = {};
+        // matrix m (0 AI^T, 1 QB): element (row, col) of the record's operand tiles
+        auto mat = [&](int m, int row, int col) { return t.mats + m * L * L + (row >> 3) * 128 + (col >> 2) * 32 + (row & 7) * 4 + (col & 3); };
+        float du[2][4] = {}, dabu[2][4] = {};
+#pragma unroll
+        for (int sb = 0; sb < 2; ++sb)
+#pragma unroll
+            for (int tb = sb; tb < 2; ++tb) {
+                FragB<1> b;
+                b.x[0].setr(*mat(1, 8 * tb + 2 * t4, 8 * sb + g)); b.x[1].setr(*mat(1, 8 * tb + 2 * t4 + 1, 8 * sb + g));
+                mma<1>(du[sb], dyf[tb], b);
+            }
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
             const float2 f = *reinterpret_cast<const float2*>(t.fw + 8 * kk + 2 * t4);
@@ -989,26 +956,29 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
 #pragma unroll
             for (int sb = 0; sb < 2; ++sb) {
                 FragB<1> b;
-                const float2 v = *reinterpret_cast<const float2*>(t.z + 8 * sb * OPS + mk(kk));
+                const float2 v = *reinterpret_cast<const float2*>(t.bwi + 8 * sb * OPS + mk(kk));
                 b.x[0].setr(v.x); b.x[1].setr(v.y);
-                mma<1>(D[2 * sb + (kk & 1)], a, b);  // (two sums: half the chain of dependent products)
+                mma<1>(du[sb], a, b);
             }
+            mma<1>(dS[kk], dyf[0], B_kn(t.wq, kk, 0));
         }
+        const FragA<1> da2[2] = {fragA_from_acc<1>(du[0]), fragA_from_acc<1>(du[1])};
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
+        for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
-            for (int kk = 0; kk < 2; ++kk) mma<1>(dS[nt], dyf[kk], B_kn(t.wq, nt, kk));
-        FragA<1> d[2];
+            for (int kb = nb; kb < 2; ++kb) {
+                FragB<1> b;
+                const float2 v = *reinterpret_cast<const float2*>(mat(0, 8 * nb + g, 8 * kb + 2 * t4));
+                b.x[0].setr(v.x); b.x[1].setr(v.y);
+                mma<1>(dabu[nb], da2[kb], b);
+            }
+        const FragA<1> dbf[2] = {fragA_from_acc<1>(dabu[0]), fragA_from_acc<1>(dabu[1])};
 #pragma unroll
-        for (int sb = 0; sb < 2; ++sb) {
+        for (int nt = 0; nt < 8; ++nt) mma<1>(dS[nt], dbf[0], B_kn(t.wa, nt, 0));
 #pragma unroll
-            for (int e = 0; e < 4; ++e) D[2 * sb][e] += D[2 * sb + 1][e];
-            d[sb] = fragA_from_acc<1>(D[2 * sb]);
-        }
+        for (int nt = 0; nt < 8; ++nt) mma<1>(dS[nt], dyf[1], B_kn(t.wq, nt, 1));
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) mma<1>(dS[nt], d[kk], B_kn(t.wa, nt, kk));
+        for (int nt = 0; nt < 8; ++nt) mma<1>(dS[nt], dbf[1], B_kn(t.wa, nt, 1));
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.free[s]);
     }
