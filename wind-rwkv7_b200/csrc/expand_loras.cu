@@ -4,32 +4,44 @@
 //     z  = tanh(z_in) @ Wz^T + k_in ;   kk = z / sqrt(max(sum_head z^2, 1e-12))
 //     a  = sigmoid(a_in @ Wa^T + a_bias)   ma, mk likewise
 //     k  = k_in * (ma + a - ma*a) * exp(w * mk) ;   b = -kk * a
-// One warp handles 16 tokens x one head (64 channels): the rank-D products are bf16 m16n8k16 MMAs
+// A warp (backward: two) handles 16 tokens x one head (64 channels): the rank-D products are bf16 m16n8k16 MMAs
 // with the head's weight slices staged in shared memory, the per-head L2 norm is a 4-lane shuffle.
 // Forward: grid (H, rows/64).  Backward: grid (H, segments), each walking its rows in 64-token tiles so the
-// weight gradients stay in registers (one LoRA per warp; bias gradients ride along as an extra
+// weight gradients stay in registers (half a LoRA per warp; bias gradients ride along as an extra
 // all-ones input column) and are flushed once with fp32 atomics; the input gradients, which
 // contract over all heads, are written as per-head partials and summed by a small kernel.
 #include "expand_loras.h"
 #include "mma_bf16.cuh"
+#include "wkv7_kernels.h"
 
 namespace wkv7 {
 
 constexpr int HC = 64;  // channels per head
 
-// The gates of one element:  a, ma, mk = sigmoid(xa, xm, xk);  w = -softplus(-v) - 0.5;  E = exp(w * mk).
-// Six special-function instructions (three tanh for the sigmoids, ex2 + lg2 for the softplus, ex2 for E) and one
-// exponential as a polynomial on the FMA pipe: the op is bound by issue slots, and the textbook forms (expf, a
-// division per sigmoid) cost three to four times the instructions.
-struct Gates { float a, ma, mk, w, E, ev; };  // ev = exp(-v) (for the backward: sigmoid(-v) = ev / (1 + ev))
-__device__ __forceinline__ Gates lora_gates(float xa, float xm, float xk, float v) {
+// The gates of two adjacent channels:  a, ma, mk = sigmoid(xa, xm, xk);  w = -softplus(-v) - 0.5;  E = exp(w * mk).
+// Seven special-function instructions an element (three tanh for the sigmoids, ex2 + lg2 for the softplus, ex2 for E), everything
+// else two elements an instruction: the op is bound by issue slots.
+struct Gates { F2 a, ma, mk, w, E; };
+__device__ __forceinline__ F2 sigmoid2(F2 x) {
+    x = mul2(x, f2(0.5f, 0.5f));
+    return fma2(f2(tanh_f(x.x), tanh_f(x.y)), f2(0.5f, 0.5f), f2(0.5f, 0.5f));
+}
+__device__ __forceinline__ F2 neg2(F2 x) { return f2(-x.x, -x.y); }
+__device__ __forceinline__ F2 bf2(const void* p) {  // two bf16 values
+    const float2 v = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(p));
+    return f2(v.x, v.y);
+}
+__device__ __forceinline__ Gates lora_gates(F2 xa, F2 xm, F2 xk, F2 v) {
+    constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     Gates o;
-    o.a = sigmoid_f(xa);
-    o.ma = sigmoid_f(xm);
-    o.mk = sigmoid_f(xk);
-    o.ev = exp_poly(-v);  // exp_poly clamps its argument to +-80
-    o.w = -0.6931471805599453f * __log2f(1.f + o.ev) - 0.5f;
-    o.E = __expf(o.w * o.mk);
+    o.a = sigmoid2(xa);
+    o.ma = sigmoid2(xm);
+    o.mk = sigmoid2(xk);
+    const F2 n = mul2(v, f2(-LOG2E, -LOG2E));
+    const F2 e = add2(f2(ex2_approx(fminf(n.x, 115.f)), ex2_approx(fminf(n.y, 115.f))), f2(1.f, 1.f));
+    o.w = fma2(f2(__log2f(e.x), __log2f(e.y)), f2(-LN2, -LN2), f2(-0.5f, -0.5f));
+    const F2 x = mul2(mul2(o.w, o.mk), f2(LOG2E, LOG2E));
+    o.E = f2(ex2_approx(x.x), ex2_approx(x.y));
     return o;
 }
 
@@ -38,10 +50,22 @@ constexpr int GLD = HC + 8;  // row stride (bf16) of the [token][channel] tiles:
 template <int D> struct LorasFwdSmem {
     bf16 W[4][HC][D + 8];  // [channel][rank]
     // [token][channel] tiles of one head: w_in, k_in on the way in (16-byte cp.async, whole 128-byte rows), the four
-    // outputs on the way out (written in the fragment pattern, stored as whole rows).  Global accesses in the
+    // outputs on the way out (at rank 16 two by two through two tiles, which makes room for six CTAs an SM: 97 -> 86 us for 32768 rows of
+    // 768 channels; at higher ranks the registers that the other two wait in cost more than that) (written in the fragment pattern, stored as whole rows).  Global accesses in the
     // fragment pattern itself would touch 16 bytes per row and instruction.
-    bf16 io[4][64][GLD];
+    static constexpr int TILES = D == 16 ? 2 : 4;
+    bf16 io[TILES][64][GLD];
 };
+
+// B fragments (rows 8 j .., k block k0) of LoRAs l and l + 1 / of LoRA l alone
+template <int D> __device__ __forceinline__ void ldW2(uint32_t (&b0)[2], uint32_t (&b1)[2], const bf16 (*W)[HC][D + 8], int l, int n0, int k0, int lane) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(b0[0]), "=r"(b0[1]), "=r"(b1[0]), "=r"(b1[1])
+                 : "r"(smem_addr(&W[l + (lane >> 4)][n0 + (lane & 7)][k0 + (lane & 8)])));
+}
+template <int D> __device__ __forceinline__ void ldW1(uint32_t (&b)[2], const bf16 (*W)[HC][D + 8], int l, int n0, int k0, int lane) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(b[0]), "=r"(b[1])
+                 : "r"(smem_addr(&W[l][n0 + (lane & 7)][k0 + (lane & 8)])));
+}
 
 // A fragments of a [16, D] input block straight from global memory (rows r0+g, r0+g+8).
 template <int D, bool TANH>
@@ -64,7 +88,7 @@ __device__ __forceinline__ void load_in_frags(uint32_t (&a)[D / 16][4], const bf
 }
 
 template <int D>
-__global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
+__global__ void __launch_bounds__(128, D == 16 ? 6 : 1) loras_fwd_kernel(LorasParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<LorasFwdSmem<D>*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -105,7 +129,7 @@ __global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
             uint32_t b[2];
-            ldB_nk(b, &sm.W[0][0][0], D + 8, 8 * j, 16 * ks, g, t4);
+            ldW1<D>(b, sm.W, 0, 8 * j, 16 * ks, lane);
             mma_bf16(z[j], az[ks], b);
         }
         const float2 k0 = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.io[1][lr + g][8 * j + 2 * t4]));
@@ -118,57 +142,68 @@ __global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
     ss1 += __shfl_xor_sync(0xffffffffu, ss1, 1); ss1 += __shfl_xor_sync(0xffffffffu, ss1, 2);
     const float in0 = rsqrtf(fmaxf(ss0, 1e-12f)), in1 = rsqrtf(fmaxf(ss1, 1e-12f));
 
+    constexpr int TILES = LorasFwdSmem<D>::TILES;
+    uint32_t kb2[TILES == 2 ? 8 : 1][2][2];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        float fa[4] = {}, fm[4] = {}, fk[4] = {};
+        const int c = h * HC + 8 * j + 2 * t4;
+        const F2 wb = bf2((const bf16*)p.w_bias + c), ab = bf2((const bf16*)p.bias[0] + c), mb = bf2((const bf16*)p.bias[1] + c), kb = bf2((const bf16*)p.bias[2] + c);
+        float fa[4] = {ab.x, ab.y, ab.x, ab.y}, fm[4] = {mb.x, mb.y, mb.x, mb.y}, fk[4] = {kb.x, kb.y, kb.x, kb.y};
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
-            uint32_t b[2];
-            ldB_nk(b, &sm.W[1][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fa, aa[ks], b);
-            ldB_nk(b, &sm.W[2][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fm, am[ks], b);
-            ldB_nk(b, &sm.W[3][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fk, ak[ks], b);
+            uint32_t ba[2], bm[2], bk[2];
+            ldW2<D>(ba, bm, sm.W, 1, 8 * j, 16 * ks, lane);
+            ldW1<D>(bk, sm.W, 3, 8 * j, 16 * ks, lane);
+            mma_bf16(fa, aa[ks], ba);
+            mma_bf16(fm, am[ks], bm);
+            mma_bf16(fk, ak[ks], bk);
         }
-        const int c = h * HC + 8 * j + 2 * t4;
-        const float2 wb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.w_bias + c));
-        const float2 ab = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[0] + c));
-        const float2 mb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[1] + c));
-        const float2 kb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[2] + c));
 #pragma unroll
         for (int hrow = 0; hrow < 2; ++hrow) {
             const int tr = lr + g + 8 * hrow, tc = 8 * j + 2 * t4;
-            const float2 wi = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.io[0][tr][tc]));
-            const float2 ki = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.io[1][tr][tc]));
-            const float inorm = hrow ? in1 : in0;
-            float ow[2], ok[2], okk[2], ob[2];
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                const int i = 2 * hrow + x;
-                const Gates gt = lora_gates(fa[i] + (x ? ab.y : ab.x), fm[i] + (x ? mb.y : mb.x), fk[i] + (x ? kb.y : kb.x),
-                                            (x ? wb.y : wb.x) + (x ? wi.y : wi.x));
-                const float kk = z[j][i] * inorm;
-                ow[x] = gt.w;
-                ok[x] = (x ? ki.y : ki.x) * (gt.ma + gt.a - gt.ma * gt.a) * gt.E;
-                okk[x] = kk;
-                ob[x] = -kk * gt.a;
+            const F2 ki = bf2(&sm.io[1][tr][tc]);
+            const float in = hrow ? in1 : in0;
+            const Gates gt = lora_gates(f2(fa[2 * hrow], fa[2 * hrow + 1]), f2(fm[2 * hrow], fm[2 * hrow + 1]), f2(fk[2 * hrow], fk[2 * hrow + 1]),
+                                        add2(wb, bf2(&sm.io[0][tr][tc])));
+            const F2 kk = mul2(f2(z[j][2 * hrow], z[j][2 * hrow + 1]), f2(in, in)), nkk = neg2(kk);
+            const F2 ok = mul2(mul2(ki, fma2(neg2(gt.ma), gt.a, add2(gt.ma, gt.a))), gt.E), ob = mul2(nkk, gt.a);
+            // w and k replace w_in and k_in in their tiles (this thread's element, already read); kk and b wait in registers
+            *reinterpret_cast<uint32_t*>(&sm.io[0][tr][tc]) = pack_bf16x2(gt.w.x, gt.w.y);
+            *reinterpret_cast<uint32_t*>(&sm.io[1][tr][tc]) = pack_bf16x2(ok.x, ok.y);
+            if (TILES == 2) {
+                kb2[TILES == 2 ? j : 0][hrow][0] = pack_bf16x2(kk.x, kk.y);
+                kb2[TILES == 2 ? j : 0][hrow][1] = pack_bf16x2(ob.x, ob.y);
+            } else {
+                *reinterpret_cast<uint32_t*>(&sm.io[TILES - 2][tr][tc]) = pack_bf16x2(kk.x, kk.y);
+                *reinterpret_cast<uint32_t*>(&sm.io[TILES - 1][tr][tc]) = pack_bf16x2(ob.x, ob.y);
             }
-            // w and k replace w_in and k_in in their tiles (this thread's element, already read); kk and b get their own
-            *reinterpret_cast<uint32_t*>(&sm.io[0][tr][tc]) = pack_bf16x2(ow[0], ow[1]);
-            *reinterpret_cast<uint32_t*>(&sm.io[1][tr][tc]) = pack_bf16x2(ok[0], ok[1]);
-            *reinterpret_cast<uint32_t*>(&sm.io[2][tr][tc]) = pack_bf16x2(okk[0], okk[1]);
-            *reinterpret_cast<uint32_t*>(&sm.io[3][tr][tc]) = pack_bf16x2(ob[0], ob[1]);
         }
     }
-    __syncwarp();
-    {   // the warp's 16 rows of the four outputs leave as whole 128-byte rows (live rows only)
-        bf16* outs[4] = {(bf16*)p.w_out, (bf16*)p.k_out, (bf16*)p.kk_out, (bf16*)p.b_out};
+    // the warp's 16 rows of two outputs at a time leave as whole 128-byte rows (live rows only)
 #pragma unroll
-        for (int ten = 0; ten < 4; ++ten)
+    for (int pair = 0; pair < 2; ++pair) {
+        __syncwarp();
+        if (pair && TILES == 2) {
+#pragma unroll
+            for (int j = 0; j < (TILES == 2 ? 8 : 0); ++j)
+#pragma unroll
+                for (int hrow = 0; hrow < 2; ++hrow) {
+                    const int tr = lr + g + 8 * hrow, tc = 8 * j + 2 * t4;
+                    *reinterpret_cast<uint32_t*>(&sm.io[0][tr][tc]) = kb2[j][hrow][0];
+                    *reinterpret_cast<uint32_t*>(&sm.io[1][tr][tc]) = kb2[j][hrow][1];
+                }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int ten = 0; ten < 2; ++ten) {
+            bf16* out = (bf16*)(pair ? (ten ? p.b_out : p.kk_out) : (ten ? p.k_out : p.w_out));
 #pragma unroll
             for (int it = 0; it < 4; ++it) {
                 const int r = lr + 4 * it + (lane >> 3), ch = lane & 7;
                 const long long row = t0 + r;
-                if (row < p.rows) *reinterpret_cast<uint4*>(outs[ten] + row * C + h * HC + ch * 8) = *reinterpret_cast<const uint4*>(&sm.io[ten][r][ch * 8]);
+                if (row < p.rows) *reinterpret_cast<uint4*>(out + row * C + h * HC + ch * 8) = *reinterpret_cast<const uint4*>(&sm.io[TILES == 2 ? ten : 2 * pair + ten][r][ch * 8]);
             }
+        }
     }
 }
 
@@ -176,35 +211,42 @@ __global__ void __launch_bounds__(128) loras_fwd_kernel(LorasParams p) {
 
 template <int D> struct LorasBwdSmem {
     bf16 W[4][HC][D + 8];        // [channel][rank]: B operand of the forward, [k][n] operand of d(input)
-    bf16 in[4][64][D + 16];      // tanh(z_in), a_in, ma_in, mk_in; column D is all ones (bias gradient)
+    bf16 in[4][64][D + 8];       // tanh(z_in), a_in, ma_in, mk_in; column D is all ones (bias gradient)
     // [token][channel] tiles of one head.  On the way in (16-byte cp.async, whole 128-byte rows) tiles 0..5 hold
     // w_in, k_in, dw_out, dk_out, db_out, dkk_out.  Each thread replaces, element by element, what it has read: tiles
     // 0..4 become the pre-activation gradients of z, a, ma, mk and dw_in (the gradient of w_in), tile 5 becomes dk_in.
     bf16 gr[6][64][GLD];
+    float rs[2][64][2];          // row sums of the two channel halves
 };
 
+// Eight warps: warps rg and rg + 4 share the 16 tokens rg of a tile, 32 channels each (the row sums meet in shared memory), so that
+// the per-thread state fits 128 registers and 16 warps are resident (four warps of all channels: 212 registers and 8 warps
+// an SM).  Bound by instruction latency (0.46 instructions a cycle and scheduler) at 188 us for 32768 rows x 12 heads of rank 16, 254 us
+// with four warps, unpacked arithmetic and conflicting row pitches.
+constexpr int BWD_THREADS = 256;
 template <int D>
-__global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
+__global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel(LorasParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<LorasBwdSmem<D>*>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int tid = threadIdx.x, warp = (tid >> 5) & 3, half = tid >> 7, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + warp) : "memory"); };
     const int h = blockIdx.x, C = (int)p.C, H = C / HC;
     const long long T = p.rows;
 
-    for (int i = tid; i < 4 * HC * (D / 8); i += 128) {
+    for (int i = tid; i < 4 * HC * (D / 8); i += BWD_THREADS) {
         const int l = i / (HC * (D / 8)), r = (i / (D / 8)) % HC, ch = i % (D / 8);
         cp_async16(&sm.W[l][r][ch * 8], (const bf16*)p.W[l] + (long long)(h * HC + r) * D + ch * 8);
     }
     cp_async_commit();
-    for (int i = tid; i < 4 * 64 * 16; i += 128) {  // ones column and padding
-        const int l = i / (64 * 16), r = (i / 16) % 64, c = i % 16;
+    for (int i = tid; i < 4 * 64 * 8; i += BWD_THREADS) {  // ones column and padding
+        const int l = i / (64 * 8), r = (i / 8) % 64, c = i % 8;
         sm.in[l][r][D + c] = __float2bfloat16(c == 0 ? 1.f : 0.f);
     }
 
-    // weight-gradient accumulators: warp w owns LoRA w: [64 channels] x [D ranks + ones column],
-    // plus channel m-tile w of the dw_bias column
+    // weight-gradient accumulators: warps w, w + 4 own LoRA w: 32 channels each x [D ranks + ones column], plus channel
+    // m-tile w of the dw_bias column, two of the four token blocks each
     constexpr int NT = D / 8 + 1;
-    float dWacc[4][NT][4] = {};
+    float dWacc[2][NT][4] = {};
     float dwb[4] = {};
 
     // gridDim.y CTAs share a head's rows: each walks a contiguous range of 64-token tiles (more resident
@@ -218,7 +260,7 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
         {
             const bf16* src6[6] = {(const bf16*)p.w_in, (const bf16*)p.k_in, (const bf16*)p.dw_out, (const bf16*)p.dk_out,
                                    (const bf16*)p.db_out, (const bf16*)p.dkk_out};
-            for (int i = tid; i < 6 * 64 * 8; i += 128) {
+            for (int i = tid; i < 6 * 64 * 8; i += BWD_THREADS) {
                 const int ten = i / 512, r = (i / 8) % 64, ch = i % 8;
                 const bool live = t0 + r < T;
                 cp_async16_zfill(&sm.gr[ten][r][ch * 8], src6[ten] + (live ? t0 + r : 0) * C + h * HC + ch * 8, live);
@@ -227,21 +269,21 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
         }
         // LoRA inputs (tanh applied to z_in): the loads of a group of four are issued together, so that their latencies overlap
         {
-            constexpr int ITEMS = 4 * 64 * (D / 8) / 128;  // per thread
-            static_assert(ITEMS % 4 == 0, "groups of four loads per thread");
+            constexpr int ITEMS = 4 * 64 * (D / 8) / BWD_THREADS, G = ITEMS < 4 ? ITEMS : 4;  // per thread
+            static_assert(ITEMS % G == 0, "whole groups of loads per thread");
 #pragma unroll
-            for (int i0 = 0; i0 < ITEMS; i0 += 4) {
-                uint4 v[4];
+            for (int i0 = 0; i0 < ITEMS; i0 += G) {
+                uint4 v[G];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = tid + 128 * (i0 + u);
+                for (int u = 0; u < G; ++u) {
+                    const int i = tid + BWD_THREADS * (i0 + u);
                     const int l = i / (64 * (D / 8)), r = (i / (D / 8)) % 64, ch = i % (D / 8);
                     v[u] = make_uint4(0, 0, 0, 0);
                     if (t0 + r < T) v[u] = *reinterpret_cast<const uint4*>((const bf16*)p.lin[l] + (t0 + r) * p.ld[l] + ch * 8);
                 }
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int i = tid + 128 * (i0 + u);
+                for (int u = 0; u < G; ++u) {
+                    const int i = tid + BWD_THREADS * (i0 + u);
                     const int l = i / (64 * (D / 8)), r = (i / (D / 8)) % 64, ch = i % (D / 8);
                     if (l == 0) {
                         float f[8];
@@ -262,109 +304,100 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
             uint32_t az[D / 16][4], aa[D / 16][4], am[D / 16][4], ak[D / 16][4];
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
-                ldA_mk(az[ks], &sm.in[0][0][0], D + 16, lr, 16 * ks, g, t4);
-                ldA_mk(aa[ks], &sm.in[1][0][0], D + 16, lr, 16 * ks, g, t4);
-                ldA_mk(am[ks], &sm.in[2][0][0], D + 16, lr, 16 * ks, g, t4);
-                ldA_mk(ak[ks], &sm.in[3][0][0], D + 16, lr, 16 * ks, g, t4);
+                ldA_mk(az[ks], &sm.in[0][0][0], D + 8, lr, 16 * ks, g, t4);
+                ldA_mk(aa[ks], &sm.in[1][0][0], D + 8, lr, 16 * ks, g, t4);
+                ldA_mk(am[ks], &sm.in[2][0][0], D + 8, lr, 16 * ks, g, t4);
+                ldA_mk(ak[ks], &sm.in[3][0][0], D + 8, lr, 16 * ks, g, t4);
             }
             // ---- pass A: z, a; row sums for the norm and its gradient -----------------------------------
-            float z[8][4], dzo[8][4];
-            float ss[2] = {0.f, 0.f}, dn[2] = {0.f, 0.f};
+            float z[4][4], dzo[4][4];
+            F2 ss2[2] = {}, dn2[2] = {};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float fa[4] = {};
+            for (int j = 0; j < 4; ++j) {
+                const F2 ab = bf2((const bf16*)p.bias[0] + h * HC + 32 * half + 8 * j + 2 * t4);
+                float fa[4] = {ab.x, ab.y, ab.x, ab.y};
                 z[j][0] = z[j][1] = z[j][2] = z[j][3] = 0.f;
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    uint32_t b[2];
-                    ldB_nk(b, &sm.W[0][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(z[j], az[ks], b);
-                    ldB_nk(b, &sm.W[1][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fa, aa[ks], b);
+                    uint32_t bz[2], ba[2];
+                    ldW2<D>(bz, ba, sm.W, 0, 8 * j + 32 * half, 16 * ks, lane);
+                    mma_bf16(z[j], az[ks], bz);
+                    mma_bf16(fa, aa[ks], ba);
                 }
-                const float2 ab = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[0] + h * HC + 8 * j + 2 * t4));
 #pragma unroll
                 for (int hrow = 0; hrow < 2; ++hrow) {
-                    const int tr = lr + g + 8 * hrow, tc = 8 * j + 2 * t4;
-                    const float2 ki = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[1][tr][tc]));
-                    const float2 dk = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[5][tr][tc]));
-                    const float2 db = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[4][tr][tc]));
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const int i = 2 * hrow + x;
-                        z[j][i] += x ? ki.y : ki.x;
-                        const float a = sigmoid_f(fa[i] + (x ? ab.y : ab.x));
-                        dzo[j][i] = (x ? dk.y : dk.x) - (x ? db.y : db.x) * a;  // gradient of kk
-                        ss[hrow] += z[j][i] * z[j][i];
-                        dn[hrow] += dzo[j][i] * z[j][i];
-                    }
+                    const int tr = lr + g + 8 * hrow, tc = 32 * half + 8 * j + 2 * t4;
+                    const F2 zz = add2(f2(z[j][2 * hrow], z[j][2 * hrow + 1]), bf2(&sm.gr[1][tr][tc]));
+                    const F2 a = sigmoid2(f2(fa[2 * hrow], fa[2 * hrow + 1]));
+                    const F2 dz = fma2(neg2(bf2(&sm.gr[4][tr][tc])), a, bf2(&sm.gr[5][tr][tc]));  // gradient of kk
+                    ss2[hrow] = fma2(zz, zz, ss2[hrow]);
+                    dn2[hrow] = fma2(dz, zz, dn2[hrow]);
+                    z[j][2 * hrow] = zz.x; z[j][2 * hrow + 1] = zz.y;
+                    dzo[j][2 * hrow] = dz.x; dzo[j][2 * hrow + 1] = dz.y;
                 }
             }
+            float ss[2] = {ss2[0].x + ss2[0].y, ss2[1].x + ss2[1].y}, dn[2] = {dn2[0].x + dn2[0].y, dn2[1].x + dn2[1].y};
 #pragma unroll
             for (int hrow = 0; hrow < 2; ++hrow) {
                 ss[hrow] += __shfl_xor_sync(0xffffffffu, ss[hrow], 1); ss[hrow] += __shfl_xor_sync(0xffffffffu, ss[hrow], 2);
                 dn[hrow] += __shfl_xor_sync(0xffffffffu, dn[hrow], 1); dn[hrow] += __shfl_xor_sync(0xffffffffu, dn[hrow], 2);
             }
+            if (t4 == 0) {
+#pragma unroll
+                for (int hrow = 0; hrow < 2; ++hrow)
+                    *reinterpret_cast<float2*>(sm.rs[half][lr + g + 8 * hrow]) = make_float2(ss[hrow], dn[hrow]);
+            }
+            pair_sync();
+#pragma unroll
+            for (int hrow = 0; hrow < 2; ++hrow) {
+                const float2 o = *reinterpret_cast<const float2*>(sm.rs[half ^ 1][lr + g + 8 * hrow]);
+                ss[hrow] += o.x;
+                dn[hrow] += o.y;
+            }
             const float inorm[2] = {rsqrtf(fmaxf(ss[0], 1e-12f)), rsqrtf(fmaxf(ss[1], 1e-12f))};
+            const float ncorr[2] = {-dn[0] * inorm[0] * inorm[0] * inorm[0], -dn[1] * inorm[1] * inorm[1] * inorm[1]};
             // ---- pass B: everything elementwise, gradients into the shared tiles ----------------------------
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float fa[4] = {}, fm[4] = {}, fk[4] = {};
+            for (int j = 0; j < 4; ++j) {
+                const int c = h * HC + 32 * half + 8 * j + 2 * t4;
+                const F2 wb = bf2((const bf16*)p.w_bias + c), ab = bf2((const bf16*)p.bias[0] + c), mb = bf2((const bf16*)p.bias[1] + c), kb = bf2((const bf16*)p.bias[2] + c);
+                float fa[4] = {ab.x, ab.y, ab.x, ab.y}, fm[4] = {mb.x, mb.y, mb.x, mb.y}, fk[4] = {kb.x, kb.y, kb.x, kb.y};
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    uint32_t b[2];
-                    ldB_nk(b, &sm.W[1][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fa, aa[ks], b);
-                    ldB_nk(b, &sm.W[2][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fm, am[ks], b);
-                    ldB_nk(b, &sm.W[3][0][0], D + 8, 8 * j, 16 * ks, g, t4); mma_bf16(fk, ak[ks], b);
+                    uint32_t ba[2], bm[2], bk[2];
+                    ldW2<D>(ba, bm, sm.W, 1, 8 * j + 32 * half, 16 * ks, lane);
+                    ldW1<D>(bk, sm.W, 3, 8 * j + 32 * half, 16 * ks, lane);
+                    mma_bf16(fa, aa[ks], ba);
+                    mma_bf16(fm, am[ks], bm);
+                    mma_bf16(fk, ak[ks], bk);
                 }
-                const int c = h * HC + 8 * j + 2 * t4;
-                const float2 wb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.w_bias + c));
-                const float2 ab = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[0] + c));
-                const float2 mb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[1] + c));
-                const float2 kb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>((const bf16*)p.bias[2] + c));
 #pragma unroll
                 for (int hrow = 0; hrow < 2; ++hrow) {
-                    const int tr = lr + g + 8 * hrow, tc = 8 * j + 2 * t4;
-                    const float2 wi = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[0][tr][tc]));
-                    const float2 ki = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[1][tr][tc]));
-                    const float2 gw = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[2][tr][tc]));
-                    const float2 gk = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[3][tr][tc]));
-                    const float2 gb = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(&sm.gr[4][tr][tc]));
-                    float o_dw[2], o_dk[2], o_z[2], o_a[2], o_m[2], o_k[2];
-#pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        const int i = 2 * hrow + x;
-                        const float v = (x ? wb.y : wb.x) + (x ? wi.y : wi.x);
-                        const Gates gt = lora_gates(fa[i] + (x ? ab.y : ab.x), fm[i] + (x ? mb.y : mb.x), fk[i] + (x ? kb.y : kb.x), v);
-                        const float a = gt.a, ma = gt.ma, mk = gt.mk, w = gt.w, E = gt.E;
-                        const float kin = x ? ki.y : ki.x;
-                        const float kmix = ma + a - ma * a;
-                        const float zz = z[j][i], kk = zz * inorm[hrow];
-                        const float dkE = (x ? gk.y : gk.x) * E;
-                        const float de = dkE * kin * kmix;                       // gradient of w*mk
-                        const float dwt = (x ? gw.y : gw.x) + de * mk;
-                        const float dmk = de * w;
-                        const float dma = dkE * (kin - kin * a);
-                        const float da = -(x ? gb.y : gb.x) * kk + dkE * (kin - kin * ma);
-                        const float in3 = inorm[hrow] * inorm[hrow] * inorm[hrow];
-                        const float dz = dzo[j][i] * inorm[hrow] - in3 * dn[hrow] * zz;
-                        o_dw[x] = dwt * sigmoid_f(-v);
-                        o_dk[x] = dkE * kmix + dz;
-                        o_z[x] = dz;
-                        o_a[x] = da * a * (1.f - a);
-                        o_m[x] = dma * ma * (1.f - ma);
-                        o_k[x] = dmk * mk * (1.f - mk);
-                    }
-                    *reinterpret_cast<uint32_t*>(&sm.gr[5][tr][tc]) = pack_bf16x2(o_dk[0], o_dk[1]);
-                    *reinterpret_cast<uint32_t*>(&sm.gr[0][tr][tc]) = pack_bf16x2(o_z[0], o_z[1]);
-                    *reinterpret_cast<uint32_t*>(&sm.gr[1][tr][tc]) = pack_bf16x2(o_a[0], o_a[1]);
-                    *reinterpret_cast<uint32_t*>(&sm.gr[2][tr][tc]) = pack_bf16x2(o_m[0], o_m[1]);
-                    *reinterpret_cast<uint32_t*>(&sm.gr[3][tr][tc]) = pack_bf16x2(o_k[0], o_k[1]);
-                    *reinterpret_cast<uint32_t*>(&sm.gr[4][tr][tc]) = pack_bf16x2(o_dw[0], o_dw[1]);
+                    const int tr = lr + g + 8 * hrow, tc = 32 * half + 8 * j + 2 * t4;
+                    const F2 ki = bf2(&sm.gr[1][tr][tc]), v = add2(wb, bf2(&sm.gr[0][tr][tc]));
+                    const Gates gt = lora_gates(f2(fa[2 * hrow], fa[2 * hrow + 1]), f2(fm[2 * hrow], fm[2 * hrow + 1]), f2(fk[2 * hrow], fk[2 * hrow + 1]), v);
+                    const F2 kmix = fma2(neg2(gt.ma), gt.a, add2(gt.ma, gt.a));
+                    const F2 zz = f2(z[j][2 * hrow], z[j][2 * hrow + 1]), in = f2(inorm[hrow], inorm[hrow]);
+                    const F2 dkE = mul2(bf2(&sm.gr[3][tr][tc]), gt.E), dkin = mul2(dkE, ki);
+                    const F2 de = mul2(dkin, kmix);                                      // gradient of w * mk
+                    const F2 dwt = fma2(de, gt.mk, bf2(&sm.gr[2][tr][tc])), dmk = mul2(de, gt.w);
+                    const F2 dma = fma2(neg2(dkin), gt.a, dkin);
+                    const F2 da = fma2(neg2(bf2(&sm.gr[4][tr][tc])), mul2(zz, in), fma2(neg2(dkin), gt.ma, dkin));
+                    const F2 o_z = fma2(f2(dzo[j][2 * hrow], dzo[j][2 * hrow + 1]), in, mul2(zz, f2(ncorr[hrow], ncorr[hrow])));
+                    const F2 o_dw = mul2(dwt, sigmoid2(neg2(v))), o_dk = fma2(dkE, kmix, o_z);
+                    const F2 o_a = mul2(da, fma2(neg2(gt.a), gt.a, gt.a)), o_m = mul2(dma, fma2(neg2(gt.ma), gt.ma, gt.ma));
+                    const F2 o_k = mul2(dmk, fma2(neg2(gt.mk), gt.mk, gt.mk));
+                    *reinterpret_cast<uint32_t*>(&sm.gr[5][tr][tc]) = pack_bf16x2(o_dk.x, o_dk.y);
+                    *reinterpret_cast<uint32_t*>(&sm.gr[0][tr][tc]) = pack_bf16x2(o_z.x, o_z.y);
+                    *reinterpret_cast<uint32_t*>(&sm.gr[1][tr][tc]) = pack_bf16x2(o_a.x, o_a.y);
+                    *reinterpret_cast<uint32_t*>(&sm.gr[2][tr][tc]) = pack_bf16x2(o_m.x, o_m.y);
+                    *reinterpret_cast<uint32_t*>(&sm.gr[3][tr][tc]) = pack_bf16x2(o_k.x, o_k.y);
+                    *reinterpret_cast<uint32_t*>(&sm.gr[4][tr][tc]) = pack_bf16x2(o_dw.x, o_dw.y);
                 }
             }
-            __syncwarp();
-            {   // dw_in (tile 4) and dk_in (tile 5) of the warp's 16 rows leave as whole 128-byte rows (live rows only)
-#pragma unroll
-                for (int ten = 4; ten < 6; ++ten)
+            pair_sync();
+            {   // dw_in (tile 4, one warp) and dk_in (tile 5, the other) leave as whole 128-byte rows (live rows only)
+                const int ten = 4 + half;
 #pragma unroll
                     for (int it = 0; it < 4; ++it) {
                         const int r = lr + 4 * it + (lane >> 3), ch = lane & 7;
@@ -375,7 +408,8 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
             }
             // ---- d(input) partial of this head: [16, D] = grad[16, 64] @ W[64, D] ----------------------------
 #pragma unroll
-            for (int l = 0; l < 4; ++l) {
+            for (int l2 = 0; l2 < 2; ++l2) {
+                const int l = 2 * half + l2;
                 float acc[D / 8][4] = {};
 #pragma unroll
                 for (int ks = 0; ks < HC / 16; ++ks) {
@@ -404,7 +438,7 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
             }
         } else {
             // rows past the end of the sequence contribute nothing to the weight gradients
-            for (int i = lane; i < 5 * 16 * (HC / 8); i += 32) {
+            for (int i = lane + 32 * half; i < 5 * 16 * (HC / 8); i += 64) {
                 const int l = i / (16 * (HC / 8)), r = (i / (HC / 8)) % 16, ch = i % (HC / 8);
                 *reinterpret_cast<uint4*>(&sm.gr[l][16 * warp + r][ch * 8]) = make_uint4(0, 0, 0, 0);
             }
@@ -415,17 +449,19 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
         for (int ks = 0; ks < 4; ++ks) {
             uint32_t b[NT][2];
 #pragma unroll
-            for (int j = 0; j < NT; ++j) ldB_kn_trans(b[j], &sm.in[warp][0][0], D + 16, 8 * j, 16 * ks, lane);
+            for (int j = 0; j < NT; ++j) ldB_kn_trans(b[j], &sm.in[warp][0][0], D + 8, 8 * j, 16 * ks, lane);
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt) {
+            for (int mt = 0; mt < 2; ++mt) {
                 uint32_t a[4];
-                ldA_km_trans(a, &sm.gr[warp][0][0], GLD, 16 * mt, 16 * ks, lane);
+                ldA_km_trans(a, &sm.gr[warp][0][0], GLD, 32 * half + 16 * mt, 16 * ks, lane);
 #pragma unroll
                 for (int j = 0; j < NT; ++j) mma_bf16(dWacc[mt][j], a, b[j]);
             }
-            uint32_t a[4];
-            ldA_km_trans(a, &sm.gr[4][0][0], GLD, 16 * warp, 16 * ks, lane);
-            mma_bf16(dwb, a, b[NT - 1]);
+            if ((ks & 1) == half) {
+                uint32_t a[4];
+                ldA_km_trans(a, &sm.gr[4][0][0], GLD, 16 * warp, 16 * ks, lane);
+                mma_bf16(dwb, a, b[NT - 1]);
+            }
         }
         __syncthreads();
     }
@@ -434,10 +470,10 @@ __global__ void __launch_bounds__(128) loras_bwd_kernel(LorasParams p) {
     float* dWo = p.dW[warp];
     float* dbo = warp == 0 ? nullptr : p.dbias[warp - 1];  // LoRA 0 (z) has no bias
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
         for (int hrow = 0; hrow < 2; ++hrow) {
-            const int ch = h * HC + 16 * mt + g + 8 * hrow;
+            const int ch = h * HC + 32 * half + 16 * mt + g + 8 * hrow;
 #pragma unroll
             for (int j = 0; j < D / 8; ++j) {
                 atomicAdd(dWo + (long long)ch * D + 8 * j + 2 * t4, dWacc[mt][j][2 * hrow]);
@@ -495,12 +531,17 @@ template <int D> static int launch_loras_bwd_t(const LorasParams& p, cudaStream_
     auto kern = loras_bwd_kernel<D>;
     const int smem = (int)sizeof(LorasBwdSmem<D>);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
-    // enough CTAs for about eight per SM (three are resident at a time), at most one per 64-token tile
+    // one round of resident CTAs, at most one per 64-token tile: each flushes its weight-gradient sums once, and a second round
+    // would rarely be full (32768 rows x 12 heads, 1188 CTAs on 296 places: 5 % slower)
+    static const int resident = [&] {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, BWD_THREADS, smem) == cudaSuccess && n > 0 ? n : 1;
+    }();
     const long long tiles = (p.rows + 63) / 64;
-    long long nseg = (8 * 148 + H - 1) / H;
+    long long nseg = (long long)resident * sm_count() / H;
     if (nseg > tiles) nseg = tiles;
     if (nseg < 1) nseg = 1;
-    kern<<<dim3((unsigned)H, (unsigned)nseg), 128, smem, stream>>>(p);
+    kern<<<dim3((unsigned)H, (unsigned)nseg), BWD_THREADS, smem, stream>>>(p);
     if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
     const long long n = p.rows * (D / 8);
     loras_reduce_heads_kernel<<<dim3((unsigned)((n + 255) / 256), 4), 256, 0, stream>>>(p, H, D);

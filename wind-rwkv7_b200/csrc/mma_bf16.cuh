@@ -16,7 +16,7 @@ using bf16 = __nv_bfloat16;
 //   B 16x8 : b0 (k=2t..2t+1, n=g)  b1 (k=2t+8.., n=g)
 //   C 16x8 : c0 (g,2t) c1 (g,2t+1) c2 (g+8,2t) c3 (g+8,2t+1)
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
@@ -66,13 +66,12 @@ __device__ __forceinline__ void ldA_km_trans(uint32_t (&a)[4], const bf16* p, in
 }
 
 // tanh on the special-function unit (one MUFU instruction, relative error 2^-11: below the bf16 rounding of every value
-// these kernels pass through it), and the logistic function through it: sigmoid(x) = 0.5 tanh(x / 2) + 0.5.
+// these kernels pass through it).
 __device__ __forceinline__ float tanh_f(float x) {
     float y;
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float sigmoid_f(float x) { return fmaf(0.5f, tanh_f(0.5f * x), 0.5f); }
 
 // 8 consecutive bf16 <-> 8 floats
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {

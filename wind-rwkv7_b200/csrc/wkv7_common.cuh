@@ -183,33 +183,8 @@ __device__ __forceinline__ FragB<PREC> fragB_kn(const float* p, int ld, int n0, 
     return f;
 }
 
-// exp(x) on the FMA and integer pipes only (for kernels whose special-function unit is the busier pipe: expand_loras,
-// with seven transcendentals per element, splits them between the two).  2^t with t = x*log2(e): round(t) goes into the
-// exponent field (the low mantissa bits of t + 1.5*2^23 are round(t); shifted left by 23 they land on the exponent, the
-// constant's own bits fall off the top), the fraction in [-0.5, 0.5] through a degree-5 polynomial (relative error 2e-6,
-// far below TF32 operand rounding).  x is clamped to [-80, 80].
-__device__ __forceinline__ float exp_poly(float x) {
-    const float t = fminf(fmaxf(x, -80.f), 80.f) * 1.4426950408889634f;
-    const float tm = t + 12582912.f;
-    const float f = t - (tm - 12582912.f);
-    float p = 1.3333558e-3f;
-    p = fmaf(p, f, 9.6181291e-3f);
-    p = fmaf(p, f, 5.5504109e-2f);
-    p = fmaf(p, f, 2.4022651e-1f);
-    p = fmaf(p, f, 6.9314718e-1f);
-    p = fmaf(p, f, 1.f);
-    return __int_as_float(__float_as_int(p) + (__float_as_int(tm) << 23));
-}
-// 1/x for positive normal x without MUFU: exponent-flip seed (12% error), three Newton steps.
-__device__ __forceinline__ float rcp_newton(float x) {
-    float y = __int_as_float(0x7EF311C7 - __float_as_int(x));
-    y = y * fmaf(-x, y, 2.f);
-    y = y * fmaf(-x, y, 2.f);
-    y = y * fmaf(-x, y, 2.f);
-    return y;
-}
-// The same two functions on the special-function unit (one MUFU instruction each, relative error about 2^-22): what the
-// WKV7 kernels use, whose XU pipe is otherwise idle (TF32 rounding is done with integer instructions).
+// exp and reciprocal on the special-function unit (one MUFU instruction each, relative error about 2^-22) for the
+// WKV7 kernels, whose XU pipe is otherwise idle (TF32 rounding is done with integer instructions).
 __device__ __forceinline__ float exp_mufu(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fminf(fmaxf(x, -80.f), 80.f) * 1.4426950408889634f));
