@@ -126,6 +126,16 @@ int wkv7_attn_ln_fwd_ws(const void* r, const void* w, const void* k, const void*
                         const void* g, const float* params, const float* s0, void* y, float* sT, float* ckpt,
                         float eps, int64_t B, int64_t T, int64_t H, int64_t N,
                         int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
+/*
+ * Forward of bf16 tensors with every sequence cut into nseg >= 2 equal segments that run as chains of their own (T % nseg == 0; batch
+ * stride T * stride_t, head stride N): for B*H far below the number of SMs.  No checkpoints.  The state at a segment's start is formed
+ * from an affine map of the segments before it, so results agree with wkv7_fwd's within the rounding of its operands, not bit for
+ * bit.  Workspace: wkv7_fwd_time_split_workspace_bytes(B, H, nseg), 16-byte aligned.
+ */
+int64_t wkv7_fwd_time_split_workspace_bytes(int64_t B, int64_t H, int64_t nseg);
+int wkv7_fwd_time_split(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                        const float* s0, void* y, float* sT, int64_t B, int64_t T, int64_t H, int64_t N, int64_t nseg,
+                        int64_t stride_t, void* workspace, void* stream);
 /* The backward's scratch is wkv7_bwd_ws_bytes() bytes.  It keeps a cut chain's state gradient in ds0, which must be given for a
  * cut.  Where there are few chains (bf16), the scratch also passes each chunk's state gradient from the CTA that walks the chain
  * to the CTAs that do the rest of the chunk's work. */

@@ -76,3 +76,18 @@ def test_backward(extra, T, dsT, ln):
         else:
             assert th.equal(a, b)
     assert L.wkv7_device_status() == 0
+
+
+@pytest.mark.parametrize('B,T,H,nseg', [(1, 34, 2, 2), (1, 3, 1, 3), (2, 99, 2, 3), (1, 256, 5, 16), (3, 1024, 7, 8)])
+@pytest.mark.parametrize('s0', [False, True])
+def test_time_split(B, T, H, nseg, s0):
+    """Sequences cut into parallel segments: one and several sequences, ragged segments, against the uncut forward."""
+    from wind_rwkv.rwkv7 import _lib, attn, synthetic
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=T, dtype=th.bfloat16, device='cuda', s0_std=0.1)
+    ins, s = [d[n] for n in 'rwkvab'], d['s0'] if s0 else None
+    with th.no_grad():
+        want = attn(*ins, N, s0=s, return_state=True)
+        got = attn(*ins, N, s0=s, return_state=True, time_split=nseg)
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and (a.float() - b.float()).norm() <= 4e-3 * b.float().norm()
+    assert _lib.lib().wkv7_device_status() == 0

@@ -228,6 +228,33 @@ int wkv7_fwd_ws(const void* r, const void* w, const void* k, const void* v, cons
                       stride_h, io_dtype, workspace, stream);
 }
 
+int64_t wkv7_fwd_time_split_workspace_bytes(int64_t B, int64_t H, int64_t nseg) {
+    return B < 0 || H < 0 || nseg < 0 ? 0 : (int64_t)wkv7::time_split_workspace_bytes(B, H, (int)nseg);
+}
+
+int wkv7_fwd_time_split(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                        const float* s0, void* y, float* sT, int64_t B, int64_t T, int64_t H, int64_t N, int64_t nseg,
+                        int64_t stride_t, void* workspace, void* stream) {
+    int rc = check_common(B, T, H, N, T * stride_t, stride_t, N, WKV7_BF16);
+    if (rc) return rc;
+    if (nseg < 2 || nseg > 4096 || T % nseg != 0) return WKV7_ERR_SHAPE;
+    if (B == 0 || H == 0 || T == 0) return WKV7_ERR_SHAPE;
+    if (!r || !w || !k || !v || !a || !b || !y || !workspace) return WKV7_ERR_NULL;
+    const void* ptrs[] = {r, w, k, v, a, b, y, s0, sT, workspace};
+    for (const void* p : ptrs)
+        if (p && !aligned16(p)) return WKV7_ERR_ALIGN;
+    if (B * nseg * H > 0x7fffffff) return WKV7_ERR_TOO_LARGE;
+    const int groups = fwd_impl().load(std::memory_order_relaxed);
+    wkv7::FwdParams p{};
+    p.r = r; p.w = w; p.k = k; p.v = v; p.a = a; p.b = b; p.s0 = s0; p.y = y; p.sT = sT;
+    p.B = B; p.T = T; p.H = H;
+    p.st = wkv7::Strides{T * stride_t, stride_t, N};
+    p.flags = (unsigned*)workspace;
+    p.status = status_ptr();
+    if (!p.status) return WKV7_ERR_LAUNCH;
+    return wkv7::launch_fwd_time_split(p, (int)nseg, groups ? groups : 4, (cudaStream_t)stream);
+}
+
 int wkv7_step(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* s0,
               void* y, float* sT, int64_t B, int64_t T, int64_t H, int64_t N, int64_t stride_b, int64_t stride_t,
               int64_t stride_h, int io_dtype, void* stream) {

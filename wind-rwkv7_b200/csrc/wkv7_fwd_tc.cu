@@ -856,6 +856,8 @@ static bool encode_checkpoint_map(CUtensorMap* m, float* base, long long records
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+__device__ __align__(128) __nv_bfloat16 g_zero_row[N];
+
 template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdParams& p, cudaStream_t stream) {
     auto kern = wkv7_fwd_tc_kernel<G, RND, LN, TAIL>;
     const int smem = G * (LN ? G_BYTES_LN : G_BYTES_PLAIN) + (int)sizeof(Ctrl) + 1024;
@@ -866,7 +868,11 @@ template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdPar
     const void* ins[8] = {p.y, p.r, p.w, p.k, p.a, p.b, p.v, p.g};
     CUtensorMap* const ms[8] = {&maps.y, &maps.in[0], &maps.in[1], &maps.in[2], &maps.in[3], &maps.in[4], &maps.in[5], &maps.g};
     for (int i = 0; i < (LN ? 8 : 7); ++i)
-        if (!encode_bthn_map(ms[i], const_cast<void*>(ins[i]), p.B, p.T, p.H, p.st)) return kLaunchFailed;
+        if (ins[i] && !encode_bthn_map(ms[i], const_cast<void*>(ins[i]), p.B, p.T, p.H, p.st)) return kLaunchFailed;
+    if (!p.v) {  // v = 0: a tensor of one zero row; what lies beyond it reads as zero
+        void* zeros = nullptr;
+        if (cudaGetSymbolAddress(&zeros, g_zero_row) != cudaSuccess || !encode_bthn_map(&maps.in[5], zeros, 1, 1, 1, Strides{N, N, N})) return kLaunchFailed;
+    }
     const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 1, p.sT ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
     kern<<<(unsigned)ws.ctas, 128 * (G + 1), smem, stream>>>(p, ws, maps);

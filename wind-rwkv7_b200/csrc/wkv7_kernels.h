@@ -67,9 +67,12 @@ int launch_bwd_bf16(const BwdParams& p, bool ln, cudaStream_t stream);
 size_t bwd_workspace_bytes(long long B, long long T, long long H);  // what launch_bwd wants at p.flags for bf16 tensors (attn)
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
-// tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
+// tcgen05 forward (bf16 IO; v null: zeros; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
 // not rounded to TF32 by their producer (the tensor core truncates them)
 int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream);
+// bf16 forward with the sequences cut into nseg segments each (wkv7_time_split.cu)
+size_t time_split_workspace_bytes(long long B, long long H, int nseg);
+int launch_fwd_time_split(const FwdParams& p, int nseg, int groups, cudaStream_t stream);
 // C[M,N] = act(A[M,K] W[N,K]^T), bf16, tanh on columns [tanh_from, tanh_to); tcgen05 + TMA (proj_gemm.cu)
 int launch_proj_gemm(const void* A, const void* W, void* C, long long M, long long N, long long K, int tanh_from, int tanh_to,
                      int* status, cudaStream_t stream);

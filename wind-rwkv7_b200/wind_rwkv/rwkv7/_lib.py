@@ -42,6 +42,8 @@ _SIGNATURES = {
     'wkv7_get_fwd_impl': (_int, []),
     'wkv7_fwd': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp]),
     'wkv7_workspace_bytes': (ctypes.c_size_t, []),
+    'wkv7_fwd_time_split_workspace_bytes': (_i64, [_i64] * 3),
+    'wkv7_fwd_time_split': (_int, [_vp] * 9 + [_i64] * 6 + [_vp] * 2),
     'wkv7_bwd_ws_bytes': (_i64, [_i64] * 4 + [_int]),
     'wkv7_fwd_ws': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_bwd_ws': (_int, [_vp] * 17 + [_i64] * 7 + [_int, _vp, _vp]),

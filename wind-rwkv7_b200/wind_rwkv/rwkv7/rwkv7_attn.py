@@ -133,6 +133,7 @@ def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
     number of SMs: one CTA walks one chain, so a single long sequence otherwise occupies H SMs).
 
     The recurrence is affine in the state: over a segment S_end = S_start M + R, with M and R independent of S_start.
+    bf16 tensors: csrc/wkv7_time_split.cu does the whole of it.  Otherwise here:
     Pass 1 runs every segment twice (two concurrent launches of nseg*B*H chains): from the zero state with the real inputs
     (final state = R) and from the identity state with v = 0 (final state = M).  A short host loop of nseg - 1 batched
     64x64 products gives every segment's start state; pass 2 is the ordinary forward over the segments with those.
@@ -141,6 +142,19 @@ def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
     B, T, HC = w.shape
     H = HC // C
     assert T % nseg == 0, 'time_split must divide T'
+    if w.dtype == th.bfloat16 and all(i.dtype == th.bfloat16 and i.shape == w.shape for i in (r, k, v, a, b)) and w.numel() and _lib.lib().wkv7_get_fwd_impl():
+        _lib.require_cuda(r, w, k, v, a, b, s0)
+        r, w, k, v, a, b = [i.detach().contiguous() for i in (r, w, k, v, a, b)]
+        s0 = None if s0 is None else s0.detach().float().contiguous()
+        assert s0 is None or list(s0.shape) == [B, H, C, C]
+        y = th.empty_like(v)
+        sT = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
+        ws = th.empty(_lib.lib().wkv7_fwd_time_split_workspace_bytes(B, H, nseg), dtype=th.uint8, device=w.device)
+        with _lib.on_device(r, w, k, v, a, b, s0):
+            rc = _lib.lib().wkv7_fwd_time_split(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), _lib.ptr(s0),
+                                                y.data_ptr(), sT.data_ptr(), B, T, H, C, nseg, HC, ws.data_ptr(), _lib.stream_of(w))
+        _lib.check(rc, 'wkv7_fwd_time_split')
+        return y, sT
     Ts = T // nseg
     ins = [i.contiguous().view(B * nseg, Ts, H, C) for i in (w, r, k, v, a, b)]   # segments become batch entries: no copy
     dev = w.device
