@@ -112,3 +112,21 @@ def test_cast():
     for s, d in zip(src, dst):
         assert th.equal(s.to(d.dtype), d)
     assert _lib.lib().wkv7_cast(None, None, None, None, 33, None) != 0
+
+
+@pytest.mark.parametrize('M', [1, 130])
+def test_proj_group(M):
+    """Products of different widths in one launch: tiles that some of them do not have."""
+    import ctypes
+    from wind_rwkv.rwkv7 import _lib, proj
+    K, widths, tanh = 72, [8, 136, 96], [(0, 8), (0, 0), (0, 64)]
+    x = [th.randn(M, K, device='cuda').bfloat16() for _ in widths]
+    w = [(th.randn(n, K, device='cuda') / 8).bfloat16() for n in widths]
+    out = [th.empty(M, n, device='cuda', dtype=th.bfloat16) for n in widths]
+    ptrs = lambda ts: (ctypes.c_void_p * 3)(*[t.data_ptr() for t in ts])
+    ints = lambda v: (ctypes.c_int64 * 3)(*v)
+    assert _lib.lib().wkv7_proj_gemm_group(3, ptrs(x), ptrs(w), ptrs(out), ints(widths), ints([f for f, _ in tanh]), ints([t for _, t in tanh]), M, K,
+                                           th.cuda.current_stream().cuda_stream) == 0
+    for a, b, o, t in zip(x, w, out, tanh):
+        assert th.equal(proj(a, b, t), o)
+    assert _lib.lib().wkv7_proj_gemm_group(5, None, None, None, None, None, None, M, K, None) != 0

@@ -405,10 +405,19 @@ enum { WR, WK, WV, WO, GATE1, GATE2, KKK1, MK1, DECAY1, AAA1, MA1, DECAY2, MAAX,
        LNW = NBF, LNB, FAAAA, NPAR };
 constexpr int64_t MIX = 32, DEC = 64, SMALL = 16, GATE = 128, WAM = DEC + 2 * SMALL;
 
-Tensor proj(const Tensor& x, const Tensor& w, int64_t from, int64_t to) {
-    Tensor out = at::empty({x.size(0), w.size(0)}, x.options());
-    check(wkv7_proj_gemm(x.data_ptr(), w.data_ptr(), out.data_ptr(), x.size(0), w.size(0), x.size(1), from, to, stream()), "wkv7_proj_gemm");
-    return out;
+// tanh on the first `to` columns
+struct Proj { const Tensor &x, &w; int64_t to; Tensor* out; };
+void proj(std::initializer_list<Proj> ps) {
+    const void *a[WKV7_PROJ_MAX], *b[WKV7_PROJ_MAX];
+    void* c[WKV7_PROJ_MAX];
+    int64_t n[WKV7_PROJ_MAX], from[WKV7_PROJ_MAX] = {}, to[WKV7_PROJ_MAX];
+    int i = 0;
+    for (const Proj& p : ps) {
+        *p.out = at::empty({p.x.size(0), p.w.size(0)}, p.x.options());
+        a[i] = p.x.data_ptr(); b[i] = p.w.data_ptr(); c[i] = p.out->data_ptr(); n[i] = p.w.size(0); to[i++] = p.to;
+    }
+    const Tensor& x = ps.begin()->x;
+    check(wkv7_proj_gemm_group(i, a, b, c, n, from, to, x.size(0), x.size(1), stream()), "wkv7_proj_gemm_group");
 }
 struct Mixer {
     int64_t B, T, C;
@@ -452,12 +461,10 @@ struct Mixer {
         ddlerp_forward(x, ddlerp_par(), m, y4);
         const Tensor xrg = in4(0), xwa = in4(1), xk = in4(2), xv = in4(3);
         r = seq(at::mm(xrg, p[WR].t()));
-        g1 = proj(xrg, p[GATE1], 0, GATE);
+        proj({{xrg, p[GATE1], GATE, &g1}, {xk, kkmk_w, 0, &kkmk}, {xwa, wam_w, DEC, &wam}});
         g = seq(at::mm(g1, p[GATE2].t()));
         k0 = seq(at::mm(xk, p[WK].t()));
-        kkmk = proj(xk, kkmk_w, 0, 0);
         v = seq(at::mm(xv, p[WV].t()));
-        wam = proj(xwa, wam_w, 0, DEC);
         w2 = seq(at::mm(wam.narrow(1, 0, DEC), p[DECAY2].t()));
         if (!save) y4 = m = Tensor();
         const int64_t ld[4] = {2 * SMALL, WAM, WAM, 2 * SMALL};
