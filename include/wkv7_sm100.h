@@ -136,17 +136,19 @@ int64_t wkv7_fwd_time_split_workspace_bytes(int64_t B, int64_t H, int64_t nseg);
 int wkv7_fwd_time_split(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                         const float* s0, void* y, float* sT, int64_t B, int64_t T, int64_t H, int64_t N, int64_t nseg,
                         int64_t stride_t, void* workspace, void* stream);
-/* The backward's scratch is wkv7_bwd_ws_bytes() bytes.  It keeps a cut chain's state gradient in ds0, which must be given for a
- * cut.  Where there are few chains (bf16), the scratch also passes each chunk's state gradient from the CTA that walks the chain
- * to the CTAs that do the rest of the chunk's work. */
+/* The backward's scratch is wkv7_bwd_ws_bytes() bytes, asked for with the call's device current (it depends on the number of SMs).
+ * The backward keeps a cut chain's state gradient in ds0, which must be given for a cut.  Where there are few chains (bf16), the
+ * scratch also passes each chunk's state gradient from the CTA that walks the chain to the CTAs that do the rest of the chunk's work. */
 int64_t wkv7_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype);
 int wkv7_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                 const void* dy, const float* ckpt, const float* dsT, const float* sT,
                 void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* ds0,
                 int64_t B, int64_t T, int64_t H, int64_t N,
                 int64_t stride_b, int64_t stride_t, int64_t stride_h, int io_dtype, void* workspace, void* stream);
-/* As wkv7_attn_ln_bwd; dparams_workspace is that call's workspace.  Where a chain is cut or shared, its part of dparams is summed in
+/* As wkv7_attn_ln_bwd; dparams_workspace is that call's workspace, workspace is wkv7_attn_ln_bwd_ws_bytes() bytes of scratch (less
+ * than wkv7_bwd_ws_bytes() asks for: this backward never walks the state gradient ahead).  Where a chain is cut or shared, its part of dparams is summed in
  * pieces: dparams then agrees with the plain call's up to fp32 rounding (and is still deterministic). */
+int64_t wkv7_attn_ln_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype);
 int wkv7_attn_ln_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                         const void* g, const float* params, const void* dy, const float* ckpt, const float* dsT,
                         const float* sT, void* dr, void* dw, void* dk, void* dv, void* da, void* db, void* dg,

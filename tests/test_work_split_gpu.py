@@ -52,7 +52,7 @@ def test_backward(extra, T, dsT, ln):
     g, params = synthetic.attn_ln_extras(B, T, H, N, seed=T, dtype=th.bfloat16, device='cuda')
     _, sT, ck = fw_attn(*[d[n].view(B, T, H, N) for n in 'wrkvab'], d['s0'])
     gs = th.randn(B, H, N, N, device='cuda') if dsT else None
-    ws = th.full((L.wkv7_bwd_ws_bytes(B, T, H, N, 0),), 255, dtype=th.uint8, device='cuda')
+    ws = th.full(((L.wkv7_attn_ln_bwd_ws_bytes if ln else L.wkv7_bwd_ws_bytes)(B, T, H, N, 0),), 255, dtype=th.uint8, device='cuda')
     part = th.empty(B, 3, H * N, device='cuda')
 
     def call(split):
@@ -76,6 +76,31 @@ def test_backward(extra, T, dsT, ln):
         else:
             assert th.equal(a, b)
     assert L.wkv7_device_status() == 0
+
+
+@pytest.mark.parametrize('form', ['c++', 'python'])
+def test_backward_scratch_of_few_chains(form, monkeypatch):
+    """The tiles of the walked state gradients are asked for where they are used (attn), not by attn_ln, which is not walked."""
+    from wind_rwkv.rwkv7 import _lib, attn, attn_ln, synthetic
+    if form == 'python':
+        _lib.ext()
+        monkeypatch.setattr(_lib, '_ext', type('Nothing', (), {'__getattr__': lambda self, name: lambda *a: None})())
+    L = _lib.lib()
+    B, T, H = 1, 4096, 12
+    tiles = B * H * (T // 16) * 64 * 72 * 4
+    assert L.wkv7_bwd_ws_bytes(B, T, H, N, 0) == L.wkv7_workspace_bytes() + tiles
+    assert L.wkv7_attn_ln_bwd_ws_bytes(B, T, H, N, 0) == L.wkv7_workspace_bytes()
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=1, dtype=th.bfloat16, device='cuda')
+    ins = [d[n].requires_grad_() for n in 'rwkvab']
+    g, params = [x.requires_grad_() for x in synthetic.attn_ln_extras(B, T, H, N, seed=1, dtype=th.bfloat16, device='cuda')]
+    for y, wrt in ((attn_ln(*ins, g, params, N), ins + [g, params]), (attn(*ins, N), ins)):
+        th.cuda.synchronize()
+        th.cuda.reset_peak_memory_stats()
+        before = th.cuda.memory_allocated()
+        grads = th.autograd.grad(y, wrt, d['dy'])
+        extra = th.cuda.max_memory_allocated() - before - sum(x.numel() * x.element_size() for x in grads)
+        assert extra < tiles // 8 if len(wrt) == 8 else extra >= tiles  # (attn_ln's rest: ds0, partial sums)
+        del grads
 
 
 @pytest.mark.parametrize('B,T,H,nseg', [(1, 34, 2, 2), (1, 3, 1, 3), (2, 99, 2, 3), (1, 256, 5, 16), (3, 1024, 7, 8)])

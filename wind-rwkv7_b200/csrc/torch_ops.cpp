@@ -111,7 +111,7 @@ variable_list wkv_backward(Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Ten
     Rows q;
     rows_of({&w}, q);
     Tensor dr = like_rows(w), dw = like_rows(w), dk = like_rows(w), dv = like_rows(w), da = like_rows(w), db = like_rows(w), ds0 = states(w, q);
-    Tensor ws = at::empty({wkv7_bwd_ws_bytes(q.B, q.T, q.H, N, q.io)}, w.options().dtype(at::kByte));
+    Tensor ws = at::empty({(g.defined() ? wkv7_attn_ln_bwd_ws_bytes : wkv7_bwd_ws_bytes)(q.B, q.T, q.H, N, q.io)}, w.options().dtype(at::kByte));
     const float* sTp = dsT.defined() ? f32(sT) : nullptr;
     if (!g.defined()) {
         check(wkv7_bwd_ws(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), dy.data_ptr(), f32(ck), f32(dsT), sTp,

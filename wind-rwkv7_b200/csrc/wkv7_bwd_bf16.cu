@@ -996,18 +996,19 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
 // all of a chunk's work in it is bound by the latency of a chunk (6200 cycles) while SMs are idle; the walk takes 1/5 of that and
 // the rest spreads over the machine.  With as many chains as SMs it still pays; beyond, a walk has its second round.
 // The tiles of a pass are kept below 512 MB; longer sequences take several passes, the walk going on from ds0.
-static int walk_chunks(long long chains, long long chunks) {
-    if (chains == 0 || chains > sm_count() || chunks < 4) return 0;
+// attn_ln is never walked: its walk would need the gradient of the recurrence output first.
+static int walk_chunks(long long chains, long long chunks, bool ln) {
+    if (ln || chains == 0 || chains > sm_count() || chunks < 4) return 0;
     return (int)std::min(chunks, std::max(1LL, (512LL << 20) / (chains * bf16bwd::TILE_FLOATS * 4)));
 }
-size_t bwd_workspace_bytes(long long B, long long T, long long H) {
-    return WORK_FLAG_BYTES + (size_t)(B * H * walk_chunks(B * H, (T + L - 1) / L)) * bf16bwd::TILE_FLOATS * sizeof(float);
+size_t bwd_workspace_bytes(long long B, long long T, long long H, bool ln) {
+    return WORK_FLAG_BYTES + (size_t)(B * H * walk_chunks(B * H, (T + L - 1) / L, ln)) * bf16bwd::TILE_FLOATS * sizeof(float);
 }
 
 template <bool LN> static int launch_bwd_bf16_t(const BwdParams& p, cudaStream_t stream) {
     using namespace bf16bwd;
     const long long chains = p.B * p.H, chunks = (p.T + L - 1) / L;
-    const int walked = !LN && p.flags && p.ds0 ? walk_chunks(chains, chunks) : 0;
+    const int walked = p.flags && p.ds0 ? walk_chunks(chains, chunks, LN) : 0;
     auto kern = p.T % L ? wkv7_bwd_bf16_kernel<true, LN, false> : wkv7_bwd_bf16_kernel<false, LN, false>;
     if (walked) kern = p.T % L ? wkv7_bwd_bf16_kernel<true, LN, !LN> : wkv7_bwd_bf16_kernel<false, LN, !LN>;
     const int smem = (int)sizeof(Smem<LN>) + 1024;

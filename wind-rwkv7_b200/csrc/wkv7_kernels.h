@@ -64,7 +64,7 @@ int launch_step(const StepParams& p, int io_dtype, cudaStream_t stream);
 bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long records);
 bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long records);
 int launch_bwd_bf16(const BwdParams& p, bool ln, cudaStream_t stream);
-size_t bwd_workspace_bytes(long long B, long long T, long long H);  // what launch_bwd wants at p.flags for bf16 tensors (attn)
+size_t bwd_workspace_bytes(long long B, long long T, long long H, bool ln);  // what launch_bwd wants at p.flags for bf16 tensors
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
 // tcgen05 forward (bf16 IO; v null: zeros; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are

@@ -45,6 +45,7 @@ _SIGNATURES = {
     'wkv7_fwd_time_split_workspace_bytes': (_i64, [_i64] * 3),
     'wkv7_fwd_time_split': (_int, [_vp] * 9 + [_i64] * 6 + [_vp] * 2),
     'wkv7_bwd_ws_bytes': (_i64, [_i64] * 4 + [_int]),
+    'wkv7_attn_ln_bwd_ws_bytes': (_i64, [_i64] * 4 + [_int]),
     'wkv7_fwd_ws': (_int, [_vp] * 10 + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_bwd_ws': (_int, [_vp] * 17 + [_i64] * 7 + [_int, _vp, _vp]),
     'wkv7_attn_ln_bwd_ws': (_int, [_vp] * 22 + [_f32] + [_i64] * 7 + [_int, _vp, _vp]),
@@ -145,9 +146,11 @@ def io_dtype(t):
 _SCRATCH_BYTES = None
 
 
-def bwd_scratch(w):
-    """Device scratch of one backward *_ws call for [B,T,H,N] tensors like w."""
-    return th.empty(lib().wkv7_bwd_ws_bytes(*w.shape, io_dtype(w)), dtype=th.uint8, device=w.device)
+def bwd_scratch(w, ln=False):
+    """Device scratch of one backward *_ws call (ln: of attn_ln) for [B,T,H,N] tensors like w, whose device must be current: the
+    size depends on its number of SMs."""
+    size = lib().wkv7_attn_ln_bwd_ws_bytes if ln else lib().wkv7_bwd_ws_bytes
+    return th.empty(size(*w.shape, io_dtype(w)), dtype=th.uint8, device=w.device)
 
 
 def scratch(device):

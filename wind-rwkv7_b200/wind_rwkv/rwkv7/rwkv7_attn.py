@@ -46,9 +46,9 @@ def bw_attn(w, q, k, v, a, b, s, dy, dsT, sT):
         w, q, k, v, a, b, dy = [i.contiguous() for i in (w, q, k, v, a, b, dy)]
     dw, dq, dk, dv, da, db = [th.empty_strided(w.shape, w.stride(), dtype=w.dtype, device=w.device) for _ in range(6)]
     ds0 = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
-    ws = _lib.bwd_scratch(w)
     sb, st, sh = _lib.strides4(w)
     with _lib.on_device(w, q, k, v, a, b, s, dy, dsT):
+        ws = _lib.bwd_scratch(w)
         rc = _lib.lib().wkv7_bwd_ws(q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(),
                                     dy.data_ptr(), s.data_ptr(), _lib.ptr(dsT), _lib.ptr(sT if dsT is not None else None),
                                     dq.data_ptr(), dw.data_ptr(), dk.data_ptr(), dv.data_ptr(), da.data_ptr(), db.data_ptr(),

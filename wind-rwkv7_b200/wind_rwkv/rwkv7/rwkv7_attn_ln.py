@@ -41,9 +41,9 @@ def bw_attn_ln(w, q, k, v, a, b, g, params, s, dy, dsT, sT):
     dparams = th.empty(3, H * C, dtype=th.float32, device=w.device)
     ws = th.empty(B, 3, H * C, dtype=th.float32, device=w.device)
     ds0 = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
-    sched = _lib.bwd_scratch(w)
     sb, st, sh = _lib.strides4(w)
     with _lib.on_device(w, q, k, v, a, b, g, params, s, dy, dsT):
+        sched = _lib.bwd_scratch(w, ln=True)
         rc = _lib.lib().wkv7_attn_ln_bwd_ws(
             q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), g.data_ptr(),
             params.data_ptr(), dy.data_ptr(), s.data_ptr(), _lib.ptr(dsT), _lib.ptr(sT if dsT is not None else None),
