@@ -97,6 +97,38 @@ def test_attn_state_and_slices(dtype, monkeypatch):
         assert th.equal(g, w)
 
 
+def _ops():
+    """name -> (function, inputs) of every entry point with an autograd function, at small sizes."""
+    from wind_rwkv.rwkv7 import TimeMixer, attn, attn_ln, ddlerp, expand_loras, synthetic
+    B, T, H, D = 2, 20, 2, 16
+    C = H * N
+    th.manual_seed(2)
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=4, dtype=th.bfloat16, device='cuda', s0_std=0.1)
+    g, params = synthetic.attn_ln_extras(B, T, H, N, seed=4, dtype=th.bfloat16, device='cuda')
+    x = th.randn(B, T, C, device='cuda').bfloat16()
+    mixer = TimeMixer(types.SimpleNamespace(n_layer=4, n_head=H, n_embd=C), 1).cuda().requires_grad_(False)
+    rkv = [d[n] for n in 'rwkvab']
+    par = [th.rand(C, device='cuda'), th.randn(4 * D, C, device='cuda'), th.randn(4, C, D, device='cuda'), th.rand(4, 1, 1, C, device='cuda')]
+    lora = [x.flip(1)] + [th.randn(B, T, D, device='cuda').bfloat16() for _ in range(4)]
+    lora += [th.randn(C, D, device='cuda') for _ in range(4)] + [th.randn(C, device='cuda') for _ in range(4)]
+    return {'attn': (lambda *a: attn(*a[:6], N, s0=a[6]), rkv + [d['s0']]), 'attn_ln': (lambda *a: attn_ln(*a, N), rkv + [g, params]),
+            'ddlerp': (ddlerp, [x] + par), 'expand_loras': (lambda *a: expand_loras(*a, N), [x] + lora), 'mixer': (mixer, [x])}
+
+
+@pytest.mark.parametrize('op', ['attn', 'attn_ln', 'ddlerp', 'expand_loras', 'mixer'])
+def test_forward_mode_raises(op):
+    """No forward-mode derivative is implemented: a dual tensor in any place raises, with and without requires_grad anywhere, and
+    no output comes back without its tangent."""
+    import torch.autograd.forward_ad as fwd
+    f, ins = _ops()[op]
+    for i in {0, 1, len(ins) // 2, len(ins) - 1} & set(range(len(ins))):
+        for grad in (False, True):
+            with fwd.dual_level():
+                dual = [fwd.make_dual(t.clone().requires_grad_(grad), th.ones_like(t)) if j == i else t for j, t in enumerate(ins)]
+                with pytest.raises((NotImplementedError, RuntimeError), match='jvp'):
+                    f(*dual)
+
+
 def test_cast():
     from wind_rwkv.rwkv7 import _lib
     import ctypes

@@ -43,12 +43,13 @@ bool grad_wanted(std::initializer_list<const Tensor*> ts) {
         if (t->defined() && t->requires_grad()) return true;
     return false;
 }
-// a dense CUDA tensor of its own: no subclass or transform wrapper, whose meaning only the Python path's operators see
+// a dense CUDA tensor of its own: no subclass or transform wrapper, whose meaning only the Python path's operators see, and no
+// forward-mode dual, for which the Python path's autograd functions raise
 bool plain(const Tensor& t) {
     using c10::DispatchKey;
     const auto keys = t.key_set();
     return t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !keys.has(DispatchKey::Python) && !keys.has(DispatchKey::FuncTorchGradWrapper) &&
-           !keys.has(DispatchKey::FuncTorchBatched);
+           !keys.has(DispatchKey::FuncTorchBatched) && !t._fw_grad(0).defined();
 }
 
 // F::apply on the first sizeof...(I) tensors of a list: autograd sees tensors that are arguments of their own, not those in a list
