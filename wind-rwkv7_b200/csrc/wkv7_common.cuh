@@ -360,7 +360,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // CTA's abort flag (every later wait then falls through), records kDeviceTimeout in the device status word and
 // returns: a lost copy or a missing arrival ends with an error code, never with a hung GPU.
 // SLEEP: the thread is suspended by the hardware (try_wait with a time hint) instead of polling.
-constexpr long long MBAR_WAIT_LIMIT = 1LL << 28;  // clocks (~0.15 s): far beyond any legitimate wait
+constexpr long long MBAR_WAIT_LIMIT = 1LL << 28;  // clocks (~0.14 s): far beyond any legitimate wait within a CTA
+// The wait for another CTA's half of a cut chain (wait_handoff below) may legitimately take longer: the CTAs of one launch run at
+// different speeds when other work shares the GPU with them, and a range of work can be 0.1 s long.  The waits of the same CTA that
+// stand still meanwhile are given more again, so that the one that gives up is the one whose condition is missing.
+constexpr long long HANDOFF_WAIT_LIMIT = 4 * MBAR_WAIT_LIMIT;         // 0.55 s
+constexpr long long ACROSS_HANDOFF_LIMIT = 2 * HANDOFF_WAIT_LIMIT;    // 1.1 s
+static_assert(MBAR_WAIT_LIMIT < HANDOFF_WAIT_LIMIT && HANDOFF_WAIT_LIMIT < ACROSS_HANDOFF_LIMIT, "see above");
+static_assert(ACROSS_HANDOFF_LIMIT <= 1LL << 31, "mbar_wait_bounded counts in 32 bits");
 __device__ __forceinline__ void give_up(volatile int* abort, int* status) {
     *abort = 1;
     *reinterpret_cast<volatile int*>(status) = (int)kDeviceTimeout;  // the launchers always pass the status word (host-visible)
@@ -447,14 +454,14 @@ struct WorkRange {
 __device__ __forceinline__ void publish_handoff(unsigned* flag) {
     asm volatile("st.release.gpu.global.u32 [%0], 1;" ::"l"(flag) : "memory");
 }
-// Bounded like every wait of this library (see mbar_wait_bounded).
+// Bounded like every wait of this library (see mbar_wait_bounded and HANDOFF_WAIT_LIMIT).
 __device__ __forceinline__ void wait_handoff(const unsigned* flag, volatile int* abort, int* status) {
     const long long start = clock64();
     for (;;) {
         unsigned ready;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(ready) : "l"(flag) : "memory");
         if (ready || *abort) return;
-        if (clock64() - start > 16 * MBAR_WAIT_LIMIT) {  // a whole range of work may lie in between when the GPU is shared
+        if (clock64() - start > HANDOFF_WAIT_LIMIT) {
             give_up(abort, status);
             return;
         }

@@ -84,7 +84,9 @@ constexpr int C_XY = 320;    // + 32 * group: X (16) | Y (16) of the group's chu
                              // [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47, and then QB AI in lanes 32-47 of columns 16-31
 constexpr int C_FOLD = 448;  // AI^T bwf (64) in lanes 0-15
 
-constexpr long long WAIT_LIMIT = MBAR_WAIT_LIMIT;
+// Any wait of this kernel may stand still while one of its groups waits for the state of a cut chain: the chain warp (full), the
+// score and inverse warps (score, fold, mats, fread), and the other groups (done).
+constexpr long long WAIT_LIMIT = ACROSS_HANDOFF_LIMIT;
 
 // One chunk of the CTA's work list, as its preparation group (and the chain thread) need it.
 struct ChunkDesc {
