@@ -13,7 +13,7 @@
  *   (stride_b, stride_t, stride_h, 1); N == 64.  A contiguous [B, T, H*N] tensor has
  *   stride_b = T*H*N, stride_t = H*N, stride_h = N.  Head- or batch-sharded views are
  *   expressed through the strides.  Base pointers and strides must keep every row 16-byte
- *   aligned.  States s0, sT, dsT, ds0: fp32 [B, H, N, N] contiguous, S[value][key].
+ *   aligned, and keep the rows of y and of the gradients, which have the inputs' strides, apart.  States s0, sT, dsT, ds0: fp32 [B, H, N, N] contiguous, S[value][key].
  *   Checkpoints: fp32 [B, H, ceil(T/16), WKV7_CHECKPOINT_FLOATS] contiguous, one record per 16-step chunk; the
  *   contents are private to the library.  Size the buffer with wkv7_checkpoint_bytes() and nothing else.
  *   io_dtype: WKV7_BF16 (bf16 tensors, single-TF32 tensor-core products, fp32 state) or

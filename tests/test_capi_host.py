@@ -92,3 +92,13 @@ def test_status_word_is_readable_without_a_device(lib):
     """wkv7_peek_status is a host load of a managed variable; without a GPU it reports a launch error rather than
     crashing."""
     assert lib.wkv7_peek_status() in (0, -7)
+
+
+def test_layouts_that_share_memory_are_told_apart():
+    import torch as th
+    from wind_rwkv.rwkv7.rwkv7_attn import _apart
+    t = th.zeros(4096)
+    for size, stride, want in [((3, 4, 2, 8), (64, 16, 8, 1), True), ((3, 4, 2, 8), (32, 16, 8, 1), False), ((3, 4, 2, 8), (0, 16, 8, 1), False),
+                               ((3, 4, 2, 8), (16, 48, 8, 1), True), ((1, 4, 2, 8), (0, 16, 8, 1), True), ((3, 1, 2, 8), (16, 1, 8, 1), True),
+                               ((3, 4, 2, 8), (128, 32, 8, 1), True), ((3, 4, 2, 8), (64, 16, 4, 1), False)]:
+        assert _apart(t.as_strided(size, stride)) is want, (size, stride)

@@ -97,6 +97,38 @@ def test_attn_state_and_slices(dtype, monkeypatch):
         assert th.equal(g, w)
 
 
+def _layouts(t, B, T, HC):
+    """[B,T,HC] views of the flat tensor t: windows that overlap by half, one sequence expanded to a batch, time outside the batch."""
+    return {'windows': t.as_strided((B, T, HC), (T // 2 * HC, HC, 1)), 'expanded': t.as_strided((B, T, HC), (0, HC, 1)),
+            'sliding': t.as_strided((B, T, HC), (HC, HC, 1)), 'time first': t.as_strided((B, T, HC), (HC, B * HC, 1)),
+            'halves': t.as_strided((B, T, HC), (T * 2 * HC, 2 * HC, 1))}
+
+
+@pytest.mark.parametrize('form', ['c++', 'python'])
+@pytest.mark.parametrize('layout', ['windows', 'expanded', 'sliding', 'time first', 'halves'])
+def test_layouts(layout, form, monkeypatch):
+    """Inputs whose rows share memory or lie in another order give what their contiguous copies give, bit for bit."""
+    from wind_rwkv.rwkv7 import attn, attn_ln, attn_step, synthetic
+    B, T, H = 3, 32, 2
+    HC = H * N
+    flat = synthetic.wkv7_inputs(1, 2 * B * T, H, N, seed=6, dtype=th.bfloat16, device='cuda')
+    g, params = synthetic.attn_ln_extras(1, 2 * B * T, H, N, seed=6, dtype=th.bfloat16, device='cuda')
+    s0 = th.randn(B, H, N, N, device='cuda')
+    views = [_layouts(x, B, T, HC)[layout] for x in [flat[n] for n in 'rwkvab'] + [g]]
+
+    def run(ins):
+        ins = [i.detach().requires_grad_() for i in ins]
+        res = [o.detach() for o in attn_step(*ins[:6], N, s0)]
+        for outs in (attn(*ins[:6], N, s0=s0, return_state=True), attn_ln(*ins, params, N, s0=s0, return_state=True)):
+            res += [o.detach() for o in outs] + list(_grads(list(outs), ins if len(res) > 2 else ins[:6], 11))
+        return res
+
+    want = run([v.contiguous() for v in views])
+    got = run(views) if form == 'c++' else _python_form(monkeypatch, lambda: run(views))
+    for a, b in zip(got, want, strict=True):
+        assert th.equal(a, b)
+
+
 def _ops():
     """name -> (function, inputs) of every entry point with an autograd function, at small sizes."""
     from wind_rwkv.rwkv7 import TimeMixer, attn, attn_ln, ddlerp, expand_loras, synthetic

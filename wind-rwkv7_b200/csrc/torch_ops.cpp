@@ -57,7 +57,8 @@ template <typename F, size_t... I>
 auto apply_list(const variable_list& in, std::index_sequence<I...>) { return F::apply(in[I]...); }
 
 // ---- WKV7 ------------------------------------------------------------------------------------------
-// [B,T,H*64] tensors with one layout whose rows are whole and 16-byte aligned
+// [B,T,H*64] tensors with one layout whose rows are whole, 16-byte aligned and apart: outputs and gradients take the same layout, and
+// rows of windows or expanded batches that share memory would be written over one another
 struct Rows { int64_t B, T, H, sb, st; int io; };
 bool rows_of(std::initializer_list<const Tensor*> ts, Rows& r) {
     const Tensor& w = **ts.begin();
@@ -67,7 +68,9 @@ bool rows_of(std::initializer_list<const Tensor*> ts, Rows& r) {
     const int64_t per16 = dt == at::kBFloat16 ? 8 : 4;
     if (w.size(2) % N != 0 || w.size(0) == 0 || w.size(1) == 0 || w.size(2) == 0) return false;
     r = Rows{w.size(0), w.size(1), w.size(2) / N, w.stride(0), w.stride(1), dt == at::kBFloat16 ? WKV7_BF16 : WKV7_F32};
-    if (w.stride(2) != 1 || r.sb % per16 || r.st % per16 || r.st < w.size(2) || (r.B > 1 && r.sb < w.size(2))) return false;
+    if (w.stride(2) != 1 || r.sb % per16 || r.st % per16 || r.st < w.size(2)) return false;
+    const int64_t row = w.size(2);
+    if (r.B > 1 && r.sb < (r.T - 1) * r.st + row && (r.sb < row || r.st < (r.B - 1) * r.sb + row)) return false;  // [B][T] or [T][B] order
     for (const Tensor* t : ts)
         if (!plain(*t) || t->scalar_type() != dt || t->sizes() != w.sizes() || t->strides() != w.strides() || t->device() != w.device() ||
             (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15))

@@ -11,9 +11,20 @@ import torch as th
 from . import _lib
 
 
+def _apart(t):
+    """No two elements share memory (dimensions nested in some order): what a layout that outputs take over has to guarantee."""
+    span = 1
+    for stride, n in sorted((s, n) for s, n in zip(t.stride(), t.shape) if n > 1):
+        if stride < span:
+            return False
+        span += (n - 1) * stride
+    return True
+
+
 def _same_layout(ts):
+    """One layout that the kernels can read and the outputs can have."""
     s = ts[0].stride()
-    return all(t.stride() == s and t.stride(3) == 1 for t in ts)
+    return all(t.stride() == s and t.stride(3) == 1 for t in ts) and _apart(ts[0])
 
 
 def fw_attn(w, q, k, v, a, b, s0, save_checkpoints=True):
