@@ -139,6 +139,8 @@ def _ops():
     g, params = synthetic.attn_ln_extras(B, T, H, N, seed=4, dtype=th.bfloat16, device='cuda')
     x = th.randn(B, T, C, device='cuda').bfloat16()
     mixer = TimeMixer(types.SimpleNamespace(n_layer=4, n_head=H, n_embd=C), 1).cuda().requires_grad_(False)
+    for p in mixer.parameters():  # (the output projection starts at zero)
+        p.add_(0.05 * th.randn_like(p))
     rkv = [d[n] for n in 'rwkvab']
     par = [th.rand(C, device='cuda'), th.randn(4 * D, C, device='cuda'), th.randn(4, C, D, device='cuda'), th.rand(4, 1, 1, C, device='cuda')]
     lora = [x.flip(1)] + [th.randn(B, T, D, device='cuda').bfloat16() for _ in range(4)]
@@ -159,6 +161,19 @@ def test_forward_mode_raises(op):
                 dual = [fwd.make_dual(t.clone().requires_grad_(grad), th.ones_like(t)) if j == i else t for j, t in enumerate(ins)]
                 with pytest.raises((NotImplementedError, RuntimeError), match='jvp'):
                     f(*dual)
+
+
+@pytest.mark.filterwarnings('ignore')
+@pytest.mark.parametrize('op', ['attn', 'attn_ln', 'ddlerp', 'expand_loras', 'mixer'])
+def test_jit_trace_replays_on_other_inputs(op):
+    f, ins = _ops()[op]
+    other = [t.flip(0).contiguous() if t.dim() > 2 else t for t in ins]
+    with th.no_grad():
+        traced = th.jit.trace(f, tuple(ins), check_trace=False)
+        got, want = traced(*other), f(*other)
+    for a, b in zip(*[o if isinstance(o, (tuple, list)) else [o] for o in (got, want)], strict=True):
+        assert not th.equal(b, th.zeros_like(b))
+        _close(a, b, 2e-2 if op == 'mixer' else 0)  # (the traced layer is the Python form, see test_mixer)
 
 
 def test_cast():

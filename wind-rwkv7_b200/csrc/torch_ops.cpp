@@ -5,6 +5,7 @@
 //
 // A function here that returns None (nothing launched) leaves the call to the Python path: other dtypes, devices, shapes or layouts than the
 // ones below, with their conversions and error messages.
+#include <ATen/TracerMode.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -43,12 +44,13 @@ bool grad_wanted(std::initializer_list<const Tensor*> ts) {
         if (t->defined() && t->requires_grad()) return true;
     return false;
 }
-// a dense CUDA tensor of its own: no subclass or transform wrapper, whose meaning only the Python path's operators see, and no
-// forward-mode dual, for which the Python path's autograd functions raise
+// a dense CUDA tensor of its own: no subclass or transform wrapper, whose meaning only the Python path's operators see, no
+// forward-mode dual, for which the Python path's autograd functions raise, and not under torch.jit.trace, which records those
+// functions but would see nothing here besides allocations
 bool plain(const Tensor& t) {
     using c10::DispatchKey;
     const auto keys = t.key_set();
-    return t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !keys.has(DispatchKey::Python) && !keys.has(DispatchKey::FuncTorchGradWrapper) &&
+    return !at::tracer::impl::is_dispatch_enabled() && t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !keys.has(DispatchKey::Python) && !keys.has(DispatchKey::FuncTorchGradWrapper) &&
            !keys.has(DispatchKey::FuncTorchBatched) && !t._fw_grad(0).defined();
 }
 
