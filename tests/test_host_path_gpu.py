@@ -163,6 +163,32 @@ def test_forward_mode_raises(op):
                     f(*dual)
 
 
+class _Sub(th.Tensor):
+    seen = []
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        cls.seen.append(getattr(func, '__name__', ''))
+        return super().__torch_function__(func, types, args, kwargs)
+
+
+@pytest.mark.parametrize('op', ['attn', 'attn_ln', 'ddlerp', 'expand_loras', 'mixer'])
+def test_subclasses(op, monkeypatch):
+    """Subclasses of Tensor see the operators of the Python form, and outputs have the classes that it gives them."""
+    f, ins = _ops()[op]
+    for i in (0, len(ins) - 1):
+        args = [t.as_subclass(_Sub) if j == i else t for j, t in enumerate(ins)]
+
+        def run():
+            _Sub.seen.clear()
+            with th.no_grad():
+                out = f(*args)
+            return [type(o) for o in (out if isinstance(out, (tuple, list)) else [out])], list(_Sub.seen)
+
+        got, want = run(), _python_form(monkeypatch, run)
+        assert got == want and want[1]
+
+
 @pytest.mark.filterwarnings('ignore')
 @pytest.mark.parametrize('op', ['attn', 'attn_ln', 'ddlerp', 'expand_loras', 'mixer'])
 def test_jit_trace_replays_on_other_inputs(op):

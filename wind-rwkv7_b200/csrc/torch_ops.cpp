@@ -9,6 +9,7 @@
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/extension.h>
 
 #include "../../include/wkv7_sm100.h"
@@ -44,14 +45,36 @@ bool grad_wanted(std::initializer_list<const Tensor*> ts) {
         if (t->defined() && t->requires_grad()) return true;
     return false;
 }
-// a dense CUDA tensor of its own: no subclass or transform wrapper, whose meaning only the Python path's operators see, no
-// forward-mode dual, for which the Python path's autograd functions raise, and not under torch.jit.trace, which records those
-// functions but would see nothing here besides allocations
+// a dense CUDA tensor of its own: no transform wrapper, whose meaning only the Python path's operators see
 bool plain(const Tensor& t) {
     using c10::DispatchKey;
     const auto keys = t.key_set();
-    return !at::tracer::impl::is_dispatch_enabled() && t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !keys.has(DispatchKey::Python) && !keys.has(DispatchKey::FuncTorchGradWrapper) &&
-           !keys.has(DispatchKey::FuncTorchBatched) && !t._fw_grad(0).defined();
+    return t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !keys.has(DispatchKey::Python) && !keys.has(DispatchKey::FuncTorchGradWrapper) &&
+           !keys.has(DispatchKey::FuncTorchBatched);
+}
+
+// What an entry point asks first, with the GIL held (it looks at the Python objects).  The Python path has to run for Python subclasses
+// of Tensor, which see its operators; for forward-mode duals, for which its autograd functions raise; and under torch.jit.trace, which
+// records those functions but would see nothing here besides allocations.
+struct Eager {
+    // (asked tensor by tensor, the dual check costs a decode step 0.2 of its 6 us; there are no duals without a level)
+    const bool duals = torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr;
+    bool operator()(const Tensor& t) const {
+        PyObject* o = t.defined() ? t.unsafeGetTensorImpl()->pyobj_slot()->load_pyobj() : nullptr;
+        return !o || (THPVariable_CheckExact(o) && !(duals && t._fw_grad(0).defined()));
+    }
+};
+bool eager(std::initializer_list<const Tensor*> ts) {
+    const Eager ok;
+    for (const Tensor* t : ts)
+        if (!ok(*t)) return false;
+    return !at::tracer::impl::is_dispatch_enabled();
+}
+bool eager(const variable_list& ts) {
+    const Eager ok;
+    for (const Tensor& t : ts)
+        if (!ok(t)) return false;
+    return !at::tracer::impl::is_dispatch_enabled();
 }
 
 // F::apply on the first sizeof...(I) tensors of a list: autograd sees tensors that are arguments of their own, not those in a list
@@ -156,14 +179,14 @@ struct WkvFn : public Function<WkvFn> {
 py::object wkv(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b, const Tensor& g, const Tensor& params,
                const OptTensor& s0, bool return_state) {
     Rows q;
-    if (!rows_of({&w, &r, &k, &v, &a, &b}, q) || !state_ok(s0, q, w)) return py::none();
+    const Tensor st = s0.value_or(Tensor());
+    if (!eager({&r, &w, &k, &v, &a, &b, &g, &params, &st}) || !rows_of({&w, &r, &k, &v, &a, &b}, q) || !state_ok(s0, q, w)) return py::none();
     if (g.defined()) {
         if (!rows_of({&w, &g}, q)) return py::none();
         if (!plain(params) || params.scalar_type() != at::kFloat || !params.is_contiguous() || params.device() != w.device() || params.dim() != 2 ||
             params.size(0) != 3 || params.size(1) != q.H * N)
             return py::none();
     }
-    const Tensor st = s0 ? *s0 : Tensor();
     Tensor y, sT;
     {
         py::gil_scoped_release nogil;
@@ -193,15 +216,16 @@ py::object attn_ln(const Tensor& r, const Tensor& w, const Tensor& k, const Tens
 // decode: (y, state)
 py::object attn_step(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b, const OptTensor& state, bool inplace) {
     Rows q;
-    if (!rows_of({&w, &r, &k, &v, &a, &b}, q) || !state_ok(state, q, w)) return py::none();
+    const Tensor st = state.value_or(Tensor());
+    if (!eager({&r, &w, &k, &v, &a, &b, &st}) || !rows_of({&w, &r, &k, &v, &a, &b}, q) || !state_ok(state, q, w)) return py::none();
     Tensor y, sT;
     {
         py::gil_scoped_release nogil;
         const c10::cuda::CUDAGuard guard(w.device());
         at::NoGradGuard ng;
         y = like_rows(v);
-        sT = inplace && state && state->defined() ? *state : states(w, q);
-        check(wkv7_step(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), state && state->defined() ? f32(*state) : nullptr,
+        sT = inplace && st.defined() ? st : states(w, q);
+        check(wkv7_step(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), f32(st),
                         y.data_ptr(), f32(sT), q.B, q.T, q.H, N, q.sb, q.st, N, q.io, stream()), "wkv7_step");
     }
     return py::make_tuple(y, sT);
@@ -280,7 +304,7 @@ struct DdlerpFn : public Function<DdlerpFn> {
     }
 };
 py::object ddlerp(const Tensor& x, const Tensor& alpha, const Tensor& L, const Tensor& R, const Tensor& beta) {
-    if (!bf16_dense(x) || x.dim() != 3 || x.numel() == 0 || x.size(2) % 64 != 0) return py::none();
+    if (!eager({&x, &alpha, &L, &R, &beta}) || !bf16_dense(x) || x.dim() != 3 || x.numel() == 0 || x.size(2) % 64 != 0) return py::none();
     const int64_t C = x.size(2);
     for (const Tensor* t : {&alpha, &L, &R, &beta})
         if (!castable(*t, x.device())) return py::none();
@@ -373,7 +397,7 @@ struct LorasFn : public Function<LorasFn> {
 };
 py::object expand_loras(const variable_list& in) {
     const Tensor& w = in[0];
-    if (!bf16_dense(w) || w.dim() != 3 || w.numel() == 0 || w.size(2) % 64 != 0 || !bf16_dense(in[1]) || in[1].sizes() != w.sizes() || in[6].dim() != 2) return py::none();
+    if (!eager(in) || !bf16_dense(w) || w.dim() != 3 || w.numel() == 0 || w.size(2) % 64 != 0 || !bf16_dense(in[1]) || in[1].sizes() != w.sizes() || in[6].dim() != 2) return py::none();
     const int64_t C = w.size(2), D = in[6].size(1);
     int64_t ld[4];
     for (int i = 0; i < 4; ++i)
@@ -577,7 +601,7 @@ struct MixerFn : public Function<MixerFn> {
     }
 };
 py::object mixer(Tensor x, const variable_list& in) {
-    if (!plain(x) || x.dim() != 3 || x.numel() == 0 || x.size(2) % N != 0 || (int)in.size() != NPAR || at::autocast::is_autocast_enabled(at::kCUDA)) return py::none();
+    if (!eager({&x}) || !eager(in) || !plain(x) || x.dim() != 3 || x.numel() == 0 || x.size(2) % N != 0 || (int)in.size() != NPAR || at::autocast::is_autocast_enabled(at::kCUDA)) return py::none();
     if (x.scalar_type() != at::kBFloat16 && x.scalar_type() != at::kFloat) return py::none();
     const int64_t C = x.size(2);
     const std::array<std::vector<int64_t>, NPAR> shape{{{C, C}, {C, C}, {C, C}, {C, C}, {GATE, C}, {C, GATE}, {SMALL, C}, {SMALL, C}, {DEC, C}, {SMALL, C}, {SMALL, C},
