@@ -163,6 +163,41 @@ def test_forward_mode_raises(op):
                     f(*dual)
 
 
+@pytest.mark.parametrize('form', ['c++', 'python'])
+@pytest.mark.parametrize('op', ['attn', 'attn_ln', 'ddlerp', 'expand_loras', 'mixer'])
+def test_saved_tensors_come_back_in_other_layouts(op, form, monkeypatch):
+    """Hooks on saved tensors that hand back some with their dimensions stored in reverse order and (C++; the Python form lets the
+    library refuse them) some from a misaligned place in a buffer."""
+    f, ins = _ops()[op]
+
+    def run(order):
+        args = [t.detach().clone().requires_grad_() for t in ins]
+        if op == 'mixer':
+            f.requires_grad_()
+            args += list(f.parameters())
+        count = iter(range(order, 1000))
+
+        def unpack(t):
+            i = next(count) % 3 if order else None
+            if i == 0:
+                return t.permute(*reversed(range(t.dim()))).contiguous().permute(*reversed(range(t.dim())))
+            if i == 1 and form == 'c++':
+                return th.cat([t.new_zeros(3), t.reshape(-1)])[3:].view(t.shape)
+            return t
+
+        with th.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+            out = f(*args[:len(ins)])
+        return _grads(out if isinstance(out, (tuple, list)) else [out], args, 12)
+
+    def compare():
+        want = run(0)
+        for order in (1, 2, 3):
+            for a, b in zip(run(order), want, strict=True):
+                _close(a, b, 1e-5 if op in ('ddlerp', 'expand_loras', 'mixer') else 0)  # sums over rows by atomics
+
+    compare() if form == 'c++' else _python_form(monkeypatch, compare)
+
+
 class _Sub(th.Tensor):
     seen = []
 

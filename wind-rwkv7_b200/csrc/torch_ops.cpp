@@ -77,6 +77,13 @@ bool eager(const variable_list& ts) {
     return !at::tracer::impl::is_dispatch_enabled();
 }
 
+// A tensor whose elements lie back to back from a 16-byte boundary on.  Backward nodes ask it of what they have saved: hooks on
+// saved tensors hand back the same values, but in a layout of their own.
+Tensor dense(const Tensor& t) {
+    if (!t.defined() || (t.is_contiguous() && !(reinterpret_cast<uintptr_t>(t.data_ptr()) & 15))) return t;
+    return t.clone(at::MemoryFormat::Contiguous);
+}
+
 // F::apply on the first sizeof...(I) tensors of a list: autograd sees tensors that are arguments of their own, not those in a list
 template <typename F, size_t... I>
 auto apply_list(const variable_list& in, std::index_sequence<I...>) { return F::apply(in[I]...); }
@@ -85,6 +92,9 @@ auto apply_list(const variable_list& in, std::index_sequence<I...>) { return F::
 // [B,T,H*64] tensors with one layout whose rows are whole, 16-byte aligned and apart: outputs and gradients take the same layout, and
 // rows of windows or expanded batches that share memory would be written over one another
 struct Rows { int64_t B, T, H, sb, st; int io; };
+Rows rows(const Tensor& w) {
+    return Rows{w.size(0), w.size(1), w.size(2) / N, w.stride(0), w.stride(1), w.scalar_type() == at::kBFloat16 ? WKV7_BF16 : WKV7_F32};
+}
 bool rows_of(std::initializer_list<const Tensor*> ts, Rows& r) {
     const Tensor& w = **ts.begin();
     if (!plain(w) || w.dim() != 3) return false;
@@ -92,7 +102,7 @@ bool rows_of(std::initializer_list<const Tensor*> ts, Rows& r) {
     if (dt != at::kBFloat16 && dt != at::kFloat) return false;
     const int64_t per16 = dt == at::kBFloat16 ? 8 : 4;
     if (w.size(2) % N != 0 || w.size(0) == 0 || w.size(1) == 0 || w.size(2) == 0) return false;
-    r = Rows{w.size(0), w.size(1), w.size(2) / N, w.stride(0), w.stride(1), dt == at::kBFloat16 ? WKV7_BF16 : WKV7_F32};
+    r = rows(w);
     if (w.stride(2) != 1 || r.sb % per16 || r.st % per16 || r.st < w.size(2)) return false;
     const int64_t row = w.size(2);
     if (r.B > 1 && r.sb < (r.T - 1) * r.st + row && (r.sb < row || r.st < (r.B - 1) * r.sb + row)) return false;  // [B][T] or [T][B] order
@@ -113,8 +123,7 @@ Tensor states(const Tensor& like, const Rows& r) { return at::empty({r.B, r.H, N
 // forward; g, params defined: attn_ln.  Returns y, sT, checkpoints (undefined without save)
 variable_list wkv_forward(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b, const Tensor& g,
                           const Tensor& params, const Tensor& s0, bool save) {
-    Rows q;
-    rows_of({&w}, q);
+    const Rows q = rows(w);
     Tensor y = like_rows(v), sT = states(w, q), ck;
     if (save) ck = at::empty({wkv7_checkpoint_bytes(q.B, q.T, q.H, N) / 4}, sT.options());
     Tensor ws = scratch(w);
@@ -127,8 +136,13 @@ variable_list wkv_forward(const Tensor& r, const Tensor& w, const Tensor& k, con
     return {y, sT, ck};
 }
 // backward.  Returns dr, dw, dk, dv, da, db, ds0 (, dg, dparams)
-variable_list wkv_backward(Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Tensor b, Tensor g, const Tensor& params, const Tensor& ck, const Tensor& sT,
-                           Tensor dy, Tensor dsT) {
+variable_list wkv_backward(Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Tensor b, Tensor g, Tensor params, Tensor ck, Tensor sT, Tensor dy, Tensor dsT) {
+    Rows q;
+    if (!rows_of({&w, &r, &k, &v, &a, &b}, q) || (g.defined() && !rows_of({&w, &g}, q))) {
+        for (Tensor* t : {&r, &w, &k, &v, &a, &b, &g}) *t = dense(*t);
+        q = rows(w);
+    }
+    for (Tensor* t : {&params, &ck, &sT}) *t = dense(*t);
     if (!dy.defined()) dy = at::zeros_like(v);
     if (dy.scalar_type() != w.scalar_type()) dy = dy.to(w.scalar_type());
     if (dy.strides() != w.strides() || (reinterpret_cast<uintptr_t>(dy.data_ptr()) & 15)) {
@@ -137,8 +151,6 @@ variable_list wkv_backward(Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Ten
         dy = d;
     }
     if (dsT.defined()) dsT = dsT.to(at::kFloat).contiguous();
-    Rows q;
-    rows_of({&w}, q);
     Tensor dr = like_rows(w), dw = like_rows(w), dk = like_rows(w), dv = like_rows(w), da = like_rows(w), db = like_rows(w), ds0 = states(w, q);
     Tensor ws = at::empty({(g.defined() ? wkv7_attn_ln_bwd_ws_bytes : wkv7_bwd_ws_bytes)(q.B, q.T, q.H, N, q.io)}, w.options().dtype(at::kByte));
     const float* sTp = dsT.defined() ? f32(sT) : nullptr;
@@ -297,9 +309,10 @@ struct DdlerpFn : public Function<DdlerpFn> {
         return y.unbind(0);
     }
     static variable_list backward(AutogradContext* ctx, variable_list go) {
-        const variable_list s = ctx->get_saved_variables();
+        variable_list s = ctx->get_saved_variables();
         const c10::cuda::CUDAGuard guard(s[0].device());
         at::NoGradGuard ng;
+        for (Tensor& t : s) t = dense(t);
         return ddlerp_backward(s[0], {s[1], s[2], s[3], s[4]}, s[5], dense_bf16(go[0], s[0]), dense_bf16(go[1], s[0]), dense_bf16(go[2], s[0]), dense_bf16(go[3], s[0]));
     }
 };
@@ -381,13 +394,19 @@ struct LorasFn : public Function<LorasFn> {
         const variable_list s = ctx->get_saved_variables();
         const c10::cuda::CUDAGuard guard(s[0].device());
         at::NoGradGuard ng;
-        const variable_list a(s.begin(), s.begin() + 6);
-        const std::vector<Tensor> p(s.begin() + 6, s.end());
+        variable_list a(s.begin(), s.begin() + 6);
+        std::vector<Tensor> p(s.begin() + 6, s.end());
+        for (Tensor& t : p) t = dense(t);
+        a[0] = dense(a[0]);
+        a[1] = dense(a[1]);
         const int64_t B = a[0].size(0), T = a[0].size(1), D = p[0].size(1);
         int64_t ld[4];
         variable_list d, da;
         for (int i = 0; i < 4; ++i) {
-            pitched(a[2 + i], B, T, D, ld + i);
+            if (!pitched(a[2 + i], B, T, D, ld + i)) {
+                a[2 + i] = dense(a[2 + i]);
+                ld[i] = D;
+            }
             d.push_back(dense_bf16(go[i], a[0]));
             da.push_back(at::empty({B, T, D}, a[0].options()));
         }
@@ -513,8 +532,8 @@ struct Mixer {
     explicit Mixer(const variable_list& s) {
         Tensor* f[] = {&params, &kkmk_w, &wam_w, &m, &y4, &r, &g1, &g, &k0, &kkmk, &v, &wam, &w2, &w, &k, &kk, &b, &y, &sT, &ck};
         size_t i = 0;
-        for (Tensor* t : f) *t = s[i++];
-        p.assign(s.begin() + i, s.end());
+        for (Tensor* t : f) *t = dense(s[i++]);
+        for (; i < s.size(); ++i) p.push_back(dense(s[i]));
         B = r.size(0); T = r.size(1); C = r.size(2);
     }
     Mixer() = default;
@@ -593,7 +612,7 @@ struct MixerFn : public Function<MixerFn> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list go) {
         variable_list s = ctx->get_saved_variables();
-        const Tensor x = s.back();
+        const Tensor x = dense(s.back());
         s.pop_back();
         const c10::cuda::CUDAGuard guard(x.device());
         at::NoGradGuard ng;

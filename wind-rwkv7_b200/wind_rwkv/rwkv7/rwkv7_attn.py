@@ -55,6 +55,7 @@ def bw_attn(w, q, k, v, a, b, s, dy, dsT, sT):
     B, T, H, C = w.shape
     if not _same_layout([w, q, k, v, a, b, dy]):
         w, q, k, v, a, b, dy = [i.contiguous() for i in (w, q, k, v, a, b, dy)]
+    s, sT = s.contiguous(), sT.contiguous()  # (hooks on saved tensors may hand back other layouts)
     dw, dq, dk, dv, da, db = [th.empty_strided(w.shape, w.stride(), dtype=w.dtype, device=w.device) for _ in range(6)]
     ds0 = th.empty(B, H, C, C, dtype=th.float32, device=w.device)
     sb, st, sh = _lib.strides4(w)

@@ -37,6 +37,7 @@ def bw_attn_ln(w, q, k, v, a, b, g, params, s, dy, dsT, sT):
     B, T, H, C = w.shape
     if not _same_layout([w, q, k, v, a, b, g, dy]):
         w, q, k, v, a, b, g, dy = [i.contiguous() for i in (w, q, k, v, a, b, g, dy)]
+    params, s, sT = params.contiguous(), s.contiguous(), sT.contiguous()  # (hooks on saved tensors may hand back other layouts)
     dw, dq, dk, dv, da, db, dg = [th.empty_strided(w.shape, w.stride(), dtype=w.dtype, device=w.device) for _ in range(7)]
     dparams = th.empty(3, H * C, dtype=th.float32, device=w.device)
     ws = th.empty(B, 3, H * C, dtype=th.float32, device=w.device)

@@ -82,7 +82,7 @@ class DDLerp(th.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy0, dy1, dy2, dy3):
-        x, ab, Lb, Rb, bb, m = ctx.saved_tensors
+        x, ab, Lb, Rb, bb, m = [i.contiguous() for i in ctx.saved_tensors]  # (hooks on saved tensors may hand back other layouts)
         dys = [th.zeros_like(x) if d is None else d.to(th.bfloat16).contiguous() for d in (dy0, dy1, dy2, dy3)]
         dx, dalpha, dL, dR, dbeta = _lib.call(_bw_op, bw_ddlerp, x, ab, Lb, Rb, bb, m, *dys)
         ta, tL, tR, tb = ctx.param_dtypes

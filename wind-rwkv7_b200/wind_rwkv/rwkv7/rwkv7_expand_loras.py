@@ -80,7 +80,7 @@ class ExpandLoras(th.autograd.Function):
 
     @staticmethod
     def backward(ctx, dw_out, dk_out, dz_out, db_out):
-        saved = ctx.saved_tensors
+        saved = [i.contiguous() for i in ctx.saved_tensors]  # (hooks on saved tensors may hand back other layouts)
         douts = [None if d is None else d.to(th.bfloat16) for d in (dw_out, dk_out, dz_out, db_out)]
         douts = [th.zeros_like(saved[0]) if d is None else d.contiguous() for d in douts]
         grads = _lib.call(_bw_op, bw_loras, *saved, *douts)
