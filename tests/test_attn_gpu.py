@@ -395,6 +395,46 @@ def test_time_split_forward(nseg):
     assert _lib.device_status() == 0
 
 
+def _long_memory(d, dtype):
+    """The same inputs with decays of e^-0.0009 to e^-0.007 a step (RWKV-7's slow channels): a segment's end depends on its start."""
+    d['w'] = (d['w'].float() * 0.5 - 5.7).to(dtype)
+    return [d[n] for n in NAMES]
+
+
+@pytest.mark.parametrize('dtype', [th.float32, th.bfloat16])
+@pytest.mark.parametrize('nseg', [2, 8])
+def test_time_split_with_long_memory(nseg, dtype):
+    """time_split where the maps of the segments matter (at the other tests' decays a segment has forgotten its start): against
+    the oracle, within the bounds of the uncut call; the process's TF32 setting is neither used nor touched."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    c_oracle, _lib, attn, synthetic, _ = _mods()
+    B, T, H = 2, 1024, 3
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=33, dtype=dtype, device='cuda', s0_std=1.0)
+    ins = _long_memory(d, dtype)
+    seen = set()
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.add(th.backends.cuda.matmul.allow_tf32)
+            return func(*args, **(kwargs or {}))
+
+    old = th.backends.cuda.matmul.allow_tf32
+    th.backends.cuda.matmul.allow_tf32 = True
+    try:
+        with th.no_grad(), Watch():
+            y, sT = attn(*ins, N, s0=d['s0'], return_state=True, time_split=nseg)
+    finally:
+        th.backends.cuda.matmul.allow_tf32 = old
+    assert seen == {True}
+    cpu = [x.double().cpu().numpy().reshape(B, T, H, N) for x in ins]
+    yo, sTo = c_oracle.wkv7_fwd(*cpu, s0=d['s0'].double().cpu().numpy())
+    yz, sTz = c_oracle.wkv7_fwd(*cpu)
+    assert np.linalg.norm(yo - yz) > 0.01 * np.linalg.norm(yo)  # the start state reaches through the segments
+    check('y', y.view(B, T, H, N), yo, dtype)
+    assert maxabs_rms(sT, sTo) <= (1e-4 if dtype == th.float32 else 2e-2)
+    assert _lib.device_status() == 0
+
+
 def test_tail_split_forward():
     """attn(..., time_split='tail'): the chains of the last, partly filled round of SMs are cut in time, the others run
     as usual, all into views of one output.  Against the unsplit call on every chain (they differ only on the split

@@ -140,6 +140,17 @@ def load_attn(HEAD_SIZE):
     _lib.lib()
 
 
+def _segment_starts(S, M, R):
+    """fp32 states at the starts of the segments, S_{j+1} = S_j M_j + R_j, the products in 64 bits: fp32 ones would depend on the
+    process's TF32 setting, and the states of sequences that forget slowly are sums over many segments."""
+    S = S.double()
+    starts = [S]
+    for m, r in zip(M[:-1], R[:-1]):
+        S = S @ m.double() + r.double()
+        starts.append(S)
+    return [s.float() for s in starts]
+
+
 def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
     """Forward only, the sequence cut into `nseg` equal segments that run as separate chains (for B*H far below the
     number of SMs: one CTA walks one chain, so a single long sequence otherwise occupies H SMs).
@@ -184,17 +195,8 @@ def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
     main.wait_stream(side)
     for t in insM + [M]:
         t.record_stream(main)
-    R, M = R.view(B, nseg, H, C, C), M.view(B, nseg, H, C, C)
-    S = th.zeros(B, H, C, C, dtype=th.float32, device=dev) if s0 is None else s0.float()
-    starts = [S]
-    prev = th.backends.cuda.matmul.allow_tf32
-    th.backends.cuda.matmul.allow_tf32 = False
-    try:
-        for j in range(nseg - 1):
-            S = S @ M[:, j] + R[:, j]
-            starts.append(S)
-    finally:
-        th.backends.cuda.matmul.allow_tf32 = prev
+    S = th.zeros(B, H, C, C, dtype=th.float32, device=dev) if s0 is None else s0
+    starts = _segment_starts(S, M.view(B, nseg, H, C, C).unbind(1), R.view(B, nseg, H, C, C).unbind(1))
     y, sT, _ = fw_attn(*ins, th.stack(starts, 1).reshape(B * nseg, H, C, C).contiguous(), save_checkpoints=False)
     return y.view(B, T, HC), sT.view(B, nseg, H, C, C)[:, -1].contiguous()
 
@@ -287,15 +289,7 @@ def _attn_tail_split(r, w, k, v, a, b, C, s0):
         R = _fw_into(*sin, None, sy)
         M = _fw_into(*sin, eye, sy) - R
         S = th.zeros(tail, C, C, dtype=th.float32, device=dev) if s0 is None else s0[B - 1, h0:]
-        starts = [S]
-        prev = th.backends.cuda.matmul.allow_tf32
-        th.backends.cuda.matmul.allow_tf32 = False
-        try:
-            for j in range(n - 1):
-                S = S @ M[j] + R[j]
-                starts.append(S)
-        finally:
-            th.backends.cuda.matmul.allow_tf32 = prev
+        starts = _segment_starts(S, M.unbind(0), R.unbind(0))
         sT[B - 1, h0:] = _fw_into(*sin, th.stack(starts, 0).contiguous(), sy)[-1]
     if B > 1:  # whole batch entries
         sT[:B - 1] = _fw_into(*[i[:B - 1] for i in ins], None if s0 is None else s0[:B - 1].contiguous(), y[:B - 1])
