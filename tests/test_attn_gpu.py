@@ -435,20 +435,26 @@ def test_time_split_with_long_memory(nseg, dtype):
     assert _lib.device_status() == 0
 
 
-def test_tail_split_forward():
+@pytest.mark.parametrize('dtype', [th.bfloat16, th.float32])
+def test_tail_split_forward(dtype, fwd_impl):
     """attn(..., time_split='tail'): the chains of the last, partly filled round of SMs are cut in time, the others run
-    as usual, all into views of one output.  Against the unsplit call on every chain (they differ only on the split
+    as usual, all into views of one output (fp32 tensors, and bf16 ones with the warp-MMA forward; the tcgen05 forward has no
+    such round and its call is the plain one).  Against the unsplit call on every chain (they differ only on the split
     chains, by the rounding of M) and against the oracle on the last batch entry (which holds the split heads and,
     next to them, plainly run ones).  Without such a tail the call is the plain forward."""
     c_oracle, _lib, attn, synthetic, _ = _mods()
     from wind_rwkv.rwkv7.rwkv7_attn import tail_split_plan
+    if dtype == th.float32 and fwd_impl == 0:
+        pytest.skip('fp32 tensors ignore fwd_impl')
+    cut = dtype == th.float32 or fwd_impl == 0
+    bound = 1e-4 if dtype == th.float32 else 2e-2
     sms = th.cuda.get_device_properties(0).multi_processor_count
     H, T = 40, 8192                        # (the split only pays for long sequences: tail_split_plan declines T = 1024)
     B = sms // H + 1                       # one round of SMs and a few heads of the last batch entry
     plan = tail_split_plan(B, T, H, sms)
     assert plan is not None and plan[0] == B * H - sms
-    d = synthetic.wkv7_inputs(B, T, H, N, seed=41, dtype=th.bfloat16, device='cuda', s0_std=0.1)
-    ins = [d[n] for n in NAMES]
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=41, dtype=dtype, device='cuda', s0_std=0.1)
+    ins = _long_memory(d, dtype)
     with th.no_grad():
         y, sT = attn(*ins, N, s0=d['s0'], return_state=True, time_split='tail')
         y1, sT1 = attn(*ins, N, s0=d['s0'], return_state=True)
@@ -457,14 +463,15 @@ def test_tail_split_forward():
     y4, y14 = y.view(B, T, H, N), y1.view(B, T, H, N)
     assert th.equal(y4[:B - 1], y14[:B - 1]) and th.equal(y4[B - 1, :, :h0], y14[B - 1, :, :h0])   # plainly run chains: same kernel, same inputs
     assert th.equal(sT[:B - 1], sT1[:B - 1]) and th.equal(sT[B - 1, :h0], sT1[B - 1, :h0])
+    assert th.equal(sT, sT1) != cut        # the split chains did run as segments, or nothing did
     hs = slice(h0 - 2, H)                  # two plainly run heads and the split ones
     cpu = [x.view(B, T, H, N)[B - 1:, :, hs].double().cpu().numpy() for x in ins]
     yo, sTo = c_oracle.wkv7_fwd(*cpu, s0=d['s0'][B - 1:, hs].double().cpu().numpy())
-    check('y', y4[B - 1:, :, hs], yo, th.bfloat16)
-    assert maxabs_rms(sT[B - 1:, hs], sTo) <= 2e-2
-    assert maxabs_rms(sT[B - 1:, h0:], sT1[B - 1:, h0:].double().cpu().numpy()) <= 2e-2
+    check('y', y4[B - 1:, :, hs], yo, dtype)
+    assert maxabs_rms(sT[B - 1:, hs], sTo) <= bound
+    assert maxabs_rms(sT[B - 1:, h0:], sT1[B - 1:, h0:].double().cpu().numpy()) <= bound
     # no tail: plain forward, bit for bit
-    d = synthetic.wkv7_inputs(2, 256, 3, N, seed=42, dtype=th.bfloat16, device='cuda')
+    d = synthetic.wkv7_inputs(2, 256, 3, N, seed=42, dtype=dtype, device='cuda')
     ins = [d[n] for n in NAMES]
     with th.no_grad():
         assert th.equal(attn(*ins, N, time_split='tail'), attn(*ins, N))

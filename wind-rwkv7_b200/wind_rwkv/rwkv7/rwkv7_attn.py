@@ -141,14 +141,14 @@ def load_attn(HEAD_SIZE):
 
 
 def _segment_starts(S, M, R):
-    """fp32 states at the starts of the segments, S_{j+1} = S_j M_j + R_j, the products in 64 bits: fp32 ones would depend on the
-    process's TF32 setting, and the states of sequences that forget slowly are sums over many segments."""
-    S = S.double()
-    starts = [S]
-    for m, r in zip(M[:-1], R[:-1]):
-        S = S @ m.double() + r.double()
-        starts.append(S)
-    return [s.float() for s in starts]
+    """fp32 states [n, ..., C, C] at the starts of n segments with maps M and R of that shape, S_{j+1} = S_j M_j + R_j.  In 64 bits:
+    fp32 products would depend on the process's TF32 setting, and the states of sequences that forget slowly are sums over many segments."""
+    C = S.shape[-1]
+    S64, M64, R64 = S.double().reshape(-1, C, C), M.double().reshape(len(M), -1, C, C), R.double().reshape(len(M), -1, C, C)
+    starts = [S64]
+    for m, r in zip(M64[:-1], R64[:-1]):
+        starts.append(th.baddbmm(r, starts[-1], m))
+    return th.stack(starts).float().view(M.shape)
 
 
 def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
@@ -196,8 +196,8 @@ def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
     for t in insM + [M]:
         t.record_stream(main)
     S = th.zeros(B, H, C, C, dtype=th.float32, device=dev) if s0 is None else s0
-    starts = _segment_starts(S, M.view(B, nseg, H, C, C).unbind(1), R.view(B, nseg, H, C, C).unbind(1))
-    y, sT, _ = fw_attn(*ins, th.stack(starts, 1).reshape(B * nseg, H, C, C).contiguous(), save_checkpoints=False)
+    starts = _segment_starts(S, M.view(B, nseg, H, C, C).transpose(0, 1), R.view(B, nseg, H, C, C).transpose(0, 1))
+    y, sT, _ = fw_attn(*ins, starts.transpose(0, 1).reshape(B * nseg, H, C, C).contiguous(), save_checkpoints=False)
     return y.view(B, T, HC), sT.view(B, nseg, H, C, C)[:, -1].contiguous()
 
 
@@ -254,8 +254,7 @@ def _tail_streams(dev):
 
 def _attn_tail_split(r, w, k, v, a, b, C, s0):
     """Forward only.  All chains but those of the last, partly filled round of SMs run as usual; the rest are cut in
-    time (see tail_split_plan and _attn_time_split; here M comes from a pass that starts at the identity state with
-    the real inputs, S_end = M + R, so no zero copy of v is needed).  The three groups of launches go to three
+    time (see tail_split_plan and _attn_time_split).  The three groups of launches go to three
     streams, write into views of one output tensor (head slices of the last batch entry, no copies) and share the
     SMs.  Falls back to the plain call when the shape gives no such tail, and for bf16 tensors, whose kernel needs none of this."""
     B, T, HC = w.shape
@@ -286,11 +285,14 @@ def _attn_tail_split(r, w, k, v, a, b, C, s0):
             return x.as_strided((n, Ts, tail, C), (Ts * HC, HC, C, 1), x[B - 1, 0, h0, 0].storage_offset())
         sin, sy = [seg(i) for i in ins], seg(y)
         eye = th.eye(C, dtype=th.float32, device=dev).expand(n, tail, C, C).contiguous()
+        # v = 0 for M, in the layout of the other inputs (as a difference of two passes with v it would carry R's rounding errors,
+        # which are as large as M itself where the state is large)
+        sinM = list(sin)
+        sinM[3] = seg(th.zeros(1, T, H, C, dtype=w.dtype, device=dev).expand(B, T, H, C))
         R = _fw_into(*sin, None, sy)
-        M = _fw_into(*sin, eye, sy) - R
+        M = _fw_into(*sinM, eye, sy)
         S = th.zeros(tail, C, C, dtype=th.float32, device=dev) if s0 is None else s0[B - 1, h0:]
-        starts = _segment_starts(S, M.unbind(0), R.unbind(0))
-        sT[B - 1, h0:] = _fw_into(*sin, th.stack(starts, 0).contiguous(), sy)[-1]
+        sT[B - 1, h0:] = _fw_into(*sin, _segment_starts(S, M, R), sy)[-1]
     if B > 1:  # whole batch entries
         sT[:B - 1] = _fw_into(*[i[:B - 1] for i in ins], None if s0 is None else s0[:B - 1].contiguous(), y[:B - 1])
     if h0 > 0:  # the last entry's heads that still fit the full rounds
