@@ -238,6 +238,30 @@ def test_strong_decay(fwd_impl):
             assert maxabs_rms(y.view(B, T, H, N), yo) <= 5e-3 and maxabs_rms(sT, sTo) <= 5e-3   # measured 2e-3
 
 
+@pytest.mark.parametrize('w_mean,w_std,b_scale', [(-5, 0.25, 1.0), (-7, 0.25, 1.0), (-7, 0.0, 1.0), (-7, 0.25, 0.1), (-9, 0.0, 0.3)])
+def test_slow_decay(w_mean, w_std, b_scale):
+    """States that last for 150 to several thousand steps (RWKV-7's slow channels start near w = -7), decays constant in time among
+    them, little removed by a and b: nothing may add up over the chunks.  The usual bounds, forward and backward."""
+    c_oracle, _lib, attn, synthetic, _ = _mods()
+    B, T, H = 1, 4096, 2
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=14, dtype=th.bfloat16, device='cuda', s0_std=0.1)
+    level = w_mean + 0.3 * th.randn(H * N, generator=th.Generator('cuda').manual_seed(15), device='cuda')
+    d['w'] = ((d['w'].float() + 0.6) * 2 * w_std + level).bfloat16()
+    d['b'] = (d['b'].float() * b_scale).bfloat16()
+    ins = [d[n].requires_grad_() for n in NAMES]
+    y, sT = attn(*ins, N, s0=d['s0'], return_state=True)
+    grads = th.autograd.grad(y, ins, d['dy'])
+    cpu = [x.detach().double().cpu().numpy().reshape(B, T, H, N) for x in ins + [d['dy']]]
+    s0 = d['s0'].double().cpu().numpy()
+    yo, sTo = c_oracle.wkv7_fwd(*cpu[:6], s0=s0)
+    go = c_oracle.wkv7_bwd(*cpu[:6], cpu[6], s0=s0)
+    check('y', y, yo, th.bfloat16)
+    assert maxabs_rms(sT, sTo) <= 2e-2
+    for n, x, ref in zip(NAMES, grads, go):
+        check('d' + n, x, ref, th.bfloat16)
+    assert _lib.device_status() == 0
+
+
 def test_bounded_wait_gives_up_and_reports(fwd_impl):
     """A device-side wait that can never be satisfied runs out after its limit, raises the CTA's abort
     flag (later waits return at once), leaves WKV7_ERR_DEVICE_TIMEOUT in the status word and the
