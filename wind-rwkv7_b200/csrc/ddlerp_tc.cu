@@ -157,15 +157,17 @@ __global__ void __launch_bounds__(g1::THREADS) ddlerp_gemm1_kernel(const __grid_
 
     if (warp == 4) {
         if (elect_one()) {
-            for (int kb = 0; kb < nkb; ++kb) {
+            int kb = 0;
+            for (; kb < nkb; ++kb) {
                 const int s = kb % STAGES, round = kb / STAGES;
-                if (round > 0) mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status);
+                if (round > 0 && !mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status)) break;
                 const uint32_t dst = smem_u32(sm + s * STAGE_BYTES);
                 mbar_expect(&ctrl->full[s], (uint32_t)STAGE_BYTES);
                 const bool prev = kb >= nkh;
                 tma_load_3d(dst, &mapX, &ctrl->full[s], (prev ? kb - nkh : kb) * BK, prev ? t0 - 1 : t0, bi);
                 tma_load_2d(dst + A_BYTES, &mapW, &ctrl->full[s], kb * BK, n0);
             }
+            ring_landed<STAGES>(ctrl->full, kb, &ctrl->zero, status);
         }
         __syncwarp();
     } else if (warp == 5) {
@@ -297,16 +299,18 @@ __global__ void __launch_bounds__(g2::THREADS, 1) ddlerp_lerp_kernel(const __gri
     if (warp == EPI_WARPS) {
         if (elect_one()) {
             int mslot = 1, mtile = -1;   // m buffer and token tile of the unit whose loads were issued last
+            int units_loaded = 0, m_loaded = 0;
             auto issue_loads = [&](int n) {
                 const int u = u_lo + n, s = n & 1;
                 const int cb = u % ncb, tile = u / ncb, t0 = (tile % tiles_per_seq) * BM, bi = tile / tiles_per_seq;
                 unsigned char* st = smSt + s * stage_bytes(D);
                 if (tile != mtile) {  // the buffer's previous tile was read by products that completed before the stage_free wait
-                    mtile = tile; mslot ^= 1;
+                    mtile = tile; mslot ^= 1; ++m_loaded;
                     mbar_expect(&ctrl->mfull[mslot], (uint32_t)m_bytes(D));
 #pragma unroll
                     for (int kb = 0; kb < KB; ++kb) tma_load_3d(smem_u32(sm + mslot * m_bytes(D) + kb * (BM * 128)), &mapM, &ctrl->mfull[mslot], kb * 64, t0, bi);
                 }
+                ++units_loaded;
                 mbar_expect(&ctrl->ops[s], (uint32_t)r_bytes(D));
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) tma_load_2d(smem_u32(st + kb * (BN * 128)), &mapR, &ctrl->ops[s], kb * 64, cb * BN);
@@ -320,14 +324,14 @@ __global__ void __launch_bounds__(g2::THREADS, 1) ddlerp_lerp_kernel(const __gri
                 const bool tile_first = n == 0 || (u_lo + n - 1) / ncb != (u_lo + n) / ncb;  // buffers alternate from tile to tile, as in issue_loads
                 if (tile_first) cur_slot ^= 1;
                 if (n + 1 < nmine) {  // the other stage was last used by unit n - 1
-                    if (n >= 1) mbar_wait_bounded<true>(&ctrl->stage_free[s ^ 1], ((n - 1) >> 1) & 1, &ctrl->abort, status);
+                    if (n >= 1 && !mbar_wait_bounded<true>(&ctrl->stage_free[s ^ 1], ((n - 1) >> 1) & 1, &ctrl->abort, status)) break;
                     issue_loads(n + 1);
                 }
                 if (tile_first) {  // its m tile must have landed: load number waited + 1 of this buffer
-                    mbar_wait_bounded<false>(&ctrl->mfull[cur_slot], waited[cur_slot] & 1, &ctrl->abort, status);
+                    if (!mbar_wait_bounded<false>(&ctrl->mfull[cur_slot], waited[cur_slot] & 1, &ctrl->abort, status)) break;
                     ++waited[cur_slot];
                 }
-                mbar_wait_bounded<false>(&ctrl->ops[s], (n >> 1) & 1, &ctrl->abort, status);
+                if (!mbar_wait_bounded<false>(&ctrl->ops[s], (n >> 1) & 1, &ctrl->abort, status)) break;
                 if (n >= 2) mbar_wait_bounded<true>(&ctrl->acc_free[s], ((n - 2) >> 1) & 1, &ctrl->abort, status);  // set s was last read for unit n - 2
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 unsigned char* st = smSt + s * stage_bytes(D);
@@ -343,6 +347,9 @@ __global__ void __launch_bounds__(g2::THREADS, 1) ddlerp_lerp_kernel(const __gri
                 }
                 tc_commit(&ctrl->accum[s]);
             }
+            ring_landed<2>(ctrl->mfull, m_loaded, &ctrl->zero, status);
+            ring_landed<2>(ctrl->ops, units_loaded, &ctrl->zero, status);
+            ring_landed<2>(ctrl->xs, units_loaded, &ctrl->zero, status);
             if (ctrl->abort) drain_products(&ctrl->drain, &ctrl->zero, status);
         }
         __syncwarp();
@@ -496,10 +503,11 @@ __global__ void __launch_bounds__(g3::THREADS) ddlerp_dw12_kernel(const __grid_c
 
     if (warp == 4) {
         if (elect_one()) {
-            for (int i = lo; i < hi; ++i) {
+            int i = lo;
+            for (; i < hi; ++i) {
                 const int n = i - lo, s = n % STAGES, round = n / STAGES;
                 const int t0 = (i % tiles_per_seq) * BM, bi = i / tiles_per_seq;
-                if (round > 0) mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status);
+                if (round > 0 && !mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status)) break;
                 const uint32_t dst = smem_u32(sm + s * STAGE_BYTES);
                 mbar_expect(&ctrl->full[s], (uint32_t)STAGE_BYTES);
 #pragma unroll
@@ -507,6 +515,7 @@ __global__ void __launch_bounds__(g3::THREADS) ddlerp_dw12_kernel(const __grid_c
 #pragma unroll
                 for (int b = 0; b < BN / 64; ++b) tma_load_3d(dst + A_BYTES + b * (BM * 128), &mapX, &ctrl->full[s], c0 + 64 * b, t0 - half, bi);
             }
+            ring_landed<STAGES>(ctrl->full, i - lo, &ctrl->zero, status);
         }
         __syncwarp();
     } else if (warp == 5) {
@@ -647,9 +656,10 @@ __global__ void __launch_bounds__(g4::THREADS, 1) ddlerp_dpre_tc_kernel(const __
 
     if (warp == 8) {
         if (elect_one()) {
-            for (int cb = 0; cb < ncb; ++cb) {
+            int cb = 0;
+            for (; cb < ncb; ++cb) {
                 const int s = cb % STAGES, round = cb / STAGES;
-                if (round > 0) mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status);
+                if (round > 0 && !mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status)) break;
                 const uint32_t dst = smem_u32(sm + s * stage_bytes(D));
                 mbar_expect(&ctrl->full[s], (uint32_t)(4 * DY_BYTES + (BM + 1) * 128 + rt_bytes(D)));
 #pragma unroll
@@ -657,6 +667,7 @@ __global__ void __launch_bounds__(g4::THREADS, 1) ddlerp_dpre_tc_kernel(const __
                 tma_load_3d(dst + 4 * DY_BYTES, &mapX, &ctrl->full[s], cb * 64, t0 - 1, bi);   // row r: x_{t0 + r - 1}; before the sequence: zeros
                 tma_load_2d(dst + 4 * DY_BYTES + X_BYTES, &mapRt, &ctrl->full[s], cb * 64, 0);
             }
+            ring_landed<STAGES>(ctrl->full, cb, &ctrl->zero, status);
         }
         __syncwarp();
     } else if (warp == 9) {
@@ -841,24 +852,26 @@ __global__ void __launch_bounds__(g5::THREADS, 1) ddlerp_main_tc_kernel(const __
 
     if (warp == EPI_WARPS) {
         if (elect_one()) {
-            int cb_prev = -1, nw = 0;
+            int cb_prev = -1, nw = 0, na = 0, nx = 0, nf = 0;  // loads issued: weights, dpre, x, m and dy
             // The dpre tile is only read by products 1 and the x tile only by the epilogue's first phase: the next unit's copies
             // of the two are requested as soon as those are done, ahead of the m and dy tiles, which products 2 still read.
             auto load_dpre = [&](int n) {
                 const int tile = (u_lo + n) % tiles, t0 = (tile % tiles_per_seq) * BM, bi = tile / tiles_per_seq;
+                ++na;
                 mbar_expect(&ctrl->full_a, (uint32_t)(KB * TILE));
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) tma_load_3d(sb + kb * TILE, &maps.dpre, &ctrl->full_a, kb * 64, t0, bi);
             };
             auto load_x = [&](int n) {
                 const int u = u_lo + n, cb = u / tiles, tile = u % tiles, t0 = (tile % tiles_per_seq) * BM, bi = tile / tiles_per_seq;
+                ++nx;
                 mbar_expect(&ctrl->full_x, (uint32_t)((BM + 1) * 128));
                 tma_load_3d(sb + off_x(D), &maps.x, &ctrl->full_x, cb * 64, t0 - 1, bi);
             };
             if (nmine > 0) { load_dpre(0); load_x(0); }
             for (int n = 0; n < nmine; ++n) {
                 const int u = u_lo + n, cb = u / tiles, tile = u % tiles, t0 = (tile % tiles_per_seq) * BM, bi = tile / tiles_per_seq;
-                if (n > 0) mbar_wait_bounded<true>(&ctrl->unit_free, (n - 1) & 1, &ctrl->abort, status);  // products 2 of the previous unit have read the tiles
+                if (n > 0 && !mbar_wait_bounded<true>(&ctrl->unit_free, (n - 1) & 1, &ctrl->abort, status)) break;  // products 2 of the previous unit have read the tiles
                 if (cb != cb_prev) {
                     // the weights may be replaced as soon as the previous unit's products are complete (unit_free)
                     cb_prev = cb; ++nw;
@@ -869,19 +882,23 @@ __global__ void __launch_bounds__(g5::THREADS, 1) ddlerp_main_tc_kernel(const __
                         tma_load_2d(sb + off_rp(D) + kb * 64 * 128, &maps.rp, &ctrl->wfull, kb * 64, cb * 64);
                     }
                 }
+                ++nf;
                 mbar_expect(&ctrl->full, (uint32_t)(KB * TILE + 4 * TILE));
 #pragma unroll
                 for (int kb = 0; kb < KB; ++kb) tma_load_3d(sb + off_m(D) + kb * TILE, &maps.m, &ctrl->full, kb * 64, t0, bi);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) tma_load_3d(sb + off_dy(D) + k * TILE, &maps.dy[k], &ctrl->full, cb * 64, t0, bi);
                 if (n + 1 < nmine) {
-                    mbar_wait_bounded<true>(&ctrl->acc1, n & 1, &ctrl->abort, status);       // products 1 of this unit have read the dpre tile
+                    if (!mbar_wait_bounded<true>(&ctrl->acc1, n & 1, &ctrl->abort, status)) break;      // products 1 of this unit have read the dpre tile
                     load_dpre(n + 1);
-                    mbar_wait_bounded<true>(&ctrl->dz_ready, n & 1, &ctrl->abort, status);   // every epilogue warp is past the x tile
+                    if (!mbar_wait_bounded<true>(&ctrl->dz_ready, n & 1, &ctrl->abort, status)) break;  // every epilogue warp is past the x tile
                     load_x(n + 1);
                 }
             }
-            (void)nw;
+            mbar_landed(&ctrl->wfull, nw, &ctrl->zero, status);
+            mbar_landed(&ctrl->full_a, na, &ctrl->zero, status);
+            mbar_landed(&ctrl->full_x, nx, &ctrl->zero, status);
+            mbar_landed(&ctrl->full, nf, &ctrl->zero, status);
         }
         __syncwarp();
     } else if (warp == EPI_WARPS + 1) {

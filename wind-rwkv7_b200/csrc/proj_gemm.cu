@@ -93,9 +93,10 @@ __global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constan
 
     if (warp == 4) {
         if (elect_one()) {  // producer: one TMA request per operand block
-            for (int kb = 0; kb < nkb; ++kb) {
+            int kb = 0;
+            for (; kb < nkb; ++kb) {
                 const int s = kb % STAGES, round = kb / STAGES;
-                if (round > 0) mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status);
+                if (round > 0 && !mbar_wait_bounded<true>(&ctrl->empty[s], (round - 1) & 1, &ctrl->abort, status)) break;
                 const uint32_t bar = smem_u32(&ctrl->full[s]), dst = smem_u32(sm + s * STAGE_BYTES);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)STAGE_BYTES) : "memory");
                 asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constan
                 asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                              ::"r"(dst + A_BYTES), "l"(&mapB), "r"(bar), "r"(kb * BK), "r"(n0) : "memory");
             }
+            ring_landed<STAGES>(ctrl->full, kb, &ctrl->zero, status);
         }
         __syncwarp();
     } else if (warp == 5) {

@@ -89,7 +89,7 @@ template <typename IoT, int PREC, bool LN> struct BwdSmem {
     alignas(128) float S0s[N * SS];
     alignas(16) float dSs[N * SS];  // dSf as [value][key], column swizzle 1
     alignas(8) uint64_t s0_bar;     // completion of the state loads
-    volatile int abort;             // set when a bounded wait gave up
+    volatile int abort, zero;       // abort: set when a bounded wait gave up; zero stays 0 (see mbar_landed_uncounted)
     alignas(16) float fw[N];
     alignas(16) float Gp[2][WARPS][N];
     alignas(16) float lnp[LN ? 3 * N : 4];
@@ -169,8 +169,8 @@ static_assert(SS == N + 8, "the state loads copy boxes of N + 8 floats per row")
 
 // Waits (polling, bounded) for a phase of the state-load barrier: the library's common wait, which the forward's
 // self-test exercises on barriers nothing arrives on.
-__device__ __forceinline__ void s0_wait(uint64_t* bar, uint32_t parity, volatile int* abort, int* status) {
-    mbar_wait_bounded<false>(bar, parity, abort, status);
+__device__ __forceinline__ bool s0_wait(uint64_t* bar, uint32_t parity, volatile int* abort, int* status) {
+    return mbar_wait_bounded<false>(bar, parity, abort, status);
 }
 
 // TAIL: the sequence length is not a multiple of 16 (an instantiation of its own, so that whole-chunk sequences carry
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
     // Carried decay term for the last chunk: sum_i dsT[i,:] * sT[i,:] (zero without dsT).
     for (int i = tid; i < WARPS * N; i += THREADS) sm.Gp[1][i / N][i % N] = 0.f;
     if (tid == 0) {
-        sm.abort = 0;
+        sm.abort = sm.zero = 0;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.s0_bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -312,6 +312,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         f.x[0].setr(q[0]); f.x[1].setr(q[SCS]);
         return f;
     };
+    bool live = true;  // this thread has not given up a wait for a record: none is requested after that
     for (int it = 0; it < nchunks; ++it) {
         const int c = nchunks - 1 - it;
         const int vs = it & 1;
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         // attn kernel does it before it waits for the state's copy; attn_ln needs the state first (for dy).
         float du[2][4] = {}, dV[2][4] = {};
         float X[2][4] = {};
-        if (!LN) s0_wait(&sm.s0_bar, it & 1, &sm.abort, p.status);  // this chunk's start state has landed
+        if (!LN) live = s0_wait(&sm.s0_bar, it & 1, &sm.abort, p.status) && live;  // this chunk's start state has landed
         // attn: the X = S0 wa^T products ride in the same loop, six independent accumulator chains instead of four, then two
         auto du_dv = [&]() {
 #pragma unroll
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             }
         };
         if (!LN) du_dv();
-        if (LN) s0_wait(&sm.s0_bar, it & 1, &sm.abort, p.status);
+        if (LN) live = s0_wait(&sm.s0_bar, it & 1, &sm.abort, p.status) && live;
         float U[2][4] = {};
         float dvx[2][4] = {};  // LN: bonus-term contribution to dv
         {
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             }
         }
         __syncthreads();  // (C2) score gradients visible; S0s free
-        if (c > 0) issue_s0(c - 1);
+        if (c > 0 && live) issue_s0(c - 1);
         cp_async_commit();
 
 #pragma unroll 1
@@ -841,6 +842,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             *reinterpret_cast<float2*>(o + (16 * warp + g + 8) * N + 8 * nt + 2 * t4) = make_float2(dS[nt][2] * STATE_SCALE, dS[nt][3] * STATE_SCALE);
         }
     }
+    if (tid == 0 && sm.abort) mbar_landed_uncounted(&sm.s0_bar, &sm.zero, p.status);
 }
 
 // dparams[i][c] = sum over batch of the per-(batch, head) partials, in a fixed order.

@@ -61,7 +61,7 @@ template <bool LN> struct Smem {
     alignas(16) float fw[N];
     alignas(8) uint64_t raw_full, rec_full;
     Desc desc[4];
-    volatile int abort;
+    volatile int abort, zero;                      // zero stays 0 (see mbar_landed)
     float bdot[LN ? WARPS : 1][L], sbon[L];        // attn_ln: per-warp parts of sum_j r k bonus; sum_i dz v
     __device__ __forceinline__ float* yt() { return reinterpret_cast<float*>(raw[0]); }  // attn_ln: [time][value], pitch OPS
 };
@@ -185,13 +185,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
     if (tid == 0) {
         mbar_init(&sm.raw_full, 1);
         mbar_init(&sm.rec_full, 1);
-        sm.abort = 0;
+        sm.abort = sm.zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     if (warp == WARPS) {
         // ---- copy warp: a bulk tensor copy takes its thread some 200 cycles, which a working warp would make the others wait
         // for at the next barrier.  Takes part in the working warps' barriers.
+        int inputs = 1, records = 1;  // loads issued
         if (lane == 0) {
             load_inputs(0);
             load_record(0);
@@ -201,7 +202,10 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous chunk's output tiles have been read
             __syncthreads();  // (A)
             if (lane == 0) {
-                if (!LN && n + 1 < work.n) load_inputs(n + 1);
+                if (!LN && n + 1 < work.n && !sm.abort) {
+                    load_inputs(n + 1);
+                    ++inputs;
+                }
                 Desc e = sm.desc[(n + 1) & 3];
                 if (e.left > (PAR ? 0 : 1)) {  // (not the last but one: the last has flags)
                     --e.c; --e.left;
@@ -216,10 +220,15 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
                 __syncthreads();  // (D2)
             }
             __syncthreads();  // (C1)
+            const bool more = lane == 0 && n + 1 < work.n && !sm.abort;  // (the working warps are past this chunk's waits for loads)
             __syncthreads();  // (C2)
-            if (lane == 0 && n + 1 < work.n) {
-                if (LN) load_inputs(n + 1);
+            if (more) {
+                if (LN) {
+                    load_inputs(n + 1);
+                    ++inputs;
+                }
                 load_record(n + 1);
+                ++records;
             }
             __syncthreads();  // (E)
             if (lane == 0) {
@@ -229,7 +238,11 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
             }
             if ((d.flags & (LAST | CUT_AFTER)) == (LAST | CUT_AFTER) && p.ds0) __syncthreads();
         }
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last stores
+        if (lane == 0) {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last stores
+            mbar_landed(&sm.raw_full, inputs, &sm.zero, p.status);
+            mbar_landed(&sm.rec_full, records, &sm.zero, p.status);
+        }
         return;
     }
 
@@ -832,9 +845,10 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
         // ---- loads
         if (lane != 0) return;
         const int map_of[5] = {0, 1, 3, 4, 6};
-        for (int n = warp & 1; n < count; n += 2) {
+        int n = warp & 1;
+        for (; n < count; n += 2) {
             const int s = n % SLOTS, c = c0 - n;
-            if (n >= SLOTS) mbar_wait_bounded<true>(&sm.free[s], (n / SLOTS - 1) & 1, &sm.abort, p.status);
+            if (n >= SLOTS && !mbar_wait_bounded<true>(&sm.free[s], (n / SLOTS - 1) & 1, &sm.abort, p.status)) break;
             WalkSlot& t = sm.slot[s];
             expect(&sm.raw_full[s], 5 * TILE + sizeof(t.mats));
 #pragma unroll
@@ -843,9 +857,8 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
                          ::"r"(smem_u32(t.mats)), "l"(p.ckpt + ((long long)bh * nchunks + c) * CK_FLOATS + CK_AI), "r"((int)sizeof(t.mats)), "r"(smem_u32(&sm.raw_full[s]))
                          : "memory");
         }
-        // shared memory must outlive the loads, also where a wait has given up
-        for (int n = max(0, count - SLOTS); n < count; ++n)
-            if ((n & 1) == (warp & 1)) mbar_wait_bounded<true>(&sm.raw_full[n % SLOTS], (n / SLOTS) & 1, &sm.drain, p.status);
+        // shared memory must outlive the loads, also where a wait has given up (n: the first of this warp's loads not issued)
+        for (int i = max(warp & 1, n - SLOTS); i < n; i += 2) mbar_wait_bounded<true>(&sm.raw_full[i % SLOTS], (i / SLOTS) & 1, &sm.drain, p.status);
         return;
     }
     if (warp >= WARPS) {

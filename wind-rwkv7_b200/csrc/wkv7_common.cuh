@@ -356,7 +356,7 @@ template <int PREC, int X = 0> __device__ __forceinline__ void tri_inverse_colum
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Bounded wait for the phase of an mbarrier with the given parity; the one wait every kernel of this library uses.
-// Returns at once when the CTA has aborted.  When `limit` clocks pass without the phase completing it raises the
+// Returns at once, false, when the CTA has aborted.  When `limit` clocks pass without the phase completing it raises the
 // CTA's abort flag (every later wait then falls through), records kDeviceTimeout in the device status word and
 // returns: a lost copy or a missing arrival ends with an error code, never with a hung GPU.
 // SLEEP: the thread is suspended by the hardware (try_wait with a time hint) instead of polling.
@@ -374,7 +374,7 @@ __device__ __forceinline__ void give_up(volatile int* abort, int* status) {
     __threadfence_system();
 }
 template <bool SLEEP>
-__device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort, int* status, long long limit = MBAR_WAIT_LIMIT) {
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* abort, int* status, long long limit = MBAR_WAIT_LIMIT) {
     const uint32_t addr = smem_u32(bar);
     const uint32_t start = clock(), most = (uint32_t)limit;
     uint32_t spin = 0;
@@ -386,12 +386,32 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
         uint32_t ok;
         asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
                      : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
-        if (ok) return;
-        if (*abort) return;
+        if (ok) return true;
+        if (*abort) return false;
         if (SLEEP) __nanosleep(100);
         if ((SLEEP || (++spin & 63) == 0) && (uint32_t)clock() - start > most) break;
     }
     give_up(abort, status);
+    return false;
+}
+
+// Every thread that issues bulk loads ends with one of these: shared memory must outlive the loads also where a wait has given up and
+// nobody waits for them any more (otherwise they landed long ago).  They rely on no load being issued on a barrier whose last phase is
+// still open, so a thread whose wait returned false issues no more.  `never_set` takes the place of the abort flag.
+// The `issued` loads that went to `bar`, a phase each:
+__device__ __forceinline__ void mbar_landed(uint64_t* bar, int issued, volatile int* never_set, int* status) {
+    if (issued > 0) mbar_wait_bounded<true>(bar, (issued - 1) & 1, never_set, status);
+}
+// the same for a ring of S barriers that take the loads in turn:
+template <int S> __device__ __forceinline__ void ring_landed(uint64_t* ring, int issued, volatile int* never_set, int* status) {
+#pragma unroll 1
+    for (int s = 0; s < S; ++s) mbar_landed(ring + s, (issued + S - 1 - s) / S, never_set, status);
+}
+// and where nobody has counted, in a CTA that has aborted: the open phase, if there is one, has one of the two parities; the wait
+// for the other one returns at once before it and runs out after it.
+__device__ __forceinline__ void mbar_landed_uncounted(uint64_t* bar, volatile int* never_set, int* status) {
+    mbar_wait_bounded<true>(bar, 0, never_set, status);
+    mbar_wait_bounded<true>(bar, 1, never_set, status);
 }
 
 __device__ __forceinline__ uint32_t elect_one() {

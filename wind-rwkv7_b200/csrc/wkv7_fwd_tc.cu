@@ -41,8 +41,8 @@
 // thread issues two tensor-map bulk stores (cp.async.bulk.tensor.2d, shared -> global), which undo the
 // swizzle: the record in global memory stays plain row-major.
 // Every wait on an mbarrier is bounded; a wait that runs out raises an abort flag that makes all
-// later waits of the CTA return at once, records kDeviceTimeout and lets the CTA finish (tensor
-// memory is still released).
+// later waits of the CTA return at once, records kDeviceTimeout and lets the CTA finish (its loads and products
+// in flight are waited for, tensor memory is released).
 #include <cuda.h>
 #include <cstring>
 
@@ -115,12 +115,13 @@ enum : int { SEG_FIRST = 1, SEG_LAST = 2 };  // first / last chunk of a segment
 
 struct Ctrl {
     uint64_t full[4], done[4], score[4], raw[4], gate[4], mats[4], fold[4], rec[4], fread, hop;
-    uint64_t drain;            // abort path only: completion of the chain thread's outstanding tensor-core work
     uint32_t tmem_base;
     volatile int abort;
-    volatile int zero;         // stays 0: the abort-path drain waits with this in place of the abort flag
     ChunkDesc desc[4][4];      // [group][own-chunk number mod 4]: where the chunk lies (written one iteration ahead by the group)
     float bdot[4][2][4][L];    // attn_ln: per-warp partial bonus dots [group][iteration parity][warp][time]
+    // abort path only, a set per warp: completion of its products, and what its waits take in place of the abort flag
+    uint64_t drain[20];
+    volatile int never_set[20];
 };
 
 // Bounded wait for the phase with the given parity.  Returns at once when the CTA has aborted.
@@ -136,11 +137,17 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Abort path: commits everything this thread has issued to the tensor core to a barrier of its own and waits for
-// it, bounded and regardless of the CTA's abort flag, so that tensor memory is not released under products in flight.
-__device__ __forceinline__ void drain_tensor_work(uint64_t* bar, volatile int* never_set, int* status) {
-    tc_commit(bar);
-    mbar_wait_bounded<false>(bar, 0, never_set, status);
+// Abort path, by the thread of each warp that issues: waits, bounded and regardless of the CTA's abort flag, for the products and the
+// load that this warp may have in flight, so that neither tensor memory nor shared memory is released under them.
+__device__ __forceinline__ void abort_drain(Ctrl* ctrl, int warp, uint64_t* load, int* status) {
+    volatile int* never_set = &ctrl->never_set[warp];
+    *never_set = 0;
+    mbar_init(&ctrl->drain[warp], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_async_smem();
+    tc_commit(&ctrl->drain[warp]);
+    mbar_wait_bounded<true>(&ctrl->drain[warp], 0, never_set, status);
+    if (load) mbar_landed_uncounted(load, never_set, status);
 }
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {  // has the phase completed? (whole warp)
     uint32_t ok;
@@ -307,9 +314,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         }
         mbar_init(&ctrl->hop, 1);
         mbar_init(&ctrl->fread, 1);
-        mbar_init(&ctrl->drain, 1);
         ctrl->abort = 0;
-        ctrl->zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // descriptors of every group's first two chunks
@@ -417,7 +422,6 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 mbar_wait<false>(&ctrl->done[g], k & 1, ctrl, p.status);  // S' is the next chunk's A operand
                 tc_fence_after();
             }
-            if (ctrl->abort) drain_tensor_work(&ctrl->drain, &ctrl->zero, p.status);
           }
         } else if (warp < 4 * G + 2) {
             // ---- score warps: warp 4G reads [AK|AB] and later AI^T bwf (tensor-memory lanes 0-15), warp 4G + 1 reads [QK|QB]
@@ -547,6 +551,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
         };
         auto load_raw = [&](int ko) {
+            if (ctrl->abort) return;  // (the last one's wait may have given up)
             const ChunkDesc& d = ctrl->desc[grp][ko & 3];
             expect_bytes(&ctrl->raw[grp], 6 * RAW_TILE);
 #pragma unroll
@@ -744,7 +749,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 tc_fence_before();
                 group_bar(grp);
                 tc_fence_after();
-                if (LN && wg == 2 && elect_one()) {
+                if (LN && wg == 2 && elect_one() && !ctrl->abort) {
                     expect_bytes(&ctrl->gate[grp], RAW_TILE);
                     load_tile(maps.g, G_GRAW, ctrl->desc[grp][k & 3], &ctrl->gate[grp]);
                 }
@@ -842,6 +847,10 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last copies
     }
 
+    if (ctrl->abort && elect_one()) {
+        const bool prep = warp < 4 * G;  // of a group, warp 2's thread issues the loads
+        abort_drain(ctrl, warp, prep && (warp & 3) == 2 ? &ctrl->raw[warp >> 2] : LN && prep && (warp & 3) == 3 ? &ctrl->gate[warp >> 2] : nullptr, p.status);
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
