@@ -58,6 +58,11 @@ def test_validation_happens_before_any_launch(lib):
     assert _fwd(lib, st=(1024, 60, 64)) == -4      # stride breaks 16-byte rows
     assert _fwd(lib, p=0x1004) == -4               # misaligned pointer
     assert _fwd(lib, T=-16) == -1
+    assert _fwd(lib, st=(1024, 0, 64)) == -1       # 16 time steps in one place
+    p = 0x1000
+    for f, n in ((lib.wkv7_fwd, 10), (lib.wkv7_step, 9)):
+        for strides in ((0, 128, 64), (2048, 128, 0)):  # two batch entries, two heads
+            assert f(*([p] * n), 2, 16, 2, 64, *strides, 0, None) == -1
     assert lib.wkv7_fwd(None, None, None, None, None, None, None, None, None, None,
                         1, 16, 1, 64, 1024, 64, 64, 0, None) == -6
     # empty problems succeed without a launch

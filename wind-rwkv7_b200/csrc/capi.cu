@@ -71,6 +71,8 @@ int check_common(int64_t B, int64_t T, int64_t H, int64_t N, int64_t sb, int64_t
     const int64_t per16 = io_dtype == WKV7_BF16 ? 8 : 4;  // elements per 16 bytes
     if (sb % per16 || st % per16 || sh % per16) return wkv7::kBadAlign;
     if (sb < 0 || st < 0 || sh < 0) return wkv7::kBadShape;
+    // entries that all lie in one place: outputs cannot, and a tensor map has no such stride
+    if ((B > 1 && sb == 0) || (T > 1 && st == 0) || (H > 1 && sh == 0)) return wkv7::kBadShape;
     if (B * H > 0x7fffffffLL) return wkv7::kTooLarge;
     // the kernels address checkpoint records through 32-bit row coordinates of their tensor maps (80 rows of 64 floats
     // per record)
