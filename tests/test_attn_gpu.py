@@ -3,10 +3,11 @@ the reference-shaped Python entry points, which call the C ABI of libwkv7_sm100.
 
 Tolerances (max-abs error relative to the RMS of the oracle tensor, the metric of the task):
   fp32 path (3xTF32 products)                       <= 1e-4
-  bf16 path arithmetic (single-TF32 products),
-  observed on fp32 outputs                          <= 2e-2   (measured: y, sT, dr, dk, dv <= 7e-3; da, db <= 1.5e-2;
+  fp32 tensors, single-TF32 products (F32_TF32)     <= 2e-2   (measured: y, sT, dr, dk, dv <= 7e-3; da, db <= 1.5e-2;
                                                                dw <= 1.9e-2)
-  bf16 outputs: rounding the exact result to bf16 already costs about 2.5e-2 of RMS (half an ulp
+  bf16 tensors, the arithmetic alone: distance of an element from the oracle beyond half a unit of its last place,
+  i.e. of the value that was rounded to it          <= 2e-2   (measured: y, dr, dk, dv <= 3.4e-3, dw <= 6.3e-3, da, db <= 1.1e-2)
+  bf16 outputs as they are: rounding the exact result to bf16 already costs about 2.5e-2 of RMS (half an ulp
   of the largest elements; 3e-2 to 7e-2 for the heavy-tailed da, db, dw), above the 2e-2 bound, so the
   literal metric cannot hold for any bf16 output.  A bf16 output is the rounding of a value that the
   arithmetic bound allows to lie 2e-2 of RMS from the oracle, so it is held to (rounding floor measured
@@ -161,8 +162,8 @@ def test_golden_config0(golden):
 
 
 def _single_tf32_on_fp32_outputs(B, T, H, seed, dist, w=None):
-    """Runs forward + backward of the WKV7_F32_TF32 class (fp32 tensors, single-TF32 products: the bf16 path's
-    arithmetic without bf16 output rounding) through the C ABI and returns max-abs/RMS errors against the oracle."""
+    """Runs forward + backward of the WKV7_F32_TF32 class (fp32 tensors, single-TF32 products, in kernels of its own) through
+    the C ABI and returns max-abs/RMS errors against the oracle."""
     c_oracle, _lib, _, synthetic, _ = _mods()
     d = synthetic.wkv7_inputs(B, T, H, N, seed=seed, dtype=th.bfloat16, dist=dist)  # bf16-representable values
     if w is not None:
@@ -192,14 +193,53 @@ def _single_tf32_on_fp32_outputs(B, T, H, seed, dist, w=None):
 
 
 @pytest.mark.parametrize('dist', ['baseline', 'upstream'])
-def test_bf16_arithmetic_on_fp32_outputs(dist, fwd_impl):
-    """The bf16 path's arithmetic meets the stated 2e-2 bound on all eight tensors at T = 1024, both input
-    distributions, when bf16 output rounding is taken out of the picture."""
+def test_single_tf32_on_fp32_outputs(dist, fwd_impl):
+    """Single-TF32 products on fp32 tensors meet the stated 2e-2 bound on all eight tensors at T = 1024, both input
+    distributions."""
     if fwd_impl == 0:
         pytest.skip('fp32 tensors always run the warp-MMA forward: one run is enough')
     errs = _single_tf32_on_fp32_outputs(2, 1024, 2, 9, dist)
     for k, v in errs.items():
         assert v <= 2e-2, f'{k}: {v:.2e}'
+
+
+def beyond_rounding(x, ref):
+    """How far the value that was rounded to each bf16 element lies at least from the oracle's, largest over the RMS."""
+    x = x.detach().double().cpu().numpy().reshape(-1)
+    ref = np.asarray(ref, np.float64).reshape(-1)
+    half_ulp = np.exp2(np.floor(np.log2(np.maximum(np.abs(x), 2.0 ** -126))) - 8)  # 8 bits of mantissa
+    return float(np.maximum(np.abs(x - ref) - half_ulp, 0).max() / np.sqrt(np.mean(ref ** 2)))
+
+
+@pytest.mark.parametrize('dist', ['baseline', 'upstream', 'strong', 'floored'])
+@pytest.mark.parametrize('B,T,heads', [(2, 1024, 2), (1, 1003, 3), (1, 512, 150), (3, 400, 100)])
+def test_bf16_arithmetic(B, T, heads, dist, fwd_impl):
+    """The bf16 kernels' arithmetic meets the stated 2e-2 bound on all eight tensors with the rounding of the outputs taken out: few
+    chains (state gradients walked ahead), more chains than SMs, ragged lengths.  `strong`, `floored`: the decays of test_strong_decay;
+    where steps are at the floor, dw is the gradient of another function there (0.5 as in that test)."""
+    if fwd_impl == 0 and heads != 2:
+        pytest.skip('one size is enough for the warp-MMA forward')
+    c_oracle, _lib, attn, synthetic, _ = _mods()
+    d = synthetic.wkv7_inputs(B, T, heads, N, seed=9, dtype=th.bfloat16, dist='upstream' if dist == 'upstream' else 'baseline')
+    w = th.randn(B, T, heads * N, generator=th.Generator().manual_seed(13))
+    if dist == 'strong':
+        d['w'] = (w + 0.5).clamp(max=2.0).bfloat16()
+    elif dist == 'floored':
+        d['w'] = (w + 1.0).bfloat16()
+    ins = [d[n].cuda().requires_grad_() for n in NAMES]
+    y, sT = attn(*ins, N, return_state=True)
+    grads = th.autograd.grad(y, ins, d['dy'].cuda())
+    few = slice(heads - 2, heads)  # the oracle on two heads
+    part = lambda x: x.detach().view(B, T, heads, N)[:, :, few]
+    cpu = [part(d[n]).double().numpy() for n in list(NAMES) + ['dy']]
+    yo, sTo = c_oracle.wkv7_fwd(*cpu[:6])
+    go = c_oracle.wkv7_bwd(*cpu[:6], cpu[6])
+    assert beyond_rounding(part(y), yo) <= 2e-2
+    assert maxabs_rms(sT[:, few], sTo) <= 2e-2
+    for n, x, ref in zip(NAMES, grads, go):
+        e = beyond_rounding(part(x), ref)
+        assert e <= (0.5 if dist == 'floored' and n == 'w' else 2e-2), f'd{n}: {e:.2e}'
+    assert _lib.device_status() == 0
 
 
 def test_strong_decay(fwd_impl):
@@ -221,7 +261,7 @@ def test_strong_decay(fwd_impl):
     errs = _single_tf32_on_fp32_outputs(B, T, H, 13, 'baseline', w=w)
     for k, v in errs.items():
         assert v <= (0.5 if k == 'dw' else 2e-2), f'{k}: {v:.2e}'
-    # the same inputs through the bf16 kernels (tcgen05 forward) and the fp32 kernels
+    # the same inputs through the bf16 kernels (tcgen05 forward; gradients: test_bf16_arithmetic) and the fp32 kernels
     c_oracle, _lib, attn, synthetic, _ = _mods()
     for dtype in (th.bfloat16, th.float32):
         d = synthetic.wkv7_inputs(B, T, H, N, seed=13, dtype=dtype, device='cuda')
