@@ -1,5 +1,6 @@
-// Several tensors converted between fp32 and bf16 in one launch: the time mixer's parameters (about thirty, from 64 to C*C
-// elements) to bf16 before its kernels, the weight gradients back to fp32 after them.  A thread takes 8 elements (one
+// Several tensors converted between fp32 and bf16, or copied, in one launch: the time mixer's parameters (about thirty, from 64 to
+// C*C elements) before its kernels, to bf16 and, those of the GroupNorm and the bonus, to one fp32 tensor.  (Weight gradients need none:
+// they come out of their products in fp32.  bf16 -> fp32 is there for callers of the C ABI.)  A thread takes 8 elements (one
 // 16-byte and one 32-byte access), a CTA a tile of 2048; the tiles of all tensors are numbered through.  Bound by DRAM: 18 MB
 // at C = 768 take 5.4 us (torch's multi-tensor copy, which cuts tensors into tiles of 65536 elements for 46 CTAs: 18 us).
 #include "expand_loras.h"

@@ -46,27 +46,16 @@ static_assert(SCS == L + 8, "the matrix loads copy boxes of L + 8 floats per row
 // carry the column swizzle xcol<1>() of wkv7_common.cuh: each is read both along and across its
 // contraction index.
 
-// Staging tiles [time][channel] in the IO dtype.  bf16: 128-byte rows, the eight 16-byte segments of a
-// row XOR-ed with (row % 8) (cp.async then writes whole aligned 128-byte lines: padded rows cost it
-// 2.5 times the shared-memory wavefronts); fp32: 256-byte rows padded by 16 bytes.
-template <typename IoT> struct BwdLayout {
-    static constexpr bool SWZ = sizeof(IoT) == 2;
-    static constexpr int ROWB = N * (int)sizeof(IoT) + (SWZ ? 0 : 16);
-    // byte offset of element (row, col)
-    __device__ static __forceinline__ int at(int row, int col) {
-        const int b = col * (int)sizeof(IoT);
-        return SWZ ? row * ROWB + ((((b >> 4) ^ (row & 7)) << 4) | (b & 15)) : row * ROWB + b;
-    }
-    static constexpr int TILEB = L * ROWB;
-    static constexpr int YS = (sizeof(IoT) == 2) ? 24 : 20;
-};
+// Staging tiles [time][channel]: 256-byte rows padded by 16 bytes.
+constexpr int ROWB = N * 4 + 16, TILEB = L * ROWB;
+constexpr int YS = 20;  // row stride (floats) of the per-warp transposition scratch
+__device__ __forceinline__ int st_at(int row, int col) { return row * ROWB + col * 4; }  // byte offset of element (row, col)
 
-template <typename IoT, int PREC, bool LN> struct BwdSmem {
-    using Lay = BwdLayout<IoT>;
-    alignas(16) unsigned char st_in[5][Lay::TILEB];  // q, w, k, a, b (dead after the scan)
-    alignas(16) unsigned char st_v[2][Lay::TILEB];
-    alignas(16) unsigned char st_dy[2][Lay::TILEB];
-    alignas(16) unsigned char st_g[LN ? 2 : 1][LN ? Lay::TILEB : 16];
+template <int PREC, bool LN> struct BwdSmem {
+    alignas(16) unsigned char st_in[5][TILEB];  // q, w, k, a, b (dead after the scan)
+    alignas(16) unsigned char st_v[2][TILEB];
+    alignas(16) unsigned char st_dy[2][TILEB];
+    alignas(16) unsigned char st_g[LN ? 2 : 1][LN ? TILEB : 16];
     alignas(16) float wq[L * OPS], wa[L * OPS], kwi[L * OPS], bwi[L * OPS];
     alignas(16) float cum[L * OPS];
     alignas(16) float lw[PREC == 3 ? L * OPS : 4];   // single-TF32 path derives it from cum
@@ -76,7 +65,7 @@ template <typename IoT, int PREC, bool LN> struct BwdSmem {
     alignas(128) float mats[2 * MAT_BLK];
     // Score gradients (stage C).  While stage B runs they are dead, and the same bytes serve as
     // the per-warp transposition scratch for dv / dg and as the GroupNorm reduction buffers.
-    static constexpr int SCRATCH_FLOATS = WARPS * L * Lay::YS * (int)sizeof(IoT) / 4 + WARPS * L * 5;
+    static constexpr int SCRATCH_FLOATS = WARPS * L * YS + WARPS * L * 5;
     static constexpr int SGRAD_FLOATS = 4 * L * SCS > SCRATCH_FLOATS ? 4 * L * SCS : SCRATCH_FLOATS;
     alignas(16) float sgrad[SGRAD_FLOATS];  // score gradient i at sgrad + i * L * SCS
     // attn_ln: Ut, Dt, Yt are dead between stage C and the next chunk's stage B and double as the output staging tiles
@@ -96,53 +85,38 @@ template <typename IoT, int PREC, bool LN> struct BwdSmem {
     float bdot[L], sbon[L];
 };
 
-template <typename IoT> __device__ __forceinline__ float bst_elem(const unsigned char* tile, int row, int col) {
-    return to_f32<IoT>(*reinterpret_cast<const IoT*>(tile + BwdLayout<IoT>::at(row, col)));
-}
+__device__ __forceinline__ float bst_elem(const unsigned char* tile, int row, int col) { return *reinterpret_cast<const float*>(tile + st_at(row, col)); }
 // two adjacent elements (col even) of a staging tile
-template <typename IoT> __device__ __forceinline__ float2 bst_pair(const unsigned char* tile, int row, int col);
-template <> __device__ __forceinline__ float2 bst_pair<float>(const unsigned char* tile, int row, int col) {
-    return *reinterpret_cast<const float2*>(tile + BwdLayout<float>::at(row, col));
-}
+__device__ __forceinline__ float2 bst_pair(const unsigned char* tile, int row, int col) { return *reinterpret_cast<const float2*>(tile + st_at(row, col)); }
 // A operand [m = time][k = value] straight from a staging tile laid out [time][value]
-template <typename IoT, int PREC>
-__device__ __forceinline__ FragA<PREC> fragA_mk_st(const unsigned char* tile, int k0, int g, int t4) {
+template <int PREC> __device__ __forceinline__ FragA<PREC> fragA_mk_st(const unsigned char* tile, int k0, int g, int t4) {
     FragA<PREC> f;
-    float2 lo = bst_pair<IoT>(tile, g, k0 + 2 * t4), hi = bst_pair<IoT>(tile, g + 8, k0 + 2 * t4);
-    constexpr bool EXACT = sizeof(IoT) == 2;  // a bf16 value is a TF32 value
-    f.x[0].template put<EXACT>(lo.x); f.x[1].template put<EXACT>(hi.x); f.x[2].template put<EXACT>(lo.y); f.x[3].template put<EXACT>(hi.y);
+    float2 lo = bst_pair(tile, g, k0 + 2 * t4), hi = bst_pair(tile, g + 8, k0 + 2 * t4);
+    f.x[0].set(lo.x); f.x[1].set(hi.x); f.x[2].set(lo.y); f.x[3].set(hi.y);
     return f;
 }
 // B operand [k = value][n = time] from a staging tile laid out [time][value]
-template <typename IoT, int PREC>
-__device__ __forceinline__ FragB<PREC> fragB_nk_st(const unsigned char* tile, int n0, int k0, int g, int t4) {
+template <int PREC> __device__ __forceinline__ FragB<PREC> fragB_nk_st(const unsigned char* tile, int n0, int k0, int g, int t4) {
     FragB<PREC> f;
-    float2 v = bst_pair<IoT>(tile, n0 + g, k0 + 2 * t4);
-    constexpr bool EXACT = sizeof(IoT) == 2;
-    f.x[0].template put<EXACT>(v.x); f.x[1].template put<EXACT>(v.y);
+    float2 v = bst_pair(tile, n0 + g, k0 + 2 * t4);
+    f.x[0].set(v.x); f.x[1].set(v.y);
     return f;
 }
 // A operand [m = value][k = time] (the transpose) from a staging tile laid out [time][value]
-template <typename IoT, int PREC>
-__device__ __forceinline__ FragA<PREC> fragA_km_st(const unsigned char* tile, int m0, int k0, int g, int t4) {
+template <int PREC> __device__ __forceinline__ FragA<PREC> fragA_km_st(const unsigned char* tile, int m0, int k0, int g, int t4) {
     FragA<PREC> f;
     const int tr = k0 + 2 * t4, vc = m0 + g;
-    constexpr bool EXACT = sizeof(IoT) == 2;
-    f.x[0].template put<EXACT>(bst_elem<IoT>(tile, tr, vc));
-    f.x[1].template put<EXACT>(bst_elem<IoT>(tile, tr, vc + 8));
-    f.x[2].template put<EXACT>(bst_elem<IoT>(tile, tr + 1, vc));
-    f.x[3].template put<EXACT>(bst_elem<IoT>(tile, tr + 1, vc + 8));
+    f.x[0].set(bst_elem(tile, tr, vc));
+    f.x[1].set(bst_elem(tile, tr, vc + 8));
+    f.x[2].set(bst_elem(tile, tr + 1, vc));
+    f.x[3].set(bst_elem(tile, tr + 1, vc + 8));
     return f;
 }
 
-template <typename IoT> __device__ __forceinline__ void store_pair(IoT* p, float x, float y);
-template <> __device__ __forceinline__ void store_pair<float>(float* p, float x, float y) {
-    *reinterpret_cast<float2*>(p) = make_float2(x, y);
-}
 // Epilogue stores.  A thread holds columns (2*t4, 2*t4+1) of two adjacent 8-column tiles; stored as they
 // are, a warp-wide store writes 16 bytes per row (half a 32-byte sector).  Lanes t4 and t4^1 swap one
 // pair, after which the even lane holds columns 4m..4m+3 of the first tile and the odd lane the same
-// columns of the second tile (m = t4 / 2): 8-byte stores (bf16), whole sectors per row.
+// columns of the second tile (m = t4 / 2): 16-byte stores, whole sectors per row.
 // `row` points at column 16*warp of the output row; live = false (rows beyond the end of the sequence) keeps the
 // exchange but skips the store.
 __device__ __forceinline__ void store_quad(float* row, float a0, float a1, float b0, float b1, int t4, bool live) {
@@ -175,10 +149,9 @@ __device__ __forceinline__ bool s0_wait(uint64_t* bar, uint32_t parity, volatile
 
 // TAIL: the sequence length is not a multiple of 16 (an instantiation of its own, so that whole-chunk sequences carry
 // none of the row tests).
-template <typename IoT, int PREC, bool LN, bool TAIL>
+template <int PREC, bool LN, bool TAIL>
 __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __grid_constant__ CkptMaps cmaps) {
-    using Lay = BwdLayout<IoT>;
-    using Smem = BwdSmem<IoT, PREC, LN>;
+    using Smem = BwdSmem<PREC, LN>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
 
@@ -188,22 +161,22 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
     const long long base = bi * p.st.b + hi * p.st.h;
     const int nchunks = (int)((p.T + L - 1) / L);  // the last chunk may be partial: its missing rows read as zeros
     constexpr bool has_tail = TAIL;
-    const IoT* gin[5] = {(const IoT*)p.r + base, (const IoT*)p.w + base, (const IoT*)p.k + base,
-                         (const IoT*)p.a + base, (const IoT*)p.b + base};
-    const IoT* gv = (const IoT*)p.v + base;
-    const IoT* gdy = (const IoT*)p.dy + base;
-    IoT* gout[5] = {(IoT*)p.dr + base, (IoT*)p.dw + base, (IoT*)p.dk + base, (IoT*)p.da + base, (IoT*)p.db + base};
-    IoT* gdv = (IoT*)p.dv + base;
-    const IoT* gg = LN ? (const IoT*)p.g + base : nullptr;
-    IoT* gdg = LN ? (IoT*)p.dg + base : nullptr;
-    constexpr uint32_t ROW_BYTES = N * sizeof(IoT);
+    const float* gin[5] = {(const float*)p.r + base, (const float*)p.w + base, (const float*)p.k + base,
+                         (const float*)p.a + base, (const float*)p.b + base};
+    const float* gv = (const float*)p.v + base;
+    const float* gdy = (const float*)p.dy + base;
+    float* gout[5] = {(float*)p.dr + base, (float*)p.dw + base, (float*)p.dk + base, (float*)p.da + base, (float*)p.db + base};
+    float* gdv = (float*)p.dv + base;
+    const float* gg = LN ? (const float*)p.g + base : nullptr;
+    float* gdg = LN ? (float*)p.dg + base : nullptr;
+    constexpr uint32_t ROW_BYTES = N * 4;
 
     if (LN) {
         for (int i = tid; i < 3 * N; i += THREADS) sm.lnp[i] = p.params[(long long)(i / N) * p.H * N + hi * N + (i % N)];
     }
     // stage-B scratch aliased onto the score-gradient buffers
-    IoT* const dvsc = reinterpret_cast<IoT*>(sm.sgrad) + warp * (L * Lay::YS);
-    float* const red = sm.sgrad + (WARPS * L * Lay::YS * (int)sizeof(IoT)) / 4;  // [WARPS][L][2]
+    float* const dvsc = sm.sgrad + warp * (L * YS);
+    float* const red = sm.sgrad + WARPS * L * YS;  // [WARPS][L][2]
     float* const red2 = red + WARPS * L * 2;                                             // [WARPS][L][3]
     float dlnw_acc[2] = {0.f, 0.f}, dlnb_acc[2] = {0.f, 0.f}, dbon_acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
     // Carried decay term for the last chunk: sum_i dsT[i,:] * sT[i,:] (zero without dsT).
@@ -230,17 +203,17 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         for (int i = tid; i < 5 * L * CH; i += THREADS) {
             const int ten = i / (L * CH), row = (i / CH) % L, ch = i % CH;
             const long long tt = (long long)c * L + row;
-            if (has_tail) cp_async16_zfill(sm.st_in[ten] + Lay::at(row, ch * (16 / (int)sizeof(IoT))),
+            if (has_tail) cp_async16_zfill(sm.st_in[ten] + st_at(row, ch * 4),
                              reinterpret_cast<const unsigned char*>(gin[ten] + (tt < p.T ? tt : p.T - 1) * p.st.t) + ch * 16, tt < p.T);
-            else cp_async16(sm.st_in[ten] + Lay::at(row, ch * (16 / (int)sizeof(IoT))), reinterpret_cast<const unsigned char*>(gin[ten] + tt * p.st.t) + ch * 16);
+            else cp_async16(sm.st_in[ten] + st_at(row, ch * 4), reinterpret_cast<const unsigned char*>(gin[ten] + tt * p.st.t) + ch * 16);
         }
     };
     auto issue_vdy = [&](int c, int s) {
         for (int i = tid; i < (LN ? 3 : 2) * L * CH; i += THREADS) {
             const int ten = i / (L * CH), row = (i / CH) % L, ch = i % CH;
             const long long tt = (long long)c * L + row;
-            const IoT* src = (ten == 0 ? gv : ten == 1 ? gdy : gg) + (!TAIL || tt < p.T ? tt : p.T - 1) * p.st.t;
-            unsigned char* dst = (ten == 0 ? sm.st_v[s] : ten == 1 ? sm.st_dy[s] : sm.st_g[LN ? s : 0]) + Lay::at(row, ch * (16 / (int)sizeof(IoT)));
+            const float* src = (ten == 0 ? gv : ten == 1 ? gdy : gg) + (!TAIL || tt < p.T ? tt : p.T - 1) * p.st.t;
+            unsigned char* dst = (ten == 0 ? sm.st_v[s] : ten == 1 ? sm.st_dy[s] : sm.st_g[LN ? s : 0]) + st_at(row, ch * 4);
             if (has_tail) cp_async16_zfill(dst, reinterpret_cast<const unsigned char*>(src) + ch * 16, tt < p.T);
             else cp_async16(dst, reinterpret_cast<const unsigned char*>(src) + ch * 16);
         }
@@ -318,7 +291,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         const int vs = it & 1;
         // ---------------- P1: decay scan and scaled operands -------------------------------------
         {
-            decay_scan<IoT, PREC, 1, Lay::SWZ>(sm.st_in[0], sm.st_in[1], sm.st_in[2], sm.st_in[3], sm.st_in[4], Lay::ROWB, sm.wq, sm.wa,
+            decay_scan<float, PREC, 1>(sm.st_in[0], sm.st_in[1], sm.st_in[2], sm.st_in[3], sm.st_in[4], ROWB, sm.wq, sm.wa,
                                   sm.kwi, sm.bwi, sm.fw, sm.cum, PREC == 3 ? sm.lw : nullptr, warp, lane,
                                   TAIL ? (int)min((long long)L, p.T - (long long)c * L) : L);
             if (LN) {  // bonus dot  sum_j r_j k_j bonus_j  per time step: 8 threads per row
@@ -327,7 +300,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int ch = part * 8 + i;
-                    acc += bst_elem<IoT>(sm.st_in[0], row, ch) * bst_elem<IoT>(sm.st_in[2], row, ch) * sm.lnp[2 * N + ch];
+                    acc += bst_elem(sm.st_in[0], row, ch) * bst_elem(sm.st_in[2], row, ch) * sm.lnp[2 * N + ch];
                 }
                 acc += __shfl_xor_sync(0xffffffffu, acc, 1);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 2);
@@ -347,8 +320,8 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         FragA<PREC> vf[2], dyf[2];
 #pragma unroll
         for (int kk = 0; kk < 2; ++kk) {
-            vf[kk] = fragA_km_st<IoT, PREC>(vt, 16 * warp, 8 * kk, g, t4);
-            if (!LN) dyf[kk] = fragA_km_st<IoT, PREC>(dyt, 16 * warp, 8 * kk, g, t4);
+            vf[kk] = fragA_km_st<PREC>(vt, 16 * warp, 8 * kk, g, t4);
+            if (!LN) dyf[kk] = fragA_km_st<PREC>(dyt, 16 * warp, 8 * kk, g, t4);
         }
         // dS <- dSf = dS * fw, then du and the first part of dV.  None of this needs the chunk-start state, so the
         // attn kernel does it before it waits for the state's copy; attn_ln needs the state first (for dy).
@@ -485,7 +458,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                     for (int hrow = 0; hrow < 2; ++hrow) {
                         const int vc = 16 * warp + g + 8 * hrow, i = e + 2 * hrow;
                         const float x = (Y[nt][i] - mu) * rstd;
-                        const float ve = bst_elem<IoT>(vt, tq, vc), ge = bst_elem<IoT>(gt, tq, vc), de = bst_elem<IoT>(dyt, tq, vc);
+                        const float ve = bst_elem(vt, tq, vc), ge = bst_elem(gt, tq, vc), de = bst_elem(dyt, tq, vc);
                         const float z = x * sm.lnp[vc] + sm.lnp[N + vc] + bd * ve;
                         const float dz = de * ge;
                         Y[nt][i] = de * z;  // dg, stored below
@@ -525,22 +498,22 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 }
                 // dg out, through the per-warp scratch tile for 16-byte stores
                 {
-                    IoT* sc = dvsc;
+                    float* sc = dvsc;
 #pragma unroll
                     for (int nt = 0; nt < 2; ++nt) {
                         const int tq = 8 * nt + 2 * t4;
-                        sc[tq * Lay::YS + g] = from_f32<IoT>(Y[nt][0]);
-                        sc[(tq + 1) * Lay::YS + g] = from_f32<IoT>(Y[nt][1]);
-                        sc[tq * Lay::YS + g + 8] = from_f32<IoT>(Y[nt][2]);
-                        sc[(tq + 1) * Lay::YS + g + 8] = from_f32<IoT>(Y[nt][3]);
+                        sc[tq * YS + g] = Y[nt][0];
+                        sc[(tq + 1) * YS + g] = Y[nt][1];
+                        sc[tq * YS + g + 8] = Y[nt][2];
+                        sc[(tq + 1) * YS + g + 8] = Y[nt][3];
                     }
                     __syncwarp();
                     const int row = lane >> 1, hf = lane & 1;
-                    const uint4* src = reinterpret_cast<const uint4*>(sc + row * Lay::YS + 8 * hf);
+                    const uint4* src = reinterpret_cast<const uint4*>(sc + row * YS + 8 * hf);
                     uint4* dst = reinterpret_cast<uint4*>(gdg + ((long long)c * L + row) * p.st.t + 16 * warp + 8 * hf);
                     if (!TAIL || (long long)c * L + row < p.T) {
                         dst[0] = src[0];
-                        if (sizeof(IoT) == 4) dst[1] = src[1];
+                        dst[1] = src[1];
                     }
                     __syncwarp();
                 }
@@ -590,22 +563,22 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 
         // dv out, transposed through a per-warp scratch tile for 16-byte stores
         {
-            IoT* sc = dvsc;
+            float* sc = dvsc;
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 const int tq = 8 * nt + 2 * t4;
-                sc[tq * Lay::YS + g] = from_f32<IoT>(dV[nt][0] + dvx[nt][0]);
-                sc[(tq + 1) * Lay::YS + g] = from_f32<IoT>(dV[nt][1] + dvx[nt][1]);
-                sc[tq * Lay::YS + g + 8] = from_f32<IoT>(dV[nt][2] + dvx[nt][2]);
-                sc[(tq + 1) * Lay::YS + g + 8] = from_f32<IoT>(dV[nt][3] + dvx[nt][3]);
+                sc[tq * YS + g] = dV[nt][0] + dvx[nt][0];
+                sc[(tq + 1) * YS + g] = dV[nt][1] + dvx[nt][1];
+                sc[tq * YS + g + 8] = dV[nt][2] + dvx[nt][2];
+                sc[(tq + 1) * YS + g + 8] = dV[nt][3] + dvx[nt][3];
             }
             __syncwarp();
             const int row = lane >> 1, hf = lane & 1;
-            const uint4* src = reinterpret_cast<const uint4*>(sc + row * Lay::YS + 8 * hf);
+            const uint4* src = reinterpret_cast<const uint4*>(sc + row * YS + 8 * hf);
             uint4* dst = reinterpret_cast<uint4*>(gdv + ((long long)c * L + row) * p.st.t + 16 * warp + 8 * hf);
             if (!TAIL || (long long)c * L + row < p.T) {
                 dst[0] = src[0];
-                if (sizeof(IoT) == 4) dst[1] = src[1];
+                dst[1] = src[1];
             }
         }
         // dSf, U, dabu to shared memory for stage C
@@ -673,13 +646,13 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll 2
             for (int kk = 0; kk < 8; ++kk) {
                 FragA<PREC> aD = fragA_mk<PREC, true, 1>(sm.Dt, OPS, 0, 8 * kk, g, t4);
-                FragA<PREC> aY = LN ? fragA_mk<PREC, true, 1>(sm.Yt, OPS, 0, 8 * kk, g, t4) : fragA_mk_st<IoT, PREC>(dyt, 8 * kk, g, t4);
+                FragA<PREC> aY = LN ? fragA_mk<PREC, true, 1>(sm.Yt, OPS, 0, 8 * kk, g, t4) : fragA_mk_st<PREC>(dyt, 8 * kk, g, t4);
                 FragA<PREC> aU = fragA_mk<PREC, true, 1>(sm.Ut, OPS, 0, 8 * kk, g, t4);
-                FragA<PREC> aV = fragA_mk_st<IoT, PREC>(vt, 8 * kk, g, t4);
+                FragA<PREC> aV = fragA_mk_st<PREC>(vt, 8 * kk, g, t4);
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
                     FragB<PREC> bsc = (warp >> 1) ? fragB_nk<PREC, true, 1>(sm.Ut, OPS, 8 * nt, 8 * kk, g, t4)
-                                                  : fragB_nk_st<IoT, PREC>(vt, 8 * nt, 8 * kk, g, t4);
+                                                  : fragB_nk_st<PREC>(vt, 8 * nt, 8 * kk, g, t4);
                     mma<PREC>(d[nt], strict ? aD : aY, bsc);
                     FragB<PREC> bS;
                     bS.x[0].setr(s0_kn[4 * kk * SS + 8 * nt]); bS.x[1].setr(s0_kn[(4 * kk + 1) * SS + 8 * nt]);
@@ -909,9 +882,9 @@ bool encode_bthn_map(CUtensorMap* m, void* base, long long B, long long T, long 
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename IoT, int PREC, bool LN> static int launch_bwd_t(const BwdParams& p, cudaStream_t stream) {
-    using Smem = BwdSmem<IoT, PREC, LN>;
-    auto kern = p.T % L ? wkv7_bwd_kernel<IoT, PREC, LN, true> : wkv7_bwd_kernel<IoT, PREC, LN, false>;
+template <int PREC, bool LN> static int launch_bwd_t(const BwdParams& p, cudaStream_t stream) {
+    using Smem = BwdSmem<PREC, LN>;
+    auto kern = p.T % L ? wkv7_bwd_kernel<PREC, LN, true> : wkv7_bwd_kernel<PREC, LN, false>;
     const int smem = (int)sizeof(Smem);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return kLaunchFailed;
@@ -933,8 +906,8 @@ int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream) {
 
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream) {
     if (io_dtype == 0) return launch_bwd_bf16(p, ln, stream);
-    if (io_dtype == 2) return ln ? launch_bwd_t<float, 1, true>(p, stream) : launch_bwd_t<float, 1, false>(p, stream);
-    return ln ? launch_bwd_t<float, 3, true>(p, stream) : launch_bwd_t<float, 3, false>(p, stream);
+    if (io_dtype == 2) return ln ? launch_bwd_t<1, true>(p, stream) : launch_bwd_t<1, false>(p, stream);
+    return ln ? launch_bwd_t<3, true>(p, stream) : launch_bwd_t<3, false>(p, stream);
 }
 
 }  // namespace wkv7

@@ -48,7 +48,7 @@ enum Status : int {
     kOk = 0,
     kBadShape = -1,        // negative or inconsistent dimensions
     kBadHeadSize = -2,     // only N == 64 is built
-    kBadChunk = -3,        // T is not a multiple of 16
+    kBadChunk = -3,        // ddlerp, expand_loras: C is not a multiple of 64
     kBadAlign = -4,        // pointer or stride not 16-byte aligned
     kBadDtype = -5,
     kNullPointer = -6,
@@ -128,18 +128,15 @@ template <int PREC> __device__ __forceinline__ FragA<PREC> fragA_from_acc(const 
     return f;
 }
 
-// Column swizzles of the fp32 tiles of the backward kernel.  A tile is read in two ways: along the
+// Column swizzle of the fp32 tiles of the backward kernels.  A tile is read in two ways: along the
 // contraction index (lanes = rows g, 8-byte loads at columns 2t) and across it (lanes = columns g,
 // rows 2t and 2t+1).
 // X = 1, for row strides of 8 or 24 mod 32 words (the padded operand and score tiles): the first
 //   pattern is conflict-free by the padding, in the second rows 2t and 2t+4 fall on the same banks;
 //   XOR-ing the column with 8 for rows 4..7 of every block of 8 rows separates them.
-// X = 2, for unpadded 64-float rows: the column is XOR-ed with 8 * ((row ^ (row >> 2)) & 3), which gives
-//   rows g = 0..3, rows g = 4..7, rows 0,2,4,6 and rows 1,3,5,7 four different values each, so both
-//   patterns are conflict-free.
-// Groups of 8 floats stay contiguous under both.  X = 0: plain layout.
+// Groups of 8 floats stay contiguous under it.  X = 0: plain layout.
 template <int X> __device__ __forceinline__ int xcol(int row, int col) {
-    return X == 1 ? (col ^ ((row & 4) << 1)) : X == 2 ? (col ^ (((row ^ (row >> 2)) & 3) << 3)) : col;
+    return X == 1 ? (col ^ ((row & 4) << 1)) : col;
 }
 
 // A operand from memory laid out [m][k] (row stride ld floats), rows m0+g, m0+g+8, block k0.
@@ -243,18 +240,16 @@ __device__ __forceinline__ void store8(float* p, const float (&f)[8], bool flip 
 // bytes wide.  Writes wq = q*P_t, wa = a*P_{t-1}, kwi = k/P_t, bwi = b/P_t (row stride OPS), the
 // chunk decay fw = P_L, and optionally the running log-decay and the per-step log-decay.
 // tq/tw/tk/ta/tb: staging tiles with row stride `rowb` bytes.
-// RAWX: the staging tiles have unpadded 128-byte rows (bf16) whose eight 16-byte segments are XOR-ed
-// with (row % 8), so that cp.async writes whole aligned lines and these 16-byte reads stay conflict-free.
 // live: number of time steps of this chunk that exist (16 except in the last chunk of a sequence whose length
 // is not a multiple of 16); rows beyond it carry zero inputs and a per-step log-decay of zero, so that the state
 // passes through them unchanged.
-template <typename IoT, int PREC, int X = 0, bool RAWX = false>
+template <typename IoT, int PREC, int X = 0>
 __device__ __forceinline__ void decay_scan(const unsigned char* tq, const unsigned char* tw, const unsigned char* tk,
                                            const unsigned char* ta, const unsigned char* tb, int rowb, float* wq, float* wa,
                                            float* kwi, float* bwi, float* fw, float* cum_out, float* lw_out, int warp, int lane,
                                            int live = L) {
     const int row = lane & 15, j0 = 16 * warp + 8 * (lane >> 4);
-    const int off = RAWX ? row * rowb + ((((j0 * (int)sizeof(IoT)) >> 4) ^ (row & 7)) << 4) : row * rowb + j0 * (int)sizeof(IoT);
+    const int off = row * rowb + j0 * (int)sizeof(IoT);
     float lw[8], cum[8], q[8], k[8], a[8], b[8];
     load8<IoT>(tw + off, lw);
     load8<IoT>(tq + off, q);
