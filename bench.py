@@ -36,9 +36,10 @@ BWD_BYTES_PER_TOKEN_HEAD = 13 * N * 2   # r,w,k,v,a,b,dy in + six gradients out,
 # Fallback copy of the pool's measured STREAM-style bandwidth, used when MEASURED_PEAKS.json is absent.
 FALLBACK_HBM_GBS = 6650.0
 # dram__bytes_read.sum + dram__bytes_write.sum of one backward launch at this workload, from an ncu capture of
-# `python bench.py --no-e2e --no-cpu-baseline --steps 1 --warmup 1 --batch 16`: 428.1 MB read + 130.8 MB written at
-# B = 16, scaled by 4 (traffic is proportional to the number of chains; the B = 64 workload is too large to capture).
-BWD_DRAM_TRAFFIC_BYTES = 2_235_450_000
+# `python bench.py --no-e2e --no-cpu-baseline --no-secondary --steps 1 --warmup 1 --batch 25`: 668.6 MB read + 219.5 MB written by
+# wkv7_bwd_bf16_kernel at B = 25 (the smallest batch that fills the machine), scaled by 64 / 25: traffic is proportional to the number
+# of chains, and the B = 64 workload is too large to capture.
+BWD_DRAM_TRAFFIC_BYTES = 2_273_530_000
 
 
 def hbm_peak():
@@ -469,7 +470,7 @@ def run_ours(args):
                        'global_batch': world * B, 'parallelism': f'batch-sharded x{world}, no collective',
                        'l2': 'inputs (7 x 100 MB) and outputs exceed the 126 MB L2; no explicit flush',
                        'precision': 'single-TF32 tensor-core products, fp32 accumulate'},
-            'roofline': {'bound': 'hbm', 'kernel': 'wkv7_bwd_kernel', 'achieved': achieved, 'peak': peak,
+            'roofline': {'bound': 'hbm', 'kernel': 'wkv7_bwd_bf16_kernel', 'achieved': achieved, 'peak': peak,
                          'unit': 'GB/s', 'frac': achieved / peak, 'peak_source': which,
                          'traffic': BWD_DRAM_TRAFFIC_BYTES, 'algorithmic_bytes': bwd_bytes,
                          'kernel_ms': bwd_ms,

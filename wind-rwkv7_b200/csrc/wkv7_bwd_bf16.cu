@@ -3,8 +3,8 @@
 // a cut chain handed on through ds0).
 //
 // What bounds it.  Per 16-step chunk 840 warp-level TF32 products (8 cycles each on one of four schedulers: 1680 cycles) and
-// 3300 shared-memory wavefronts (one a cycle) meet 8200 warp instructions with the dependencies of a chain: with two CTAs an SM
-// takes 4500 cycles per chunk (attn, a full machine), the data pipe busy 73 % of them.  The form of wkv7_bwd.cu had it
+// 3300 shared-memory wavefronts (one a cycle) meet 8700 warp instructions with the dependencies of a chain: with two CTAs an SM
+// takes 4400 cycles per chunk (attn, a full machine), the data pipe busy 76 % of them.  The form of wkv7_bwd.cu had it
 // busy 81 % of 5035 cycles.  What changed:
 //  * equal shares of work instead of whole chains (768 chains on 296 CTAs are 2.6 rounds);
 //  * the term of the decay gradient that was carried from the following chunk, sum_i dS[i,:] S'[i,:] with S' = (S0 + V^T kwi +
@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
 // chain: 4 chain warps (16 value rows of dS each, no exchange between them), PREP groups of 4 preparing warps (the scan, 16 key columns
 // each) that take every PREP-th chunk, two warps that issue the loads; SLOTS chunks in flight.  Leaves dS at the end of every chunk in
 // `tiles`, for chunks it0 .. it0 + n - 1 (counted from the end of the sequence).
-// Bound by the chain of dependent products, some 1300 cycles a chunk (the one-kernel form: 6200).  Backward of 48 chains of 63 chunks
+// Bound by the chain of dependent products, some 1500 cycles a chunk (the one-kernel form: 6200).  Backward of 48 chains of 63 chunks
 // 203 -> 115 us, of 8 chains of 256 chunks 745 -> 230 us, of 148 chains of 63 chunks 236 -> 205 us.
 constexpr int SLOTS = 6, PREP = 2, WALK_THREADS = 32 * (WARPS * (1 + PREP) + 2);
 struct WalkSlot {

@@ -14,7 +14,8 @@
 // operand needs an explicit completion wait (tcgen05.commit -> mbarrier); only same-accumulator products are ordered by the
 // tensor pipe.  With three hops (U explicit) and a wait for "results of chunk c-2 read" a chunk took the chain 2000 cycles,
 // most of them waits; what bounds it now is the latency from a chunk's operand tiles to its completion over the four chunks
-// in flight (shared memory has room for four sets of tiles): 1820 cycles per chunk without checkpoints (2070 before), 2500 with (2780).
+// in flight (shared memory has room for four sets of tiles): about 1700 cycles per chunk without checkpoints (B8 T65536 H40), 2250 with
+// (B64 T1024 H12).
 //
 // Warp roles (128 (G+1) threads).  Warps 0..4G-1 are G preparation groups of four warps, each working on its own chunk
 // (position g, g+G, ... of the CTA's list): the decay scan of the six input tiles (bulk tensor loads, one chunk ahead), the

@@ -158,8 +158,8 @@ def _attn_time_split(r, w, k, v, a, b, C, s0, nseg):
     The recurrence is affine in the state: over a segment S_end = S_start M + R, with M and R independent of S_start.
     bf16 tensors: csrc/wkv7_time_split.cu does the whole of it.  Otherwise here:
     Pass 1 runs every segment twice (two concurrent launches of nseg*B*H chains): from the zero state with the real inputs
-    (final state = R) and from the identity state with v = 0 (final state = M).  A short host loop of nseg - 1 batched
-    64x64 products gives every segment's start state; pass 2 is the ordinary forward over the segments with those.
+    (final state = R) and from the identity state with v = 0 (final state = M).  nseg - 1 batched 64x64 products give
+    every segment's start state (_segment_starts); pass 2 is the ordinary forward over the segments with those.
     Three passes of length T/nseg instead of one of length T.  Results differ from the unsplit call by the rounding
     of M (single-TF32 products for bf16 tensors): y and sT agree within the path's tolerance, not bit for bit."""
     B, T, HC = w.shape
@@ -256,7 +256,7 @@ def _attn_tail_split(r, w, k, v, a, b, C, s0):
     """Forward only.  All chains but those of the last, partly filled round of SMs run as usual; the rest are cut in
     time (see tail_split_plan and _attn_time_split).  The three groups of launches go to three
     streams, write into views of one output tensor (head slices of the last batch entry, no copies) and share the
-    SMs.  Falls back to the plain call when the shape gives no such tail, and for bf16 tensors, whose kernel needs none of this."""
+    SMs.  Falls back to the plain call when the shape gives no such tail, and with the tcgen05 forward, which needs none of this."""
     B, T, HC = w.shape
     H = HC // C
     dev = w.device
@@ -311,7 +311,8 @@ def attn(r, w, k, v, a, b, HEAD_SIZE, *, s0=None, return_state=False, time_split
 
     time_split=n (no upstream counterpart; inference only, no autograd): the sequence runs as n segments in
     parallel, see _attn_time_split.  Pays when B*H is far below the number of SMs.
-    time_split='tail': only the chains of the last, partly filled round of SMs are cut in time, see _attn_tail_split."""
+    time_split='tail': only the chains of the last, partly filled round of SMs are cut in time, see _attn_tail_split (fp32
+    tensors; the bf16 forward spreads its chains evenly, there this is the plain call)."""
     if time_split is None and HEAD_SIZE == _lib.HEAD_SIZE and not th.compiler.is_compiling():
         out = _lib.ext().attn(r, w, k, v, a, b, s0, return_state)
         if out is not None:
