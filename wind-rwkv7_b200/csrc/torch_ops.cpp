@@ -57,21 +57,21 @@ bool plain(const Tensor& t) {
 // of Tensor, which see its operators; for forward-mode duals, for which its autograd functions raise; and under torch.jit.trace, which
 // records those functions but would see nothing here besides allocations.
 struct Eager {
-    // (asked tensor by tensor, the dual check costs a decode step 0.2 of its 6 us; there are no duals without a level)
-    const bool duals = torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr;
+    const bool duals;  // whether there can be any: asked tensor by tensor, it costs a decode step 0.2 of its 6 us
+    explicit Eager(bool autograd) : duals(autograd && torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr) {}
     bool operator()(const Tensor& t) const {
         PyObject* o = t.defined() ? t.unsafeGetTensorImpl()->pyobj_slot()->load_pyobj() : nullptr;
         return !o || (THPVariable_CheckExact(o) && !(duals && t._fw_grad(0).defined()));
     }
 };
-bool eager(std::initializer_list<const Tensor*> ts) {
-    const Eager ok;
+bool eager(std::initializer_list<const Tensor*> ts, bool autograd = true) {  // autograd: the Python form has an autograd function
+    const Eager ok(autograd);
     for (const Tensor* t : ts)
         if (!ok(*t)) return false;
     return !at::tracer::impl::is_dispatch_enabled();
 }
 bool eager(const variable_list& ts) {
-    const Eager ok;
+    const Eager ok(true);
     for (const Tensor& t : ts)
         if (!ok(t)) return false;
     return !at::tracer::impl::is_dispatch_enabled();
@@ -229,7 +229,7 @@ py::object attn_ln(const Tensor& r, const Tensor& w, const Tensor& k, const Tens
 py::object attn_step(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b, const OptTensor& state, bool inplace) {
     Rows q;
     const Tensor st = state.value_or(Tensor());
-    if (!eager({&r, &w, &k, &v, &a, &b, &st}) || !rows_of({&w, &r, &k, &v, &a, &b}, q) || !state_ok(state, q, w)) return py::none();
+    if (!eager({&r, &w, &k, &v, &a, &b, &st}, false) || !rows_of({&w, &r, &k, &v, &a, &b}, q) || !state_ok(state, q, w)) return py::none();
     Tensor y, sT;
     {
         py::gil_scoped_release nogil;
