@@ -307,6 +307,11 @@ __device__ __forceinline__ void load8f2(const unsigned char* p, F2 (&f)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) f[i] = f2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
 }
+__device__ __forceinline__ void load4f2(const unsigned char* p, F2 (&f)[2]) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    f[0] = f2(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u));
+    f[1] = f2(__uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

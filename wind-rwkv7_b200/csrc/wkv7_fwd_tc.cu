@@ -38,7 +38,7 @@
 // Checkpoint states leave through shared memory: tensor memory holds one state row per lane, so a warp-wide
 // store from registers can write one 32-byte sector per lane at best (512 wavefronts of the SM's L1 data
 // pipe per 16 KB state).  Instead each thread writes its row into a 128-byte-swizzled staging tile (two
-// [64 rows][32 floats] halves in the dead [wa;wq] / [kwi;bwi] tiles, conflict-free 16-byte stores) and one
+// [64 rows][32 floats] halves in the dead [wa;wq] / [kwi;bwi] tiles, conflict-free 8-byte stores) and one
 // thread issues two tensor-map bulk stores (cp.async.bulk.tensor.2d, shared -> global), which undo the
 // swizzle: the record in global memory stays plain row-major.
 // Every wait on an mbarrier is bounded; a wait that runs out raises an abort flag that makes all
@@ -241,23 +241,10 @@ __device__ __forceinline__ void tri_inverse_tc(const float* ABt, unsigned char* 
         *reinterpret_cast<float4*>(AIt + kchunk(col, q, 512)) = make_float4(rnd(r[2 * q].x), rnd(r[2 * q].y), rnd(r[2 * q + 1].x), rnd(r[2 * q + 1].y));
 }
 
-// two 16-byte chunks of an operand tile; R: round to TF32 (nearest) first, otherwise the tensor core
+// 16 bytes of an operand tile; R: round to TF32 (nearest) first, otherwise the tensor core
 // truncates the low 13 mantissa bits when it reads the operand
-template <bool R> __device__ __forceinline__ float4 quad(F2 a, F2 b) {
-    return R ? make_float4(rnd(a.x), rnd(a.y), rnd(b.x), rnd(b.y)) : make_float4(a.x, a.y, b.x, b.y);
-}
-template <bool R> __device__ __forceinline__ void store8t(unsigned char* p0, unsigned char* p1, const F2 (&f)[4]) {
-    *reinterpret_cast<float4*>(p0) = quad<R>(f[0], f[1]);
-    *reinterpret_cast<float4*>(p1) = quad<R>(f[2], f[3]);
-}
-// 32 bytes of an MN-major tile in two 16-byte stores; `flip` swaps the order of the two halves so that the
-// eight lanes of a quarter-warp (rows r..r+7, where r and r+4 share a 32-byte unit) never hit the same bank
-template <bool R> __device__ __forceinline__ void store8mn(unsigned char* p, const F2 (&f)[4], bool flip) {
-    const float4 lo = quad<R>(f[0], f[1]), hi = quad<R>(f[2], f[3]);
-    const int off = flip ? 16 : 0;
-    // selected float by float: a whole-struct select is turned back into unswapped stores (and 16-way bank conflicts)
-    *reinterpret_cast<float4*>(p + off) = make_float4(flip ? hi.x : lo.x, flip ? hi.y : lo.y, flip ? hi.z : lo.z, flip ? hi.w : lo.w);
-    *reinterpret_cast<float4*>(p + (16 - off)) = make_float4(flip ? lo.x : hi.x, flip ? lo.y : hi.y, flip ? lo.z : hi.z, flip ? lo.w : hi.w);
+template <bool R> __device__ __forceinline__ float4 quad4(const F2 (&f)[2]) {
+    return R ? make_float4(rnd(f[0].x), rnd(f[0].y), rnd(f[1].x), rnd(f[1].y)) : make_float4(f[0].x, f[0].y, f[1].x, f[1].y);
 }
 // A 16x16 matrix from its accumulator fragment into a K-major operand tile, rounded to TF32; entries with
 // column > row + keep are written as zero (keep = 16: all kept).
@@ -652,8 +639,10 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             __syncwarp();
             if (sdst && !seg_last) {
                 // checkpoint state: exact fp32 (the backward's tensor-core products read its upper 19 bits, its carried
-                // decay term all of them), staged in the 128-byte-swizzled layout the tensor-map store expects: half h = columns 32h..32h+31,
-                // row i at i*128 bytes, its 16-byte unit u at (u ^ (i & 7))
+                // decay term all of them), staged in the swizzled layout the tensor-map store expects: half h = columns 32h..32h+31,
+                // row i at i*128 bytes, its 32-byte unit u at (u ^ (i & 3)).  A half-warp's 8-byte stores cover four rows x 32 bytes: with
+                // 32-byte units they fill the 32 banks; with the 16-byte swizzle rows 2i and 2i + 1 met in the same ones (B64 T1024 H12:
+                // 372 us with them, 359 us without).
                 unsigned char* stage = gs + G_WAQ;
                 const int i = 16 * wg + (lane >> 2);  // rows i, i + 8
 #pragma unroll
@@ -665,7 +654,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     for (int j = 0; j < 4; ++j)
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
-                            *reinterpret_cast<uint2*>(stage + half * 8192 + (i + 8 * h) * 128 + (((2 * j + ((lane & 3) >> 1)) ^ (i & 7)) << 4) + (lane & 1) * 8) =
+                            *reinterpret_cast<uint2*>(stage + half * 8192 + (i + 8 * h) * 128 + ((j ^ (i & 3)) << 5) + (lane & 3) * 8) =
                                 make_uint2(x[4 * j + 2 * h], x[4 * j + 2 * h + 1]);
                 }
                 fence_async_smem();
@@ -703,13 +692,22 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 }
             }
         };
-        const int row = lane & 15, j0 = 16 * wg + 8 * (lane >> 4);
+        // Scan and operand tiles: a thread has two adjacent time steps x 4 adjacent key channels (quad), so that the running sum takes
+        // three shuffle rounds of 4 channels instead of four of 8 (a shuffle is a pass through the shared-memory pipe that this kernel
+        // is short of).  Slot 0 is the earlier or the later one (`late`) of the two steps, such that the eight lanes of a quarter-warp store to
+        // eight rows, every residue of the row mod 8 once and, with the quad's parity, all eight 16-byte units of the MN-major rows: neither
+        // the raw loads nor the tile stores have bank conflicts.  Lane bits 0, 1, 3: pair of time steps; bits 2, 4: quad.
+        // (One step x 8 channels: 359 us at B64 T1024 H12, 1904 us at B8 T16384 H40 without checkpoints; this: 354 and 1886 us.)
+        const int late = ((lane >> 1) ^ (lane >> 2) ^ (lane >> 3)) & 1;
+        const int quad = 4 * wg + ((lane >> 2) & 1) + ((lane >> 3) & 2), row0 = 2 * ((lane & 3) + ((lane >> 1) & 4)) + late;  // slot 1: row0 ^ 1
+        const int j0 = 4 * quad;
+        const float late0 = late ? 0.f : -1.f, late1 = late ? -1.f : 0.f;
         if (wg == 2 && grp < work.n && elect_one()) load_raw(0);
         __syncwarp();
         // Iteration k: read the results of own chunk k - 1, write the operand tiles of chunk k (whose scan is in registers),
         // start its score product; then scan chunk k + 1 while the score, inverse and chain warps finish chunk k.  (k = -1 only
         // scans, the last one only reads results: one copy of each piece of code.)
-        F2 o[4][4], v[4], fwv[4];  // wq, wa, kwi, bwi; kwf, bwf are formed from kwi, bwi and fw when the tiles are written
+        F2 o[4][2][2], v[2][2], fwv[2];  // [slot][channel pair] of wq, wa, kwi, bwi; kwf, bwf are formed from kwi, bwi and fw when the tiles are written
         for (int k = -1, v0 = grp - G; ; v0 += G, ++k) {
             if (k >= 0) {
                 // ---------------- results of the previous own chunk (its operand tiles are free afterwards) --
@@ -717,33 +715,38 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 if (v0 >= work.n) break;
                 // ---------------- operand tiles -----------------------------------------------------------
                 {
-                    const int jc = j0 >> 2;
-                    const int mo = (j0 >> 5) * 2048 + row * 128 + ((((j0 & 31) >> 3) ^ (row & 3)) << 5);
-                    const bool flip = (row >> 2) & 1;
-                    F2 kf[4], bf[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {  // k P_L / P_t first, then 2^-64
-                        kf[i] = mul2(mul2(o[2][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
-                        bf[i] = mul2(mul2(o[3][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                    for (int e = 0; e < 2; ++e) {
+                        const int row = row0 ^ e, mo = (quad >> 3) * 2048 + row * 128 + ((((quad >> 1) & 3) ^ (row & 3)) << 5) + (quad & 1) * 16;
+                        F2 kf[2], bf[2];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {  // k P_L / P_t first, then 2^-64
+                            kf[i] = mul2(mul2(o[2][e][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                            bf[i] = mul2(mul2(o[3][e][i], fwv[i]), f2(STATE_SCALE, STATE_SCALE));
+                        }
+                        *reinterpret_cast<float4*>(gs + G_KWF + mo) = quad4<RND>(kf);
+                        *reinterpret_cast<float4*>(gs + G_BWF + mo) = quad4<RND>(bf);
+                        *reinterpret_cast<float4*>(gs + G_V + mo) = quad4<false>(v[e]);  // bf16 values are exact in TF32
                     }
-                    store8mn<RND>(gs + G_KWF + mo, kf, flip);
-                    store8mn<RND>(gs + G_BWF + mo, bf, flip);
-                    store8mn<false>(gs + G_V + mo, v, flip);  // bf16 values are exact in TF32
-                    if (row & 8) {  // the decay blocks' entries, one per lane (see S_CUT)
-                        const F2 p01 = row & 2 ? fwv[1] : fwv[0], p23 = row & 2 ? fwv[3] : fwv[2], p4 = row & 4 ? p23 : p01;
-                        const float pl = (row & 1 ? p4.y : p4.x) * (STATE_SCALE * (1.f + S_CUT));  // where P_L underflows, so does S~ P_L
-                        const uint32_t dither = ((__float_as_uint(o[2][0].x) ^ __float_as_uint(o[3][0].x)) * 0x9e3779b1u) >> 19;
-                        *reinterpret_cast<uint32_t*>(gs + G_DF + (j0 >> 3) * 256 + ((row >> 2) & 1) * 128 + (row & 7) * 16 + (row & 3) * 4) =
+                    if (!(lane & 8)) {  // the decay blocks' entries, one per lane (see S_CUT): channel j0 + (lane & 3)
+                        const F2 p2 = lane & 2 ? fwv[1] : fwv[0];
+                        const float pl = (lane & 1 ? p2.y : p2.x) * (STATE_SCALE * (1.f + S_CUT));  // where P_L underflows, so does S~ P_L
+                        const uint32_t dither = ((__float_as_uint(o[2][0][0].x) ^ __float_as_uint(o[3][0][0].x)) * 0x9e3779b1u) >> 19;
+                        *reinterpret_cast<uint32_t*>(gs + G_DF + quad * 128 + ((quad & 1) * 4 + (lane & 3)) * 16 + (lane & 3) * 4) =
                             (__float_as_uint(pl) + dither) & 0xffffe000u;
                     }
                     if (k > 0 && p.ckpt) {  // the state's staging tiles are the next two operand tiles: wait until the bulk stores have read them
                         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                         group_bar(grp);
                     }
-                    store8t<RND>(gs + G_WAQ + kchunk(row, jc, 2048), gs + G_WAQ + kchunk(row, jc + 1, 2048), o[1]);
-                    store8t<RND>(gs + G_WAQ + kchunk(16 + row, jc, 2048), gs + G_WAQ + kchunk(16 + row, jc + 1, 2048), o[0]);
-                    store8t<RND>(gs + G_KB + kchunk(row, jc, 2048), gs + G_KB + kchunk(row, jc + 1, 2048), o[2]);
-                    store8t<RND>(gs + G_KB + kchunk(16 + row, jc, 2048), gs + G_KB + kchunk(16 + row, jc + 1, 2048), o[3]);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int at = kchunk(row0 ^ e, quad, 2048);
+                        *reinterpret_cast<float4*>(gs + G_WAQ + at) = quad4<RND>(o[1][e]);
+                        *reinterpret_cast<float4*>(gs + G_WAQ + 4096 + at) = quad4<RND>(o[0][e]);
+                        *reinterpret_cast<float4*>(gs + G_KB + at) = quad4<RND>(o[2][e]);
+                        *reinterpret_cast<float4*>(gs + G_KB + 4096 + at) = quad4<RND>(o[3][e]);
+                    }
                 }
                 if (ctrl->desc[grp][k & 3].flags & SEG_FIRST) load_state(ctrl->desc[grp][k & 3], wg);
                 fence_async_smem();
@@ -776,68 +779,85 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 __syncwarp();
             }
             // ---------------- decay scan of the next own chunk, into registers -----------------------
-            // One thread = one time step x 8 adjacent key channels.  The three transcendentals per
-            // element go to the special-function unit: with the matrix products on tcgen05 the FMA
+            // The three transcendentals per element go to the special-function unit: with the matrix products on tcgen05 the FMA
             // pipe and the issue slots are what this kernel runs out of, not MUFU throughput.
             if (v0 + G < work.n) {
                 mbar_wait<true>(&ctrl->raw[grp], (k + 1) & 1, ctrl, p.status);
-                const unsigned char* raw = gs + G_RAW + row * ROWB + (((j0 >> 3) ^ (row & 7)) << 4);
-                F2 cum[4], q[4], kk[4], a[4], b[4];
-                load8f2(raw + 1 * RAW_TILE, cum);
-                load8f2(raw + 0 * RAW_TILE, q);
-                load8f2(raw + 2 * RAW_TILE, kk);
-                load8f2(raw + 3 * RAW_TILE, a);
-                load8f2(raw + 4 * RAW_TILE, b);
-                load8f2(raw + 5 * RAW_TILE, v);
-                if (LN) {  // bonus dot sum_j r_j k_j bonus_j of this time step: 8 channels here, the rest by shuffle and in the epilogue
-                    F2 acc = f2(0.f, 0.f);
-                    const float4* bp = reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][(k + 1) & 3].hi) * N + j0);
+                F2 cum[2][2], q[2][2], kk[2][2], a[2][2], b[2][2];
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) {
-                        const float4 bo = __ldg(bp + i);
-                        acc = fma2(mul2(q[2 * i], kk[2 * i]), f2(bo.x, bo.y), acc);
-                        acc = fma2(mul2(q[2 * i + 1], kk[2 * i + 1]), f2(bo.z, bo.w), acc);
+                for (int e = 0; e < 2; ++e) {
+                    const int row = row0 ^ e;
+                    const unsigned char* raw = gs + G_RAW + row * ROWB + (((quad >> 1) ^ (row & 7)) << 4) + (quad & 1) * 8;
+                    load4f2(raw + 1 * RAW_TILE, cum[e]);
+                    load4f2(raw + 0 * RAW_TILE, q[e]);
+                    load4f2(raw + 2 * RAW_TILE, kk[e]);
+                    load4f2(raw + 3 * RAW_TILE, a[e]);
+                    load4f2(raw + 4 * RAW_TILE, b[e]);
+                    load4f2(raw + 5 * RAW_TILE, v[e]);
+                }
+                if (LN) {  // bonus dot sum_j r_j k_j bonus_j of these time steps: 4 channels here, the rest by shuffle and in the epilogue
+                    const float4 bo = __ldg(reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][(k + 1) & 3].hi) * N + j0));
+                    float dot[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const F2 acc = fma2(mul2(q[e][1], kk[e][1]), f2(bo.z, bo.w), mul2(mul2(q[e][0], kk[e][0]), f2(bo.x, bo.y)));
+                        dot[e] = acc.x + acc.y;
                     }
-                    float dot = acc.x + acc.y;
-                    dot += __shfl_xor_sync(0xffffffffu, dot, 16);
-                    if (lane < 16) ctrl->bdot[grp][(k + 1) & 1][wg][row] = dot;
+                    float first = late ? dot[1] : dot[0], second = late ? dot[0] : dot[1];  // (lanes of the other quads have them in the other slot)
+                    first += __shfl_xor_sync(0xffffffffu, first, 4);
+                    second += __shfl_xor_sync(0xffffffffu, second, 4);
+                    first += __shfl_xor_sync(0xffffffffu, first, 16);
+                    second += __shfl_xor_sync(0xffffffffu, second, 16);
+                    if (!(lane & 0x14)) *reinterpret_cast<float2*>(&ctrl->bdot[grp][(k + 1) & 1][wg][row0 & 14]) = make_float2(first, second);
                 }
                 // log2 of the per-step decay: -exp(w) * log2(e); running sum along the 16 time rows
                 constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // the per-step floor in log2 units
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    cum[i] = mul2(cum[i], f2(LOG2E, LOG2E));
-                    cum[i] = mul2(f2(ex2_approx(cum[i].x), ex2_approx(cum[i].y)), f2(-LOG2E, -LOG2E));
-                    cum[i] = f2(fmaxf(cum[i].x, FLOOR), fmaxf(cum[i].y, FLOOR));
-                }
-                if (TAIL && ctrl->desc[grp][(k + 1) & 3].c + 1 == nchunks && row >= tail) {  // a row beyond the end of the sequence: no decay, the state passes through
+                for (int e = 0; e < 2; ++e)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) cum[i] = f2(0.f, 0.f);
-                }
-                F2 step[4];  // this row's own log2 decay: P_{t-1} = 2^(cum_t - step_t), cheaper than a shuffle for the row above
+                    for (int i = 0; i < 2; ++i) {
+                        F2 x = mul2(cum[e][i], f2(LOG2E, LOG2E));
+                        x = mul2(f2(ex2_approx(x.x), ex2_approx(x.y)), f2(-LOG2E, -LOG2E));
+                        cum[e][i] = f2(fmaxf(x.x, FLOOR), fmaxf(x.y, FLOOR));
+                        // a row beyond the end of the sequence: no decay, the state passes through
+                        if (TAIL && ctrl->desc[grp][(k + 1) & 3].c + 1 == nchunks && (row0 ^ e) >= tail) cum[e][i] = f2(0.f, 0.f);
+                    }
+                F2 sum[2];  // through the later step of the pair
 #pragma unroll
-                for (int i = 0; i < 4; ++i) step[i] = cum[i];
+                for (int i = 0; i < 2; ++i) sum[i] = add2(cum[0][i], cum[1][i]);
 #pragma unroll
-                for (int d = 1; d < 16; d <<= 1)
+                for (int d = 1; d < 4; d <<= 1)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const F2 up = f2(__shfl_up_sync(0xffffffffu, cum[i].x, d, 16), __shfl_up_sync(0xffffffffu, cum[i].y, d, 16));
-                        if (row >= d) cum[i] = add2(cum[i], up);
+                    for (int i = 0; i < 2; ++i) {
+                        const F2 up = f2(__shfl_up_sync(0xffffffffu, sum[i].x, d, 4), __shfl_up_sync(0xffffffffu, sum[i].y, d, 4));
+                        if ((lane & 3) >= d) sum[i] = add2(sum[i], up);
                     }
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < 2; ++i) {
+                    const int src = (lane & 0x14) | 3;
+                    const F2 low = f2(__shfl_sync(0xffffffffu, sum[i].x, src), __shfl_sync(0xffffffffu, sum[i].y, src));
+                    if (lane & 8) sum[i] = add2(sum[i], low);
+                }
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
                     // P~_t = 2^64 P_t and its reciprocal (see ANCHOR_LN): both finite for cum >= -179 (2^-115 ~ e^-80)
-                    const F2 ca = add2(cum[i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = fma2(step[i], f2(-1.f, -1.f), ca);
-                    const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
-                    const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
-                    const F2 inv = f2(ex2_approx(-cx), ex2_approx(-cy));
-                    const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
-                    o[0][i] = mul2(q[i], incl);   // wq
-                    o[1][i] = mul2(a[i], non);    // wa
-                    o[2][i] = mul2(kk[i], inv);   // kwi
-                    o[3][i] = mul2(b[i], inv);    // bwi
+                    const F2 sa = add2(sum[i], f2(ANCHOR_LOG2, ANCHOR_LOG2));
                     // P~_L = 2^64 P_L (P_L itself may lie below fp32's normal range)
-                    fwv[i] = f2(__shfl_sync(0xffffffffu, incl.x, 15, 16), __shfl_sync(0xffffffffu, incl.y, 15, 16));
+                    const int src = (lane & 0x14) | 11;
+                    fwv[i] = f2(ex2_approx(fmaxf(__shfl_sync(0xffffffffu, sa.x, src), -115.f)), ex2_approx(fmaxf(__shfl_sync(0xffffffffu, sa.y, src), -115.f)));
+                    const F2 c[2] = {fma2(cum[1][i], f2(late0, late0), sa), fma2(cum[0][i], f2(late1, late1), sa)};  // less the later step's, in the earlier one
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const F2 cp = fma2(cum[e][i], f2(-1.f, -1.f), c[e]);  // without this step's own decay
+                        const float cx = fmaxf(c[e].x, -115.f), cy = fmaxf(c[e].y, -115.f);
+                        const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
+                        const F2 inv = f2(ex2_approx(-cx), ex2_approx(-cy));
+                        const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
+                        o[0][e][i] = mul2(q[e][i], incl);   // wq
+                        o[1][e][i] = mul2(a[e][i], non);    // wa
+                        o[2][e][i] = mul2(kk[e][i], inv);   // kwi
+                        o[3][e][i] = mul2(b[e][i], inv);    // bwi
+                    }
                 }
             }
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // y's tile has been read (its issuer only)
@@ -860,7 +880,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 }
 
 // Tensor map over the checkpoint buffer seen as an fp32 matrix [records * 80 rows][64 floats]; box = 64 rows x
-// 32 floats (128 bytes) with the 128-byte swizzle.  Encoded through the runtime's driver-entry-point query
+// 32 floats (128 bytes) with the 128-byte swizzle of 32-byte units.  Encoded through the runtime's driver-entry-point query
 // (the library does not link against libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -878,7 +898,7 @@ static bool encode_checkpoint_map(CUtensorMap* m, float* base, long long records
     const cuuint32_t box[2] = {32, (cuuint32_t)N};
     const cuuint32_t es[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+              CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 __device__ __align__(128) __nv_bfloat16 g_zero_row[N];
