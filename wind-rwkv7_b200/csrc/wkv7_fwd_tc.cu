@@ -5,33 +5,35 @@
 // different machine mapping.  One CTA per SM walks its share of the chunks (WorkSplit: whole chains and at most two pieces of
 // cut ones).  The 64x64 state S[value][key] lives in tensor memory and is never held in registers: per 16-step chunk one
 // elected thread issues 24 tcgen05.mma instructions (M = 64 value rows, TF32 operands, fp32 accumulate)
-//     hop 1   [X | Yp] = S [wa;wq]^T + V^T [AK;QK]^T        A = S straight from tensor memory
-//             S' = S diag(fw) + V^T kwf                      into the next of four state buffers; eight N = 8 products
-//                                                            apply the decay; issued while hop 1 drains
+//     ahead   [X | Yp] = V^T [AK;QK]^T,  S' = V^T kwf        needs no state: issued while the chunk before it drains; A = V^T from
+//                                                            tensor memory, S' in the next of four state buffers
+//     hop 1   [X | Yp] += S [wa;wq]^T                        A = S straight from tensor memory
+//             S' += S diag(fw)                               eight N = 8 products apply the decay; issued while hop 1 drains
 //     hop 2   S' += X (AI^T bwf),  Y = Yp + X (QB AI)^T      A = X from tensor memory
 // with kwf = kwi*fw, bwf = bwi*fw, so the column scaling of the state never touches a CUDA core.  U = X AI^T itself is never
 // formed: AI^T bwf and QB AI come from two small products off the chain.  An accumulator that the next product reads as its A
 // operand needs an explicit completion wait (tcgen05.commit -> mbarrier); only same-accumulator products are ordered by the
-// tensor pipe.  With three hops (U explicit) and a wait for "results of chunk c-2 read" a chunk took the chain 2000 cycles,
-// most of them waits; what bounds it now is the latency from a chunk's operand tiles to its completion over the four chunks
-// in flight (shared memory has room for four sets of tiles): about 1700 cycles per chunk without checkpoints (B8 T65536 H40), 2250 with
-// (B64 T1024 H12).
+// tensor pipe.
+// What bounds it: three things at once, none of which is saturated alone.  The chain's two round trips (1000 cycles a chunk in the
+// running kernel, 560 alone: 210 for a product, its commit and the wait, 5 to 38 for each further product); the latency from a chunk's
+// operand tiles to its completion, some 5500 cycles, over the four chunks in flight (shared memory has no room for a fifth);
+// and the shared-memory data pipe, some 1200 wavefronts a chunk, that both stand in.  About 1450 cycles a chunk without checkpoints
+// (B8 T65536 H40), 1800 with (B64 T1024 H12: 338 us, 5.0 TB/s of HBM traffic).  Before the V parts went ahead of the chain and off shared
+// memory, and the scores, the inverse and the fold each had warps of their own: 1550 and 1860.
 //
-// Warp roles (128 (G+1) threads).  Warps 0..4G-1 are G preparation groups of four warps, each working on its own chunk
-// (position g, g+G, ... of the CTA's list): the decay scan of the six input tiles (bulk tensor loads, one chunk ahead), the
-// operand tiles in the shared-memory layouts the tensor core reads, the four 16x16 score matrices as ONE tcgen05 product
-// ([wa;wq] x [kwi;bwi]^T, M = 64 of which 32 rows are used), and afterwards the read-back of Y (and of the chunk-end state for
-// the checkpoints).  The scan of a group's next chunk is computed into registers while its current one goes through the rest.
-// Warps 4G, 4G+1 read the scores back from their quarter of tensor memory, mask them and write AK, AB, QK, QB; warp 4G+2
-// inverts (I - AB) and issues the two fold products, whose results warps 4G, 4G+1 write as operand tiles; warp 4G+3 issues
-// the chain.  (With the scores, the inverse and the fold done by the preparation groups, three of a group's four warps
-// waited through half of its time.)  The kernel's hot code has to stay small: its warps run different parts of it at the same
+// Warp roles (128 (G+2) threads).  Warps 0..4G-1 are G preparation groups of four warps, each working on its own chunk (c, c+G, ...).
+// Eight service warps serve all groups, each a stage of a chunk's way to the chain (a warp takes some 500 cycles per stage, so that a
+// stage shared with another one makes chunks wait): 4G, 4G+1 read the scores back from their quarter of tensor memory, mask them and write
+// AK, AB, QK, QB; 4G+2, 4G+6 invert (I - AB) (even and odd groups); 4G+4, 4G+5, 4G+7 form the two fold products; 4G+3 issues
+// the chain.  The kernel's hot code has to stay small: its warps run different parts of it at the same
 // time out of one instruction cache, and 10 KB more of it cost 30 % once all SMs missed at the same time.
+// (Not better: the scores by mma.sync in the preparation warps - every operand is read four times, 1.2 times slower; forming the
+// inverse's two 8x8 blocks in lanes 0-15 only, 1 % slower.)
 //
 // Shared-memory operand layouts (the tiles are produced by threads, not copied):
 //   K-major (contraction index contiguous): 16-byte chunks [row/8][k/4][row%8][k%4], descriptor
 //     LBO = 128 B (next k-chunk), SBO = bytes per 8-row group, no swizzle.
-//   MN-major TF32 (V, kwf, bwf: contraction index = time): only the 128-byte swizzle with 32-byte
+//   MN-major TF32 (kwf, bwf: contraction index = time): only the 128-byte swizzle with 32-byte
 //     base exists for 32-bit MN-major operands: rows of 32 channels (128 B) per time step, the
 //     32-byte unit index XOR-ed with (t % 4); LBO = stride between the two 32-channel halves,
 //     SBO = 512 B (four time steps).
@@ -57,8 +59,10 @@ constexpr int RAW_TILE = L * ROWB;  // 2048
 // per-group shared memory (byte offsets; tensor-core tiles first, all 1024-byte aligned)
 constexpr int G_WAQ = 0;       // [wa;wq]   32 rows x 64, K-major            8192
 constexpr int G_KB = 8192;     // [kwi;bwi] 32 rows x 64, K-major            8192 (directly after WAQ: the M = 64 score
-                               //                                                 product reads rows 32..63 from here, unused)
-constexpr int G_V = 16384;     // V   [time][value]  MN-major                4096
+                               //                                                 product reads rows 32..63 from here, unused);
+                               // time step s of every eight in row kb_row(s): the score product's columns then come back as
+                               // 8x4 blocks with a column per lane, which stmatrix can store
+constexpr int G_V = 16384;     // attn_ln's epilogue only: V [time][value], bf16, 16-byte units XOR-ed with the row   2048 (of 4096)
 constexpr int G_KWF = 20480;   // kwf [time][key]    MN-major                4096
 constexpr int G_BWF = 24576;   // bwf [time][key]    MN-major                4096
 constexpr int G_SC = 28672;    // [AK;QK]  32 rows x 16, K-major             2048
@@ -66,7 +70,7 @@ constexpr int G_AI = 30720;    // AI^T     16 x 16, K-major                  102
 constexpr int G_QB = 31744;    // QB       16 x 16, K-major                  1024
 static_assert(G_AI == G_SC + 2048 && G_QB == G_AI + 1024, "[AK;QK], AI^T, QB must be contiguous: they leave as one bulk copy");
 constexpr int G_DF = 32768;    // eight 8x8 diagonal blocks of fw, K-major   2048
-constexpr int G_ABT = 34816;   // AB transposed, fp32 [16][SCS]              1536
+constexpr int G_ABT = 34816;   // AB transposed, fp32 [16][ABS]              1536
 constexpr int G_QBU = 34816;   // QB AI, 16 x 16, K-major (AB is dead by then) 1024
 constexpr int G_RAW = 36864;   // q, w, k, a, b, v staging                   6 * 2048
 constexpr int G_Y = 49152;            // the chunk's output as [time][value], bf16, 128-byte swizzle             2048
@@ -82,8 +86,8 @@ constexpr int LN_PART = L * LN_YS * 4;     // byte offset of the per-warp partia
 constexpr int C_S = 0;       // four 64-column state buffers: chunk c reads c % 4 and writes (c + 1) % 4
 constexpr int C_INIT = 256;  // start state of the next segment (written by the group that prepares its first chunk)
 constexpr int C_XY = 320;    // + 32 * group: X (16) | Y (16) of the group's chunk; before that its score products,
-                             // [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47, and then QB AI in lanes 32-47 of columns 16-31
-constexpr int C_FOLD = 448;  // AI^T bwf (64) in lanes 0-15
+                             // [AK|AB] in lanes 0-15, [QK|QB] in lanes 32-47 (columns permuted, see G_KB)
+constexpr int C_V = 448;     // + 16 * group: V^T [value][time] of the group's chunk
 
 // Any wait of this kernel may stand still while one of its groups waits for the state of a cut chain: the chain warp (full), the
 // score and inverse warps (score, fold, mats, fread), and the other groups (done).
@@ -115,14 +119,14 @@ struct ChunkDesc {
 enum : int { SEG_FIRST = 1, SEG_LAST = 2 };  // first / last chunk of a segment
 
 struct Ctrl {
-    uint64_t full[4], done[4], score[4], raw[4], gate[4], mats[4], fold[4], rec[4], fread, hop;
+    uint64_t full[4], done[4], score[4], raw[4], gate[4], mats[4], inv[4], rec[4], hop;
     uint32_t tmem_base;
     volatile int abort;
     ChunkDesc desc[4][4];      // [group][own-chunk number mod 4]: where the chunk lies (written one iteration ahead by the group)
     float bdot[4][2][4][L];    // attn_ln: per-warp partial bonus dots [group][iteration parity][warp][time]
     // abort path only, a set per warp: completion of its products, and what its waits take in place of the abort flag
-    uint64_t drain[20];
-    volatile int never_set[20];
+    uint64_t drain[24];
+    volatile int never_set[24];
 };
 
 // Bounded wait for the phase with the given parity.  Returns at once when the CTA has aborted.
@@ -193,6 +197,10 @@ __device__ __forceinline__ void tmem_ld_frag4(uint32_t ta, uint32_t* v) {  // 32
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(v[0]),"=r"(v[1]),"=r"(v[2]),"=r"(v[3]),"=r"(v[4]),"=r"(v[5]),"=r"(v[6]),"=r"(v[7]),"=r"(v[8]),"=r"(v[9]),"=r"(v[10]),"=r"(v[11]),"=r"(v[12]),"=r"(v[13]),"=r"(v[14]),"=r"(v[15]) : "r"(ta));
 }
+__device__ __forceinline__ void tmem_st_frag(uint32_t ta, const uint32_t* v) {  // the layout of tmem_ld_frag
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
+        :: "r"(v[0]),"r"(v[1]),"r"(v[2]),"r"(v[3]),"r"(v[4]),"r"(v[5]),"r"(v[6]),"r"(v[7]), "r"(ta) : "memory");
+}
 __device__ __forceinline__ void tmem_st16(uint32_t ta, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
         :: "r"(v[0]),"r"(v[1]),"r"(v[2]),"r"(v[3]),"r"(v[4]),"r"(v[5]),"r"(v[6]),"r"(v[7]),"r"(v[8]),"r"(v[9]),"r"(v[10]),"r"(v[11]),"r"(v[12]),"r"(v[13]),"r"(v[14]),"r"(v[15]), "r"(ta) : "memory");
@@ -204,41 +212,76 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // without.)
 __device__ __forceinline__ float rnd(float x) { return __uint_as_float(tf32_rna(x)); }
 
+__device__ __forceinline__ int kb_row(int s) { return (s & 8) | ((s & 3) << 1) | ((s >> 2) & 1); }
 // byte offset of the 16-byte chunk holding (row, k..k+3) in a K-major tile; sbo = bytes per 8-row group
 __device__ __forceinline__ int kchunk(int row, int kc, int sbo) { return (row >> 3) * sbo + kc * 128 + (row & 7) * 16; }
 
-// Column `col` of AI = (I - AB)^-1 (AB strictly lower triangular), written as row `col` of the K-major tile of AI^T.
-// Right-looking substitution as in tri_inverse_column().
-template <int S_> __device__ __forceinline__ void tri_fetch_tc(F2 (&dst)[L / 2], const float* ABt) {  // row S_ of ABt, entries > S_
+constexpr int ABS = 20;  // row pitch (floats) of the transposed AB: rows of 16-byte pieces and single columns are both conflict-free
+// AI = (I - AB)^-1 (AB strictly lower triangular) into the K-major tile of AI^T, one warp.  In 8x8 blocks, AI = [X11, 0; X21, X22] with
+// X21 = X22 A21 X11: the two diagonal blocks by right-looking substitution side by side (7 dependent steps instead of 15, a lane per
+// column), then the two products, all 32 lanes.  ABt[s][t] = AB[t][s]; its blocks are overwritten once they have been used.
+template <int S_> __device__ __forceinline__ void tri_fetch_tc(F2 (&dst)[4], const float* At) {  // row S_ of the block, entries > S_
 #pragma unroll
-    for (int v = (S_ + 1) / 4; v < L / 4; ++v) {
-        const float4 x = *reinterpret_cast<const float4*>(ABt + S_ * SCS + 4 * v);
+    for (int v = (S_ + 1) / 4; v < 2; ++v) {
+        const float4 x = *reinterpret_cast<const float4*>(At + S_ * ABS + 4 * v);
         dst[2 * v] = f2(x.x, x.y); dst[2 * v + 1] = f2(x.z, x.w);
     }
 }
-template <int S_> __device__ __forceinline__ void tri_step_tc(F2 (&r)[L / 2], const F2 (&c)[L / 2], F2 (&cn)[L / 2], const float* ABt) {
-    if (S_ + 1 < L - 1) tri_fetch_tc<(S_ + 1 < L - 1 ? S_ + 1 : 0)>(cn, ABt);
+template <int S_> __device__ __forceinline__ void tri_step_tc(F2 (&r)[4], const F2 (&c)[4], F2 (&cn)[4], const float* At) {
+    if (S_ + 1 < 7) tri_fetch_tc<(S_ + 1 < 7 ? S_ + 1 : 0)>(cn, At);
     const float ms = S_ & 1 ? r[S_ / 2].y : r[S_ / 2].x;
     if (!(S_ & 1)) r[S_ / 2].y = fmaf(c[S_ / 2].y, ms, r[S_ / 2].y);
 #pragma unroll
-    for (int h = S_ / 2 + 1; h < L / 2; ++h) r[h] = fma2(c[h], f2(ms, ms), r[h]);
+    for (int h = S_ / 2 + 1; h < 4; ++h) r[h] = fma2(c[h], f2(ms, ms), r[h]);
 }
-__device__ __forceinline__ void tri_inverse_tc(const float* ABt, unsigned char* AIt, int col) {
-    F2 r[L / 2], ca[L / 2], cb[L / 2];
+__device__ __forceinline__ void tri_inverse_tc(float* ABt, unsigned char* AIt, int lane) {
+    const int c = lane & 7, blk = (lane >> 3) & 1, p = lane >> 3;  // (lanes 16..31 repeat 0..15 up to the products)
+    {
+        const float* At = ABt + 8 * blk * (ABS + 1);
+        F2 r[4], ca[4], cb[4];
 #pragma unroll
-    for (int h = 0; h < L / 2; ++h) r[h] = f2(2 * h == col ? 1.f : 0.f, 2 * h + 1 == col ? 1.f : 0.f);
-    tri_fetch_tc<0>(ca, ABt);
-    tri_step_tc<0>(r, ca, cb, ABt);   tri_step_tc<1>(r, cb, ca, ABt);
-    tri_step_tc<2>(r, ca, cb, ABt);   tri_step_tc<3>(r, cb, ca, ABt);
-    tri_step_tc<4>(r, ca, cb, ABt);   tri_step_tc<5>(r, cb, ca, ABt);
-    tri_step_tc<6>(r, ca, cb, ABt);   tri_step_tc<7>(r, cb, ca, ABt);
-    tri_step_tc<8>(r, ca, cb, ABt);   tri_step_tc<9>(r, cb, ca, ABt);
-    tri_step_tc<10>(r, ca, cb, ABt);  tri_step_tc<11>(r, cb, ca, ABt);
-    tri_step_tc<12>(r, ca, cb, ABt);  tri_step_tc<13>(r, cb, ca, ABt);
-    tri_step_tc<14>(r, ca, cb, ABt);
+        for (int h = 0; h < 4; ++h) r[h] = f2(2 * h == c ? 1.f : 0.f, 2 * h + 1 == c ? 1.f : 0.f);
+        tri_fetch_tc<0>(ca, At);
+        tri_step_tc<0>(r, ca, cb, At);  tri_step_tc<1>(r, cb, ca, At);
+        tri_step_tc<2>(r, ca, cb, At);  tri_step_tc<3>(r, cb, ca, At);
+        tri_step_tc<4>(r, ca, cb, At);  tri_step_tc<5>(r, cb, ca, At);
+        tri_step_tc<6>(r, ca, cb, At);
+        __syncwarp();
+        if (lane < 16) {
+            // X11[.][c] to row 8 + c (zeros and unused until now), X22[.][c] to row c (A11's place)
+            float* x = ABt + (8 * (1 - blk) + c) * ABS;
+            *reinterpret_cast<float4*>(x) = make_float4(r[0].x, r[0].y, r[1].x, r[1].y);
+            *reinterpret_cast<float4*>(x + 4) = make_float4(r[2].x, r[2].y, r[3].x, r[3].y);
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-        *reinterpret_cast<float4*>(AIt + kchunk(col, q, 512)) = make_float4(rnd(r[2 * q].x), rnd(r[2 * q].y), rnd(r[2 * q + 1].x), rnd(r[2 * q + 1].y));
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float4*>(AIt + blk * 512 + (2 * blk + q) * 128 + c * 16) =
+                    make_float4(rnd(r[2 * q].x), rnd(r[2 * q].y), rnd(r[2 * q + 1].x), rnd(r[2 * q + 1].y));
+        } else {  // AI^T below its diagonal blocks
+            *reinterpret_cast<float4*>(AIt + 512 + blk * 128 + c * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+    }
+    // column c, rows 2 p, 2 p + 1 of T = A21 X11 and of X21 = X22 T
+    auto col_product = [&](const float* mt, const float* col) {
+        F2 acc[2] = {f2(0.f, 0.f), f2(0.f, 0.f)};
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+            const float4 x = *reinterpret_cast<const float4*>(col + 4 * v);
+            const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 m = *reinterpret_cast<const float2*>(mt + (4 * v + i) * ABS + 2 * p);
+                acc[i & 1] = fma2(f2(m.x, m.y), f2(xs[i], xs[i]), acc[i & 1]);
+            }
+        }
+        return add2(acc[0], acc[1]);
+    };
+    float* t = ABt + (8 + c) * ABS + 8;
+    const F2 tc = col_product(ABt + 8, ABt + (8 + c) * ABS);
+    *reinterpret_cast<float2*>(t + 2 * p) = make_float2(tc.x, tc.y);  // (A22's place)
+    __syncwarp();
+    const F2 x = col_product(ABt, t);
+    *reinterpret_cast<float2*>(AIt + (2 + (p >> 1)) * 128 + c * 16 + (p & 1) * 8) = make_float2(rnd(x.x), rnd(x.y));
 }
 
 // 16 bytes of an operand tile; R: round to TF32 (nearest) first, otherwise the tensor core
@@ -246,17 +289,28 @@ __device__ __forceinline__ void tri_inverse_tc(const float* ABt, unsigned char* 
 template <bool R> __device__ __forceinline__ float4 quad4(const F2 (&f)[2]) {
     return R ? make_float4(rnd(f[0].x), rnd(f[0].y), rnd(f[1].x), rnd(f[1].y)) : make_float4(f[0].x, f[0].y, f[1].x, f[1].y);
 }
-// A 16x16 matrix from its accumulator fragment into a K-major operand tile, rounded to TF32; entries with
-// column > row + keep are written as zero (keep = 16: all kept).
-__device__ __forceinline__ void store_frag16(unsigned char* tile, const uint32_t* x, int r0, int c0, int keep) {
+template <bool R> __device__ __forceinline__ F2 rnd2(F2 a) { return R ? f2(rnd(a.x), rnd(a.y)) : a; }
+// four 8x4 blocks of 32-bit elements, 16 bytes of each of their rows at the address of lane 8 * block + row: lane 4 r + c has element (r, c)
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t saddr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
+}
+__device__ __forceinline__ void stmatrix4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// A 16x16 matrix into a K-major operand tile, rounded to TF32: x[4 j + 2 h + e] is row lane / 4 + 8 h, column 8 j + 4 e + lane % 4.
+// Entries with column > row + keep are written as zero.
+__device__ __forceinline__ void store_frag16(uint32_t tile, const uint32_t* x, int lane, int keep) {
+    const uint32_t at = tile + ((lane >> 3) & 1) * 128 + (lane >> 4) * 512 + (lane & 7) * 16;  // blocks (h, e) = (0, 0), (0, 1), (1, 0), (1, 1)
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < 2; ++j) {
+        uint32_t v[4];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int row = r0 + 8 * h, col = 8 * j + c0;
-            *reinterpret_cast<float2*>(tile + kchunk(row, col >> 2, 512) + (col & 3) * 4) =
-                make_float2(col <= row + keep ? rnd(__uint_as_float(x[4 * j + 2 * h])) : 0.f, col + 1 <= row + keep ? rnd(__uint_as_float(x[4 * j + 2 * h + 1])) : 0.f);
+        for (int i = 0; i < 4; ++i) {
+            const int row = (lane >> 2) + 8 * (i >> 1), col = 8 * j + 4 * (i & 1) + (lane & 3);
+            v[i] = col <= row + keep ? tf32_rna(__uint_as_float(x[4 * j + i])) : 0u;
         }
+        stmatrix4(at + j * 256, v[0], v[1], v[2], v[3]);
+    }
 }
 __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
@@ -268,17 +322,17 @@ __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi) {
 struct alignas(64) FwdMaps { CUtensorMap ck, y, in[6], g; };  // checkpoint states; output; q, w, k, a, b, v; gate
 
 template <int G, bool RND, bool LN, bool TAIL>
-__global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams p, WorkSplit ws, const __grid_constant__ FwdMaps maps) {
+__global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams p, WorkSplit ws, const __grid_constant__ FwdMaps maps) {
     using IoT = __nv_bfloat16;
     constexpr int G_BYTES = LN ? G_BYTES_LN : G_BYTES_PLAIN;
     constexpr int NCOLS = 512;
-    static_assert(C_XY + 32 * G <= C_FOLD && C_FOLD + 64 <= NCOLS, "tensor memory columns");
+    static_assert(C_XY + 32 * G <= C_V && C_V + 16 * G <= NCOLS, "tensor memory columns");
     // Register reallocation (G == 4 only).  setmaxnreg.inc blocks, without a bound, until the CTA's
-    // register pool can satisfy it, and the pool is what the CTA was launched with: 640 threads x 96
-    // registers (65536 / 640 rounded down to a multiple of 8; build.py checks that ptxas reports 96).
+    // register pool can satisfy it, and the pool is what the CTA was launched with: 768 threads x 80
+    // registers (65536 / 768 rounded down to a multiple of 8; build.py checks that ptxas reports 80).
     // The raised and lowered counts must therefore fit into that pool exactly or with room to spare.
-    constexpr int LAUNCH_REGS = 96, PREP_REGS = 104, CHAIN_REGS = 64;
-    static_assert(G != 4 || 128 * G * PREP_REGS + 128 * CHAIN_REGS <= 128 * (G + 1) * LAUNCH_REGS, "setmaxnreg would never be satisfied");
+    constexpr int LAUNCH_REGS = 80, PREP_REGS = 96, SERVICE_REGS = 48;
+    static_assert(G != 4 || 128 * G * PREP_REGS + 256 * SERVICE_REGS <= 128 * (G + 2) * LAUNCH_REGS, "setmaxnreg would never be satisfied");
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* sm = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     Ctrl* ctrl = reinterpret_cast<Ctrl*>(sm + G * G_BYTES);
@@ -291,9 +345,9 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 
     if (tid == 0) {
         for (int g = 0; g < G; ++g) {
-            mbar_init(&ctrl->full[g], 2);
+            mbar_init(&ctrl->full[g], 3);
             mbar_init(&ctrl->mats[g], 2);
-            mbar_init(&ctrl->fold[g], 1);
+            mbar_init(&ctrl->inv[g], 1);
             mbar_init(&ctrl->rec[g], 1);
             mbar_init(&ctrl->done[g], 1);
             mbar_init(&ctrl->score[g], 1);
@@ -301,7 +355,6 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
             mbar_init(&ctrl->gate[g], 1);
         }
         mbar_init(&ctrl->hop, 1);
-        mbar_init(&ctrl->fread, 1);
         ctrl->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -366,39 +419,48 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
     };
 
     if (warp >= 4 * G) {
-        // ------------------------------ chain warp group -----------------------------------------
-        if (G == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CHAIN_REGS));
+        // ------------------------------ service warps -----------------------------------------
+        if (G == 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SERVICE_REGS));
+        const int q = warp & 3;  // (of the score and fold warps:) tensor-memory lanes 0-15 or 32-47
+        const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);
         if (warp == 4 * G + 3) {
           if (elect_one()) {
             const uint32_t sb = smem_u32(sm);
             int seg_first = 0;  // list position at which the next segment begins
+            // The V parts of chunk c's products, X | Yp and S', need no state: they are issued while the chunk before it drains.
+            // The group has read the results of its previous chunk by the time it is full, so the buffers about to be written
+            // (X | Y of this group, and the state buffer, last read for chunk c - 4) are free.
+            auto start_chunk = [&](int c) {
+                const int g = c % G;
+                const uint32_t gb = sb + g * G_BYTES, Sn = tmem + C_S + 64 * ((c + 1) & 3), XY = tmem + C_XY + 32 * g;
+                const uint64_t dSC = desc_kmajor(gb + G_SC, 512), dKWF = desc_mnmajor(gb + G_KWF);
+                const uint32_t V = tmem + C_V + 16 * g;
+                mbar_wait<false>(&ctrl->full[g], (c / G) & 1, ctrl, p.status);
+                tc_fence_after();
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks) mma_ts(XY, V + 8 * ks, dSC + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
+#pragma unroll
+                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, V + 8 * ks, dKWF + (uint64_t)(ks * 64), idesc(64, false, true), ks > 0);
+            };
+            start_chunk(0);
             for (int c = 0; c < work.n; ++c) {  // position in the CTA's list
                 const int g = c % G, k = c / G;
                 const uint32_t gb = sb + g * G_BYTES;
-                const uint64_t dWAQ = desc_kmajor(gb + G_WAQ, 2048), dSC = desc_kmajor(gb + G_SC, 512),
-                               dQBU = desc_kmajor(gb + G_QBU, 512), dDF = desc_kmajor(gb + G_DF, 256);
-                const uint64_t dV = desc_mnmajor(gb + G_V), dKWF = desc_mnmajor(gb + G_KWF), dBWU = desc_mnmajor(gb + G_BWF);
+                const uint64_t dWAQ = desc_kmajor(gb + G_WAQ, 2048), dQBU = desc_kmajor(gb + G_QBU, 512), dDF = desc_kmajor(gb + G_DF, 256);
+                const uint64_t dBWU = desc_mnmajor(gb + G_BWF);
                 const uint32_t Sn = tmem + C_S + 64 * ((c + 1) & 3), XY = tmem + C_XY + 32 * g;
                 uint32_t Sa = tmem + C_S + 64 * (c & 3);
                 if (c == seg_first) {
                     Sa = tmem + C_INIT;
                     seg_first = c < work.h ? work.h : c < work.n - work.t ? min(c + nchunks, work.n - work.t) : work.n;
                 }
-                // The group has also read the results of its previous chunk by then, so the buffers about to be written
-                // (X | Y of this group, and the state buffer, last read for chunk c - 4) are free.
-                mbar_wait<false>(&ctrl->full[g], k & 1, ctrl, p.status);
-                tc_fence_after();
                 // hop 1
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) mma_ts(XY, Sa + 8 * ks, dWAQ + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ss(XY, dV + (uint64_t)(ks * 64), dSC + (uint64_t)(ks * 16), idesc(32, true, false), 1);
+                for (int ks = 0; ks < 8; ++ks) mma_ts(XY, Sa + 8 * ks, dWAQ + (uint64_t)(ks * 16), idesc(32, false, false), 1);
                 tc_commit(&ctrl->hop);
-                // the decay of the old state and the V part of the update go into the other buffer while hop 1 drains
+                // the decay of the old state goes into the other buffer while hop 1 drains
 #pragma unroll
-                for (int s = 0; s < 8; ++s) mma_ts(Sn + 8 * s, Sa + 8 * s, dDF + (uint64_t)(s * 16), idesc(8, false, false), 0);
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ss(Sn, dV + (uint64_t)(ks * 64), dKWF + (uint64_t)(ks * 64), idesc(64, true, true), 1);
+                for (int s = 0; s < 8; ++s) mma_ts(Sn + 8 * s, Sa + 8 * s, dDF + (uint64_t)(s * 16), idesc(8, false, false), 1);
                 mbar_wait<false>(&ctrl->hop, c & 1, ctrl, p.status);
                 tc_fence_after();
                 // hop 2: the X part of the state update and of Y
@@ -407,107 +469,51 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
                 for (int ks = 0; ks < 2; ++ks) mma_ts(XY + 16, XY + 8 * ks, dQBU + (uint64_t)(ks * 16), idesc(16, false, false), 1);
                 tc_commit(&ctrl->done[g]);
+                if (c + 1 < work.n) start_chunk(c + 1);
                 mbar_wait<false>(&ctrl->done[g], k & 1, ctrl, p.status);  // S' is the next chunk's A operand
                 tc_fence_after();
             }
           }
-        } else if (warp < 4 * G + 2) {
-            // ---- score warps: warp 4G reads [AK|AB] and later AI^T bwf (tensor-memory lanes 0-15), warp 4G + 1 reads [QK|QB]
-            // and later QB AI (lanes 32-47).  Both take whatever is ready: the fold products of the older chunk first.
-            const int q = warp - 4 * G;
-            const uint32_t tq = tmem + ((uint32_t)(32 * q) << 16);
-            const int r0 = lane >> 2, c0 = 2 * (lane & 3);  // this lane's fragment: rows r0, r0 + 8, columns c0, c0 + 1 of every 8
-            int r = 0, f = 0;
-            uint32_t since = clock();
-            while (f < work.n) {
-                const int gf = f % G, gr = r % G;
-                if (f < r && mbar_test(&ctrl->fold[gf], (f / G) & 1)) {
-                    unsigned char* gs = sm + gf * G_BYTES;
-                    tc_fence_after();
-                    if (q == 0) {
+        } else if (warp == 4 * G || warp == 4 * G + 1) {
+            // ---- score warps: warp 4G reads [AK|AB], warp 4G + 1 reads [QK|QB]
+            for (int r = 0; r < work.n; ++r) {
+                const int gr = r % G;
+                unsigned char* gs = sm + gr * G_BYTES;
+                mbar_wait<true>(&ctrl->score[gr], (r / G) & 1, ctrl, p.status);
+                tc_fence_after();
+                uint32_t x[16];
+                tmem_ld_frag4(tq + C_XY + 32 * gr, x);
+                tmem_ld_wait();
+                tc_fence_before();
+                // the previous chunk's matrices have left for its checkpoint record
+                if (p.ckpt && r >= G) mbar_wait<true>(&ctrl->rec[gr], (r / G - 1) & 1, ctrl, p.status);
+                if (q == 0) {  // AB, strictly lower, kept transposed for the inverse
+                    float* ABt = reinterpret_cast<float*>(gs + G_ABT);
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            uint32_t x[16];
-                            tmem_ld_frag4(tq + C_FOLD + 32 * half, x);
-                            tmem_ld_wait();
-                            if (half == 1) {
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) mbar_arrive(&ctrl->fread);
-                            }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                                for (int h = 0; h < 2; ++h)  // time step r0 + 8h, keys 32 half + 8j + c0, +1
-                                    *reinterpret_cast<float2*>(gs + G_BWF + half * 2048 + (r0 + 8 * h) * 128 + ((j ^ (r0 & 3)) << 5) + c0 * 4) =
-                                        make_float2(rnd(__uint_as_float(x[4 * j + 2 * h])), rnd(__uint_as_float(x[4 * j + 2 * h + 1])));
-                        }
-                    } else {
-                        uint32_t x[8];
-                        tmem_ld_frag(tq + C_XY + 32 * gf + 16, x);
-                        tmem_ld_wait();
-                        tc_fence_before();
-                        store_frag16(gs + G_QBU, x, r0, c0, 16);
+                    for (int i = 0; i < 8; ++i) {
+                        const int row = (lane >> 2) + 8 * ((i >> 1) & 1), col = 8 * (i >> 2) + 4 * (i & 1) + (lane & 3);
+                        ABt[col * ABS + row] = col < row ? __uint_as_float(x[8 + i]) : 0.f;
                     }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctrl->full[gf]);
-                    ++f;
-                } else if (r < work.n && mbar_test(&ctrl->score[gr], (r / G) & 1)) {
-                    unsigned char* gs = sm + gr * G_BYTES;
-                    tc_fence_after();
-                    uint32_t x[16];
-                    tmem_ld_frag4(tq + C_XY + 32 * gr, x);
-                    tmem_ld_wait();
-                    tc_fence_before();
-                    // the previous chunk's matrices have left for its checkpoint record
-                    if (p.ckpt && r >= G) mbar_wait<true>(&ctrl->rec[gr], (r / G - 1) & 1, ctrl, p.status);
-                    store_frag16(gs + G_SC + 1024 * q, x, r0, c0, q ? 0 : -1);          // AK (strictly lower) or QK (lower triangular)
-                    if (q == 0) {  // AB, strictly lower, kept transposed for the inverse
-                        float* ABt = reinterpret_cast<float*>(gs + G_ABT);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const int row = r0 + 8 * ((i >> 1) & 1), col = 8 * (i >> 2) + c0 + (i & 1);
-                            ABt[col * SCS + row] = col < row ? __uint_as_float(x[8 + i]) : 0.f;
-                        }
-                    } else {
-                        store_frag16(gs + G_QB, x + 8, r0, c0, 0);
-                    }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctrl->mats[gr]);
-                    ++r;
                 } else {
-                    if (ctrl->abort) break;
-                    if ((uint32_t)clock() - since > (uint32_t)WAIT_LIMIT) give_up(&ctrl->abort, p.status);
-                    continue;
+                    store_frag16(smem_u32(gs + G_QB), x + 8, lane, 0);
                 }
-                since = clock();
+                store_frag16(smem_u32(gs + G_SC + 1024 * q), x, lane, q ? 0 : -1);          // AK (strictly lower) or QK (lower triangular)
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ctrl->mats[gr]);
             }
-        } else if (warp == 4 * G + 2) {
-            // ---- inverse warp: AI^T, then the two products that fold U into its consumers: U = X AI^T, so U bwf = X (AI^T bwf)
-            // and U QB^T = X (QB AI)^T (one dependent tensor-core round trip per chunk less for the chain).  A = [AI^T; QB] for both.
+        } else if (q == 2) {
+            // ---- inverse warps (even and odd groups: each barrier has one warp that sees all its phases)
             for (int c = 0; c < work.n; ++c) {
                 const int g = c % G, k = c / G;
+                if ((g ^ (warp >> 2)) & 1) continue;
                 unsigned char* gs = sm + g * G_BYTES;
-                mbar_wait<false>(&ctrl->mats[g], k & 1, ctrl, p.status);
-                if (p.ckpt && c > 0) {  // the previous chunk's record copy has read its tiles
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&ctrl->rec[(c - 1) % G]);
-                }
-                if (lane < 16) tri_inverse_tc(reinterpret_cast<const float*>(gs + G_ABT), gs + G_AI, lane);
+                mbar_wait<true>(&ctrl->mats[g], k & 1, ctrl, p.status);
+                tri_inverse_tc(reinterpret_cast<float*>(gs + G_ABT), gs + G_AI, lane);
                 fence_async_smem();
-                if (c > 0) mbar_wait<false>(&ctrl->fread, (c - 1) & 1, ctrl, p.status);
-                tc_fence_after();
                 __syncwarp();
                 if (elect_one()) {
-                    const uint64_t dA = desc_kmajor(smem_u32(gs + G_AI), 512), dB = desc_mnmajor(smem_u32(gs + G_BWF));
-#pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_FOLD, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 64), idesc(64, false, true), ks > 0);
-#pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) mma_ss(tmem + C_XY + 32 * g + 16, dA + (uint64_t)(ks * 16), dA + (uint64_t)(ks * 16), idesc(16, false, false), ks > 0);
-                    tc_commit(&ctrl->fold[g]);
+                    mbar_arrive(&ctrl->inv[g]);
                     // The chunk's four 16x16 matrices go into its checkpoint record: the three tiles [AK;QK], AI^T, QB are
                     // contiguous in shared memory and are stored as they are, by one bulk copy.
                     if (p.ckpt) {
@@ -516,11 +522,61 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                         asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
                                      ::"l"(__cvta_generic_to_global(ckm)), "r"(smem_u32(gs + G_SC)), "n"(4 * L * L * 4) : "memory");
                         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                        mbar_arrive(&ctrl->rec[g]);
                     }
                 }
                 __syncwarp();
             }
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // shared memory must outlive the last copy
+        } else {
+            // ---- fold warps: U = X AI^T, so U bwf = X (AI^T bwf) and U QB^T = X (QB AI)^T: one dependent tensor-core round trip per chunk
+            // less for the chain.  Warps 4G + 4, 4G + 5 form 32 key columns of AI^T bwf each, in the place of bwf, warp 4G + 7 QB AI.
+            // (mma.sync: as tcgen05 products they read 104 wavefronts of operands instead of 64, 64 rows of A for 32 or 16 used ones, and
+            // the results came back through tensor memory.)
+            const int g8 = lane >> 2, t4 = lane & 3;
+            const uint32_t at = (lane >> 4) * 512 + ((lane >> 3) & 1) * 128 + (lane & 7) * 16;  // A operands: 8x4 blocks (rows 0-7 | 8-15) x (4 columns | the next 4)
+            for (int c = 0; c < work.n; ++c) {
+                const int g = c % G;
+                unsigned char* gs = sm + g * G_BYTES;
+                mbar_wait<true>(&ctrl->inv[g], (c / G) & 1, ctrl, p.status);
+                uint32_t ai[2][4];
+#pragma unroll
+                for (int kb = 0; kb < 2; ++kb) ldmatrix4(ai[kb], smem_u32(gs + G_AI) + at + kb * 256);
+                if (q == 3) {
+                    float acc[2][4] = {};
+#pragma unroll
+                    for (int kb = 0; kb < 2; ++kb) {
+                        uint32_t a[4];
+                        ldmatrix4(a, smem_u32(gs + G_QB) + at + kb * 256);
+#pragma unroll
+                        for (int nt = 0; nt < 2; ++nt) mma_tf32_raw(acc[nt], a[0], a[2], a[1], a[3], ai[kb][2 * nt], ai[kb][2 * nt + 1]);  // B = AI^T by rows
+                    }
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            *reinterpret_cast<float2*>(gs + G_QBU + kchunk(g8 + 8 * h, 2 * nt + (t4 >> 1), 512) + (t4 & 1) * 8) = make_float2(rnd(acc[nt][2 * h]), rnd(acc[nt][2 * h + 1]));
+                } else {
+                    unsigned char* bw = gs + G_BWF + q * 2048;
+                    float acc[4][4] = {};
+#pragma unroll
+                    for (int kb = 0; kb < 2; ++kb)
+#pragma unroll
+                        for (int nt = 0; nt < 4; ++nt) {  // contraction slots t4, t4 + 4 are time steps t4, t4 + 4 of the eight
+                            const unsigned char* b = bw + (8 * kb + t4) * 128 + ((nt ^ t4) << 5) + g8 * 4;
+                            mma_tf32_raw(acc[nt], ai[kb][0], ai[kb][2], ai[kb][1], ai[kb][3], *reinterpret_cast<const uint32_t*>(b), *reinterpret_cast<const uint32_t*>(b + 512));
+                        }
+                    __syncwarp();  // bwf has been read
+#pragma unroll
+                    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            *reinterpret_cast<float2*>(bw + (g8 + 8 * h) * 128 + ((nt ^ (g8 & 3)) << 5) + t4 * 8) = make_float2(rnd(acc[nt][2 * h]), rnd(acc[nt][2 * h + 1]));
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&ctrl->full[g]);
+            }
         }
         __syncwarp();
     } else {
@@ -545,8 +601,18 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
             for (int ten = 0; ten < 6; ++ten) load_tile(maps.in[ten], G_RAW + ten * RAW_TILE, d, &ctrl->raw[grp]);
         };
-        // Results of own chunk number kk (list position vv): Y^T into registers, the chunk-end state straight to the
-        // checkpoint (or the final state).  All of it is read before the group announces its next chunk.
+        // The output tile of own chunk number kk, once all of the group's warps have written it.
+        auto store_y = [&](int kk) {
+            if (wg == 1 && elect_one()) {
+                const ChunkDesc& d = ctrl->desc[grp][kk & 3];
+                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+                             ::"l"(&maps.y), "r"(0), "r"(d.hi), "r"(d.c * L), "r"(d.bi), "r"(smem_u32(gs + G_Y)) : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            __syncwarp();
+        };
+        // Results of own chunk number kk (list position vv): Y^T into the output tile (which leaves after the group's next barrier),
+        // the chunk-end state to the checkpoint (or the final state).  All of it is read before the group announces its next chunk.
         auto read_results = [&](int kk) {
             mbar_wait<true>(&ctrl->done[grp], kk & 1, ctrl, p.status);
             if (LN) mbar_wait<true>(&ctrl->gate[grp], kk & 1, ctrl, p.status);
@@ -610,10 +676,8 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     const float md = a1 * (1.f / N);
                     const float mu = pivot + md;
                     const float rstd = rsqrtf(fmaxf(a2 * (1.f / N) - md * md, 0.f) + p.eps);
-                    // v of this chunk is still in the fp32 MN-major tile, the gate in its own double buffer
-                    const int mo = (i0 >> 5) * 2048 + t * 128 + ((((i0 & 31) >> 3) ^ (t & 3)) << 5);
-                    const float4 v0 = *reinterpret_cast<const float4*>(gs + G_V + mo), v1 = *reinterpret_cast<const float4*>(gs + G_V + mo + 16);
-                    const float vval[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                    float vval[8];  // v of this chunk was kept aside, the gate has its own double buffer
+                    load8<IoT>(gs + G_V + t * 128 + (((i0 >> 3) ^ (t & 7)) << 4), vval);
                     float gv[8];
                     load8<IoT>(gs + G_GRAW + t * ROWB + (((i0 >> 3) ^ (t & 7)) << 4), gv);
                     float o8[8];
@@ -629,14 +693,11 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     *reinterpret_cast<uint4*>(gs + G_Y + t * 128 + (((i0 >> 3) ^ (t & 7)) << 4)) = pk;
                 }
             }
-            fence_async_smem();
-            group_bar(grp);
-            if (wg == 0 && elect_one()) {
-                asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
-                             ::"l"(&maps.y), "r"(0), "r"(d.hi), "r"(cc * L), "r"(d.bi), "r"(smem_u32(gs + G_Y)) : "memory");
-                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            if (LN) {  // (the staging tiles are about to be written again)
+                fence_async_smem();
+                group_bar(grp);
+                store_y(kk);
             }
-            __syncwarp();
             if (sdst && !seg_last) {
                 // checkpoint state: exact fp32 (the backward's tensor-core products read its upper 19 bits, its carried
                 // decay term all of them), staged in the swizzled layout the tensor-map store expects: half h = columns 32h..32h+31,
@@ -707,12 +768,20 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
         // Iteration k: read the results of own chunk k - 1, write the operand tiles of chunk k (whose scan is in registers),
         // start its score product; then scan chunk k + 1 while the score, inverse and chain warps finish chunk k.  (k = -1 only
         // scans, the last one only reads results: one copy of each piece of code.)
-        F2 o[4][2][2], v[2][2], fwv[2];  // [slot][channel pair] of wq, wa, kwi, bwi; kwf, bwf are formed from kwi, bwi and fw when the tiles are written
+        F2 o[4][2][2], fwv[2];  // [slot][channel pair] of wq, wa, kwi, bwi; kwf, bwf are formed from kwi, bwi and fw when the tiles are written
+        uint32_t v[4];          // V^T: values 16 wg + lane / 4 (+ 8) x time steps 2 (lane % 4), + 1; then time steps 8 ..
         for (int k = -1, v0 = grp - G; ; v0 += G, ++k) {
             if (k >= 0) {
                 // ---------------- results of the previous own chunk (its operand tiles are free afterwards) --
                 if (k > 0) read_results(k - 1);
-                if (v0 >= work.n) break;
+                if (v0 >= work.n) {
+                    if (!LN && k > 0) {
+                        fence_async_smem();
+                        group_bar(grp);
+                        store_y(k - 1);
+                    }
+                    break;
+                }
                 // ---------------- operand tiles -----------------------------------------------------------
                 {
 #pragma unroll
@@ -726,7 +795,15 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                         }
                         *reinterpret_cast<float4*>(gs + G_KWF + mo) = quad4<RND>(kf);
                         *reinterpret_cast<float4*>(gs + G_BWF + mo) = quad4<RND>(bf);
-                        *reinterpret_cast<float4*>(gs + G_V + mo) = quad4<false>(v[e]);  // bf16 values are exact in TF32
+                    }
+                    uint32_t vf[8];  // bf16 values are exact in TF32
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { vf[2 * i] = v[i] << 16; vf[2 * i + 1] = v[i] & 0xffff0000u; }
+                    tmem_st_frag(tlane + C_V + 16 * grp, vf);
+                    if (LN) {  // the epilogue's v: as the raw tile had it
+                        const int t = (lane & 7) + 8 * (lane >> 4), unit = 2 * wg + ((lane >> 3) & 1);
+                        asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
+                                     ::"r"(smem_u32(gs + G_V + t * 128 + ((unit ^ (t & 7)) << 4))), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
                     }
                     if (!(lane & 8)) {  // the decay blocks' entries, one per lane (see S_CUT): channel j0 + (lane & 3)
                         const F2 p2 = lane & 2 ? fwv[1] : fwv[0];
@@ -742,12 +819,14 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const int at = kchunk(row0 ^ e, quad, 2048);
-                        *reinterpret_cast<float4*>(gs + G_WAQ + at) = quad4<RND>(o[1][e]);
-                        *reinterpret_cast<float4*>(gs + G_WAQ + 4096 + at) = quad4<RND>(o[0][e]);
-                        *reinterpret_cast<float4*>(gs + G_KB + at) = quad4<RND>(o[2][e]);
-                        *reinterpret_cast<float4*>(gs + G_KB + 4096 + at) = quad4<RND>(o[3][e]);
+                        *reinterpret_cast<float4*>(gs + G_WAQ + at) = quad4<false>(o[1][e]);
+                        *reinterpret_cast<float4*>(gs + G_WAQ + 4096 + at) = quad4<false>(o[0][e]);
+                        const int ak = kchunk(kb_row(row0 ^ e), quad, 2048);
+                        *reinterpret_cast<float4*>(gs + G_KB + ak) = quad4<RND>(o[2][e]);
+                        *reinterpret_cast<float4*>(gs + G_KB + 4096 + ak) = quad4<RND>(o[3][e]);
                     }
                 }
+                tmem_st_wait();  // V
                 if (ctrl->desc[grp][k & 3].flags & SEG_FIRST) load_state(ctrl->desc[grp][k & 3], wg);
                 fence_async_smem();
                 tc_fence_before();
@@ -770,6 +849,7 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                 }
                 __syncwarp();
                 // ---------------- the four score matrices as one product ---------------------------------
+                if (!LN && k > 0) store_y(k - 1);
                 if (wg == 0 && elect_one()) {
                     const uint64_t dA = desc_kmajor(smem_u32(gs + G_WAQ), 2048), dB = desc_kmajor(smem_u32(gs + G_KB), 2048);
 #pragma unroll
@@ -793,7 +873,11 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                     load4f2(raw + 2 * RAW_TILE, kk[e]);
                     load4f2(raw + 3 * RAW_TILE, a[e]);
                     load4f2(raw + 4 * RAW_TILE, b[e]);
-                    load4f2(raw + 5 * RAW_TILE, v[e]);
+                }
+                {
+                    const int t = 8 * (lane >> 4) + (lane & 7), unit = 2 * wg + ((lane >> 3) & 1);
+                    const uint32_t at = smem_u32(gs + G_RAW + 5 * RAW_TILE + t * ROWB + ((unit ^ (t & 7)) << 4));
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at) : "memory");
                 }
                 if (LN) {  // bonus dot sum_j r_j k_j bonus_j of these time steps: 4 channels here, the rest by shuffle and in the epilogue
                     const float4 bo = __ldg(reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][(k + 1) & 3].hi) * N + j0));
@@ -853,8 +937,8 @@ __global__ void __launch_bounds__(128 * (G + 1), 1) wkv7_fwd_tc_kernel(FwdParams
                         const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
                         const F2 inv = f2(ex2_approx(-cx), ex2_approx(-cy));
                         const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
-                        o[0][e][i] = mul2(q[e][i], incl);   // wq
-                        o[1][e][i] = mul2(a[e][i], non);    // wa
+                        o[0][e][i] = rnd2<RND>(mul2(q[e][i], incl));   // wq (rounded here already: writing the tiles is on the way to the chain, this is not)
+                        o[1][e][i] = rnd2<RND>(mul2(a[e][i], non));    // wa
                         o[2][e][i] = mul2(kk[e][i], inv);   // kwi
                         o[3][e][i] = mul2(b[e][i], inv);    // bwi
                     }
@@ -920,7 +1004,7 @@ template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdPar
     }
     const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 1, p.sT ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
-    kern<<<(unsigned)ws.ctas, 128 * (G + 1), smem, stream>>>(p, ws, maps);
+    kern<<<(unsigned)ws.ctas, 128 * (G + 2), smem, stream>>>(p, ws, maps);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 
