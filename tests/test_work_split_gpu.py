@@ -117,3 +117,20 @@ def test_time_split(B, T, H, nseg, s0):
     for a, b in zip(got, want):
         assert a.dtype == b.dtype and (a.float() - b.float()).norm() <= 4e-3 * b.float().norm()
     assert _lib.lib().wkv7_device_status() == 0
+
+
+@pytest.mark.parametrize('B,T,H', [(1, 1024, 12), (1, 1008, 12), (2, 1024, 12), (1, 1008, 2)])
+def test_time_split_maps_of_cut_chains(B, T, H):
+    """The segments' maps where they matter (slow decays, start states of size 1) and where CTAs hand half-walked ones on (180 and 384
+    segments on 148 SMs, whole and partial last chunks), against the uncut forward.  M's products are single TF32 like the uncut
+    call's: the bound is that of test_time_split."""
+    from wind_rwkv.rwkv7 import _lib, attn, synthetic
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=T + B, dtype=th.bfloat16, device='cuda', s0_std=1.0)
+    d['w'] = (d['w'].float() * 0.5 - 5.7).bfloat16()
+    ins = [d[n] for n in 'rwkvab']
+    with th.no_grad():
+        want = attn(*ins, N, s0=d['s0'], return_state=True)
+        got = attn(*ins, N, s0=d['s0'], return_state=True, time_split=16)
+    for a, b in zip(got, want):
+        assert (a.float() - b.float()).norm() <= 4e-3 * b.float().norm()
+    assert _lib.lib().wkv7_device_status() == 0

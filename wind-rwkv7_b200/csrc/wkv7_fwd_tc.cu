@@ -76,6 +76,8 @@ constexpr int G_RAW = 36864;   // q, w, k, a, b, v staging                   6 *
 constexpr int G_Y = 49152;            // the chunk's output as [time][value], bf16, 128-byte swizzle             2048
 constexpr int G_GRAW = G_Y + 2048;    // attn_ln only: the gate tile                                            2048
 constexpr int G_BYTES_PLAIN = G_GRAW;  // 50 KB
+constexpr int G_Z0 = G_QB, G_Z1 = G_Y;  // affine maps only (which have neither): zeros                          2 * 256
+static_assert(G_Z0 < G_DF && G_DF + 2048 <= G_Z1, "descriptors have positive strides");
 constexpr int G_BYTES_LN = G_GRAW + RAW_TILE;  // 52 KB
 static_assert(G_RAW % 1024 == 0 && G_RAW + 6 * RAW_TILE <= G_Y && G_Y % 1024 == 0 && G_BYTES_PLAIN % 1024 == 0 && G_BYTES_LN % 1024 == 0, "tile alignment");
 // attn_ln epilogue scratch inside the kwf / bwf tiles, which are dead once the chain step has completed
@@ -170,9 +172,9 @@ __device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr, uint32_t sbo) {
 __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t saddr) {  // 128-byte swizzle with 32-byte base
     return (uint64_t)((saddr >> 4) & 0x3fff) | ((uint64_t)(2048 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (1ull << 61);
 }
-// instruction descriptor: fp32 accumulate, TF32 operands, M = 64
-__host__ __device__ constexpr uint32_t idesc(int n, bool a_mn, bool b_mn) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | (4u << 24);
+// instruction descriptor: fp32 accumulate, TF32 operands
+__host__ __device__ constexpr uint32_t idesc(int n, bool b_mn, int m = 64) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 __device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t acc) {
     asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n"
@@ -317,15 +319,20 @@ __device__ __forceinline__ uint32_t pack_bf16x2_rn(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// AFF: the segments of a sequence cut in time as affine maps, S -> S M + R (wkv7_time_split.cu).  The state has 128 rows, R in lanes 0-63 and
+// M in lanes 64-127 of tensor memory (M = 128 products; V^T has zeros there): one walk over the chunks instead of two, and without the
+// output's products, tiles and stores.  R starts from zero (a sequence's first segment: from s0), M from the identity; they leave
+// through sT and sM.
 // TAIL: the sequence length is not a multiple of 16 (a build of its own, so that whole-chunk sequences carry none of
 // the row tests in their register budget).
 struct alignas(64) FwdMaps { CUtensorMap ck, y, in[6], g; };  // checkpoint states; output; q, w, k, a, b, v; gate
 
-template <int G, bool RND, bool LN, bool TAIL>
+template <int G, bool RND, bool LN, bool TAIL, bool AFF>
 __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams p, WorkSplit ws, const __grid_constant__ FwdMaps maps) {
     using IoT = __nv_bfloat16;
     constexpr int G_BYTES = LN ? G_BYTES_LN : G_BYTES_PLAIN;
-    constexpr int NCOLS = 512;
+    constexpr int NCOLS = 512, M = AFF ? 128 : 64, NX = AFF ? 16 : 32;  // rows of the state; columns X | Yp or X alone
+    static_assert(!(AFF && LN), "the maps have no output");
     static_assert(C_XY + 32 * G <= C_V && C_V + 16 * G <= NCOLS, "tensor memory columns");
     // Register reallocation (G == 4 only).  setmaxnreg.inc blocks, without a bound, until the CTA's
     // register pool can satisfy it, and the pool is what the CTA was launched with: 768 threads x 80
@@ -345,8 +352,8 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
 
     if (tid == 0) {
         for (int g = 0; g < G; ++g) {
-            mbar_init(&ctrl->full[g], 3);
-            mbar_init(&ctrl->mats[g], 2);
+            mbar_init(&ctrl->full[g], AFF ? 2 : 3);
+            mbar_init(&ctrl->mats[g], AFF ? 1 : 2);
             mbar_init(&ctrl->inv[g], 1);
             mbar_init(&ctrl->rec[g], 1);
             mbar_init(&ctrl->done[g], 1);
@@ -382,6 +389,9 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
     // the off-diagonal zeros of the decay blocks are written once
     for (int i = tid; i < G * (2048 / 16); i += blockDim.x)
         *reinterpret_cast<uint4*>(sm + (i / 128) * G_BYTES + G_DF + (i % 128) * 16) = make_uint4(0, 0, 0, 0);
+    if (AFF)  // zeros before and after them: products of 16 columns (the least with 128 rows) take a block and one of these
+        for (int i = tid; i < G * 32; i += blockDim.x)
+            *reinterpret_cast<uint4*>(sm + (i / 32) * G_BYTES + (i & 16 ? G_Z1 : G_Z0) + (i & 15) * 16) = make_uint4(0, 0, 0, 0);
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctrl->tmem_base)), "r"(NCOLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -398,10 +408,17 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
         const int sbh = d.bh, sc = d.c;
         const uint32_t ta = tmem + C_INIT;
         if (d.prev_first >= 0) mbar_wait<true>(&ctrl->done[d.prev_first % G], (d.prev_first / G) & 1, ctrl, p.status);  // its start state has been used
-        const int i = 16 * wq + (lane & 15);
+        const int row = AFF ? 32 * wq + lane : 16 * wq + (lane & 15), i = row & 63;
         if (sc > 0) wait_handoff(ws.flags + blockIdx.x - 1, &ctrl->abort, p.status);
         const float* src = sc > 0 ? p.sT : p.s0;
-        if (src) src += (long long)sbh * N * N + i * N;
+        if (AFF) {
+            const int entry = (int)((unsigned)d.bi / (unsigned)p.nseg);
+            if (sc > 0) src = (row < 64 ? p.sT : p.sM) + (long long)sbh * N * N;
+            else src = row < 64 && p.s0 && d.bi == entry * p.nseg ? p.s0 + (long long)(entry * (int)p.H + d.hi) * N * N : nullptr;
+            if (src) src += i * N;
+        } else if (src) {
+            src += (long long)sbh * N * N + i * N;
+        }
         float* ck = (p.ckpt && lane < 16) ? p.ckpt + ((long long)sbh * nchunks + sc) * CK_FLOATS + i * N : nullptr;
 #pragma unroll 1
         for (int cb = 0; cb < N; cb += 16) {
@@ -409,6 +426,10 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 float4 x = src ? __ldcg(reinterpret_cast<const float4*>(src + cb + 4 * q)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (AFF && sc == 0 && row >= 64) {  // identity
+                    const int j = i - cb - 4 * q;
+                    x = make_float4(j == 0, j == 1, j == 2, j == 3);
+                }
                 x.x *= STATE_SCALE; x.y *= STATE_SCALE; x.z *= STATE_SCALE; x.w *= STATE_SCALE;  // the state is carried as S~ = 2^-64 S (see ANCHOR_LN)
                 v[4 * q] = __float_as_uint(x.x); v[4 * q + 1] = __float_as_uint(x.y); v[4 * q + 2] = __float_as_uint(x.z); v[4 * q + 3] = __float_as_uint(x.w);
                 if (ck) *reinterpret_cast<float4*>(ck + cb + 4 * q) = x;
@@ -438,9 +459,9 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                 mbar_wait<false>(&ctrl->full[g], (c / G) & 1, ctrl, p.status);
                 tc_fence_after();
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(XY, V + 8 * ks, dSC + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
+                for (int ks = 0; ks < 2; ++ks) mma_ts(XY, V + 8 * ks, dSC + (uint64_t)(ks * 16), idesc(NX, false, M), ks > 0);
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, V + 8 * ks, dKWF + (uint64_t)(ks * 64), idesc(64, false, true), ks > 0);
+                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, V + 8 * ks, dKWF + (uint64_t)(ks * 64), idesc(64, true, M), ks > 0);
             };
             start_chunk(0);
             for (int c = 0; c < work.n; ++c) {  // position in the CTA's list
@@ -456,24 +477,33 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                 }
                 // hop 1
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) mma_ts(XY, Sa + 8 * ks, dWAQ + (uint64_t)(ks * 16), idesc(32, false, false), 1);
+                for (int ks = 0; ks < 8; ++ks) mma_ts(XY, Sa + 8 * ks, dWAQ + (uint64_t)(ks * 16), idesc(NX, false, M), 1);
                 tc_commit(&ctrl->hop);
                 // the decay of the old state goes into the other buffer while hop 1 drains
 #pragma unroll
-                for (int s = 0; s < 8; ++s) mma_ts(Sn + 8 * s, Sa + 8 * s, dDF + (uint64_t)(s * 16), idesc(8, false, false), 1);
+                for (int s = 0; s < 8; ++s) {
+                    if (!AFF) {
+                        mma_ts(Sn + 8 * s, Sa + 8 * s, dDF + (uint64_t)(s * 16), idesc(8, false), 1);
+                    } else {  // rows 0-7 and 8-15 of the operand: the block and zeros, or zeros and the block
+                        const uint32_t blk = gb + G_DF + 256 * s;
+                        mma_ts(Sn + 16 * (s >> 1), Sa + 8 * s, s & 1 ? desc_kmajor(gb + G_Z0, blk - (gb + G_Z0)) : desc_kmajor(blk, gb + G_Z1 - blk), idesc(16, false, M), 1);
+                    }
+                }
                 mbar_wait<false>(&ctrl->hop, c & 1, ctrl, p.status);
                 tc_fence_after();
                 // hop 2: the X part of the state update and of Y
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, XY + 8 * ks, dBWU + (uint64_t)(ks * 64), idesc(64, false, true), 1);
+                for (int ks = 0; ks < 2; ++ks) mma_ts(Sn, XY + 8 * ks, dBWU + (uint64_t)(ks * 64), idesc(64, true, M), 1);
 #pragma unroll
-                for (int ks = 0; ks < 2; ++ks) mma_ts(XY + 16, XY + 8 * ks, dQBU + (uint64_t)(ks * 16), idesc(16, false, false), 1);
+                for (int ks = 0; ks < (AFF ? 0 : 2); ++ks) mma_ts(XY + 16, XY + 8 * ks, dQBU + (uint64_t)(ks * 16), idesc(16, false, M), 1);
                 tc_commit(&ctrl->done[g]);
                 if (c + 1 < work.n) start_chunk(c + 1);
                 mbar_wait<false>(&ctrl->done[g], k & 1, ctrl, p.status);  // S' is the next chunk's A operand
                 tc_fence_after();
             }
           }
+        } else if (AFF && (warp == 4 * G + 1 || warp == 4 * G + 7)) {
+            // (QK, QB and QB AI are for the output)
         } else if (warp == 4 * G || warp == 4 * G + 1) {
             // ---- score warps: warp 4G reads [AK|AB], warp 4G + 1 reads [QK|QB]
             for (int r = 0; r < work.n; ++r) {
@@ -597,9 +627,9 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
         auto load_raw = [&](int ko) {
             if (ctrl->abort) return;  // (the last one's wait may have given up)
             const ChunkDesc& d = ctrl->desc[grp][ko & 3];
-            expect_bytes(&ctrl->raw[grp], 6 * RAW_TILE);
+            expect_bytes(&ctrl->raw[grp], (AFF ? 5 : 6) * RAW_TILE);
 #pragma unroll
-            for (int ten = 0; ten < 6; ++ten) load_tile(maps.in[ten], G_RAW + ten * RAW_TILE, d, &ctrl->raw[grp]);
+            for (int ten = AFF ? 1 : 0; ten < 6; ++ten) load_tile(maps.in[ten], G_RAW + ten * RAW_TILE, d, &ctrl->raw[grp]);
         };
         // The output tile of own chunk number kk, once all of the group's warps have written it.
         auto store_y = [&](int kk) {
@@ -620,9 +650,11 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
             const ChunkDesc& d = ctrl->desc[grp][kk & 3];
             const int vv = grp + kk * G, cc = d.c;
             const bool seg_last = d.flags & SEG_LAST;
-            float* sdst = seg_last ? (p.sT ? p.sT + (long long)d.bh * N * N : nullptr)
+            float* sdst = AFF ? (seg_last ? (wg < 2 ? p.sT : p.sM) + (long long)d.bh * N * N : nullptr)
+                        : seg_last ? (p.sT ? p.sT + (long long)d.bh * N * N : nullptr)
                                    : (p.ckpt ? p.ckpt + ((long long)d.bh * nchunks + cc + 1) * CK_FLOATS : nullptr);
-            if (!LN) {
+            if (AFF) {
+            } else if (!LN) {
                 // Y^T [value][time], read as accumulator fragments, goes as bf16 through a transposing matrix store into the
                 // [time][value] tile (128-byte rows, 16-byte units XOR-ed with the row as the tensor map's swizzle wants), which
                 // leaves by one bulk tensor store; the map clips rows beyond the end of the sequence.
@@ -731,7 +763,7 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                 __syncwarp();
             } else if (sdst) {
                 // final state: exact, straight from registers (32-byte stores: whole sectors of the lane's 256-byte row)
-                float* d = sdst + (16 * wg + (lane & 15)) * N;
+                float* d = sdst + (AFF ? 32 * (wg & 1) + lane : 16 * wg + (lane & 15)) * N;
 #pragma unroll
                 for (int qt = 0; qt < 4; ++qt) {
                     uint32_t sv[16];
@@ -739,7 +771,7 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                     tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 16; ++e) sv[e] = __float_as_uint(__uint_as_float(sv[e]) * STATE_UNSCALE);  // S = 2^64 S~
-                    if (lane < 16) {
+                    if (AFF || lane < 16) {
 #pragma unroll
                         for (int q8 = 0; q8 < 2; ++q8)
                             asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(d + 16 * qt + 8 * q8), "r"(sv[8 * q8]), "r"(sv[8 * q8 + 1]),
@@ -765,17 +797,23 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
         const float late0 = late ? 0.f : -1.f, late1 = late ? -1.f : 0.f;
         if (wg == 2 && grp < work.n && elect_one()) load_raw(0);
         __syncwarp();
+        if (AFF && wg >= 2) {
+            const uint32_t zeros[16] = {};
+            tmem_st16(tlane + C_V + 16 * grp, zeros);
+            tmem_st_wait();
+        }
         // Iteration k: read the results of own chunk k - 1, write the operand tiles of chunk k (whose scan is in registers),
         // start its score product; then scan chunk k + 1 while the score, inverse and chain warps finish chunk k.  (k = -1 only
         // scans, the last one only reads results: one copy of each piece of code.)
         F2 o[4][2][2], fwv[2];  // [slot][channel pair] of wq, wa, kwi, bwi; kwf, bwf are formed from kwi, bwi and fw when the tiles are written
-        uint32_t v[4];          // V^T: values 16 wg + lane / 4 (+ 8) x time steps 2 (lane % 4), + 1; then time steps 8 ..
+        uint32_t v[4], v2[AFF ? 4 : 1];  // (AFF: values 32 wg + .. and 32 wg + 16 + .., warps 0 and 1)
+                                // V^T: values 16 wg + lane / 4 (+ 8) x time steps 2 (lane % 4), + 1; then time steps 8 ..
         for (int k = -1, v0 = grp - G; ; v0 += G, ++k) {
             if (k >= 0) {
                 // ---------------- results of the previous own chunk (its operand tiles are free afterwards) --
                 if (k > 0) read_results(k - 1);
                 if (v0 >= work.n) {
-                    if (!LN && k > 0) {
+                    if (!LN && !AFF && k > 0) {
                         fence_async_smem();
                         group_bar(grp);
                         store_y(k - 1);
@@ -799,7 +837,12 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                     uint32_t vf[8];  // bf16 values are exact in TF32
 #pragma unroll
                     for (int i = 0; i < 4; ++i) { vf[2 * i] = v[i] << 16; vf[2 * i + 1] = v[i] & 0xffff0000u; }
-                    tmem_st_frag(tlane + C_V + 16 * grp, vf);
+                    if (!AFF || wg < 2) tmem_st_frag(tlane + C_V + 16 * grp, vf);
+                    if (AFF && wg < 2) {
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) { vf[2 * i] = v2[AFF ? i : 0] << 16; vf[2 * i + 1] = v2[AFF ? i : 0] & 0xffff0000u; }
+                        tmem_st_frag(tlane + (16u << 16) + C_V + 16 * grp, vf);
+                    }
                     if (LN) {  // the epilogue's v: as the raw tile had it
                         const int t = (lane & 7) + 8 * (lane >> 4), unit = 2 * wg + ((lane >> 3) & 1);
                         asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
@@ -820,7 +863,7 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                     for (int e = 0; e < 2; ++e) {
                         const int at = kchunk(row0 ^ e, quad, 2048);
                         *reinterpret_cast<float4*>(gs + G_WAQ + at) = quad4<false>(o[1][e]);
-                        *reinterpret_cast<float4*>(gs + G_WAQ + 4096 + at) = quad4<false>(o[0][e]);
+                        if (!AFF) *reinterpret_cast<float4*>(gs + G_WAQ + 4096 + at) = quad4<false>(o[0][e]);
                         const int ak = kchunk(kb_row(row0 ^ e), quad, 2048);
                         *reinterpret_cast<float4*>(gs + G_KB + ak) = quad4<RND>(o[2][e]);
                         *reinterpret_cast<float4*>(gs + G_KB + 4096 + ak) = quad4<RND>(o[3][e]);
@@ -849,11 +892,11 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                 }
                 __syncwarp();
                 // ---------------- the four score matrices as one product ---------------------------------
-                if (!LN && k > 0) store_y(k - 1);
+                if (!LN && !AFF && k > 0) store_y(k - 1);
                 if (wg == 0 && elect_one()) {
                     const uint64_t dA = desc_kmajor(smem_u32(gs + G_WAQ), 2048), dB = desc_kmajor(smem_u32(gs + G_KB), 2048);
 #pragma unroll
-                    for (int ks = 0; ks < 8; ++ks) mma_ss(tmem + C_XY + 32 * grp, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 16), idesc(32, false, false), ks > 0);
+                    for (int ks = 0; ks < 8; ++ks) mma_ss(tmem + C_XY + 32 * grp, dA + (uint64_t)(ks * 16), dB + (uint64_t)(ks * 16), idesc(32, false), ks > 0);
                     tc_commit(&ctrl->score[grp]);
                 }
                 __syncwarp();
@@ -869,15 +912,17 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                     const int row = row0 ^ e;
                     const unsigned char* raw = gs + G_RAW + row * ROWB + (((quad >> 1) ^ (row & 7)) << 4) + (quad & 1) * 8;
                     load4f2(raw + 1 * RAW_TILE, cum[e]);
-                    load4f2(raw + 0 * RAW_TILE, q[e]);
+                    if (!AFF) load4f2(raw + 0 * RAW_TILE, q[e]);
                     load4f2(raw + 2 * RAW_TILE, kk[e]);
                     load4f2(raw + 3 * RAW_TILE, a[e]);
                     load4f2(raw + 4 * RAW_TILE, b[e]);
                 }
                 {
-                    const int t = 8 * (lane >> 4) + (lane & 7), unit = 2 * wg + ((lane >> 3) & 1);
-                    const uint32_t at = smem_u32(gs + G_RAW + 5 * RAW_TILE + t * ROWB + ((unit ^ (t & 7)) << 4));
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at) : "memory");
+                    const int t = 8 * (lane >> 4) + (lane & 7), unit = (AFF ? 4 * (wg & 1) : 2 * wg) + ((lane >> 3) & 1);
+                    const uint32_t at = smem_u32(gs + G_RAW + 5 * RAW_TILE + t * ROWB);
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at + ((unit ^ (t & 7)) << 4)) : "memory");
+                    if (AFF)
+                        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(v2[0]), "=r"(v2[AFF ? 1 : 0]), "=r"(v2[AFF ? 2 : 0]), "=r"(v2[AFF ? 3 : 0]) : "r"(at + (((unit + 2) ^ (t & 7)) << 4)) : "memory");
                 }
                 if (LN) {  // bonus dot sum_j r_j k_j bonus_j of these time steps: 4 channels here, the rest by shuffle and in the epilogue
                     const float4 bo = __ldg(reinterpret_cast<const float4*>(p.params + (2 * p.H + ctrl->desc[grp][(k + 1) & 3].hi) * N + j0));
@@ -937,7 +982,7 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                         const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
                         const F2 inv = f2(ex2_approx(-cx), ex2_approx(-cy));
                         const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
-                        o[0][e][i] = rnd2<RND>(mul2(q[e][i], incl));   // wq (rounded here already: writing the tiles is on the way to the chain, this is not)
+                        if (!AFF) o[0][e][i] = rnd2<RND>(mul2(q[e][i], incl));   // wq (rounded here already: writing the tiles is on the way to the chain, this is not)
                         o[1][e][i] = rnd2<RND>(mul2(a[e][i], non));    // wa
                         o[2][e][i] = mul2(kk[e][i], inv);   // kwi
                         o[3][e][i] = mul2(b[e][i], inv);    // bwi
@@ -985,10 +1030,8 @@ static bool encode_checkpoint_map(CUtensorMap* m, float* base, long long records
               CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-__device__ __align__(128) __nv_bfloat16 g_zero_row[N];
-
-template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdParams& p, cudaStream_t stream) {
-    auto kern = wkv7_fwd_tc_kernel<G, RND, LN, TAIL>;
+template <int G, bool RND, bool LN, bool TAIL, bool AFF = false> static int launch_tt(const FwdParams& p, cudaStream_t stream) {
+    auto kern = wkv7_fwd_tc_kernel<G, RND, LN, TAIL, AFF>;
     const int smem = G * (LN ? G_BYTES_LN : G_BYTES_PLAIN) + (int)sizeof(Ctrl) + 1024;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
     FwdMaps maps;
@@ -998,10 +1041,6 @@ template <int G, bool RND, bool LN, bool TAIL> static int launch_tt(const FwdPar
     CUtensorMap* const ms[8] = {&maps.y, &maps.in[0], &maps.in[1], &maps.in[2], &maps.in[3], &maps.in[4], &maps.in[5], &maps.g};
     for (int i = 0; i < (LN ? 8 : 7); ++i)
         if (ins[i] && !encode_bthn_map(ms[i], const_cast<void*>(ins[i]), p.B, p.T, p.H, p.st)) return kLaunchFailed;
-    if (!p.v) {  // v = 0: a tensor of one zero row; what lies beyond it reads as zero
-        void* zeros = nullptr;
-        if (cudaGetSymbolAddress(&zeros, g_zero_row) != cudaSuccess || !encode_bthn_map(&maps.in[5], zeros, 1, 1, 1, Strides{N, N, N})) return kLaunchFailed;
-    }
     const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 1, p.sT ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
     kern<<<(unsigned)ws.ctas, 128 * (G + 2), smem, stream>>>(p, ws, maps);
@@ -1057,6 +1096,7 @@ template <bool LN> static int launch_ln(const FwdParams& p, int groups, cudaStre
 }
 
 int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream) {
+    if (p.sM) return p.T % L ? tc::launch_tt<4, true, false, true, true>(p, stream) : tc::launch_tt<4, true, false, false, true>(p, stream);
     return ln ? launch_ln<true>(p, groups, stream) : launch_ln<false>(p, groups, stream);
 }
 

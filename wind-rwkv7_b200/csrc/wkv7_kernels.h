@@ -18,6 +18,10 @@ struct FwdParams {
     float eps;
     int* status;                        // device status word
     unsigned* flags;                    // scratch for cut chains (WorkSplit), or null: every chain is worked by one CTA
+    // tcgen05 forward: the chains as affine maps S -> S M + R, R to sT [B,H,N,N] and M to sM, no y.  The batch entries are segments of
+    // sequences, nseg of each; R of a sequence's first one starts from s0 [B/nseg,H,N,N] (or null: zeros).  Null: the ordinary forward
+    float* sM;
+    int nseg;
 };
 
 struct BwdParams {
@@ -67,7 +71,7 @@ int launch_bwd_bf16(const BwdParams& p, bool ln, cudaStream_t stream);
 size_t bwd_workspace_bytes(long long B, long long T, long long H, bool ln);  // what launch_bwd wants at p.flags for bf16 tensors
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
-// tcgen05 forward (bf16 IO; v null: zeros; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
+// tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
 // not rounded to TF32 by their producer (the tensor core truncates them)
 int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream);
 // bf16 forward with the sequences cut into nseg segments each (wkv7_time_split.cu)
