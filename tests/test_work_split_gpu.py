@@ -79,6 +79,34 @@ def test_backward(extra, T, dsT, ln):
     assert L.wkv7_device_status() == 0
 
 
+@pytest.mark.parametrize('chains,T,dsT', [(1, 48, True), (1, 49, False), (1, 64, True), (5, 100, True), (149, 49, True), (300, 65, False), (12, 38900, True)])
+def test_backward_f32_walked(chains, T, dsT):
+    """fp32 tensors: the state gradient walked by a kernel of its own (from four chunks on, any number of chains, in several passes where the
+    tiles would take more than 512 MB), then all chunks in parallel, against the one-kernel form of the entry point without scratch.
+    The same products to 2^-22 each, summed in another order: 1e-5 of the norm."""
+    from wind_rwkv.rwkv7 import _lib, synthetic
+    from wind_rwkv.rwkv7.rwkv7_attn import fw_attn
+    L = _lib.lib()
+    B, H = 1, chains
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=T, dtype=th.float32, device='cuda', s0_std=0.1)
+    _, sT, ck = fw_attn(*[d[n].view(B, T, H, N) for n in 'wrkvab'], d['s0'])
+    gs = th.randn(B, H, N, N, device='cuda') if dsT else None
+    ws = th.full((L.wkv7_bwd_ws_bytes(B, T, H, N, 1),), 255, dtype=th.uint8, device='cuda')
+    assert (ws.numel() > L.wkv7_workspace_bytes()) == (T > 48)
+
+    def call(walk):
+        outs = [th.full_like(d['r'], float('nan')) for _ in range(6)] + [th.full((B, H, N, N), float('nan'), device='cuda')]
+        a = [d[n].data_ptr() for n in 'rwkvab'] + [d['dy'].data_ptr(), ck.data_ptr(), _lib.ptr(gs), _lib.ptr(sT if dsT else None)]
+        a += [o.data_ptr() for o in outs] + [B, T, H, N, T * H * N, H * N, N, 1] + ([ws.data_ptr()] if walk else []) + [None]
+        assert getattr(L, 'wkv7_bwd' + ('_ws' if walk else ''))(*a) == 0
+        th.cuda.synchronize()
+        return outs
+
+    for a, b in zip(call(False), call(True)):
+        assert bool(th.isfinite(a).all()) and (a - b).norm() <= 1e-5 * a.norm()
+    assert L.wkv7_device_status() == 0
+
+
 @pytest.mark.parametrize('form', ['c++', 'python'])
 def test_backward_scratch_of_few_chains(form, monkeypatch):
     """The tiles of the walked state gradients are asked for where they are used (attn), not by attn_ln, which is not walked."""

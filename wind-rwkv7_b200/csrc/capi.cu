@@ -220,7 +220,8 @@ size_t wkv7_workspace_bytes(void) { return wkv7::WORK_FLAG_BYTES; }
 
 static int64_t bwd_scratch_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype, bool ln) {
     if (B < 0 || T < 0 || H < 0 || N != wkv7::N) return 0;
-    return (int64_t)(io_dtype == WKV7_BF16 ? wkv7::bwd_workspace_bytes(B, T, H, ln) : wkv7::WORK_FLAG_BYTES);
+    if (io_dtype == WKV7_BF16) return (int64_t)wkv7::bwd_workspace_bytes(B, T, H, ln);
+    return (int64_t)(io_dtype == WKV7_F32 && !ln ? wkv7::bwd32_workspace_bytes(B, T, H) : wkv7::WORK_FLAG_BYTES);
 }
 int64_t wkv7_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype) { return bwd_scratch_bytes(B, T, H, N, io_dtype, false); }
 int64_t wkv7_attn_ln_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype) { return bwd_scratch_bytes(B, T, H, N, io_dtype, true); }

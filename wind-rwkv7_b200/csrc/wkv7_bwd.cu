@@ -1,5 +1,7 @@
 // WKV7 backward for sm_100a, fp32 tensors (single or triple TF32 products; bf16 tensors: wkv7_bwd_bf16.cu): one CTA per
 // (batch, head) chain, 4 warps, chunks of 16 time steps walked in reverse; the gradient dS of the state stays in registers.
+// attn with triple TF32 and scratch: dS is walked by a kernel of its own (wkv7_bwd_walk32_kernel), then all chunks are worked in
+// parallel (PAR).
 //
 // Replaces the reference's backward_kernel (wind_rwkv/rwkv7/attn.cu:131-326).  The forward
 // intermediates of a chunk are rebuilt from the fp32 chunk-start state S0 the forward wrote (exact fp32; in the
@@ -30,6 +32,7 @@
 // Stage C (contractions over the value index, warp owns 16 key columns): the four score
 // gradients and DA, DQ, DB, DK with S0 and dSf read from shared memory.
 #include <cuda.h>
+#include <algorithm>
 #include <cstddef>
 #include <cstring>
 
@@ -51,13 +54,16 @@ constexpr int ROWB = N * 4 + 16, TILEB = L * ROWB;
 constexpr int YS = 20;  // row stride (floats) of the per-warp transposition scratch
 __device__ __forceinline__ int st_at(int row, int col) { return row * ROWB + col * 4; }  // byte offset of element (row, col)
 
-template <int PREC, bool LN> struct BwdSmem {
+// PAR: two CTAs an SM (3072 chunks: 148 us; with one, 233): v and dy in one set, requested after stage C; the score gradients in the place of
+// the matrices, which come after the chunk's last barrier.
+template <int PREC, bool LN, bool PAR> struct BwdSmem {
+    static constexpr int SETS = PAR ? 1 : 2;
     alignas(16) unsigned char st_in[5][TILEB];  // q, w, k, a, b (dead after the scan)
-    alignas(16) unsigned char st_v[2][TILEB];
-    alignas(16) unsigned char st_dy[2][TILEB];
+    alignas(16) unsigned char st_v[SETS][TILEB];
+    alignas(16) unsigned char st_dy[SETS][TILEB];
     alignas(16) unsigned char st_g[LN ? 2 : 1][LN ? TILEB : 16];
     alignas(16) float wq[L * OPS], wa[L * OPS], kwi[L * OPS], bwi[L * OPS];
-    alignas(16) float cum[L * OPS];
+    alignas(16) float cum[L * OPS];                  // running log-decay; fp32 class: P~_t
     alignas(16) float lw[PREC == 3 ? L * OPS : 4];   // single-TF32 path derives it from cum
     // The chunk's four 16x16 matrices AK, QK, AI^T, QB (matrix m, row r: row group 2m + r/8 of the record's 64-row operand
     // tile), filled by two bulk tensor loads: rows with (r & 4) == 0 form a dense block of [8 row groups][4 rows][24 floats]
@@ -67,7 +73,9 @@ template <int PREC, bool LN> struct BwdSmem {
     // the per-warp transposition scratch for dv / dg and as the GroupNorm reduction buffers.
     static constexpr int SCRATCH_FLOATS = WARPS * L * YS + WARPS * L * 5;
     static constexpr int SGRAD_FLOATS = 4 * L * SCS > SCRATCH_FLOATS ? 4 * L * SCS : SCRATCH_FLOATS;
-    alignas(16) float sgrad[SGRAD_FLOATS];  // score gradient i at sgrad + i * L * SCS
+    alignas(16) float sgrad_[PAR ? 4 : SGRAD_FLOATS];
+    __device__ __forceinline__ float* sgrad() { return PAR ? mats : sgrad_; }  // score gradient i at sgrad() + i * L * SCS
+    static_assert(!PAR || 4 * L * SCS <= 2 * MAT_BLK, "room for the score gradients");
     // attn_ln: Ut, Dt, Yt are dead between stage C and the next chunk's stage B and double as the output staging tiles
     alignas(LN ? 1024 : 16) float Ut[L * OPS];  // U and dabu as [time][value]
     alignas(16) float Dt[L * OPS];
@@ -147,18 +155,34 @@ __device__ __forceinline__ bool s0_wait(uint64_t* bar, uint32_t parity, volatile
     return mbar_wait_bounded<false>(bar, parity, abort, status);
 }
 
+// PAR: the state gradients at the chunks' ends are given (wkv7_bwd_walk32_kernel), so that no chunk depends on another one and a CTA
+// takes `per` of the list of all chains' steps it0 .. it0 + count - 1 (counted from the end of the sequence).
+struct Walked { const float* tiles; int it0, count, per, total; };
+constexpr int TILE_FLOATS = N * SS;  // a state gradient as the kernel keeps it in shared memory: pitch SS, columns xcol<1>
+// d += a b; with SPLIT the products with a lower part go to d2
+template <int PREC, bool SPLIT> __device__ __forceinline__ void mma2(float (&d)[4], float (&d2)[4], const FragA<PREC>& a, const FragB<PREC>& b) {
+    if (!SPLIT) {
+        mma<PREC>(d, a, b);
+        return;
+    }
+    mma_tf32_raw(d2, a.x[0].l, a.x[1].l, a.x[2].l, a.x[3].l, b.x[0].h, b.x[1].h);
+    mma_tf32_raw(d, a.x[0].h, a.x[1].h, a.x[2].h, a.x[3].h, b.x[0].h, b.x[1].h);
+    mma_tf32_raw(d2, a.x[0].h, a.x[1].h, a.x[2].h, a.x[3].h, b.x[0].l, b.x[1].l);
+}
 // TAIL: the sequence length is not a multiple of 16 (an instantiation of its own, so that whole-chunk sequences carry
 // none of the row tests).
-template <int PREC, bool LN, bool TAIL>
-__global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __grid_constant__ CkptMaps cmaps) {
-    using Smem = BwdSmem<PREC, LN>;
+template <int PREC, bool LN, bool TAIL, bool PAR>
+__global__ void __launch_bounds__(THREADS, PAR ? 2 : 1) wkv7_bwd_kernel(BwdParams p, Walked wk, const __grid_constant__ CkptMaps cmaps) {
+    static_assert(!(PAR && LN), "attn_ln's state gradient needs the gradient of the recurrence output first");
+    using Smem = BwdSmem<PREC, LN, PAR>;
+    static_assert(!PAR || sizeof(Smem) + 1024 <= 116736, "two CTAs per SM");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const long long bh = blockIdx.x;
+    const long long bh = blockIdx.x;  // (not PAR)
     const long long bi = bh / p.H, hi = bh % p.H;
-    const long long base = bi * p.st.b + hi * p.st.h;
+    const long long base = PAR ? 0 : bi * p.st.b + hi * p.st.h;
     const int nchunks = (int)((p.T + L - 1) / L);  // the last chunk may be partial: its missing rows read as zeros
     constexpr bool has_tail = TAIL;
     const float* gin[5] = {(const float*)p.r + base, (const float*)p.w + base, (const float*)p.k + base,
@@ -167,6 +191,15 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
     const float* gdy = (const float*)p.dy + base;
     float* gout[5] = {(float*)p.dr + base, (float*)p.dw + base, (float*)p.dk + base, (float*)p.da + base, (float*)p.db + base};
     float* gdv = (float*)p.dv + base;
+    // position `it` of the CTA's list: chain, chunk, and (PAR) element offset of the chain
+    struct Item { long long bh, off; int c, t; };
+    const int items = PAR ? min(wk.per, wk.total - (int)blockIdx.x * wk.per) : nchunks;
+    auto item = [&](int it) {
+        if (!PAR) return Item{bh, 0, nchunks - 1 - it, it};
+        const int x = (int)blockIdx.x * wk.per + it, chain = (int)((unsigned)x / (unsigned)wk.count), t = x - chain * wk.count;
+        const int b = (int)((unsigned)chain / (unsigned)p.H);
+        return Item{chain, b * p.st.b + (chain - b * (int)p.H) * p.st.h, nchunks - 1 - wk.it0 - t, t};
+    };
     const float* gg = LN ? (const float*)p.g + base : nullptr;
     float* gdg = LN ? (float*)p.dg + base : nullptr;
     constexpr uint32_t ROW_BYTES = N * 4;
@@ -175,8 +208,8 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         for (int i = tid; i < 3 * N; i += THREADS) sm.lnp[i] = p.params[(long long)(i / N) * p.H * N + hi * N + (i % N)];
     }
     // stage-B scratch aliased onto the score-gradient buffers
-    float* const dvsc = sm.sgrad + warp * (L * YS);
-    float* const red = sm.sgrad + WARPS * L * YS;  // [WARPS][L][2]
+    float* const dvsc = sm.sgrad_ + (PAR ? 0 : warp * (L * YS));  // (PAR has neither)
+    float* const red = sm.sgrad_ + (PAR ? 0 : WARPS * L * YS);  // [WARPS][L][2]
     float* const red2 = red + WARPS * L * 2;                                             // [WARPS][L][3]
     float dlnw_acc[2] = {0.f, 0.f}, dlnb_acc[2] = {0.f, 0.f}, dbon_acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
     // Carried decay term for the last chunk: sum_i dsT[i,:] * sT[i,:] (zero without dsT).
@@ -187,7 +220,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (p.dsT && p.sT && tid < N) {
+    if (!PAR && p.dsT && p.sT && tid < N) {
         const float* d = p.dsT + bh * N * N;
         const float* s = p.sT + bh * N * N;
         float acc = 0.f;
@@ -199,51 +232,63 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
     // cp.async; a chunk's loads are issued one iteration ahead and waited for before the barrier
     // that ends the iteration.
     constexpr int CH = ROW_BYTES / 16;
-    auto issue_in = [&](int c) {
+    auto issue_in = [&](const Item& n) {
+        const int c = n.c;
         for (int i = tid; i < 5 * L * CH; i += THREADS) {
             const int ten = i / (L * CH), row = (i / CH) % L, ch = i % CH;
             const long long tt = (long long)c * L + row;
             if (has_tail) cp_async16_zfill(sm.st_in[ten] + st_at(row, ch * 4),
-                             reinterpret_cast<const unsigned char*>(gin[ten] + (tt < p.T ? tt : p.T - 1) * p.st.t) + ch * 16, tt < p.T);
-            else cp_async16(sm.st_in[ten] + st_at(row, ch * 4), reinterpret_cast<const unsigned char*>(gin[ten] + tt * p.st.t) + ch * 16);
+                             reinterpret_cast<const unsigned char*>(gin[ten] + n.off + (tt < p.T ? tt : p.T - 1) * p.st.t) + ch * 16, tt < p.T);
+            else cp_async16(sm.st_in[ten] + st_at(row, ch * 4), reinterpret_cast<const unsigned char*>(gin[ten] + n.off + tt * p.st.t) + ch * 16);
         }
     };
-    auto issue_vdy = [&](int c, int s) {
+    auto issue_vdy = [&](const Item& n, int s) {
+        const int c = n.c;
         for (int i = tid; i < (LN ? 3 : 2) * L * CH; i += THREADS) {
             const int ten = i / (L * CH), row = (i / CH) % L, ch = i % CH;
             const long long tt = (long long)c * L + row;
-            const float* src = (ten == 0 ? gv : ten == 1 ? gdy : gg) + (!TAIL || tt < p.T ? tt : p.T - 1) * p.st.t;
+            const float* src = (ten == 0 ? gv : ten == 1 ? gdy : gg) + n.off + (!TAIL || tt < p.T ? tt : p.T - 1) * p.st.t;
             unsigned char* dst = (ten == 0 ? sm.st_v[s] : ten == 1 ? sm.st_dy[s] : sm.st_g[LN ? s : 0]) + st_at(row, ch * 4);
             if (has_tail) cp_async16_zfill(dst, reinterpret_cast<const unsigned char*>(src) + ch * 16, tt < p.T);
             else cp_async16(dst, reinterpret_cast<const unsigned char*>(src) + ch * 16);
         }
     };
+    // (by thread 0, after the expectation that counts their bytes, too)
+    auto issue_mats = [&](const Item& n) {
+        const uint32_t bar = smem_u32(&sm.s0_bar);
+        const int record = (int)(n.bh * nchunks + n.c);
+        // the matrices: the record keeps them as the forward's operand tiles, 16-byte pieces [row / 8][column / 4][row % 8];
+        // seen as [row group][row bit 2][row % 4][piece][4 floats], a box of 6 pieces per row (2 of them beyond the
+        // row: zero fill) lands as rows of 24 floats; the second block starts at piece -2
+#pragma unroll
+        for (int blk = 0; blk < 2; ++blk)
+            asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+                         ::"r"(smem_u32(sm.mats + blk * MAT_BLK)), "l"(&cmaps.ckm), "r"(bar), "r"(0), "r"(-2 * blk), "r"(0), "r"(blk), "r"(record * (CK_FLOATS / 128) + CK_MATS / 128) : "memory");
+    };
     // the checkpoint record of chunk c: its start state and its four 16x16 matrices (QK, QB, AK, AI), which the
     // forward left there so that the scores and the triangular inverse are not rebuilt here
-    auto issue_s0 = [&](int c) {
+    auto issue_s0 = [&](const Item& n) {
         if (tid == 0) {
             // two boxes of [8][4 rows][72 floats]: rows 8a + b and rows 8a + 4 + b (a < 8, b < 4); the second starts at
             // column -8, so that its fill comes first in each row
             const uint32_t bar = smem_u32(&sm.s0_bar);
-            const int record = (int)(bh * nchunks + c);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)((N * SS + 2 * MAT_BLK) * 4)) : "memory");
+            const int record = (int)(n.bh * nchunks + n.c);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)(((PAR ? 2 : 1) * N * SS + 2 * MAT_BLK) * 4)) : "memory");
+            if (PAR)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(smem_u32(sm.dSs)), "l"(wk.tiles + (n.bh * wk.count + n.t) * TILE_FLOATS), "r"(TILE_FLOATS * 4), "r"(bar) : "memory");
 #pragma unroll
             for (int blk = 0; blk < 2; ++blk)
                 asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
                              ::"r"(smem_u32(sm.S0s + blk * S0_BLK)), "l"(&cmaps.ck), "r"(bar), "r"(-8 * blk), "r"(0), "r"(blk), "r"(0), "r"(record) : "memory");
-            // the matrices: the record keeps them as the forward's operand tiles, 16-byte pieces [row / 8][column / 4][row % 8];
-            // seen as [row group][row bit 2][row % 4][piece][4 floats], a box of 6 pieces per row (2 of them beyond the
-            // row: zero fill) lands as rows of 24 floats; the second block starts at piece -2
-#pragma unroll
-            for (int blk = 0; blk < 2; ++blk)
-                asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
-                             ::"r"(smem_u32(sm.mats + blk * MAT_BLK)), "l"(&cmaps.ckm), "r"(bar), "r"(0), "r"(-2 * blk), "r"(0), "r"(blk), "r"(record * (CK_FLOATS / 128) + CK_MATS / 128) : "memory");
+            if (!PAR) issue_mats(n);
         }
     };
-    if (nchunks > 0) {
-        issue_in(nchunks - 1);
-        issue_vdy(nchunks - 1, 0);
-        issue_s0(nchunks - 1);
+    if (items > 0) {
+        issue_in(item(0));
+        issue_vdy(item(0), 0);
+        issue_s0(item(0));
+        if (PAR && tid == 0) issue_mats(item(0));
         cp_async_commit();
         cp_async_wait<0>();
     }
@@ -251,7 +296,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 
     // dS: warp owns value rows 16*warp + {g, g+8}; tile nt covers key columns 8nt..8nt+7.
     float dS[8][4];
-    {
+    if (!PAR) {
         const float* d = p.dsT ? p.dsT + bh * N * N : nullptr;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
@@ -286,9 +331,25 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         return f;
     };
     bool live = true;  // this thread has not given up a wait for a record: none is requested after that
-    for (int it = 0; it < nchunks; ++it) {
-        const int c = nchunks - 1 - it;
-        const int vs = it & 1;
+    for (int it = 0; it < items; ++it) {
+        const Item now = item(it);
+        const int c = now.c;
+        const int vs = PAR ? 0 : it & 1, gp_set = it & 1;
+        // PAR: this thread's entries of the state at the chunk's end, for the carried decay term (zero for a final state that is not given)
+        float2 nx[PAR ? 8 : 1][2];
+        if (PAR) {
+            const bool last = c + 1 == nchunks;
+            const float* q = last ? (p.dsT && p.sT ? p.sT + now.bh * N * N : nullptr) : p.ckpt + (now.bh * nchunks + c + 1) * CK_FLOATS + CK_STATE;
+            const float sc = last ? STATE_SCALE : 1.f;
+            if (q) q += (16 * warp + g) * N + 2 * t4;
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float2 v = q ? *reinterpret_cast<const float2*>(q + 8 * h * N + 8 * nt) : make_float2(0.f, 0.f);
+                    nx[PAR ? nt : 0][h] = make_float2(v.x * sc, v.y * sc);
+                }
+        }
         // ---------------- P1: decay scan and scaled operands -------------------------------------
         {
             decay_scan<float, PREC, 1>(sm.st_in[0], sm.st_in[1], sm.st_in[2], sm.st_in[3], sm.st_in[4], ROWB, sm.wq, sm.wa,
@@ -309,9 +370,9 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             }
         }
         __syncthreads();  // (A)
-        if (c > 0) {
-            issue_in(c - 1);
-            issue_vdy(c - 1, vs ^ 1);
+        if (it + 1 < items) {
+            issue_in(item(it + 1));
+            if (!PAR) issue_vdy(item(it + 1), vs ^ 1);
         }
 
         // ---------------- stage B: rows = value index -----------------------------------------
@@ -329,9 +390,47 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         float X[2][4] = {};
         if (!LN) live = s0_wait(&sm.s0_bar, it & 1, &sm.abort, p.status) && live;  // this chunk's start state has landed
         // attn: the X = S0 wa^T products ride in the same loop, six independent accumulator chains instead of four, then two
-        auto du_dv = [&]() {
+        auto carry = [&](float (&gp)[16]) {  // sum over the rows of gp, a thread's part of it: [2 * nt + e] for key column 8 * nt + 2 * t4 + e
+            // Sum over the eight row lanes g as a reduce-scatter: every step halves the values a lane carries (8 + 4 + 2
+            // shuffles instead of 3 per value), and lane g ends with the two sums of tile nt = bit-reversed g.
+            const bool b0 = g & 1, b1 = g & 2, b2 = g & 4;
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
+            for (int i = 0; i < 8; ++i) {
+                const float send = b0 ? gp[i] : gp[i + 8], keep = b0 ? gp[i + 8] : gp[i];
+                gp[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float send = b1 ? gp[i] : gp[i + 4], keep = b1 ? gp[i + 4] : gp[i];
+                gp[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float send = b2 ? gp[i] : gp[i + 2], keep = b2 ? gp[i + 2] : gp[i];
+                gp[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+            }
+            const int nt_own = (b2 ? 1 : 0) + (b1 ? 2 : 0) + (b0 ? 4 : 0);
+            *reinterpret_cast<float2*>(&sm.Gp[PAR ? gp_set ^ 1 : gp_set][warp][8 * nt_own + 2 * t4]) = make_float2(gp[0], gp[1]);
+        };
+        auto du_dv = [&]() {
+            float* const own = sm.dSs + (16 * warp + g) * SS;  // PAR: dS comes through shared memory, dSf goes there at once
+            if (PAR) {
+                float gp[16];
+#pragma unroll
+                for (int nt = 0; nt < 8; ++nt) {
+                    float* q = own + xcol<1>(g, 8 * nt + 2 * t4);
+                    const float2 f = *reinterpret_cast<const float2*>(sm.fw + 8 * nt + 2 * t4), lo = *reinterpret_cast<const float2*>(q), hi2 = *reinterpret_cast<const float2*>(q + 8 * SS);
+                    const float2 (&n2)[2] = nx[PAR ? nt : 0];
+                    gp[2 * nt] = lo.x * n2[0].x + hi2.x * n2[1].x;
+                    gp[2 * nt + 1] = lo.y * n2[0].y + hi2.y * n2[1].y;
+                    *reinterpret_cast<float2*>(q) = make_float2(lo.x * STATE_SCALE * f.x, lo.y * STATE_SCALE * f.y);
+                    *reinterpret_cast<float2*>(q + 8 * SS) = make_float2(hi2.x * STATE_SCALE * f.x, hi2.y * STATE_SCALE * f.y);
+                }
+                carry(gp);
+                __syncwarp();
+            }
+#pragma unroll
+            for (int nt = 0; nt < (PAR ? 0 : 8); ++nt) {
                 const float2 f = *reinterpret_cast<const float2*>(sm.fw + 8 * nt + 2 * t4);  // P~_L = 2^64 P_L
                 dS[nt][0] = dS[nt][0] * STATE_SCALE * f.x; dS[nt][1] = dS[nt][1] * STATE_SCALE * f.y;
                 dS[nt][2] = dS[nt][2] * STATE_SCALE * f.x; dS[nt][3] = dS[nt][3] * STATE_SCALE * f.y;
@@ -343,21 +442,36 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                     mma<PREC>(du[sb], dyf[tb], mat_kn(3, sb, tb));
                     mma<PREC>(dV[sb], dyf[tb], mat_kn(1, sb, tb));
                 }
-#pragma unroll
+            // (PAR: rolled, so that a chunk's code fits the instruction cache; the small terms apart, a third of the dependent products)
+            float small[PAR ? 6 : 1][4] = {};
+#pragma unroll PAR ? 1 : 8
             for (int kk = 0; kk < 8; ++kk) {
-                FragA<PREC> a = fragA_from_acc<PREC>(dS[kk]);
+                FragA<PREC> a;
+                if (PAR) {
+                    const float* q = own + xcol<1>(g, 8 * kk + 2 * t4);
+                    const float2 lo = *reinterpret_cast<const float2*>(q), hi2 = *reinterpret_cast<const float2*>(q + 8 * SS);
+                    a.x[0].set(lo.x); a.x[1].set(hi2.x); a.x[2].set(lo.y); a.x[3].set(hi2.y);
+                } else {
+                    a = fragA_from_acc<PREC>(dS[PAR ? 0 : kk]);
+                }
 #pragma unroll
                 for (int sb = 0; sb < 2; ++sb) {
-                    mma<PREC>(du[sb], a, fragB_nk<PREC, true, 1>(sm.bwi, OPS, 8 * sb, 8 * kk, g, t4));
-                    mma<PREC>(dV[sb], a, fragB_nk<PREC, true, 1>(sm.kwi, OPS, 8 * sb, 8 * kk, g, t4));
+                    mma2<PREC, PAR>(du[sb], small[PAR ? sb : 0], a, fragB_nk<PREC, true, 1>(sm.bwi, OPS, 8 * sb, 8 * kk, g, t4));
+                    mma2<PREC, PAR>(dV[sb], small[PAR ? 2 + sb : 0], a, fragB_nk<PREC, true, 1>(sm.kwi, OPS, 8 * sb, 8 * kk, g, t4));
                 }
                 if (!LN) {
                     FragA<PREC> a0;
                     const float2 lo = *reinterpret_cast<const float2*>(s0_mk + 8 * kk), hi2 = *reinterpret_cast<const float2*>(s0_mk + 4 * SS + 8 * kk);
                     a0.x[0].setr(lo.x); a0.x[1].setr(hi2.x); a0.x[2].setr(lo.y); a0.x[3].setr(hi2.y);
 #pragma unroll
-                    for (int nt = 0; nt < 2; ++nt) mma<PREC>(X[nt], a0, fragB_nk<PREC, true, 1>(sm.wa, OPS, 8 * nt, 8 * kk, g, t4));
+                    for (int nt = 0; nt < 2; ++nt) mma2<PREC, PAR>(X[nt], small[PAR ? 4 + nt : 0], a0, fragB_nk<PREC, true, 1>(sm.wa, OPS, 8 * nt, 8 * kk, g, t4));
                 }
+            }
+#pragma unroll
+            for (int i = 0; i < (PAR ? 8 : 0); ++i) {
+                du[i >> 2][i & 3] += small[PAR ? i >> 2 : 0][i & 3];
+                dV[i >> 2][i & 3] += small[PAR ? 2 + (i >> 2) : 0][i & 3];
+                X[i >> 2][i & 3] += small[PAR ? 4 + (i >> 2) : 0][i & 3];
             }
         };
         if (!LN) du_dv();
@@ -561,8 +675,16 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
             for (int tb = sb; tb < 2; ++tb) mma<PREC>(dV[sb], dbf[tb], mat_kn(0, sb, tb));
 
-        // dv out, transposed through a per-warp scratch tile for 16-byte stores
-        {
+        if (PAR) {  // dv out, whole sectors of eight values
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const long long row = (long long)c * L + 8 * nt + 2 * t4 + e;
+                    float* q = gdv + now.off + row * p.st.t + 16 * warp + g;
+                    if (!TAIL || row < p.T) { q[0] = dV[nt][e]; q[8] = dV[nt][e + 2]; }
+                }
+        } else {  // transposed through a per-warp scratch tile for 16-byte stores
             float* sc = dvsc;
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
@@ -575,7 +697,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             __syncwarp();
             const int row = lane >> 1, hf = lane & 1;
             const uint4* src = reinterpret_cast<const uint4*>(sc + row * YS + 8 * hf);
-            uint4* dst = reinterpret_cast<uint4*>(gdv + ((long long)c * L + row) * p.st.t + 16 * warp + 8 * hf);
+            uint4* dst = reinterpret_cast<uint4*>(gdv + now.off + ((long long)c * L + row) * p.st.t + 16 * warp + 8 * hf);
             if (!TAIL || (long long)c * L + row < p.T) {
                 dst[0] = src[0];
                 dst[1] = src[1];
@@ -583,7 +705,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         }
         // dSf, U, dabu to shared memory for stage C
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
+        for (int nt = 0; nt < (PAR ? 0 : 8); ++nt) {
             *reinterpret_cast<float2*>(sm.dSs + (16 * warp + g) * SS + xcol<1>(g, 8 * nt + 2 * t4)) = make_float2(pre<PREC>(dS[nt][0]), pre<PREC>(dS[nt][1]));
             *reinterpret_cast<float2*>(sm.dSs + (16 * warp + g + 8) * SS + xcol<1>(g, 8 * nt + 2 * t4)) = make_float2(pre<PREC>(dS[nt][2]), pre<PREC>(dS[nt][3]));
         }
@@ -597,8 +719,8 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             sm.Dt[tq * OPS + c1] = pre<PREC>(dabu[nt][2]); sm.Dt[(tq + 1) * OPS + c1] = pre<PREC>(dabu[nt][3]);
         }
         // dS0 = dSf + dY^T wq + dabu^T wa ; carried decay term sum_i dS0[i,:] S0[i,:]
-        {
-            float gp[16];  // this thread's two rows: [2 * nt + e] for key column 8 * nt + 2 * t4 + e
+        if (!PAR) {
+            float gp[16];  // this thread's two rows
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
 #pragma unroll
@@ -611,26 +733,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 gp[2 * nt] = dS[nt][0] * lo.x + dS[nt][2] * hi2.x;
                 gp[2 * nt + 1] = dS[nt][1] * lo.y + dS[nt][3] * hi2.y;
             }
-            // Sum over the eight row lanes g as a reduce-scatter: every step halves the values a lane carries (8 + 4 + 2
-            // shuffles instead of 3 per value), and lane g ends with the two sums of tile nt = bit-reversed g.
-            const bool b0 = g & 1, b1 = g & 2, b2 = g & 4;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float send = b0 ? gp[i] : gp[i + 8], keep = b0 ? gp[i + 8] : gp[i];
-                gp[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float send = b1 ? gp[i] : gp[i + 4], keep = b1 ? gp[i + 4] : gp[i];
-                gp[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float send = b2 ? gp[i] : gp[i + 2], keep = b2 ? gp[i + 2] : gp[i];
-                gp[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-            }
-            const int nt_own = (b2 ? 1 : 0) + (b1 ? 2 : 0) + (b0 ? 4 : 0);
-            *reinterpret_cast<float2*>(&sm.Gp[it & 1][warp][8 * nt_own + 2 * t4]) = make_float2(gp[0], gp[1]);
+            carry(gp);
         }
         __syncthreads();  // (C1)
         // ---------------- stage C: contractions over the value index --------------------------
@@ -640,10 +743,10 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             // 2 dQB = tril(dY U^T), 3 dAB = stril(dabu U^T)
             float d[2][4] = {};
             const bool strict = warp & 1;
-            float* dst = sm.sgrad + warp * (L * SCS);  // 0 dQK, 1 dAK, 2 dQB, 3 dAB
+            float* dst = sm.sgrad() + warp * (L * SCS);  // 0 dQK, 1 dAK, 2 dQB, 3 dAB
             // (rolled, as far as registers allow no less: the chunk loop is 100 KB of code in the triple-TF32 class, three times the
             // instruction cache; 96 chains of 32 chunks 339 -> 325 us)
-#pragma unroll 2
+#pragma unroll PAR ? 1 : 2
             for (int kk = 0; kk < 8; ++kk) {
                 FragA<PREC> aD = fragA_mk<PREC, true, 1>(sm.Dt, OPS, 0, 8 * kk, g, t4);
                 FragA<PREC> aY = LN ? fragA_mk<PREC, true, 1>(sm.Yt, OPS, 0, 8 * kk, g, t4) : fragA_mk_st<PREC>(dyt, 8 * kk, g, t4);
@@ -651,8 +754,9 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 FragA<PREC> aV = fragA_mk_st<PREC>(vt, 8 * kk, g, t4);
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt) {
-                    FragB<PREC> bsc = (warp >> 1) ? fragB_nk<PREC, true, 1>(sm.Ut, OPS, 8 * nt, 8 * kk, g, t4)
-                                                  : fragB_nk_st<PREC>(vt, 8 * nt, 8 * kk, g, t4);
+                    FragB<PREC> bsc;  // [contraction][row of half nt] of U or V: registers of its A fragment
+                    bsc.x[0] = (warp >> 1) ? aU.x[nt] : aV.x[nt];
+                    bsc.x[1] = (warp >> 1) ? aU.x[2 + nt] : aV.x[2 + nt];
                     mma<PREC>(d[nt], strict ? aD : aY, bsc);
                     FragB<PREC> bS;
                     bS.x[0].setr(s0_kn[4 * kk * SS + 8 * nt]); bS.x[1].setr(s0_kn[(4 * kk + 1) * SS + 8 * nt]);
@@ -673,13 +777,15 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                     make_float2(keep(g + 8, s) ? pre<PREC>(d[nt][2]) : 0.f, keep(g + 8, s + 1) ? pre<PREC>(d[nt][3]) : 0.f);
             }
         }
-        __syncthreads();  // (C2) score gradients visible; S0s free
-        if (c > 0 && live) issue_s0(c - 1);
+        if (PAR) fence_async_smem();  // dSs was written here and comes by bulk copy next
+        __syncthreads();  // (C2) score gradients visible; S0s (and dSs) free
+        if (it + 1 < items && live) issue_s0(item(it + 1));
+        if (PAR && it + 1 < items) issue_vdy(item(it + 1), 0);
         cp_async_commit();
 
 #pragma unroll 1
         for (int kk = 0; kk < 2; ++kk) {
-            const float *dQK = sm.sgrad, *dAK = sm.sgrad + L * SCS, *dQB = sm.sgrad + 2 * L * SCS, *dAB = sm.sgrad + 3 * L * SCS;
+            const float *dQK = sm.sgrad(), *dAK = dQK + L * SCS, *dQB = dQK + 2 * L * SCS, *dAB = dQK + 3 * L * SCS;
             FragA<PREC> aAB = fragA_mk<PREC, true, 1>(dAB, SCS, 0, 8 * kk, g, t4), aAK = fragA_mk<PREC, true, 1>(dAK, SCS, 0, 8 * kk, g, t4);
             FragA<PREC> aQB = fragA_mk<PREC, true, 1>(dQB, SCS, 0, 8 * kk, g, t4), aQK = fragA_mk<PREC, true, 1>(dQK, SCS, 0, 8 * kk, g, t4);
             FragA<PREC> tAB = fragA_km<PREC, true, 1>(dAB, SCS, 0, 8 * kk, g, t4), tAK = fragA_km<PREC, true, 1>(dAK, SCS, 0, 8 * kk, g, t4);
@@ -707,8 +813,10 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 const int kx = xcol<1>(tq, key);
                 const float2 cu = *reinterpret_cast<const float2*>(sm.cum + tq * OPS + kx);
                 float2 lwp;
+                float2 up = make_float2(STATE_UNSCALE, STATE_UNSCALE);  // P~ before the first step
                 if (PREC == 3) {
                     lwp = *reinterpret_cast<const float2*>(sm.lw + tq * OPS + kx);
+                    if (tq > 0) up = *reinterpret_cast<const float2*>(sm.cum + (tq - 1) * OPS + xcol<1>(tq - 1, key));
                 } else {  // running log-decay difference; row -1 is zero
                     const float2 cp = tq > 0 ? *reinterpret_cast<const float2*>(sm.cum + (tq - 1) * OPS + xcol<1>(tq - 1, key)) : make_float2(0.f, 0.f);
                     lwp = make_float2(cu.x - cp.x, cu.y - cp.y);
@@ -723,11 +831,11 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int i = e + 2 * hrow;
-                    const float incl = decay_up<PREC>(cuv[e]);   // P~_t, as the scan formed it
+                    const float incl = PREC == 3 ? cuv[e] : decay_up<PREC>(cuv[e]);   // P~_t, as the scan formed it
                     const float inv = rcp_p<PREC>(incl);
                     // P_{t-1} = exp(cum_{t-1}) with cum_{t-1} = cum_t - lw_t (0 for the first row): an exponential on the idle
-                    // special-function unit instead of two shuffles for the row above
-                    const float non = decay_up<PREC>(cuv[e] - lwa[e]);
+                    // special-function unit instead of two shuffles for the row above; fp32 class: from the row above (an exponential is 15 instructions)
+                    const float non = PREC == 3 ? (e ? up.y : up.x) : decay_up<PREC>(cuv[e] - lwa[e]);
                     o_a[e] = non * DA[nt][i];
                     o_q[e] = incl * DQ[nt][i];
                     o_b[e] = inv * DB[nt][i];
@@ -774,7 +882,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         {
 #pragma unroll
             for (int hrow = 0; hrow < 2; ++hrow) {
-                const long long off = ((long long)c * L + g + 8 * hrow) * p.st.t + 16 * warp;
+                const long long off = now.off + ((long long)c * L + g + 8 * hrow) * p.st.t + 16 * warp;
                 const bool live = !TAIL || (long long)c * L + g + 8 * hrow < p.T;  // uniform over the lanes that exchange values
 #pragma unroll
                 for (int ten = 0; ten < 5; ++ten)
@@ -782,7 +890,9 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
             }
         }
         cp_async_wait<0>();
+        if (PAR) fence_async_smem();  // the score gradients' place is filled by bulk copies next
         __syncthreads();  // (E)
+        if (PAR && tid == 0 && it + 1 < items && live) issue_mats(item(it + 1));
     }
 
     if (LN) {
@@ -807,7 +917,7 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
                 if (g == 0) ws[2 * p.H * N + 16 * warp + 8 * nt + 2 * t4 + e] = a;
             }
     }
-    if (p.ds0) {
+    if (!PAR && p.ds0) {
         float* o = p.ds0 + bh * N * N;
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
@@ -816,6 +926,236 @@ __global__ void __launch_bounds__(THREADS) wkv7_bwd_kernel(BwdParams p, const __
         }
     }
     if (tid == 0 && sm.abort) mbar_landed_uncounted(&sm.s0_bar, &sm.zero, p.status);
+}
+
+// ---- the state gradient alone, fp32 ------------------------------------------------------------------------------------------------
+// The products that carry dS from chunk to chunk (stage B's du, dabu and dS0), one CTA per chain, triple TF32.  Four chain warps (16 value
+// rows of dS each, no exchange between them); WALK_PREP groups of four warps fetch a chunk's inputs and scan it, and split its operands
+// into the two TF32 parts once instead of at each of their uses; WALK_SLOTS chunks in flight.  Leaves dS at the end of every chunk in
+// `tiles`, from where the chunk kernel (PAR) takes all chunks over all SMs.  With a chunk's whole work on the chain it took 20 000 cycles,
+// most of them for fetching its 90 KB of code.
+// Bound by the chain of dependent products, 3300 cycles a chunk (two preparation groups: 3700).  Backward in us, one kernel -> walk and
+// chunks: 96 chains of 32 chunks 336 -> 212, 8 of 256 2573 -> 534, 320 of 52 1461 -> 992, 2048 of 8 1095 -> 929.
+constexpr int WALK_SLOTS = 4, WALK_PREP = 3, WALK_THREADS = THREADS * (1 + WALK_PREP);
+struct Walk32Slot {
+    alignas(16) unsigned char dy[TILEB];
+    alignas(16) float mats[2 * L * L];               // AI^T, QB as the record holds them
+    alignas(16) float op[3][2][L * OPS];             // wq, wa, bwi: upper and lower part, column swizzle xcol<1>
+    alignas(16) float fw[N];
+};
+struct Walk32Smem {
+    alignas(16) unsigned char raw[WALK_PREP][4][TILEB];  // q, w, a, b
+    Walk32Slot slot[WALK_SLOTS];
+    uint64_t ready[WALK_SLOTS], free[WALK_SLOTS];
+    volatile int abort;
+};
+static_assert(sizeof(Walk32Smem) <= 232448, "one CTA per SM");
+
+template <bool TAIL>
+__global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk32_kernel(BwdParams p, float* tiles, int it0, int count) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    Walk32Smem& sm = *reinterpret_cast<Walk32Smem*>(smem_raw);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t4 = lane & 3, w = warp & 3;
+    const int bh = blockIdx.x, bi = bh / (int)p.H, hi = bh - bi * (int)p.H, nchunks = (int)((p.T + L - 1) / L), c0 = nchunks - 1 - it0;
+    const long long base = bi * p.st.b + hi * p.st.h;
+    if (tid == 0) {
+        for (int i = 0; i < WALK_SLOTS; ++i) {
+            mbar_init(&sm.ready[i], WARPS);
+            mbar_init(&sm.free[i], WARPS);
+        }
+        sm.abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (warp >= WARPS) {
+        // ---- preparation: group `grp` takes every WALK_PREP-th chunk
+        const int grp = warp / WARPS - 1, gt = tid & (THREADS - 1);
+        const float* in[5] = {(const float*)p.r + base, (const float*)p.w + base, (const float*)p.a + base, (const float*)p.b + base, (const float*)p.dy + base};
+        auto piece = [&](void* dst, const float* src, int n, int row) {  // 16 bytes of step n's chunk, rows beyond the sequence as zeros
+            const long long tt = (long long)(c0 - n) * L + row;
+            if (TAIL) cp_async16_zfill(dst, src + (tt < p.T ? tt : p.T - 1) * p.st.t, tt < p.T);
+            else cp_async16(dst, src + tt * p.st.t);
+        };
+        const int prow = gt / (N / 4), pch = 4 * (gt % (N / 4));  // a thread's pieces: rows prow, prow + 8
+        auto fetch = [&](int n) {  // q, w, a, b
+#pragma unroll
+            for (int ten = 0; ten < 4; ++ten)
+#pragma unroll
+                for (int r = prow; r < L; r += 8) piece(sm.raw[grp][ten] + st_at(r, pch), in[ten] + pch, n, r);
+        };
+        auto fetch_slot = [&](int n) {  // dy and the record's matrices
+            Walk32Slot& t = sm.slot[n % WALK_SLOTS];
+#pragma unroll
+            for (int r = prow; r < L; r += 8) piece(t.dy + st_at(r, pch), in[4] + pch, n, r);
+            cp_async16(t.mats + 4 * gt, p.ckpt + ((long long)bh * nchunks + c0 - n) * CK_FLOATS + CK_AI + 4 * gt);
+            static_assert(2 * L * L == 4 * THREADS, "a piece per thread");
+        };
+        auto group_bar = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); };
+        const int row = lane & 15, j0 = 16 * w + 8 * (lane >> 4), at = row * OPS + xcol<1>(row, j0);
+        const bool flip = (row >> 2) & 1;
+        auto split = [&](float (*op)[L * OPS], const float (&x)[8]) {
+            float h[8], l[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                h[i] = __uint_as_float(tf32_rna(x[i]));
+                l[i] = __uint_as_float(tf32_rna(x[i] - h[i]));
+            }
+            store8(op[0] + at, h, flip);
+            store8(op[1] + at, l, flip);
+        };
+        if (grp < count) fetch(grp);
+        for (int n = grp; n < count; n += WALK_PREP) {
+            if (n >= WALK_SLOTS) mbar_wait_bounded<true>(&sm.free[n % WALK_SLOTS], (n / WALK_SLOTS - 1) & 1, &sm.abort, p.status);
+            fetch_slot(n);
+            cp_async_commit();
+            cp_async_wait<0>();
+            group_bar();  // everyone's pieces have landed
+            Walk32Slot& t = sm.slot[n % WALK_SLOTS];
+            const unsigned char (*raw)[TILEB] = sm.raw[grp];
+            const int off = st_at(row, j0);
+            float lw[8], cum[8], x[8], o[8];
+            load8<float>(raw[1] + off, lw);
+            const int live = TAIL ? (int)min((long long)L, p.T - (long long)(c0 - n) * L) : L;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cum[i] = lw[i] = row < live ? fmaxf(-exp_p<3>(lw[i]), MIN_STEP_LOG_DECAY) : 0.f;  // as decay_scan()
+#pragma unroll
+            for (int d = 1; d < 16; d <<= 1)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float up = __shfl_up_sync(0xffffffffu, cum[i], d, 16);
+                    if (row >= d) cum[i] += up;
+                }
+            load8<float>(raw[2] + off, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = x[i] * decay_up<3>(cum[i] - lw[i]);
+            split(t.op[1], o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                cum[i] = decay_up<3>(cum[i]);
+                if (row == 15) t.fw[j0 + i] = cum[i];
+            }
+            load8<float>(raw[0] + off, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = x[i] * cum[i];
+            split(t.op[0], o);
+            load8<float>(raw[3] + off, x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = x[i] * rcp_p<3>(cum[i]);
+            split(t.op[2], o);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.ready[n % WALK_SLOTS]);
+            group_bar();  // the raw tiles have been read
+            if (n + WALK_PREP < count) fetch(n + WALK_PREP);
+        }
+        cp_async_wait<0>();
+        return;
+    }
+    // ---- the chain: value rows 16 w + {g, g + 8} of dS, carried as in wkv7_bwd_kernel
+    const int bg = (g >> 2) & 1, bt = (t4 >> 1) & 1;  // element offsets under xcol<1> (pitch 72)
+    const int mkE = g * OPS + 2 * t4 + 8 * bg, mkO = mkE - 16 * bg, knE = 2 * t4 * OPS + g + 8 * bt, knO = knE - 16 * bt;
+    auto mk = [&](int kk) { return (kk & 1 ? mkO : mkE) + 8 * kk; };
+    auto kn = [&](int nb) { return (nb & 1 ? knO : knE) + 8 * nb; };
+    auto put = [](FragB<3>& f, int i, float h, float l) { f.x[i].h = __float_as_uint(h); f.x[i].l = __float_as_uint(l); };
+    float dS[8][4];
+    const long long st = (long long)bh * N * N + (16 * w + g) * N + 2 * t4;
+    {
+        const float* src = it0 ? p.ds0 : p.dsT;  // a later pass goes on from where the earlier one left it
+        const float scale = it0 ? 1.f : STATE_UNSCALE;
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            const float2 lo = src ? *reinterpret_cast<const float2*>(src + st + 8 * nt) : make_float2(0.f, 0.f);
+            const float2 hi2 = src ? *reinterpret_cast<const float2*>(src + st + 8 * N + 8 * nt) : make_float2(0.f, 0.f);
+            dS[nt][0] = lo.x * scale; dS[nt][1] = lo.y * scale; dS[nt][2] = hi2.x * scale; dS[nt][3] = hi2.y * scale;
+        }
+    }
+    float* out = tiles + (long long)bh * count * TILE_FLOATS + 16 * w * SS;
+    for (int n = 0; n < count; ++n, out += TILE_FLOATS) {
+        const int s = n % WALK_SLOTS;
+        const Walk32Slot& t = sm.slot[s];
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            *reinterpret_cast<float2*>(out + mk(nt)) = make_float2(dS[nt][0], dS[nt][1]);
+            *reinterpret_cast<float2*>(out + 8 * SS + mk(nt)) = make_float2(dS[nt][2], dS[nt][3]);
+        }
+        mbar_wait_bounded<false>(&sm.ready[s], (n / WALK_SLOTS) & 1, &sm.abort, p.status);
+        const FragA<3> dyf[2] = {fragA_km_st<3>(t.dy, 16 * w, 0, g, t4), fragA_km_st<3>(t.dy, 16 * w, 8, g, t4)};
+        // matrix m (0 AI^T, 1 QB): element (row, col) of the record's operand tiles
+        auto mat = [&](int m, int row, int col) { return t.mats + m * L * L + (row >> 3) * 128 + (col >> 2) * 32 + (row & 7) * 4 + (col & 3); };
+        auto B_kn = [&](int op, int nb, int kk) {
+            const float *q = t.op[op][0] + 8 * kk * OPS + kn(nb), *l = q + L * OPS;
+            FragB<3> f;
+            put(f, 0, q[0], l[0]); put(f, 1, q[OPS], l[OPS]);
+            return f;
+        };
+        // (the three terms of a product apart: the sums over the keys are what the chain waits for)
+        float du[2][4] = {}, du_l[2][4] = {}, du_r[2][4] = {}, dabu[2][4] = {}, dabu_s[2][4] = {};
+#pragma unroll
+        for (int sb = 0; sb < 2; ++sb)
+#pragma unroll
+            for (int tb = sb; tb < 2; ++tb) {
+                FragB<3> b;
+                b.x[0].set(*mat(1, 8 * tb + 2 * t4, 8 * sb + g)); b.x[1].set(*mat(1, 8 * tb + 2 * t4 + 1, 8 * sb + g));
+                mma2<3, true>(du[sb], du_r[sb], dyf[tb], b);
+            }
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+            const float2 f = *reinterpret_cast<const float2*>(t.fw + 8 * kk + 2 * t4);
+            dS[kk][0] = dS[kk][0] * STATE_SCALE * f.x; dS[kk][1] = dS[kk][1] * STATE_SCALE * f.y;
+            dS[kk][2] = dS[kk][2] * STATE_SCALE * f.x; dS[kk][3] = dS[kk][3] * STATE_SCALE * f.y;
+            const FragA<3> a = fragA_from_acc<3>(dS[kk]);
+#pragma unroll
+            for (int sb = 0; sb < 2; ++sb) {
+                const float* q = t.op[2][0] + 8 * sb * OPS + mk(kk);
+                const float2 h = *reinterpret_cast<const float2*>(q), l = *reinterpret_cast<const float2*>(q + L * OPS);
+                FragB<3> b;
+                put(b, 0, h.x, l.x); put(b, 1, h.y, l.y);
+                mma_tf32_raw(du[sb], a.x[0].h, a.x[1].h, a.x[2].h, a.x[3].h, b.x[0].h, b.x[1].h);
+                mma_tf32_raw(du_l[sb], a.x[0].l, a.x[1].l, a.x[2].l, a.x[3].l, b.x[0].h, b.x[1].h);
+                mma_tf32_raw(du_r[sb], a.x[0].h, a.x[1].h, a.x[2].h, a.x[3].h, b.x[0].l, b.x[1].l);
+            }
+            mma<3>(dS[kk], dyf[0], B_kn(0, kk, 0));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) du[i >> 2][i & 3] += du_l[i >> 2][i & 3] + du_r[i >> 2][i & 3];
+        const FragA<3> da2[2] = {fragA_from_acc<3>(du[0]), fragA_from_acc<3>(du[1])};
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int kb = nb; kb < 2; ++kb) {
+                FragB<3> b;
+                const float2 v = *reinterpret_cast<const float2*>(mat(0, 8 * nb + g, 8 * kb + 2 * t4));
+                b.x[0].set(v.x); b.x[1].set(v.y);
+                mma2<3, true>(dabu[nb], dabu_s[nb], da2[kb], b);
+            }
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) mma<3>(dS[nt], dyf[1], B_kn(0, nt, 1));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dabu[i >> 2][i & 3] += dabu_s[i >> 2][i & 3];
+        const FragA<3> dbf[2] = {fragA_from_acc<3>(dabu[0]), fragA_from_acc<3>(dabu[1])};
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            mma<3>(dS[nt], dbf[0], B_kn(1, nt, 0));
+            mma<3>(dS[nt], dbf[1], B_kn(1, nt, 1));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.free[s]);
+    }
+    const float scale = it0 + count < nchunks ? 1.f : STATE_SCALE;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+        *reinterpret_cast<float2*>(p.ds0 + st + 8 * nt) = make_float2(dS[nt][0] * scale, dS[nt][1] * scale);
+        *reinterpret_cast<float2*>(p.ds0 + st + 8 * N + 8 * nt) = make_float2(dS[nt][2] * scale, dS[nt][3] * scale);
+    }
+}
+
+// How many chunks of each chain are walked at a time: tiles of at most 512 MB, longer sequences take several passes, the walk going on
+// from ds0.  0: not at all: with three chunks the second launch costs what it saves (144 chains: 78 us in one kernel, 81 in two).
+static int walk32_chunks(long long chains, long long chunks) {
+    if (chains == 0 || chunks < 4 || chains > 0x7fffffffLL / 2) return 0;
+    return (int)std::min(chunks, std::max(1LL, (512LL << 20) / (chains * TILE_FLOATS * 4)));
+}
+size_t bwd32_workspace_bytes(long long B, long long T, long long H) {
+    return WORK_FLAG_BYTES + (size_t)(B * H * walk32_chunks(B * H, (T + L - 1) / L)) * TILE_FLOATS * sizeof(float);
 }
 
 // dparams[i][c] = sum over batch of the per-(batch, head) partials, in a fixed order.
@@ -883,17 +1223,34 @@ bool encode_bthn_map(CUtensorMap* m, void* base, long long B, long long T, long 
 }
 
 template <int PREC, bool LN> static int launch_bwd_t(const BwdParams& p, cudaStream_t stream) {
-    using Smem = BwdSmem<PREC, LN>;
-    auto kern = p.T % L ? wkv7_bwd_kernel<PREC, LN, true> : wkv7_bwd_kernel<PREC, LN, false>;
-    const int smem = (int)sizeof(Smem);
+    constexpr bool WALK = PREC == 3 && !LN;
+    const long long chains = p.B * p.H, chunks = (p.T + L - 1) / L;
+    const int walked = WALK && p.flags && p.ds0 ? walk32_chunks(chains, chunks) : 0;
+    auto kern = p.T % L ? wkv7_bwd_kernel<PREC, LN, true, false> : wkv7_bwd_kernel<PREC, LN, false, false>;
+    if (walked) kern = p.T % L ? wkv7_bwd_kernel<PREC, LN, true, WALK> : wkv7_bwd_kernel<PREC, LN, false, WALK>;
+    const int smem = (int)(walked ? sizeof(BwdSmem<PREC, LN, WALK>) : sizeof(BwdSmem<PREC, LN, false>));
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return kLaunchFailed;
     CkptMaps cmaps;
     memset(&cmaps, 0, sizeof(cmaps));
-    const long long records = p.B * p.H * ((p.T + L - 1) / L);
+    const long long records = chains * chunks;
     if (!(encode_ckpt_state_map(&cmaps.ck, p.ckpt, records) && encode_ckpt_mats_map(&cmaps.ckm, p.ckpt, records)))
         return kLaunchFailed;
-    kern<<<(unsigned)(p.B * p.H), THREADS, smem, stream>>>(p, cmaps);
+    if (walked) {
+        auto walk = p.T % L ? wkv7_bwd_walk32_kernel<true> : wkv7_bwd_walk32_kernel<false>;
+        const int slots = 2 * sm_count();
+        if (cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Walk32Smem)) != cudaSuccess) return kLaunchFailed;
+        float* tiles = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.flags) + WORK_FLAG_BYTES);
+        for (long long it0 = 0; it0 < chunks; it0 += walked) {
+            const int n = (int)std::min<long long>(walked, chunks - it0), total = (int)chains * n, per = (total + slots - 1) / slots;
+            walk<<<(unsigned)chains, WALK_THREADS, sizeof(Walk32Smem), stream>>>(p, tiles, (int)it0, n);
+            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+            kern<<<(unsigned)((total + per - 1) / per), THREADS, smem, stream>>>(p, Walked{tiles, (int)it0, n, per, total}, cmaps);
+            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+        }
+        return kOk;
+    }
+    kern<<<(unsigned)chains, THREADS, smem, stream>>>(p, Walked{}, cmaps);
     if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
     return LN ? launch_reduce_dparams(p, stream) : kOk;
 }

@@ -81,7 +81,7 @@ template <int PREC> struct Op {  // one scalar operand
     uint32_t h, l;
     __device__ __forceinline__ void set(float x) {
         h = tf32_rna(x);
-        if (PREC == 3) l = tf32_rna(x - __uint_as_float(h));
+        if (PREC == 3) l = __float_as_uint(x - __uint_as_float(h)) + 0x1000u;  // rounded by the product, which does not look at the 13 bits below
         else l = 0;
     }
     // x was stored through pre<PREC>() or is exactly representable in TF32 (a bf16 value)
@@ -198,7 +198,7 @@ template <int PREC> __device__ __forceinline__ float rcp_p(float x) { return PRE
 // P~ = 2^64 exp(c) for a running log-decay c <= 0 (clamped at MIN_CUM_LOG_DECAY).  fp32 class: exact power-of-two scaling
 // of expf(c) wherever that has not underflowed.
 template <int PREC> __device__ __forceinline__ float decay_up(float c) {
-    if (PREC == 3) return c >= -80.f ? expf(c) * STATE_UNSCALE : expf(fmaxf(c, MIN_CUM_LOG_DECAY) + ANCHOR_LN);
+    if (PREC == 3) return expf(c >= -80.f ? c : fmaxf(c, MIN_CUM_LOG_DECAY) + ANCHOR_LN) * (c >= -80.f ? STATE_UNSCALE : 1.f);
     return exp_mufu(c + ANCHOR_LN);  // exp_mufu clamps its argument at -80
 }
 
@@ -238,7 +238,7 @@ __device__ __forceinline__ void store8(float* p, const float (&f)[8], bool flip 
 // 16-channel group).  The running log-decay along the 16 time rows is a 4-step warp-shuffle scan,
 // eight independent channels per thread keep the pipes busy, and all shared-memory traffic is 16
 // bytes wide.  Writes wq = q*P_t, wa = a*P_{t-1}, kwi = k/P_t, bwi = b/P_t (row stride OPS), the
-// chunk decay fw = P_L, and optionally the running log-decay and the per-step log-decay.
+// chunk decay fw = P_L, and optionally the running log-decay (fp32 class: P~_t itself) and the per-step log-decay.
 // tq/tw/tk/ta/tb: staging tiles with row stride `rowb` bytes.
 // live: number of time steps of this chunk that exist (16 except in the last chunk of a sequence whose length
 // is not a multiple of 16); rows beyond it carry zero inputs and a per-step log-decay of zero, so that the state
@@ -268,10 +268,10 @@ __device__ __forceinline__ void decay_scan(const unsigned char* tq, const unsign
             if (row >= d) cum[i] += up;
         }
     // P_t from one exp (argument clamped so that P_t and 1/P_t stay finite), 1/P_t from a reciprocal.
-    float o[4][8];
+    float o[4][8], pt[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const float incl = decay_up<PREC>(cum[i]);   // P~_t
+        const float incl = pt[i] = decay_up<PREC>(cum[i]);   // P~_t
         const float inv = rcp_p<PREC>(incl);
         // P_{t-1} = exp(cum_t - lw_t) (row 0: exp(0) = 1): one more exponential on the idle special-function unit is
         // cheaper here than fetching the row above with a shuffle
@@ -288,7 +288,7 @@ __device__ __forceinline__ void decay_scan(const unsigned char* tq, const unsign
     store8(wa + at, o[1], flip);
     store8(kwi + at, o[2], flip);
     store8(bwi + at, o[3], flip);
-    if (cum_out) store8(cum_out + at, cum, flip);
+    if (cum_out) store8(cum_out + at, PREC == 3 ? pt : cum, flip);
     if (lw_out) store8(lw_out + at, lw, flip);
 }
 

@@ -69,6 +69,7 @@ bool encode_ckpt_state_map(CUtensorMap* m, const float* ckpt, long long records)
 bool encode_ckpt_mats_map(CUtensorMap* m, const float* ckpt, long long records);
 int launch_bwd_bf16(const BwdParams& p, bool ln, cudaStream_t stream);
 size_t bwd_workspace_bytes(long long B, long long T, long long H, bool ln);  // what launch_bwd wants at p.flags for bf16 tensors
+size_t bwd32_workspace_bytes(long long B, long long T, long long H);         // and for fp32 ones, attn
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
 // tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
