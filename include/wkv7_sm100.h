@@ -273,6 +273,10 @@ int wkv7_proj_gemm(const void* A, const void* W, void* C, int64_t M, int64_t N, 
 #define WKV7_PROJ_MAX 4
 int wkv7_proj_gemm_group(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N,
                          const int64_t* tanh_from, const int64_t* tanh_to, int64_t M, int64_t K, void* stream);
+/* Up to WKV7_PROJ_LD_MAX of them, each with a K of its own, the rows of A lda >= K elements apart (a multiple of 8: columns of a wider tensor). */
+#define WKV7_PROJ_LD_MAX 6
+int wkv7_proj_gemm_group_ld(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* K,
+                            const int64_t* lda, const int64_t* tanh_from, const int64_t* tanh_to, int64_t M, void* stream);
 
 /*
  * expand_loras: second-stage LoRA expansion producing (w, k, kk, b) for the mixer.  Replaces

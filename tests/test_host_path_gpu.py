@@ -270,3 +270,39 @@ def test_proj_group(M):
     for a, b, o, t in zip(x, w, out, tanh):
         assert th.equal(proj(a, b, t), o)
     assert _lib.lib().wkv7_proj_gemm_group(5, None, None, None, None, None, None, M, K, None) != 0
+
+
+@pytest.mark.parametrize('M', [1, 130])
+def test_proj_group_of_several_widths_and_depths(M):
+    """Products of different K in one launch, rows of A that are columns of a wider tensor: one K block and several, whole and partial."""
+    import ctypes
+    from wind_rwkv.rwkv7 import _lib, proj
+    shapes, ld = [(8, 8), (264, 72), (96, 64), (128, 200), (16, 64), (40, 512)], [8, 72, 96, 208, 64, 520]
+    x = [th.randn(M, s, device='cuda').bfloat16()[:, :k] for (_, k), s in zip(shapes, ld)]
+    w = [(th.randn(n, k, device='cuda') / 8).bfloat16() for n, k in shapes]
+    out = [th.empty(M, n, device='cuda', dtype=th.bfloat16) for n, _ in shapes]
+    ptrs = lambda ts: (ctypes.c_void_p * 6)(*[t.data_ptr() for t in ts])
+    ints = lambda v: (ctypes.c_int64 * 6)(*v)
+    call = lambda count, k, lda: _lib.lib().wkv7_proj_gemm_group_ld(
+        count, ptrs(x), ptrs(w), ptrs(out), ints([n for n, _ in shapes]), ints(k), ints(lda), ints([0] * 6), ints([0] * 6), M, th.cuda.current_stream().cuda_stream)
+    ks = [k for _, k in shapes]
+    assert call(6, ks, ld) == 0
+    for a, b, o in zip(x, w, out):
+        assert th.equal(proj(a.contiguous(), b), o)
+    assert call(7, ks, ld) != 0 and call(6, ks, [k - 8 for k in ks]) != 0 and call(6, ks, [k + 4 for k in ld]) != 0
+
+
+@pytest.mark.parametrize('B,T,C', [(1, 1, 64), (1, 130, 512), (1, 515, 2048), (2, 1200, 2048)])
+def test_mixer_projections_of_few_rows(B, T, C, monkeypatch):
+    """The layer on both sides of the lines between this library's and the framework's projections, against the Python form (the ops one
+    by one): the bound of the layer's other tests."""
+    from collections import namedtuple
+    from wind_rwkv.rwkv7 import TimeMixer
+    th.manual_seed(T)
+    m = TimeMixer(namedtuple('Config', ['n_layer', 'n_head', 'n_embd'])(12, C // 64, C), 3).cuda()
+    with th.no_grad():
+        for p in m.parameters():
+            p.add_(th.randn_like(p) * 0.02)
+    x = th.randn(B, T, C, device='cuda').bfloat16()
+    with th.no_grad():
+        _close(m(x), _python_form(monkeypatch, lambda: m(x)), 1e-2)

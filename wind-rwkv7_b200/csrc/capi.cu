@@ -394,13 +394,13 @@ int wkv7_attn_ln_bwd_static(const void* r, const void* w, const void* k, const v
                       scratch, ds0, B, T, H, N, stride_b, stride_t, stride_h, io_dtype, nullptr, stream);
 }
 
-int wkv7_proj_gemm_group(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* tanh_from,
-                         const int64_t* tanh_to, int64_t M, int64_t K, void* stream) {
-    if (count < 1 || count > WKV7_PROJ_MAX || M < 0 || K <= 0) return WKV7_ERR_SHAPE;
+int wkv7_proj_gemm_group_ld(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* K,
+                            const int64_t* lda, const int64_t* tanh_from, const int64_t* tanh_to, int64_t M, void* stream) {
+    if (count < 1 || count > WKV7_PROJ_LD_MAX || M < 0) return WKV7_ERR_SHAPE;
     for (int i = 0; i < count; ++i) {
-        if (N[i] <= 0 || tanh_from[i] < 0 || tanh_to[i] < tanh_from[i] || tanh_to[i] > N[i]) return WKV7_ERR_SHAPE;
-        if (N[i] % 8 != 0 || K % 8 != 0) return WKV7_ERR_ALIGN;   // 16-byte rows for the bulk tensor loads and the stores
-        if (M > 0x7fffffffLL || N[i] > 0x7fffffffLL || K > 0x7fffffffLL || (M + 127) / 128 > 65535) return WKV7_ERR_TOO_LARGE;
+        if (K[i] <= 0 || lda[i] < K[i] || N[i] <= 0 || tanh_from[i] < 0 || tanh_to[i] < tanh_from[i] || tanh_to[i] > N[i]) return WKV7_ERR_SHAPE;
+        if (N[i] % 8 != 0 || K[i] % 8 != 0 || lda[i] % 8 != 0) return WKV7_ERR_ALIGN;   // 16-byte rows for the bulk tensor loads and the stores
+        if (M > 0x7fffffffLL || N[i] > 0x7fffffffLL || lda[i] > 0x7fffffffLL || (M + 127) / 128 > 65535) return WKV7_ERR_TOO_LARGE;
         if (M == 0) continue;
         if (!A[i] || !W[i] || !C[i]) return WKV7_ERR_NULL;
         if (!aligned16(A[i]) || !aligned16(W[i]) || !aligned16(C[i])) return WKV7_ERR_ALIGN;
@@ -408,7 +408,15 @@ int wkv7_proj_gemm_group(int count, const void* const* A, const void* const* W, 
     if (M == 0) return WKV7_OK;
     int* status = status_ptr();
     if (!status) return WKV7_ERR_LAUNCH;
-    return wkv7::launch_proj_gemm(count, A, W, C, N, tanh_from, tanh_to, M, K, status, (cudaStream_t)stream);
+    return wkv7::launch_proj_gemm(count, A, W, C, N, K, lda, tanh_from, tanh_to, M, status, (cudaStream_t)stream);
+}
+
+int wkv7_proj_gemm_group(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* tanh_from,
+                         const int64_t* tanh_to, int64_t M, int64_t K, void* stream) {
+    if (count < 1 || count > WKV7_PROJ_MAX) return WKV7_ERR_SHAPE;
+    int64_t k[WKV7_PROJ_MAX];
+    for (int i = 0; i < count; ++i) k[i] = K;
+    return wkv7_proj_gemm_group_ld(count, A, W, C, N, k, k, tanh_from, tanh_to, M, stream);
 }
 
 int wkv7_proj_gemm(const void* A, const void* W, void* C, int64_t M, int64_t N, int64_t K, int64_t tanh_from,
@@ -416,7 +424,7 @@ int wkv7_proj_gemm(const void* A, const void* W, void* C, int64_t M, int64_t N, 
     return wkv7_proj_gemm_group(1, &A, &W, &C, &N, &tanh_from, &tanh_to, M, K, stream);
 }
 
-static_assert(WKV7_PROJ_MAX == wkv7::PROJ_MAX, "mirrored constant");
+static_assert(WKV7_PROJ_LD_MAX == wkv7::PROJ_MAX && WKV7_PROJ_MAX <= wkv7::PROJ_MAX, "mirrored constants");
 
 static int ddlerp_check(int64_t B, int64_t T, int64_t C, int64_t D) {
     if (B < 0 || T < 0 || C <= 0 || D <= 0) return WKV7_ERR_SHAPE;

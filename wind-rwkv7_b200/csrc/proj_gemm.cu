@@ -55,14 +55,14 @@ __device__ __forceinline__ float tanh_approx(float x) {
     return y;
 }
 
-// Products of one M and K, one per blockIdx.z: a narrow product of few rows occupies a handful of SMs for the time that its K
+// Products of one M, one per blockIdx.z: a narrow product of few rows occupies a handful of SMs for the time that its K
 // loop takes, so those of one layer run side by side (three on 513 rows, K = 2048: 3 x 11.4 -> 12 us).
 struct Products {
-    struct alignas(64) One { CUtensorMap A, B, C; long long N; int tanh_from, tanh_to; } p[PROJ_MAX];
+    struct alignas(64) One { CUtensorMap A, B, C; long long N; int K, tanh_from, tanh_to; } p[PROJ_MAX];
 };
 
 template <int STAGES>
-__global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constant__ Products products, long long K, int* status) {
+__global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constant__ Products products, int* status) {
     const Products::One& one = products.p[blockIdx.z];
     const long long N = one.N;
     if (blockIdx.x * (long long)BN >= N) return;
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constan
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int nkb = (int)((K + BK - 1) / BK);
+    const int nkb = (one.K + BK - 1) / BK;
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&ctrl->full[s], 1); mbar_init(&ctrl->empty[s], 1); }
@@ -201,12 +201,12 @@ static EncodeTiledFn encode_fn() {
     }();
     return fn;
 }
-// [rows, K] bf16 row-major; box = 64 k x 128 rows, 128-byte swizzle; out-of-range parts of a box read as zeros
-static bool encode_kmajor(CUtensorMap* m, const void* base, long long rows, long long K, int box_rows = BM) {
+// [rows, K] bf16, rows ld apart; box = 64 k x 128 rows, 128-byte swizzle; out-of-range parts of a box read as zeros
+static bool encode_kmajor(CUtensorMap* m, const void* base, long long rows, long long K, long long ld, int box_rows = BM) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
     const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
     const cuuint32_t es[2] = {1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -215,8 +215,8 @@ static bool encode_kmajor(CUtensorMap* m, const void* base, long long rows, long
 
 }  // namespace gemm
 
-int launch_proj_gemm(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* tanh_from,
-                     const int64_t* tanh_to, long long M, long long K, int* status, cudaStream_t stream) {
+int launch_proj_gemm(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* K, const int64_t* lda,
+                     const int64_t* tanh_from, const int64_t* tanh_to, long long M, int* status, cudaStream_t stream) {
     using namespace gemm;
     Products ps;
     memset(&ps, 0, sizeof(ps));
@@ -224,8 +224,8 @@ int launch_proj_gemm(int count, const void* const* A, const void* const* W, void
     for (int i = 0; i < count; ++i) {
         Products::One& o = ps.p[i];
         // C [M, N]: the same kind of map (64 columns x 32 rows per store, one per warp and half tile)
-        if (!encode_kmajor(&o.A, A[i], M, K) || !encode_kmajor(&o.B, W[i], N[i], K) || !encode_kmajor(&o.C, C[i], M, N[i], 32)) return kLaunchFailed;
-        o.N = N[i]; o.tanh_from = (int)tanh_from[i]; o.tanh_to = (int)tanh_to[i];
+        if (!encode_kmajor(&o.A, A[i], M, K[i], lda[i]) || !encode_kmajor(&o.B, W[i], N[i], K[i], K[i]) || !encode_kmajor(&o.C, C[i], M, N[i], N[i], 32)) return kLaunchFailed;
+        o.N = N[i]; o.K = (int)K[i]; o.tanh_from = (int)tanh_from[i]; o.tanh_to = (int)tanh_to[i];
         const long long n = (N[i] + BN - 1) / BN;
         most = n > most ? n : most;
         tiles += n;
@@ -235,7 +235,7 @@ int launch_proj_gemm(int count, const void* const* A, const void* const* W, void
     auto kern = alone ? proj_gemm_kernel<MANY> : proj_gemm_kernel<FEW>;
     const int smem = (alone ? MANY : FEW) * STAGE_BYTES + (int)sizeof(Ctrl) + 1024;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
-    kern<<<grid, gemm::THREADS, smem, stream>>>(ps, K, status);
+    kern<<<grid, gemm::THREADS, smem, stream>>>(ps, status);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 

@@ -454,19 +454,30 @@ enum { WR, WK, WV, WO, GATE1, GATE2, KKK1, MK1, DECAY1, AAA1, MA1, DECAY2, MAAX,
        LNW = NBF, LNB, FAAAA, NPAR };
 constexpr int64_t MIX = 32, DEC = 64, SMALL = 16, GATE = 128, WAM = DEC + 2 * SMALL;
 
-// tanh on the first `to` columns
-struct Proj { const Tensor &x, &w; int64_t to; Tensor* out; };
+// rows of x may be columns of a wider tensor; tanh on the first `to` columns of the result
+struct Proj { Tensor x; const Tensor& w; int64_t to; Tensor* out; };
 void proj(std::initializer_list<Proj> ps) {
-    const void *a[WKV7_PROJ_MAX], *b[WKV7_PROJ_MAX];
-    void* c[WKV7_PROJ_MAX];
-    int64_t n[WKV7_PROJ_MAX], from[WKV7_PROJ_MAX] = {}, to[WKV7_PROJ_MAX];
+    constexpr int MAX = WKV7_PROJ_LD_MAX;
+    const void *a[MAX], *b[MAX];
+    void* c[MAX];
+    int64_t n[MAX], k[MAX], lda[MAX], from[MAX] = {}, to[MAX];
     int i = 0;
     for (const Proj& p : ps) {
         *p.out = at::empty({p.x.size(0), p.w.size(0)}, p.x.options());
-        a[i] = p.x.data_ptr(); b[i] = p.w.data_ptr(); c[i] = p.out->data_ptr(); n[i] = p.w.size(0); to[i++] = p.to;
+        a[i] = p.x.data_ptr(); b[i] = p.w.data_ptr(); c[i] = p.out->data_ptr(); n[i] = p.w.size(0); k[i] = p.x.size(1); lda[i] = p.x.stride(0); to[i++] = p.to;
     }
-    const Tensor& x = ps.begin()->x;
-    check(wkv7_proj_gemm_group(i, a, b, c, n, from, to, x.size(0), x.size(1), stream()), "wkv7_proj_gemm_group");
+    check(wkv7_proj_gemm_group_ld(i, a, b, c, n, k, lda, from, to, ps.begin()->x.size(0), stream()), "wkv7_proj_gemm_group_ld");
+}
+// Tiles of 128 x 128 an SM, times two, in one launch of all the mixer's first-stage products, three C x C ones among them: with few rows (M = B T)
+// at::mm, the better kernel with many, leaves half of the SMs idle, one product after the other, and its calls cost the host 10 us
+// each.  Up to four tiles an SM this library's kernel takes the first stages in one launch; up to one and a half, where the host is
+// what the layer waits for, the second stages (one launch) and the output projection, too.  Layer in us, all at::mm -> first -> all:
+//   C = 512, 256 rows (0.2 tiles an SM)  157 -> 130 -> 111      C = 768, 1280 rows (1.4)   159 -> 131 -> 119
+//   C = 2048, 515 rows (1.7)             174 -> 153 -> 155      C = 2048, 1280 rows (3.5)  201 -> 191 -> 198
+//   C = 2048, 1792 rows (4.8)            297 -> 296             C = 2048, 2400 rows (6.6)  277 -> 287
+int64_t half_tiles(int64_t M, int64_t C) {
+    const int64_t tiles = (M + 127) / 128 * (3 * ((C + 127) / 128) + 3), sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    return (2 * tiles + sms - 1) / sms;
 }
 struct Mixer {
     int64_t B, T, C;
@@ -509,12 +520,23 @@ struct Mixer {
         convert(in);
         ddlerp_forward(x, ddlerp_par(), m, y4);
         const Tensor xrg = in4(0), xwa = in4(1), xk = in4(2), xv = in4(3);
-        r = seq(at::mm(xrg, p[WR].t()));
-        proj({{xrg, p[GATE1], GATE, &g1}, {xk, kkmk_w, 0, &kkmk}, {xwa, wam_w, DEC, &wam}});
-        g = seq(at::mm(g1, p[GATE2].t()));
-        k0 = seq(at::mm(xk, p[WK].t()));
-        v = seq(at::mm(xv, p[WV].t()));
-        w2 = seq(at::mm(wam.narrow(1, 0, DEC), p[DECAY2].t()));
+        const int64_t load = half_tiles(B * T, C);
+        Tensor r2, k2, v2, g2, w22, out;
+        if (load <= 8) {
+            proj({{xrg, p[WR], 0, &r2}, {xk, p[WK], 0, &k2}, {xv, p[WV], 0, &v2}, {xrg, p[GATE1], GATE, &g1}, {xk, kkmk_w, 0, &kkmk}, {xwa, wam_w, DEC, &wam}});
+        } else {
+            r2 = at::mm(xrg, p[WR].t());
+            proj({{xrg, p[GATE1], GATE, &g1}, {xk, kkmk_w, 0, &kkmk}, {xwa, wam_w, DEC, &wam}});
+            k2 = at::mm(xk, p[WK].t());
+            v2 = at::mm(xv, p[WV].t());
+        }
+        if (load <= 3) {
+            proj({{g1, p[GATE2], 0, &g2}, {wam.narrow(1, 0, DEC), p[DECAY2], 0, &w22}});
+        } else {
+            g2 = at::mm(g1, p[GATE2].t());
+            w22 = at::mm(wam.narrow(1, 0, DEC), p[DECAY2].t());
+        }
+        r = seq(r2); k0 = seq(k2); v = seq(v2); g = seq(g2); w2 = seq(w22);
         if (!save) y4 = m = Tensor();
         const int64_t ld[4] = {2 * SMALL, WAM, WAM, 2 * SMALL};
         const variable_list o = loras_forward(loras_in(), ld, loras_par());
@@ -522,7 +544,9 @@ struct Mixer {
         if (!save) k0 = w2 = Tensor();
         const variable_list a = wkv_forward(r, w, k, v, kk, b, g, params, Tensor(), save);
         y = a[0]; sT = a[1]; ck = a[2];
-        return seq(at::mm(rows(y), p[WO].t()));
+        if (load > 3) return seq(at::mm(rows(y), p[WO].t()));
+        proj({{rows(y), p[WO], 0, &out}});
+        return seq(out);
     }
     variable_list saved() const {
         variable_list s{params, kkmk_w, wam_w, m, y4, r, g1, g, k0, kkmk, v, wam, w2, w, k, kk, b, y, sT, ck};

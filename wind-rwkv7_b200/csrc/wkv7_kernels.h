@@ -78,10 +78,10 @@ int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream);
 // bf16 forward with the sequences cut into nseg segments each (wkv7_time_split.cu)
 size_t time_split_workspace_bytes(long long B, long long H, int nseg);
 int launch_fwd_time_split(const FwdParams& p, int nseg, int groups, cudaStream_t stream);
-// for each of `count` products C[M,N] = act(A[M,K] W[N,K]^T), bf16, tanh on columns [tanh_from, tanh_to); tcgen05 + TMA (proj_gemm.cu)
-constexpr int PROJ_MAX = 4;
-int launch_proj_gemm(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* tanh_from,
-                     const int64_t* tanh_to, long long M, long long K, int* status, cudaStream_t stream);
+// for each of `count` products C[M,N] = act(A[M,K] W[N,K]^T), bf16, A's rows lda apart, tanh on columns [tanh_from, tanh_to); tcgen05 + TMA (proj_gemm.cu)
+constexpr int PROJ_MAX = 6;
+int launch_proj_gemm(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* K, const int64_t* lda,
+                     const int64_t* tanh_from, const int64_t* tanh_to, long long M, int* status, cudaStream_t stream);
 // one small CTA running the tcgen05 forward's bounded mbarrier wait on barriers nothing arrives on
 int launch_bounded_wait_selftest(long long limit_cycles, int* status, long long* cycles, cudaStream_t stream);
 

@@ -66,6 +66,7 @@ _SIGNATURES = {
     'wkv7_expand_loras_fwd_ld': (_int, [_vp] * 19 + [_i64] * 4 + [_vp]),
     'wkv7_expand_loras_bwd_ld': (_int, [_vp] * 35 + [_i64] * 4 + [_vp]),
     'wkv7_proj_gemm_group': (_int, [_int] + [_vp] * 6 + [_i64] * 2 + [_vp]),
+    'wkv7_proj_gemm_group_ld': (_int, [_int] + [_vp] * 8 + [_i64] + [_vp]),
     'wkv7_cast': (_int, [_vp] * 4 + [_int, _vp]),
     'wkv7_expand_loras_bwd_workspace_bytes': (_i64, [_i64] * 4),
     'wkv7_expand_loras_bwd': (_int, [_vp] * 33 + [_i64] * 4 + [_vp]),
