@@ -162,3 +162,22 @@ def test_time_split_maps_of_cut_chains(B, T, H):
     for a, b in zip(got, want):
         assert (a.float() - b.float()).norm() <= 4e-3 * b.float().norm()
     assert _lib.lib().wkv7_device_status() == 0
+
+
+@pytest.mark.parametrize('chains,T,s0', [(1, 1, False), (1, 16, True), (2, 17, True), (3, 48, False), (5, 100, True), (148, 65, True), (149, 500, True), (150, 33, False)])
+def test_forward_f32(chains, T, s0):
+    """fp32 forward on both sides of the line between its two kernels, against a float64 recurrence on the CPU: fewer chunks than preparation
+    groups, partial last chunks, as many chains as SMs and more.  1e-5 of the norm: fp32 sums of products that are right to 2^-22."""
+    from wind_rwkv.rwkv7 import _lib, attn, synthetic
+    d = synthetic.wkv7_inputs(1, T, chains, N, seed=T, dtype=th.float32, device='cuda', s0_std=0.1)
+    y, sT = attn(*[d[n] for n in 'rwkvab'], N, s0=d['s0'] if s0 else None, return_state=True)
+    r, w, k, v, a, b = [d[n].view(T, chains, N).double().cpu() for n in 'rwkvab']
+    S = d['s0'][0].double().cpu() if s0 else th.zeros(chains, N, N, dtype=th.float64)
+    ref = []
+    for t in range(T):
+        sa = S @ a[t].unsqueeze(-1)
+        S = S * th.exp(-th.exp(w[t])).unsqueeze(1) + sa @ b[t].unsqueeze(1) + v[t].unsqueeze(-1) @ k[t].unsqueeze(1)
+        ref.append((S @ r[t].unsqueeze(-1)).squeeze(-1))
+    for got, want in ((y.view(T, chains, N), th.stack(ref)), (sT[0], S)):
+        assert (got.double().cpu() - want).norm() <= 1e-5 * want.norm()
+    assert _lib.lib().wkv7_device_status() == 0
