@@ -868,6 +868,14 @@ __global__ void __launch_bounds__(g5::THREADS, 1) ddlerp_main_tc_kernel(const __
                 mbar_expect(&ctrl->full_x, (uint32_t)((BM + 1) * 128));
                 tma_load_3d(sb + off_x(D), &maps.x, &ctrl->full_x, cb * 64, t0 - 1, bi);
             };
+            // The unit after this one has no room in shared memory yet, but in L2: its dy and x tiles (ddlerp forward and backward, 32768 rows of
+            // 768: 329 -> 317 us).
+            auto prefetch = [&](int n) {
+                const int u = u_lo + n, cb = u / tiles, tile = u % tiles, t0 = (tile % tiles_per_seq) * BM, bi = tile / tiles_per_seq;
+#pragma unroll
+                for (int k = 0; k < 5; ++k)
+                    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(k < 4 ? &maps.dy[k] : &maps.x), "r"(cb * 64), "r"(t0), "r"(bi) : "memory");
+            };
             if (nmine > 0) { load_dpre(0); load_x(0); }
             for (int n = 0; n < nmine; ++n) {
                 const int u = u_lo + n, cb = u / tiles, tile = u % tiles, t0 = (tile % tiles_per_seq) * BM, bi = tile / tiles_per_seq;
@@ -889,6 +897,7 @@ __global__ void __launch_bounds__(g5::THREADS, 1) ddlerp_main_tc_kernel(const __
 #pragma unroll
                 for (int k = 0; k < 4; ++k) tma_load_3d(sb + off_dy(D) + k * TILE, &maps.dy[k], &ctrl->full, cb * 64, t0, bi);
                 if (n + 1 < nmine) {
+                    prefetch(n + 1);
                     if (!mbar_wait_bounded<true>(&ctrl->acc1, n & 1, &ctrl->abort, status)) break;      // products 1 of this unit have read the dpre tile
                     load_dpre(n + 1);
                     if (!mbar_wait_bounded<true>(&ctrl->dz_ready, n & 1, &ctrl->abort, status)) break;  // every epilogue warp is past the x tile
