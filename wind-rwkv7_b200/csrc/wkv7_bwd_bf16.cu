@@ -117,6 +117,50 @@ __device__ __forceinline__ FragB<1> as_b(const FragA<1>& f, int nt) {
     return b;
 }
 
+// The scan: a thread has two adjacent time steps x 4 adjacent key channels, so that the running sum takes three shuffle rounds of 4
+// channels instead of four of 8 (a shuffle is a pass through the data pipe).  Slot 0 is the earlier or the later one (`late`) of the two,
+// such that the raw loads (half-warps: every residue of the row mod 8 once, two channel quads) and the operand stores (quarter-warps: rows 0,
+// 2, 4, 6 or 1, 3, 5, 7 of the pitch-72 tiles x two quads) are free of bank conflicts.
+// (One step x 8 channels: 782 us at B64 T1024 H12, 117 with its walk at B3 T1003 H16; this: 776 and 115.)
+struct ScanLane {
+    int row0, quad;  // slot 1: row0 ^ 1; quad: of the head's 16
+    bool late;
+    __device__ __forceinline__ ScanLane(int w, int lane)
+        : row0(2 * ((lane & 3) + ((lane >> 1) & 4)) + ((lane >> 3) & 1)), quad(4 * w + ((lane >> 2) & 1) + ((lane >> 3) & 2)), late((lane >> 3) & 1) {}
+    __device__ __forceinline__ int raw(int e) const { const int row = row0 ^ e; return row * ROWB + (((quad >> 1) ^ (row & 7)) << 4) + (quad & 1) * 8; }
+    __device__ __forceinline__ int dst(int e) const { const int row = row0 ^ e; return row * OPS + xcol<1>(row, 4 * quad); }
+    // w -> running log2 decay through and before the slots' steps; steps from `live` on do not exist
+    __device__ __forceinline__ void decay(F2 (&cum)[2][2], F2 (&before)[2][2], int live, int lane) const {
+        constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // log2 of the per-step decay
+        F2 x[2][2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const F2 l = mul2(cum[e][i], f2(LOG2E, LOG2E)), d = mul2(f2(ex2_approx(l.x), ex2_approx(l.y)), f2(-LOG2E, -LOG2E));
+                x[e][i] = (row0 ^ e) < live ? f2(fmaxf(d.x, FLOOR), fmaxf(d.y, FLOOR)) : f2(0.f, 0.f);
+            }
+        const float f0 = late ? 0.f : -1.f, f1 = late ? -1.f : 0.f;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            F2 sum = add2(x[0][i], x[1][i]);
+#pragma unroll
+            for (int d = 1; d < 4; d <<= 1) {
+                const F2 up = f2(__shfl_up_sync(0xffffffffu, sum.x, d, 4), __shfl_up_sync(0xffffffffu, sum.y, d, 4));
+                if ((lane & 3) >= d) sum = add2(sum, up);
+            }
+            const int src = (lane & 0x14) | 3;
+            const F2 low = f2(__shfl_sync(0xffffffffu, sum.x, src), __shfl_sync(0xffffffffu, sum.y, src));
+            if (late) sum = add2(sum, low);
+            cum[0][i] = fma2(x[1][i], f2(f0, f0), sum);  // less the later step's, in the earlier one
+            cum[1][i] = fma2(x[0][i], f2(f1, f1), sum);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) before[e][i] = fma2(x[e][i], f2(-1.f, -1.f), cum[e][i]);
+        }
+    }
+};
+__device__ __forceinline__ float4 pre4(const F2 (&v)[2]) { return make_float4(pre<1>(v[0].x), pre<1>(v[0].y), pre<1>(v[1].x), pre<1>(v[1].y)); }
+
 // PAR: the state gradients at the chunks' ends are given (wkv7_bwd_walk_kernel), so that chunks are worked in any order and none is
 // carried here; the tiles of steps it0 .. it0 + ws.per_chain - 1 of each chain are in `tiles`.
 struct Tiles { const float* base; int it0; };
@@ -304,71 +348,49 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
         // ---------------- scan: one thread = one time step x 8 adjacent key channels, as in the tcgen05 forward ----------------
         mbar_wait_bounded<false>(&sm.raw_full, n & 1, &sm.abort, p.status);
         {
-            const int row = lane & 15, j0 = 16 * warp + 8 * (lane >> 4), at = row * ROWB + (((j0 >> 3) ^ (row & 7)) << 4);
-            F2 q[4], cum[4], k[4], a[4], b[4];
-            load8f2(sm.raw[1] + at, cum);
-            load8f2(sm.raw[0] + at, q);
-            load8f2(sm.raw[2] + at, k);
-            load8f2(sm.raw[3] + at, a);
-            load8f2(sm.raw[4] + at, b);
-            if (LN) {  // bonus dot sum_j r_j k_j bonus_j of this time step: this warp's 16 channels
-                F2 acc = f2(0.f, 0.f);
-                const float4* bon = reinterpret_cast<const float4*>(p.params + (2 * p.H + d.hi) * N + j0);
+            const ScanLane sl(warp, lane);
+            F2 q[2][2], cum[2][2], before[2][2], k[2][2], a[2][2], b[2][2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int at = sl.raw(e);
+                load4f2(sm.raw[1] + at, cum[e]);
+                load4f2(sm.raw[0] + at, q[e]);
+                load4f2(sm.raw[2] + at, k[e]);
+                load4f2(sm.raw[3] + at, a[e]);
+                load4f2(sm.raw[4] + at, b[e]);
+            }
+            if (LN) {  // bonus dot sum_j r_j k_j bonus_j of these time steps: this warp's 16 channels
+                const float4 bo = __ldg(reinterpret_cast<const float4*>(p.params + (2 * p.H + d.hi) * N + 4 * sl.quad));
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const F2 acc = fma2(mul2(q[e][1], k[e][1]), f2(bo.z, bo.w), mul2(mul2(q[e][0], k[e][0]), f2(bo.x, bo.y)));
+                    float dot = acc.x + acc.y;
+                    dot += __shfl_xor_sync(0xffffffffu, dot, 4);
+                    dot += __shfl_xor_sync(0xffffffffu, dot, 16);
+                    if (!(lane & 0x14)) sm.bdot[warp][sl.row0 ^ e] = dot;
+                }
+            }
+            sl.decay(cum, before, TAIL ? (int)min((long long)L, p.T - (long long)d.c * L) : L, lane);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                F2 wq[2], wa[2], kw[2], bw[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    const float4 bo = __ldg(bon + i);
-                    acc = fma2(mul2(q[2 * i], k[2 * i]), f2(bo.x, bo.y), acc);
-                    acc = fma2(mul2(q[2 * i + 1], k[2 * i + 1]), f2(bo.z, bo.w), acc);
+                    const F2 ca = add2(cum[e][i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = add2(before[e][i], f2(ANCHOR_LOG2, ANCHOR_LOG2));
+                    const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
+                    const F2 incl = f2(ex2_approx(cx), ex2_approx(cy)), inv = f2(ex2_approx(-cx), ex2_approx(-cy));
+                    const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
+                    wq[i] = mul2(q[e][i], incl); wa[i] = mul2(a[e][i], non); kw[i] = mul2(k[e][i], inv); bw[i] = mul2(b[e][i], inv);
+                    // P_L (where it underflows, so does dS P_L)
+                    if (e == 0 && (lane & 11) == 11) *reinterpret_cast<float2*>(sm.fw + 4 * sl.quad + 2 * i) = make_float2(incl.x * STATE_SCALE, incl.y * STATE_SCALE);
                 }
-                float dot = acc.x + acc.y;
-                dot += __shfl_xor_sync(0xffffffffu, dot, 16);
-                if (lane < 16) sm.bdot[warp][lane] = dot;
+                const int dst = sl.dst(e);
+                *reinterpret_cast<float4*>(sm.wq + dst) = pre4(wq);
+                *reinterpret_cast<float4*>(sm.wa + dst) = pre4(wa);
+                *reinterpret_cast<float4*>(sm.kwi + dst) = pre4(kw);
+                *reinterpret_cast<float4*>(sm.bwi + dst) = pre4(bw);
+                *reinterpret_cast<float4*>(sm.cum + dst) = make_float4(cum[e][0].x, cum[e][0].y, cum[e][1].x, cum[e][1].y);
             }
-            constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // log2 of the per-step decay
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                cum[i] = mul2(cum[i], f2(LOG2E, LOG2E));
-                cum[i] = mul2(f2(ex2_approx(cum[i].x), ex2_approx(cum[i].y)), f2(-LOG2E, -LOG2E));
-                cum[i] = f2(fmaxf(cum[i].x, FLOOR), fmaxf(cum[i].y, FLOOR));
-            }
-            if (TAIL && (long long)d.c * L + row >= p.T) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) cum[i] = f2(0.f, 0.f);
-            }
-            F2 step[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) step[i] = cum[i];
-#pragma unroll
-            for (int s = 1; s < 16; s <<= 1)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const F2 up = f2(__shfl_up_sync(0xffffffffu, cum[i].x, s, 16), __shfl_up_sync(0xffffffffu, cum[i].y, s, 16));
-                    if (row >= s) cum[i] = add2(cum[i], up);
-                }
-            float oq[8], oa[8], ok[8], ob[8], oc[8];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const F2 ca = add2(cum[i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = fma2(step[i], f2(-1.f, -1.f), ca);
-                const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
-                const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
-                const F2 inv = f2(ex2_approx(-cx), ex2_approx(-cy));
-                const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
-                const F2 wq = mul2(q[i], incl), wa = mul2(a[i], non), kw = mul2(k[i], inv), bw = mul2(b[i], inv);
-                oq[2 * i] = pre<1>(wq.x); oq[2 * i + 1] = pre<1>(wq.y);
-                oa[2 * i] = pre<1>(wa.x); oa[2 * i + 1] = pre<1>(wa.y);
-                ok[2 * i] = pre<1>(kw.x); ok[2 * i + 1] = pre<1>(kw.y);
-                ob[2 * i] = pre<1>(bw.x); ob[2 * i + 1] = pre<1>(bw.y);
-                oc[2 * i] = cum[i].x; oc[2 * i + 1] = cum[i].y;
-                // P_L (where it underflows, so does dS P_L)
-                if (row == 15) *reinterpret_cast<float2*>(sm.fw + j0 + 2 * i) = make_float2(incl.x * STATE_SCALE, incl.y * STATE_SCALE);
-            }
-            const int dst = row * OPS + xcol<1>(row, j0);
-            const bool flip = (row >> 2) & 1;
-            store8(sm.wq + dst, oq, flip);
-            store8(sm.wa + dst, oa, flip);
-            store8(sm.kwi + dst, ok, flip);
-            store8(sm.bwi + dst, ob, flip);
-            store8(sm.cum + dst, oc, flip);
         }
         __syncthreads();  // (A)
         if (!PAR && (d.flags & FIRST)) {
@@ -863,63 +885,35 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
     }
     if (warp >= WARPS) {
         // ---- preparation: this warp's 16 key columns of every PREP-th chunk
-        const int row = lane & 15, j0 = 16 * w + 8 * (lane >> 4), at = row * ROWB + (((j0 >> 3) ^ (row & 7)) << 4);
-        const int dst = row * OPS + xcol<1>(row, j0);
-        const bool flip = (row >> 2) & 1;
+        const ScanLane sl(w, lane);
         for (int n = warp / WARPS - 1; n < count; n += PREP) {
             const int s = n % SLOTS;
             WalkSlot& t = sm.slot[s];
             mbar_wait_bounded<true>(&sm.raw_full[s], (n / SLOTS) & 1, &sm.abort, p.status);
-            F2 cum[4], x[4], step[4];
-            load8f2(t.raw[1] + at, cum);
-            constexpr float LOG2E = 1.4426950408889634f, FLOOR = MIN_STEP_LOG_DECAY * LOG2E;  // the scan of wkv7_bwd_bf16_kernel
+            F2 cum[2][2], before[2][2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                cum[i] = mul2(cum[i], f2(LOG2E, LOG2E));
-                cum[i] = mul2(f2(ex2_approx(cum[i].x), ex2_approx(cum[i].y)), f2(-LOG2E, -LOG2E));
-                cum[i] = f2(fmaxf(cum[i].x, FLOOR), fmaxf(cum[i].y, FLOOR));
-            }
-            if (TAIL && (long long)(c0 - n) * L + row >= p.T) {
+            for (int e = 0; e < 2; ++e) load4f2(t.raw[1] + sl.raw(e), cum[e]);
+            sl.decay(cum, before, TAIL ? (int)min((long long)L, p.T - (long long)(c0 - n) * L) : L, lane);  // as wkv7_bwd_bf16_kernel does
 #pragma unroll
-                for (int i = 0; i < 4; ++i) cum[i] = f2(0.f, 0.f);
-            }
+            for (int e = 0; e < 2; ++e) {
+                const int at = sl.raw(e), dst = sl.dst(e);
+                F2 q[2], a[2], b[2], wq[2], wa[2], bw[2];
+                load4f2(t.raw[0] + at, q);
+                load4f2(t.raw[2] + at, a);
+                load4f2(t.raw[3] + at, b);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) step[i] = cum[i];
-#pragma unroll
-            for (int d = 1; d < 16; d <<= 1)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const F2 up = f2(__shfl_up_sync(0xffffffffu, cum[i].x, d, 16), __shfl_up_sync(0xffffffffu, cum[i].y, d, 16));
-                    if (row >= d) cum[i] = add2(cum[i], up);
+                for (int i = 0; i < 2; ++i) {
+                    const F2 ca = add2(cum[e][i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = add2(before[e][i], f2(ANCHOR_LOG2, ANCHOR_LOG2));
+                    const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
+                    const F2 incl = f2(ex2_approx(cx), ex2_approx(cy)), inv = f2(ex2_approx(-cx), ex2_approx(-cy));
+                    const F2 non = f2(ex2_approx(fmaxf(cp.x, -115.f)), ex2_approx(fmaxf(cp.y, -115.f)));
+                    wq[i] = mul2(q[i], incl); wa[i] = mul2(a[i], non); bw[i] = mul2(b[i], inv);
+                    if (e == 0 && (lane & 11) == 11) *reinterpret_cast<float2*>(t.fw + 4 * sl.quad + 2 * i) = make_float2(incl.x * STATE_SCALE, incl.y * STATE_SCALE);
                 }
-            float o[8], inv[8], non[8];
-            load8f2(t.raw[0] + at, x);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const F2 ca = add2(cum[i], f2(ANCHOR_LOG2, ANCHOR_LOG2)), cp = fma2(step[i], f2(-1.f, -1.f), ca);
-                const float cx = fmaxf(ca.x, -115.f), cy = fmaxf(ca.y, -115.f);
-                const F2 incl = f2(ex2_approx(cx), ex2_approx(cy));
-                inv[2 * i] = ex2_approx(-cx); inv[2 * i + 1] = ex2_approx(-cy);
-                non[2 * i] = ex2_approx(fmaxf(cp.x, -115.f)); non[2 * i + 1] = ex2_approx(fmaxf(cp.y, -115.f));
-                const F2 wq = mul2(x[i], incl);
-                o[2 * i] = pre<1>(wq.x); o[2 * i + 1] = pre<1>(wq.y);
-                if (row == 15) *reinterpret_cast<float2*>(t.fw + j0 + 2 * i) = make_float2(incl.x * STATE_SCALE, incl.y * STATE_SCALE);
+                *reinterpret_cast<float4*>(t.wq + dst) = pre4(wq);
+                *reinterpret_cast<float4*>(t.wa + dst) = pre4(wa);
+                *reinterpret_cast<float4*>(t.bwi + dst) = pre4(bw);
             }
-            store8(t.wq + dst, o, flip);
-            load8f2(t.raw[2] + at, x);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const F2 v = mul2(x[i], f2(non[2 * i], non[2 * i + 1]));
-                o[2 * i] = pre<1>(v.x); o[2 * i + 1] = pre<1>(v.y);
-            }
-            store8(t.wa + dst, o, flip);
-            load8f2(t.raw[3] + at, x);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const F2 v = mul2(x[i], f2(inv[2 * i], inv[2 * i + 1]));
-                o[2 * i] = pre<1>(v.x); o[2 * i + 1] = pre<1>(v.y);
-            }
-            store8(t.bwi + dst, o, flip);
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.ready[s]);
         }
