@@ -80,3 +80,21 @@ def test_zero_state_and_empty_sequence():
     e = [x[:, :0] for x in ins]
     y, s = attn_step(*e, N, d['s0'])
     assert y.shape == (1, 0, N) and th.equal(s, d['s0'])
+
+
+@pytest.mark.parametrize('extra,T,dtype', [(0, 1, th.bfloat16), (1, 1, th.bfloat16), (1, 3, th.float32), (700, 2, th.bfloat16), (1500, 1, th.float32)])
+@pytest.mark.parametrize('form', ['s0', 'inplace', 'zeros'])
+def test_many_chains(extra, T, dtype, form):
+    """More chains than twice the resident CTAs (4 an SM): CTAs that walk several, from two to four each, against the same chains in calls
+    that stay below, bit for bit."""
+    from wind_rwkv.rwkv7 import _lib, attn_step, synthetic
+    H = 7
+    B = (8 * th.cuda.get_device_properties(0).multi_processor_count + extra + H - 1) // H
+    d = synthetic.wkv7_inputs(B, T, H, 64, seed=T + extra, dtype=dtype, device='cuda', s0_std=0.5)
+    ins = [d[n] for n in 'rwkvab']
+    s0 = None if form == 'zeros' else d['s0']
+    want = [attn_step(*[x[i:i + 40] for x in ins], 64, None if s0 is None else s0[i:i + 40]) for i in range(0, B, 40)]
+    s = s0.clone() if form == 'inplace' else s0
+    y, sT = attn_step(*ins, 64, s, inplace=form == 'inplace')
+    assert th.equal(y, th.cat([a for a, _ in want])) and th.equal(sT, th.cat([b for _, b in want]))
+    assert _lib.device_status() == 0

@@ -283,6 +283,7 @@ int wkv7_step(const void* r, const void* w, const void* k, const void* v, const 
     p.r = r; p.w = w; p.k = k; p.v = v; p.a = a; p.b = b; p.s0 = s0; p.y = y; p.sT = sT;
     p.B = B; p.T = T; p.H = H;
     p.st = wkv7::Strides{stride_b, stride_t, stride_h};
+    p.status = status_ptr();
     return wkv7::launch_step(p, io_dtype == WKV7_BF16 ? 0 : 1, (cudaStream_t)stream);
 }
 

@@ -50,6 +50,7 @@ struct StepParams {
     float* sT;                          // [B,H,N,N] or null
     long long B, T, H;
     Strides st;
+    int* status;                        // device status word
 };
 
 // Work split for `chains` chains of `per_chain` chunks with `per_sm` resident CTAs per SM.  Chains are cut only when there are

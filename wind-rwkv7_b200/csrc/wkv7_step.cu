@@ -14,10 +14,36 @@
 // S r) are 16 FMAs per thread and two shuffles.  The step's vectors are loaded, converted and (the decays) exponentiated once per
 // CTA, not by each of the 64 rows (8192 exponentials per chain).
 // What is left is the state traffic: 2 * 16 KB per chain and call, all loads of it in flight before the first barrier, six CTAs an
-// SM (40 registers; at 76 registers and three CTAs 54 us): 6400 chains 54 -> 44.6 us; the same kernel without the arithmetic 36 us.
+// SM (40 registers; at 76 registers and three CTAs 1.2 times as long).  Many chains: wkv7_step_ring_kernel below.
 #include "wkv7_kernels.h"
 
 namespace wkv7 {
+
+// One step: thread (i, q)'s 16 elements of state row i, the step's vectors u.  Returns y_i (in all of the row's threads).
+__device__ __forceinline__ float step_row(float (&S)[16], const float (*u)[N], int i, int q) {
+    float sa = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 a = *reinterpret_cast<const float4*>(&u[1][16 * j + 4 * q]);
+        sa = fmaf(S[4 * j], a.x, sa); sa = fmaf(S[4 * j + 1], a.y, sa);
+        sa = fmaf(S[4 * j + 2], a.z, sa); sa = fmaf(S[4 * j + 3], a.w, sa);
+    }
+    sa += __shfl_xor_sync(0xffffffffu, sa, 1);
+    sa += __shfl_xor_sync(0xffffffffu, sa, 2);
+    const float v = u[5][i];
+    float y = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float4 d = *reinterpret_cast<const float4*>(&u[0][16 * j + 4 * q]), b = *reinterpret_cast<const float4*>(&u[2][16 * j + 4 * q]);
+        const float4 k = *reinterpret_cast<const float4*>(&u[3][16 * j + 4 * q]), r = *reinterpret_cast<const float4*>(&u[4][16 * j + 4 * q]);
+        S[4 * j] = fmaf(S[4 * j], d.x, fmaf(sa, b.x, v * k.x)); y = fmaf(S[4 * j], r.x, y);
+        S[4 * j + 1] = fmaf(S[4 * j + 1], d.y, fmaf(sa, b.y, v * k.y)); y = fmaf(S[4 * j + 1], r.y, y);
+        S[4 * j + 2] = fmaf(S[4 * j + 2], d.z, fmaf(sa, b.z, v * k.z)); y = fmaf(S[4 * j + 2], r.z, y);
+        S[4 * j + 3] = fmaf(S[4 * j + 3], d.w, fmaf(sa, b.w, v * k.w)); y = fmaf(S[4 * j + 3], r.w, y);
+    }
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    return y + __shfl_xor_sync(0xffffffffu, y, 2);
+}
 
 template <typename IoT>
 __global__ void __launch_bounds__(256, 6) wkv7_step_kernel(StepParams p) {
@@ -50,28 +76,7 @@ __global__ void __launch_bounds__(256, 6) wkv7_step_kernel(StepParams p) {
             x0 = src0[(t + 1) * p.st.t];
             if (part < 2) x1 = src1[(t + 1) * p.st.t];
         }
-        float sa = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 a = *reinterpret_cast<const float4*>(&u[1][16 * j + 4 * q]);
-            sa = fmaf(S[4 * j], a.x, sa); sa = fmaf(S[4 * j + 1], a.y, sa);
-            sa = fmaf(S[4 * j + 2], a.z, sa); sa = fmaf(S[4 * j + 3], a.w, sa);
-        }
-        sa += __shfl_xor_sync(0xffffffffu, sa, 1);
-        sa += __shfl_xor_sync(0xffffffffu, sa, 2);
-        const float v = u[5][i];
-        float y = 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 d = *reinterpret_cast<const float4*>(&u[0][16 * j + 4 * q]), b = *reinterpret_cast<const float4*>(&u[2][16 * j + 4 * q]);
-            const float4 k = *reinterpret_cast<const float4*>(&u[3][16 * j + 4 * q]), r = *reinterpret_cast<const float4*>(&u[4][16 * j + 4 * q]);
-            S[4 * j] = fmaf(S[4 * j], d.x, fmaf(sa, b.x, v * k.x)); y = fmaf(S[4 * j], r.x, y);
-            S[4 * j + 1] = fmaf(S[4 * j + 1], d.y, fmaf(sa, b.y, v * k.y)); y = fmaf(S[4 * j + 1], r.y, y);
-            S[4 * j + 2] = fmaf(S[4 * j + 2], d.z, fmaf(sa, b.z, v * k.z)); y = fmaf(S[4 * j + 2], r.z, y);
-            S[4 * j + 3] = fmaf(S[4 * j + 3], d.w, fmaf(sa, b.w, v * k.w)); y = fmaf(S[4 * j + 3], r.w, y);
-        }
-        y += __shfl_xor_sync(0xffffffffu, y, 1);
-        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        const float y = step_row(S, u, i, q);
         if (q == 0) ((IoT*)p.y)[base - (tid & 63) + t * p.st.t + i] = from_f32<IoT>(y);
     }
     if (p.sT) {
@@ -81,10 +86,92 @@ __global__ void __launch_bounds__(256, 6) wkv7_step_kernel(StepParams p) {
     }
 }
 
-int launch_step(const StepParams& p, int io_dtype, cudaStream_t stream) {
-    if (io_dtype == 0) wkv7_step_kernel<__nv_bfloat16><<<(unsigned)(p.B * p.H), 256, 0, stream>>>(p);
-    else wkv7_step_kernel<float><<<(unsigned)(p.B * p.H), 256, 0, stream>>>(p);
+// More chains than resident CTAs: each CTA walks several, and the next one's state comes by a bulk copy while this one is worked and stored
+// (a CTA per chain leaves the memory idle between its last store and its successor's first load).  Four CTAs an SM (five or six spill: 39 us): 6400
+// chains 44.0 -> 38.5 us, 10240 65.6 -> 57.8, 3200 25.1 -> 21.0, 1280 11.4 -> 10.8, 768 9.5 -> 9.9, hence the line at two chains a CTA.
+constexpr int RING_PER_SM = 4;
+template <typename IoT>
+__global__ void __launch_bounds__(256, RING_PER_SM) wkv7_step_ring_kernel(StepParams p, int chains) {
+    __shared__ __align__(128) float st[N * N];
+    __shared__ __align__(16) float vec[2][6][N];
+    __shared__ uint64_t full;
+    __shared__ volatile int abort, zero;
+    const int tid = threadIdx.x, i = tid >> 2, q = tid & 3, part = tid >> 6, H = (int)p.H;
+    const IoT* const in0 = (const IoT*)(part == 0 ? p.w : part == 1 ? p.a : part == 2 ? p.b : p.k) + (tid & 63);
+    const IoT* const in1 = (const IoT*)(part == 0 ? p.r : p.v) + (tid & 63);
+    auto offset = [&](int bh) { const int b = (int)((unsigned)bh / (unsigned)H); return b * p.st.b + (bh - b * H) * p.st.h; };
+    auto load = [&](int bh) {  // one thread
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full)), "n"(N * N * 4) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(smem_u32(st)), "l"(p.s0 + (long long)bh * N * N), "n"(N * N * 4), "r"(smem_u32(&full)) : "memory");
+    };
+    int bh = blockIdx.x, loads = 0;
+    if (tid == 0) {
+        mbar_init(&full, 1);
+        abort = zero = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (p.s0) { load(bh); ++loads; }
+    }
+    long long base = offset(bh);
+    IoT x0 = in0[base], x1 = x0;
+    if (part < 2) x1 = in1[base];
+    __syncthreads();
+    unsigned step = 0;
+    for (int n = 0; bh < chains; ++n) {
+        const int next = bh + (int)gridDim.x;
+        const long long next_base = next < chains ? offset(next) : 0;
+        float S[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) S[j] = 0.f;
+        if (p.s0) {
+            mbar_wait_bounded<false>(&full, n & 1, &abort, p.status);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float4 s = *reinterpret_cast<const float4*>(st + i * N + 16 * j + 4 * q);
+                S[4 * j] = s.x; S[4 * j + 1] = s.y; S[4 * j + 2] = s.z; S[4 * j + 3] = s.w;
+            }
+        }
+        IoT* const y = (IoT*)p.y + base + i;
+        for (long long t = 0; t < p.T; ++t, ++step) {
+            float (*u)[N] = vec[step & 1];
+            const float f0 = to_f32<IoT>(x0);
+            u[part][tid & 63] = part == 0 ? expf(-expf(f0)) : f0;
+            if (part < 2) u[4 + part][tid & 63] = to_f32<IoT>(x1);
+            __syncthreads();
+            if (t == 0 && tid == 0 && p.s0 && next < chains && !abort) {  // everyone has read the state
+                fence_async_smem();
+                load(next);
+                ++loads;
+            }
+            const bool same = t + 1 < p.T;
+            if (same || next < chains) {
+                const long long at = same ? base + (t + 1) * p.st.t : next_base;
+                x0 = in0[at];
+                if (part < 2) x1 = in1[at];
+            }
+            const float yt = step_row(S, u, i, q);
+            if (q == 0) y[t * p.st.t] = from_f32<IoT>(yt);
+        }
+        if (p.sT) {
+            float* out = p.sT + (long long)bh * N * N + i * N + 4 * q;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float4*>(out + 16 * j) = make_float4(S[4 * j], S[4 * j + 1], S[4 * j + 2], S[4 * j + 3]);
+        }
+        bh = next;
+        base = next_base;
+    }
+    if (tid == 0) mbar_landed(&full, loads, &zero, p.status);  // shared memory must outlive the loads, also where a wait has given up
+}
+
+template <typename IoT> static int launch_step_t(const StepParams& p, cudaStream_t stream) {
+    const long long chains = p.B * p.H, resident = (long long)RING_PER_SM * sm_count();
+    if (chains > 2 * resident && chains <= 0x3fffffff && p.status) wkv7_step_ring_kernel<IoT><<<(unsigned)resident, 256, 0, stream>>>(p, (int)chains);
+    else wkv7_step_kernel<IoT><<<(unsigned)chains, 256, 0, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+}
+int launch_step(const StepParams& p, int io_dtype, cudaStream_t stream) {
+    return io_dtype == 0 ? launch_step_t<__nv_bfloat16>(p, stream) : launch_step_t<float>(p, stream);
 }
 
 }  // namespace wkv7
