@@ -31,10 +31,11 @@ __device__ __forceinline__ F2 bf2(const void* p) {  // two bf16 values
     const float2 v = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(p));
     return f2(v.x, v.y);
 }
-__device__ __forceinline__ Gates lora_gates(F2 xa, F2 xm, F2 xk, F2 v) {
+// SIG = false: xa is a already.
+template <bool SIG = true> __device__ __forceinline__ Gates lora_gates(F2 xa, F2 xm, F2 xk, F2 v) {
     constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
     Gates o;
-    o.a = sigmoid2(xa);
+    o.a = SIG ? sigmoid2(xa) : xa;
     o.ma = sigmoid2(xm);
     o.mk = sigmoid2(xk);
     const F2 n = mul2(v, f2(-LOG2E, -LOG2E));
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel
             }
             // ---- pass A: z, a; row sums for the norm and its gradient -----------------------------------
             float z[4][4], dzo[4][4];
+            F2 av[4][2];  // (kept for pass B: formed again, product and sigmoid, 292 us where this is 285, forward and backward of 32768 rows of 768)
             F2 ss2[2] = {}, dn2[2] = {};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -329,6 +331,7 @@ __global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel
                     const int tr = lr + g + 8 * hrow, tc = 32 * half + 8 * j + 2 * t4;
                     const F2 zz = add2(f2(z[j][2 * hrow], z[j][2 * hrow + 1]), bf2(&sm.gr[1][tr][tc]));
                     const F2 a = sigmoid2(f2(fa[2 * hrow], fa[2 * hrow + 1]));
+                    av[j][hrow] = a;
                     const F2 dz = fma2(neg2(bf2(&sm.gr[4][tr][tc])), a, bf2(&sm.gr[5][tr][tc]));  // gradient of kk
                     ss2[hrow] = fma2(zz, zz, ss2[hrow]);
                     dn2[hrow] = fma2(dz, zz, dn2[hrow]);
@@ -360,14 +363,12 @@ __global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int c = h * HC + 32 * half + 8 * j + 2 * t4;
-                const F2 wb = bf2((const bf16*)p.w_bias + c), ab = bf2((const bf16*)p.bias[0] + c), mb = bf2((const bf16*)p.bias[1] + c), kb = bf2((const bf16*)p.bias[2] + c);
-                float fa[4] = {ab.x, ab.y, ab.x, ab.y}, fm[4] = {mb.x, mb.y, mb.x, mb.y}, fk[4] = {kb.x, kb.y, kb.x, kb.y};
+                const F2 wb = bf2((const bf16*)p.w_bias + c), mb = bf2((const bf16*)p.bias[1] + c), kb = bf2((const bf16*)p.bias[2] + c);
+                float fm[4] = {mb.x, mb.y, mb.x, mb.y}, fk[4] = {kb.x, kb.y, kb.x, kb.y};
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
-                    uint32_t ba[2], bm[2], bk[2];
-                    ldW2<D>(ba, bm, sm.W, 1, 8 * j + 32 * half, 16 * ks, lane);
-                    ldW1<D>(bk, sm.W, 3, 8 * j + 32 * half, 16 * ks, lane);
-                    mma_bf16(fa, aa[ks], ba);
+                    uint32_t bm[2], bk[2];
+                    ldW2<D>(bm, bk, sm.W, 2, 8 * j + 32 * half, 16 * ks, lane);
                     mma_bf16(fm, am[ks], bm);
                     mma_bf16(fk, ak[ks], bk);
                 }
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel
                 for (int hrow = 0; hrow < 2; ++hrow) {
                     const int tr = lr + g + 8 * hrow, tc = 32 * half + 8 * j + 2 * t4;
                     const F2 ki = bf2(&sm.gr[1][tr][tc]), v = add2(wb, bf2(&sm.gr[0][tr][tc]));
-                    const Gates gt = lora_gates(f2(fa[2 * hrow], fa[2 * hrow + 1]), f2(fm[2 * hrow], fm[2 * hrow + 1]), f2(fk[2 * hrow], fk[2 * hrow + 1]), v);
+                    const Gates gt = lora_gates<false>(av[j][hrow], f2(fm[2 * hrow], fm[2 * hrow + 1]), f2(fk[2 * hrow], fk[2 * hrow + 1]), v);
                     const F2 kmix = fma2(neg2(gt.ma), gt.a, add2(gt.ma, gt.a));
                     const F2 zz = f2(z[j][2 * hrow], z[j][2 * hrow + 1]), in = f2(inorm[hrow], inorm[hrow]);
                     const F2 dkE = mul2(bf2(&sm.gr[3][tr][tc]), gt.E), dkin = mul2(dkE, ki);
