@@ -36,10 +36,10 @@ BWD_BYTES_PER_TOKEN_HEAD = 13 * N * 2   # r,w,k,v,a,b,dy in + six gradients out,
 # Fallback copy of the pool's measured STREAM-style bandwidth, used when MEASURED_PEAKS.json is absent.
 FALLBACK_HBM_GBS = 6650.0
 # dram__bytes_read.sum + dram__bytes_write.sum of one backward launch at this workload, from an ncu capture of
-# `python bench.py --no-e2e --no-cpu-baseline --no-secondary --steps 1 --warmup 1 --batch 25`: 668.6 MB read + 219.5 MB written by
+# `python bench.py --no-e2e --no-cpu-baseline --no-secondary --steps 1 --warmup 1 --batch 25`: 668.5 MB read + 217.9 MB written by
 # wkv7_bwd_bf16_kernel at B = 25 (the smallest batch that fills the machine), scaled by 64 / 25: traffic is proportional to the number
 # of chains, and the B = 64 workload is too large to capture.
-BWD_DRAM_TRAFFIC_BYTES = 2_273_530_000
+BWD_DRAM_TRAFFIC_BYTES = 2_269_390_000
 
 
 def hbm_peak():
