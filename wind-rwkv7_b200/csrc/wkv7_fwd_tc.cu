@@ -144,6 +144,12 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {  // has the phase completed? (waits for the hardware's time limit)
+    uint32_t ok;
+    asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok;
+}
 // Abort path, by the thread of each warp that issues: waits, bounded and regardless of the CTA's abort flag, for the products and the
 // load that this warp may have in flight, so that neither tensor memory nor shared memory is released under them.
 __device__ __forceinline__ void abort_drain(Ctrl* ctrl, int warp, uint64_t* load, int* status) {
@@ -153,14 +159,10 @@ __device__ __forceinline__ void abort_drain(Ctrl* ctrl, int warp, uint64_t* load
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
     tc_commit(&ctrl->drain[warp]);
-    mbar_wait_bounded<true>(&ctrl->drain[warp], 0, never_set, status);
+    const uint32_t since = clock();  // the kernel's own limit: products may stand behind a warp that still waits for a hand-off
+    while (!mbar_test(&ctrl->drain[warp], 0) && !*never_set)
+        if ((uint32_t)clock() - since > (uint32_t)WAIT_LIMIT) give_up(never_set, status);
     if (load) mbar_landed_uncounted(load, never_set, status);
-}
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {  // has the phase completed? (whole warp)
-    uint32_t ok;
-    asm volatile("{\n.reg .pred P;\nmbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
-                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return __all_sync(0xffffffffu, ok);
 }
 // named barrier of one preparation group (the id in a register: a switch over immediate ids costs instruction-cache space)
 __device__ __forceinline__ void group_bar(int grp) { asm volatile("bar.sync %0, 128;" ::"r"(grp + 1) : "memory"); }
