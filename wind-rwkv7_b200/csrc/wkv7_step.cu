@@ -165,7 +165,9 @@ __global__ void __launch_bounds__(256, RING_PER_SM) wkv7_step_ring_kernel(StepPa
 }
 
 template <typename IoT> static int launch_step_t(const StepParams& p, cudaStream_t stream) {
-    const long long chains = p.B * p.H, resident = (long long)RING_PER_SM * sm_count();
+    const long long chains = p.B * p.H;
+    // (the smallest calls, whose time is the host's, do not ask for the number of SMs)
+    const long long resident = chains > 512 ? (long long)RING_PER_SM * sm_count() : chains;
     if (chains > 2 * resident && chains <= 0x3fffffff && p.status) wkv7_step_ring_kernel<IoT><<<(unsigned)resident, 256, 0, stream>>>(p, (int)chains);
     else wkv7_step_kernel<IoT><<<(unsigned)chains, 256, 0, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
