@@ -92,7 +92,7 @@ constexpr int C_XY = 320;    // + 32 * group: X (16) | Y (16) of the group's chu
 constexpr int C_V = 448;     // + 16 * group: V^T [value][time] of the group's chunk
 
 // Any wait of this kernel may stand still while one of its groups waits for the state of a cut chain: the chain warp (full), the
-// score and inverse warps (score, fold, mats, fread), and the other groups (done).
+// score, inverse and fold warps (score, mats, inv), and the other groups (done).
 constexpr long long WAIT_LIMIT = ACROSS_HANDOFF_LIMIT;
 
 // The decay of the state, S' = S diag(P_L), is a product of TF32 operands: the tensor core reads S cut off after 10 mantissa bits, and
