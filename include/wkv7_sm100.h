@@ -138,8 +138,9 @@ int wkv7_fwd_time_split(const void* r, const void* w, const void* k, const void*
                         const float* s0, void* y, float* sT, int64_t B, int64_t T, int64_t H, int64_t N, int64_t nseg,
                         int64_t stride_t, void* workspace, void* stream);
 /* The backward's scratch is wkv7_bwd_ws_bytes() bytes, asked for with the call's device current (it depends on the number of SMs).
- * The backward keeps a cut chain's state gradient in ds0, which must be given for a cut.  Where there are few chains (bf16), and for
- * WKV7_F32 with any number of them, the scratch also passes each chunk's state gradient from the CTA that walks the chain to the CTAs that do the rest of the chunk's work. */
+ * The backward keeps a cut chain's state gradient in ds0, which must be given for a cut.  Where there are few chains (bf16: up to the
+ * number of SMs, WKV7_F32: up to 2647), the scratch, then up to 512 MB, also passes each chunk's state gradient from the CTA that walks the chain
+ * to the CTAs that do the rest of the chunk's work.  With workspace null the call is wkv7_bwd, which needs none. */
 int64_t wkv7_bwd_ws_bytes(int64_t B, int64_t T, int64_t H, int64_t N, int io_dtype);
 int wkv7_bwd_ws(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                 const void* dy, const float* ckpt, const float* dsT, const float* sT,

@@ -107,3 +107,17 @@ def test_layouts_that_share_memory_are_told_apart():
                                ((3, 4, 2, 8), (16, 48, 8, 1), True), ((1, 4, 2, 8), (0, 16, 8, 1), True), ((3, 1, 2, 8), (16, 1, 8, 1), True),
                                ((3, 4, 2, 8), (128, 32, 8, 1), True), ((3, 4, 2, 8), (64, 16, 4, 1), False)]:
         assert _apart(t.as_strided(size, stride)) is want, (size, stride)
+
+
+def test_backward_scratch_is_bounded(lib):
+    """Tiles of the walked state gradients take 512 MB at most, whatever the number of chains and chunks, and a chain's tile of 18 KB a
+    chunk comes in passes of 11 chunks or whole sequences."""
+    flags, tile = lib.wkv7_workspace_bytes(), 64 * 72 * 4
+    for chains in [1, 12, 149, 2000, 2647, 2648, 4096, 14563, 14564, 29127, 29128, 100000, 1 << 20]:
+        for chunks in [1, 3, 4, 5, 10, 11, 12, 25, 300]:
+            for B, H in ((chains, 1), (1, chains)):
+                n = lib.wkv7_bwd_ws_bytes(B, 16 * chunks, H, 64, 1) - flags
+                assert 0 <= n <= 512 << 20 and n % (chains * tile) == 0, (chains, chunks)
+                per_pass = n // (chains * tile)
+                assert per_pass == 0 or min(chunks, 11) <= per_pass <= chunks, (chains, chunks)
+                assert per_pass or chunks < 4 or chains > 2647, (chains, chunks)

@@ -81,9 +81,14 @@ def test_backward(extra, T, dsT, ln):
 
 @pytest.mark.parametrize('chains,T,dsT', [(1, 48, True), (1, 49, False), (1, 64, True), (5, 100, True), (149, 49, True), (300, 65, False), (12, 38900, True)])
 def test_backward_f32_walked(chains, T, dsT):
-    """fp32 tensors: the state gradient walked by a kernel of its own (from four chunks on, any number of chains, in several passes where the
-    tiles would take more than 512 MB), then all chunks in parallel, against the one-kernel form of the entry point without scratch.
+    """fp32 tensors: the state gradient walked by a kernel of its own (from four chunks on, in several passes where the tiles would take more
+    than 512 MB), then all chunks in parallel, against the one-kernel form of the entry point without scratch.
     The same products to 2^-22 each, summed in another order: 1e-5 of the norm."""
+    assert backward_f32_both_ways(chains, T, dsT) == (T > 48)
+
+
+def backward_f32_both_ways(chains, T, dsT):
+    """Compares the two; whether the scratch had room for tiles."""
     from wind_rwkv.rwkv7 import _lib, synthetic
     from wind_rwkv.rwkv7.rwkv7_attn import fw_attn
     L = _lib.lib()
@@ -92,7 +97,6 @@ def test_backward_f32_walked(chains, T, dsT):
     _, sT, ck = fw_attn(*[d[n].view(B, T, H, N) for n in 'wrkvab'], d['s0'])
     gs = th.randn(B, H, N, N, device='cuda') if dsT else None
     ws = th.full((L.wkv7_bwd_ws_bytes(B, T, H, N, 1),), 255, dtype=th.uint8, device='cuda')
-    assert (ws.numel() > L.wkv7_workspace_bytes()) == (T > 48)
 
     def call(walk):
         outs = [th.full_like(d['r'], float('nan')) for _ in range(6)] + [th.full((B, H, N, N), float('nan'), device='cuda')]
@@ -105,6 +109,14 @@ def test_backward_f32_walked(chains, T, dsT):
     for a, b in zip(call(False), call(True)):
         assert bool(th.isfinite(a).all()) and (a - b).norm() <= 1e-5 * a.norm()
     assert L.wkv7_device_status() == 0
+    return ws.numel() > L.wkv7_workspace_bytes()
+
+
+@pytest.mark.parametrize('chains,T', [(2647, 11 * 16), (2647, 12 * 16 + 5), (2648, 12 * 16)])
+def test_backward_f32_walked_many_chains(chains, T):
+    """As above where the tiles' 512 MB hold 11 chunks of every chain: one pass, two (11 chunks and 2), and one chain more, which is not
+    walked and then has no scratch but the flags."""
+    assert backward_f32_both_ways(chains, T, True) == (chains == 2647)
 
 
 @pytest.mark.parametrize('form', ['c++', 'python'])

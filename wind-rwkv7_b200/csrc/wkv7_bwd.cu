@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(THREADS, PAR ? 2 : 1) wkv7_bwd_kernel(BwdParam
 // `tiles`, from where the chunk kernel (PAR) takes all chunks over all SMs.  With a chunk's whole work on the chain it took 20 000 cycles,
 // most of them for fetching its 90 KB of code.
 // Bound by the chain of dependent products, 3300 cycles a chunk (two preparation groups: 3700).  Backward in us, one kernel -> walk and
-// chunks: 96 chains of 32 chunks 336 -> 212, 8 of 256 2573 -> 534, 320 of 52 1461 -> 992, 2048 of 8 1095 -> 929.
+// chunks: 96 chains of 32 chunks 288 -> 203, 96 of 256 2251 -> 1469, 296 of 32 574 -> 513, 1024 of 32 1969 -> 1784, 2048 of 16 1867 -> 1818.
 constexpr int WALK_SLOTS = 4, WALK_PREP = 3, WALK_THREADS = THREADS * (1 + WALK_PREP);
 struct Walk32Slot {
     alignas(16) unsigned char dy[TILEB];
@@ -1149,10 +1149,14 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk32_kernel(BwdPar
 }
 
 // How many chunks of each chain are walked at a time: tiles of at most 512 MB, longer sequences take several passes, the walk going on
-// from ds0.  0: not at all: with three chunks the second launch costs what it saves (144 chains: 78 us in one kernel, 81 in two).
+// from ds0.  0: not at all.  With three chunks the second launch costs what it saves (144 chains: 78 us in one kernel, 81 in two).  Each pass
+// starts two kernels and loads and stores the whole dS, and of many chains only a few chunks fit: one kernel / walk in us, chunks a pass in
+// brackets: 2048 chains of 64 7376 / 7118 (14), 2640 of 32 4682 / 4656 (11), 2912 of 32 5176 / 5196 (10), 4096 of 64 14346 / 14626 (7), 8192
+// of 8 3654 / 3986 (3), 32000 of 8 14122 / 18143 (1).  Hence the line at 11, 2647 chains: beyond it whole sequences in one pass would gain 2 % at most.
 static int walk32_chunks(long long chains, long long chunks) {
-    if (chains == 0 || chunks < 4 || chains > 0x7fffffffLL / 2) return 0;
-    return (int)std::min(chunks, std::max(1LL, (512LL << 20) / (chains * TILE_FLOATS * 4)));
+    constexpr long long BYTES = 512LL << 20, PASS = 11;
+    if (chains == 0 || chunks < 4 || chains > BYTES / (PASS * TILE_FLOATS * 4)) return 0;
+    return (int)std::min(chunks, BYTES / (chains * TILE_FLOATS * 4));
 }
 size_t bwd32_workspace_bytes(long long B, long long T, long long H) {
     return WORK_FLAG_BYTES + (size_t)(B * H * walk32_chunks(B * H, (T + L - 1) / L)) * TILE_FLOATS * sizeof(float);
