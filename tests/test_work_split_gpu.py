@@ -144,6 +144,48 @@ def test_backward_scratch_of_few_chains(form, monkeypatch):
         del grads
 
 
+@pytest.mark.parametrize('form', ['c++', 'python'])
+@pytest.mark.parametrize('dtype', [th.bfloat16, th.float32])
+def test_backward_without_room_for_the_scratch(dtype, form, monkeypatch):
+    """Where the tiles of the walked state gradients cannot be allocated, but the gradients can, the backward takes its one-kernel form:
+    bf16 bit for bit the same, fp32 as in test_backward_f32_walked."""
+    from wind_rwkv.rwkv7 import _lib, attn, synthetic
+    if form == 'python':
+        _lib.ext()
+        monkeypatch.setattr(_lib, '_ext', type('Nothing', (), {'__getattr__': lambda self, name: lambda *a: None})())
+    B, T, H = 1, 16384, 12
+    tiles = _lib.lib().wkv7_bwd_ws_bytes(B, T, H, N, _lib.io_dtype(th.empty(0, dtype=dtype)))
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=1, dtype=dtype, device='cuda')
+    ins = [d[n].requires_grad_() for n in 'rwkvab']
+    y = attn(*ins, N)
+
+    def limit(reserved):
+        th.cuda.set_per_process_memory_fraction(min(1.0, reserved / th.cuda.get_device_properties(0).total_memory))
+
+    try:
+        th.cuda.synchronize()
+        th.cuda.empty_cache()
+        limit(th.cuda.memory_reserved())
+        holes = []  # what other tests' remains leave free of the memory that the process keeps
+        with pytest.raises(th.OutOfMemoryError):
+            while True:
+                holes.append(th.empty(tiles, dtype=th.uint8, device='cuda'))
+        limit(float('inf'))
+        want = th.autograd.grad(y, ins, d['dy'], retain_graph=True)
+        held = th.cuda.memory_reserved()  # with all that one backward allocates, the tiles last
+        want = [x.cpu() for x in want]
+        th.cuda.empty_cache()
+        asked = th.cuda.memory_stats()['num_ooms']
+        limit(held - tiles // 2)
+        got = [x.cpu() for x in th.autograd.grad(y, ins, d['dy'])]
+    finally:
+        limit(float('inf'))
+    assert th.cuda.memory_stats()['num_ooms'] == asked + 1
+    for a, b in zip(got, want):
+        assert th.equal(a, b) if dtype == th.bfloat16 else (a - b).norm() <= 1e-5 * b.norm()
+    assert _lib.lib().wkv7_device_status() == 0
+
+
 @pytest.mark.parametrize('B,T,H,nseg', [(1, 34, 2, 2), (1, 3, 1, 3), (2, 99, 2, 3), (1, 256, 5, 16), (3, 1024, 7, 8)])
 @pytest.mark.parametrize('s0', [False, True])
 def test_time_split(B, T, H, nseg, s0):

@@ -39,6 +39,16 @@ Tensor scratch(const Tensor& like) {
     static const int64_t bytes = (int64_t)wkv7_workspace_bytes();
     return at::empty({bytes}, like.options().dtype(at::kByte));
 }
+// Scratch of a backward call; undefined where the tiles of a walked state gradient, up to 512 MB, cannot be had: the kernels then take the form
+// that needs none.
+Tensor bwd_scratch(int64_t bytes, const Tensor& like) {
+    try {
+        return at::empty({bytes}, like.options().dtype(at::kByte));
+    } catch (const c10::OutOfMemoryError&) {
+        if (bytes <= (int64_t)wkv7_workspace_bytes()) throw;
+        return Tensor();
+    }
+}
 bool grad_wanted(std::initializer_list<const Tensor*> ts) {
     if (!at::GradMode::is_enabled()) return false;
     for (const Tensor* t : ts)
@@ -152,18 +162,19 @@ variable_list wkv_backward(Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Ten
     }
     if (dsT.defined()) dsT = dsT.to(at::kFloat).contiguous();
     Tensor dr = like_rows(w), dw = like_rows(w), dk = like_rows(w), dv = like_rows(w), da = like_rows(w), db = like_rows(w), ds0 = states(w, q);
-    Tensor ws = at::empty({(g.defined() ? wkv7_attn_ln_bwd_ws_bytes : wkv7_bwd_ws_bytes)(q.B, q.T, q.H, N, q.io)}, w.options().dtype(at::kByte));
+    const Tensor ws = bwd_scratch((g.defined() ? wkv7_attn_ln_bwd_ws_bytes : wkv7_bwd_ws_bytes)(q.B, q.T, q.H, N, q.io), w);
+    void* const wsp = ws.defined() ? ws.data_ptr() : nullptr;
     const float* sTp = dsT.defined() ? f32(sT) : nullptr;
     if (!g.defined()) {
         check(wkv7_bwd_ws(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), dy.data_ptr(), f32(ck), f32(dsT), sTp,
                           dr.data_ptr(), dw.data_ptr(), dk.data_ptr(), dv.data_ptr(), da.data_ptr(), db.data_ptr(), f32(ds0), q.B, q.T, q.H, N, q.sb, q.st, N,
-                          q.io, ws.data_ptr(), stream()), "wkv7_bwd_ws");
+                          q.io, wsp, stream()), "wkv7_bwd_ws");
         return {dr, dw, dk, dv, da, db, ds0};
     }
     Tensor dg = like_rows(w), dp = at::empty({3, q.H * N}, ds0.options()), part = at::empty({q.B, 3, q.H * N}, ds0.options());
     check(wkv7_attn_ln_bwd_ws(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(), g.data_ptr(), f32(params), dy.data_ptr(),
                               f32(ck), f32(dsT), sTp, dr.data_ptr(), dw.data_ptr(), dk.data_ptr(), dv.data_ptr(), da.data_ptr(), db.data_ptr(), dg.data_ptr(),
-                              f32(dp), f32(part), f32(ds0), LN_EPS, q.B, q.T, q.H, N, q.sb, q.st, N, q.io, ws.data_ptr(), stream()), "wkv7_attn_ln_bwd_ws");
+                              f32(dp), f32(part), f32(ds0), LN_EPS, q.B, q.T, q.H, N, q.sb, q.st, N, q.io, wsp, stream()), "wkv7_attn_ln_bwd_ws");
     return {dr, dw, dk, dv, da, db, ds0, dg, dp};
 }
 

@@ -149,9 +149,15 @@ _SCRATCH_BYTES = None
 
 def bwd_scratch(w, ln=False):
     """Device scratch of one backward *_ws call (ln: of attn_ln) for [B,T,H,N] tensors like w, whose device must be current: the
-    size depends on its number of SMs."""
-    size = lib().wkv7_attn_ln_bwd_ws_bytes if ln else lib().wkv7_bwd_ws_bytes
-    return th.empty(size(*w.shape, io_dtype(w)), dtype=th.uint8, device=w.device)
+    size depends on its number of SMs.  None where the tiles of a walked state gradient, up to 512 MB, cannot be had: the kernels then
+    take the form that needs none."""
+    size = (lib().wkv7_attn_ln_bwd_ws_bytes if ln else lib().wkv7_bwd_ws_bytes)(*w.shape, io_dtype(w))
+    try:
+        return th.empty(size, dtype=th.uint8, device=w.device)
+    except th.OutOfMemoryError:
+        if size <= lib().wkv7_workspace_bytes():
+            raise
+        return None
 
 
 def scratch(device):

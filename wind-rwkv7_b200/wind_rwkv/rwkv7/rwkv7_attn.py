@@ -64,7 +64,7 @@ def bw_attn(w, q, k, v, a, b, s, dy, dsT, sT):
         rc = _lib.lib().wkv7_bwd_ws(q.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(), b.data_ptr(),
                                     dy.data_ptr(), s.data_ptr(), _lib.ptr(dsT), _lib.ptr(sT if dsT is not None else None),
                                     dq.data_ptr(), dw.data_ptr(), dk.data_ptr(), dv.data_ptr(), da.data_ptr(), db.data_ptr(),
-                                    ds0.data_ptr(), B, T, H, C, sb, st, sh, _lib.io_dtype(w), ws.data_ptr(), _lib.stream_of(w))
+                                    ds0.data_ptr(), B, T, H, C, sb, st, sh, _lib.io_dtype(w), _lib.ptr(ws), _lib.stream_of(w))
     _lib.check(rc, 'wkv7_bwd_ws')
     return dw, dq, dk, dv, da, db, ds0
 
