@@ -98,3 +98,22 @@ def test_many_chains(extra, T, dtype, form):
     y, sT = attn_step(*ins, 64, s, inplace=form == 'inplace')
     assert th.equal(y, th.cat([a for a, _ in want])) and th.equal(sT, th.cat([b for _, b in want]))
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize('T', [8, 9])
+@pytest.mark.parametrize('dtype', [th.bfloat16, th.float32])
+def test_many_chains_of_several_steps(T, dtype):
+    """On both sides of the line at eight steps a call: as single steps of the same chains, bit for bit (bf16 and fp32 y come from the same
+    fp32 state)."""
+    from wind_rwkv.rwkv7 import _lib, attn_step, synthetic
+    H = 7
+    B = (8 * th.cuda.get_device_properties(0).multi_processor_count) // H + 1
+    d = synthetic.wkv7_inputs(B, T, H, 64, seed=T, dtype=dtype, device='cuda', s0_std=0.5)
+    ins = [d[n] for n in 'rwkvab']
+    y, sT = attn_step(*ins, 64, d['s0'])
+    s, ys = d['s0'], []
+    for t in range(T):
+        yt, s = attn_step(*[x[:, t:t + 1] for x in ins], 64, s)
+        ys.append(yt)
+    assert th.equal(y, th.cat(ys, 1)) and th.equal(sT, s)
+    assert _lib.device_status() == 0

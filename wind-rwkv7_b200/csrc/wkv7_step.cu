@@ -14,7 +14,7 @@
 // S r) are 16 FMAs per thread and two shuffles.  The step's vectors are loaded, converted and (the decays) exponentiated once per
 // CTA, not by each of the 64 rows (8192 exponentials per chain).
 // What is left is the state traffic: 2 * 16 KB per chain and call, all loads of it in flight before the first barrier, six CTAs an
-// SM (40 registers; at 76 registers and three CTAs 1.2 times as long).  Many chains: wkv7_step_ring_kernel below.
+// SM (40 registers; at 76 registers and three CTAs 1.2 times as long).  Many chains, up to eight steps: wkv7_step_ring_kernel below.
 #include "wkv7_kernels.h"
 
 namespace wkv7 {
@@ -89,7 +89,11 @@ __global__ void __launch_bounds__(256, 6) wkv7_step_kernel(StepParams p) {
 // More chains than resident CTAs: each CTA walks several, and the next one's state comes by a bulk copy while this one is worked and stored
 // (a CTA per chain leaves the memory idle between its last store and its successor's first load).  Four CTAs an SM (five or six spill: 39 us): 6400
 // chains 44.0 -> 38.5 us, 10240 65.6 -> 57.8, 3200 25.1 -> 21.0, 1280 11.4 -> 10.8, 768 9.5 -> 9.9, hence the line at two chains a CTA.
-constexpr int RING_PER_SM = 4;
+// More steps a call: what counts is more and more the steps' latency, which six CTAs an SM hide better than four, and how full the last round of
+// CTAs is.  A CTA per chain / here, us, at T = 4: 1280 chains 25.8 / 22.7, 1600 28.9 / 28.7, 3200 51.2 / 47.3, 6400 92.8 / 90.2; T = 8: 1280
+// 41.1 / 37.0, 1600 45.3 / 47.3, 2688 73.9 / 69.9, 6400 161.2 / 162.1; T = 12: 1280 56.1 / 51.4, 1600 61.6 / 67.6, 3200 118.9 / 120.4, 6400
+// 230.8 / 233.9; T = 16: 10240 473 / 479; hence the line at eight steps.
+constexpr int RING_PER_SM = 4, RING_STEPS = 8;
 template <typename IoT>
 __global__ void __launch_bounds__(256, RING_PER_SM) wkv7_step_ring_kernel(StepParams p, int chains) {
     __shared__ __align__(128) float st[N * N];
@@ -168,7 +172,7 @@ template <typename IoT> static int launch_step_t(const StepParams& p, cudaStream
     const long long chains = p.B * p.H;
     // (the smallest calls, whose time is the host's, do not ask for the number of SMs)
     const long long resident = chains > 512 ? (long long)RING_PER_SM * sm_count() : chains;
-    if (chains > 2 * resident && chains <= 0x3fffffff && p.status) wkv7_step_ring_kernel<IoT><<<(unsigned)resident, 256, 0, stream>>>(p, (int)chains);
+    if (chains > 2 * resident && chains <= 0x3fffffff && p.T <= RING_STEPS && p.status) wkv7_step_ring_kernel<IoT><<<(unsigned)resident, 256, 0, stream>>>(p, (int)chains);
     else wkv7_step_kernel<IoT><<<(unsigned)chains, 256, 0, stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
