@@ -270,7 +270,8 @@ int wkv7_ddlerp_bwd_tc(const void* x, const void* alpha, const void* L, const vo
  */
 int wkv7_proj_gemm(const void* A, const void* W, void* C, int64_t M, int64_t N, int64_t K,
                    int64_t tanh_from, int64_t tanh_to, void* stream);
-/* Up to WKV7_PROJ_MAX such products of one M and K in one launch (the arrays are host memory). */
+/* Up to WKV7_PROJ_MAX such products of one M and K in one launch (the arrays are host memory): the form below for callers whose products share
+ * one K and whose A are contiguous; the library itself calls the one below. */
 #define WKV7_PROJ_MAX 4
 int wkv7_proj_gemm_group(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N,
                          const int64_t* tanh_from, const int64_t* tanh_to, int64_t M, int64_t K, void* stream);

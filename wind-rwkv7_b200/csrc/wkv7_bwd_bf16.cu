@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
     bool taken_up = false;  // the segment continues another CTA's
     for (int n = 0; n < work.n; ++n) {
         const Desc d = sm.desc[n & 3];
-        // ---------------- scan: one thread = one time step x 8 adjacent key channels, as in the tcgen05 forward ----------------
+        // ---------------- scan: one thread = two adjacent time steps x 4 adjacent key channels (ScanLane) ----------------
         mbar_wait_bounded<false>(&sm.raw_full, n & 1, &sm.abort, p.status);
         {
             const ScanLane sl(warp, lane);

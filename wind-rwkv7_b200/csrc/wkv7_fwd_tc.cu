@@ -16,9 +16,10 @@
 // tensor pipe.
 // What bounds it: three things at once, none of which is saturated alone.  The chain's two round trips (1000 cycles a chunk in the
 // running kernel, 560 alone: 210 for a product, its commit and the wait, 5 to 38 for each further product); the latency from a chunk's
-// operand tiles to its completion, some 5500 cycles, over the four chunks in flight (shared memory has no room for a fifth);
-// and the shared-memory data pipe, some 1200 wavefronts a chunk, that both stand in.  About 1450 cycles a chunk without checkpoints
-// (B8 T65536 H40), 1800 with (B64 T1024 H12: 338 us, 5.0 TB/s of HBM traffic).  Before the V parts went ahead of the chain and off shared
+// operand tiles to its completion, some 5500 cycles, over the four chunks in flight (a fifth group would leave 72 registers a thread, where
+// preparation takes 96, and all 512 columns of tensor memory are in use); and the shared-memory data pipe, some 1000 wavefronts of
+// loads and stores a chunk and 360 of operand reads, that both stand in.  About 1450 cycles a chunk without checkpoints
+// (B8 T65536 H40), 1800 with (B64 T1024 H12: 338 us, 4.7 TB/s of HBM traffic).  Before the V parts went ahead of the chain and off shared
 // memory, and the scores, the inverse and the fold each had warps of their own: 1550 and 1860.
 //
 // Warp roles (128 (G+2) threads).  Warps 0..4G-1 are G preparation groups of four warps, each working on its own chunk (c, c+G, ...).
@@ -669,10 +670,10 @@ __global__ void __launch_bounds__(128 * (G + 2), 1) wkv7_fwd_tc_kernel(FwdParams
                 const int t = (lane & 7) + 8 * (lane >> 4), unit = 2 * wg + ((lane >> 3) & 1);  // row address of block lane / 8
                 asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};"
                              ::"r"(smem_u32(gs + G_Y + t * 128 + ((unit ^ (t & 7)) << 4))), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
-                        } else {
+            } else {
                 // attn_ln epilogue (reference: wind_rwkv/rwkv7/attn_ln.cu:176-205): GroupNorm over the head's 64
                 // value channels of each time step, + bonus dot * v, * gate.  Y^T goes to shared memory as
-                // fp32 [time][value] (in the dead kwf / bwf tiles); then one thread = one time step x 8 value channels, the mapping of the scan.
+                // fp32 [time][value] (in the dead kwf / bwf tiles); then one thread = one time step x 8 value channels.
                 float* ysf = reinterpret_cast<float*>(gs + G_KWF);
                 float* part = reinterpret_cast<float*>(gs + G_KWF + LN_PART);
                 {
