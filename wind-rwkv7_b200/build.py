@@ -27,21 +27,21 @@ def _deps():
 
 
 def _check_tc_launch_registers(log):
-    """The 4-group tcgen05 forward redistributes registers between its warp groups with setmaxnreg, whose
+    """The tcgen05 forward redistributes registers between its warp groups with setmaxnreg, whose
     blocking form waits without a bound for registers that must come out of the CTA's launch allocation.
     The kernel's arithmetic assumes that allocation is 80 registers per thread; stop the build if ptxas
-    chose anything else for those instantiations."""
+    chose anything else for any instantiation."""
     lines = log.splitlines()
     seen = 0
     for i, ln in enumerate(lines):
-        if 'Compiling entry function' in ln and 'wkv7_fwd_tc_kernelILi4E' in ln:
+        if 'Compiling entry function' in ln and 'wkv7_fwd_tc_kernelILi' in ln:
             used = next((l for l in lines[i + 1:i + 6] if 'Used' in l and 'registers' in l), '')
             seen += 1
             if 'Used 80 registers' not in used:
-                raise RuntimeError('wkv7_fwd_tc_kernel<4,*> must be launched with 80 registers per thread '
+                raise RuntimeError('wkv7_fwd_tc_kernel must be launched with 80 registers per thread '
                                    f'(setmaxnreg arithmetic); ptxas reports: {used.strip()!r}')
-    if seen < 8:
-        raise RuntimeError('ptxas log holds fewer wkv7_fwd_tc_kernel<4,*> entries than are built: cannot check their register count')
+    if seen < 18:
+        raise RuntimeError('ptxas log holds fewer wkv7_fwd_tc_kernel entries than are built: cannot check their register count')
 
 
 def _build_ext():

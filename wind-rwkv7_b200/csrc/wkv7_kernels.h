@@ -73,7 +73,7 @@ size_t bwd_workspace_bytes(long long B, long long T, long long H, bool ln);  // 
 size_t bwd32_workspace_bytes(long long B, long long T, long long H);         // and for fp32 ones, attn
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
-// tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| = preparation groups per CTA (2..4); negative: operands are
+// tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| + 1 = chunks in flight per CTA (2..4; attn_ln: always four chunks); negative: operands are
 // not rounded to TF32 by their producer (the tensor core truncates them)
 int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream);
 // bf16 forward with the sequences cut into nseg segments each (wkv7_time_split.cu)
