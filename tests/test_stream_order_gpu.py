@@ -1,0 +1,67 @@
+"""Kernels that may start before the one ahead of them in the stream has ended: calls in a row, each on inputs of its own, give what the same calls
+give with the device waited for after each; and sums that start from zero do so in memory that held something else."""
+import types
+
+import pytest
+import torch as th
+
+pytestmark = pytest.mark.gpu
+N = 64
+
+
+def _bf(*shape, std=1.0):
+    return (th.randn(*shape, device='cuda') * std).bfloat16()
+
+
+def _ddlerp(B, T, C, D):
+    from wind_rwkv.rwkv7 import ddlerp
+    ins = [_bf(B, T, C), th.rand(C, device='cuda'), th.randn(4 * D, C, device='cuda') * .02, th.randn(4, C, D, device='cuda') * .02, th.rand(4, 1, 1, C, device='cuda')]
+    return lambda x: ddlerp(*x), ins, [_bf(B, T, C) for _ in range(4)]
+
+
+def _attn(B, T, H):
+    from wind_rwkv.rwkv7 import attn, synthetic
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=int(th.randint(1 << 30, (1,))), dtype=th.bfloat16, device='cuda')
+    return lambda x: (attn(*x, N),), [d[n] for n in 'rwkvab'], [d['dy']]
+
+
+def _mixer(B, T, C):
+    from wind_rwkv.rwkv7 import TimeMixer
+    model = TimeMixer(types.SimpleNamespace(n_layer=4, n_head=C // N, n_embd=C), 1).cuda()
+    with th.no_grad():
+        for p in model.parameters():
+            p.add_(th.randn_like(p) * .02)
+    params = list(model.parameters())
+    return lambda x: (model(x[0]),), [_bf(B, T, C)] + params, [_bf(B, T, C)]
+
+
+@pytest.mark.parametrize('make,args', [(_ddlerp, (2, 130, 128, 16)), (_ddlerp, (3, 257, 192, 32)), (_ddlerp, (1, 65, 64, 64)),
+                                       (_attn, (1, 130, 3)), (_attn, (3, 1003, 2)), (_mixer, (1, 65, 256)), (_mixer, (2, 515, 128))])
+def test_calls_in_a_row(make, args):
+    th.manual_seed(0)
+    cases = [make(*args) for _ in range(4)]
+    for _, ins, _ in cases:
+        for t in ins:
+            t.requires_grad_()
+
+    def run(sync):
+        out = []
+        for f, ins, g in cases:
+            poison = th.full((1 << 24,), float('nan'), device='cuda')  # what the allocator hands out next holds NaN
+            del poison
+            y = f(ins)
+            if sync:
+                th.cuda.synchronize()
+            out.append((y, th.autograd.grad(y, ins, g)))
+            if sync:
+                th.cuda.synchronize()
+        th.cuda.synchronize()
+        return out
+    apart, rows = run(True), [run(False) for _ in range(3)]
+    for row in rows:
+        for (y0, d0), (y1, d1) in zip(apart, row):
+            for a, b in zip(y0, y1):
+                assert th.equal(a, b)
+            for a, b in zip(d0, d1):  # weight gradients are fp32 sums by atomics, in any order (and bf16 values behind them none)
+                assert th.isfinite(b).all()
+                assert float((a.float() - b.float()).norm()) <= 1e-5 * float(a.float().norm()) + 1e-12

@@ -5,12 +5,14 @@
 // at C = 768 take 5.4 us (torch's multi-tensor copy, which cuts tensors into tiles of 65536 elements for 46 CTAs: 18 us).
 #include "expand_loras.h"
 #include "mma_bf16.cuh"
+#include "wkv7_kernels.h"
 
 namespace wkv7 {
 
 constexpr int CAST_TILE = 2048;
 
 __global__ void __launch_bounds__(CAST_TILE / 8) cast_kernel(const __grid_constant__ CastParams p) {
+    stream_order();
     long long tile = blockIdx.x;
     int t = 0;
     for (; t < p.count; ++t) {
@@ -39,8 +41,7 @@ int launch_cast(const CastParams& p, cudaStream_t stream) {
     long long tiles = 0;
     for (int i = 0; i < p.count; ++i) tiles += (p.numel[i] + CAST_TILE - 1) / CAST_TILE;
     if (tiles > 0x7fffffffLL) return kTooLarge;
-    cast_kernel<<<(unsigned)tiles, CAST_TILE / 8, 0, stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(cast_kernel, dim3((unsigned)tiles), CAST_TILE / 8, 0, stream, p) ? kOk : kLaunchFailed;
 }
 
 }  // namespace wkv7

@@ -431,11 +431,14 @@ __global__ void __launch_bounds__(256) ddlerp_bwd_dL_kernel(DdlerpBwdParams p, l
 template <int D> static int launch_ddlerp_bwd_t(const DdlerpBwdParams& p, cudaStream_t stream, void* ws = nullptr, int* status = nullptr) {
     const long long B = p.rows / p.T;
     const int C = (int)p.C;
-    if (cudaMemsetAsync(p.dalpha, 0, sizeof(float) * C, stream) != cudaSuccess) return kLaunchFailed;
-    if (cudaMemsetAsync(p.dbeta, 0, sizeof(float) * 4 * C, stream) != cudaSuccess) return kLaunchFailed;
-    if (cudaMemsetAsync(p.dR, 0, sizeof(float) * 4 * C * D, stream) != cudaSuccess) return kLaunchFailed;
-    if (cudaMemsetAsync(p.dL, 0, sizeof(float) * 4 * D * C, stream) != cudaSuccess) return kLaunchFailed;
-    if (ws && (D == 16 || D == 32) && launch_ddlerp_prep_bwd(p, ws, stream) != kOk) return kLaunchFailed;
+    if (ws && (D == 16 || D == 32)) {
+        if (launch_ddlerp_prep_bwd(p, ws, stream) != kOk) return kLaunchFailed;  // zeroes the sums, too
+    } else {
+        if (cudaMemsetAsync(p.dalpha, 0, sizeof(float) * C, stream) != cudaSuccess) return kLaunchFailed;
+        if (cudaMemsetAsync(p.dbeta, 0, sizeof(float) * 4 * C, stream) != cudaSuccess) return kLaunchFailed;
+        if (cudaMemsetAsync(p.dR, 0, sizeof(float) * 4 * C * D, stream) != cudaSuccess) return kLaunchFailed;
+        if (cudaMemsetAsync(p.dL, 0, sizeof(float) * 4 * D * C, stream) != cudaSuccess) return kLaunchFailed;
+    }
     int dpre_rc = ws ? launch_ddlerp_dpre_tc(p, ws, status, stream) : kBadShape;  // tcgen05 form where it covers the rank
     if (dpre_rc != kOk && dpre_rc != kBadShape) return dpre_rc;
     if (dpre_rc == kBadShape) {

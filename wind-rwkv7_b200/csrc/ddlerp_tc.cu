@@ -97,6 +97,8 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
 // ---- prep: W12 = [L (1 - alpha) | L alpha]  [4D, 2C],  R' [C, 4D] -------------------------------------------------------
 __global__ void ddlerp_prep_kernel(const __nv_bfloat16* __restrict__ L, const __nv_bfloat16* __restrict__ alpha, const __nv_bfloat16* __restrict__ R,
                                    __nv_bfloat16* __restrict__ W12, __nv_bfloat16* __restrict__ Rp, int C, int D) {
+    stream_order();
+    L = after_stream_order(L); alpha = after_stream_order(alpha); R = after_stream_order(R);
     const int n4 = 4 * D;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const long long nW = (long long)n4 * 2 * C, nR = (long long)C * n4;
@@ -154,6 +156,7 @@ __global__ void __launch_bounds__(g1::THREADS) ddlerp_gemm1_kernel(const __grid_
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
 
     if (warp == 4) {
         if (elect_one()) {
@@ -293,6 +296,8 @@ __global__ void __launch_bounds__(g2::THREADS, 1) ddlerp_lerp_kernel(const __gri
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
+    beta = after_stream_order(beta);
     // this CTA's units: a contiguous range of the (token tile, channel block) list, channel blocks running fastest
     const int u_lo = (int)((long long)units * blockIdx.x / gridDim.x), nmine = (int)((long long)units * (blockIdx.x + 1) / gridDim.x) - u_lo;
 
@@ -500,6 +505,7 @@ __global__ void __launch_bounds__(g3::THREADS) ddlerp_dw12_kernel(const __grid_c
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
 
     if (warp == 4) {
         if (elect_one()) {
@@ -564,6 +570,8 @@ __global__ void __launch_bounds__(g3::THREADS) ddlerp_dw12_kernel(const __grid_c
 // nullptr (zero on entry) also dalpha[c] += sum_n L[n, c] (dW2 - dW1)[n, c]  ( = sum_t (dpre L)[t, c] (x_{t-1} - x_t)[c] ).
 __global__ void ddlerp_dl_finish_kernel(float* __restrict__ dL, const float* __restrict__ dW2, const __nv_bfloat16* __restrict__ alpha,
                                         const __nv_bfloat16* __restrict__ L, float* __restrict__ dalpha, int C, int n4) {
+    stream_order();
+    dW2 = after_stream_order(dW2); alpha = after_stream_order(alpha); L = after_stream_order(L);
     const int c = blockIdx.x * blockDim.x + threadIdx.x, n0 = blockIdx.y * 8;
     if (c >= C) return;
     const float a = __bfloat162float(alpha[c]);
@@ -605,10 +613,17 @@ __host__ __device__ constexpr int stage_bytes(int D) { return 4 * DY_BYTES + X_B
 // The backward's rearranged weights, one launch: R^T as [4D, C] (row k D + d = R[k][:, d]), L^T as [C, 4D], and R' as [C, 4D]
 // (column k D + d = R[k][c][d])
 __global__ void ddlerp_prep_bwd_kernel(const __nv_bfloat16* __restrict__ L, const __nv_bfloat16* __restrict__ R, __nv_bfloat16* __restrict__ Rt,
-                                       __nv_bfloat16* __restrict__ Lt, __nv_bfloat16* __restrict__ Rp, int C, int D) {
+                                       __nv_bfloat16* __restrict__ Lt, __nv_bfloat16* __restrict__ Rp, float* __restrict__ dalpha,
+                                       float* __restrict__ dbeta, float* __restrict__ dR, float* __restrict__ dL, float* __restrict__ dW2, int C, int D) {
+    stream_order();
+    L = after_stream_order(L); R = after_stream_order(R);
     const int n4 = 4 * D;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)C * n4) return;
+    // the sums that the following kernels add to start from zero (as five memsets they were 18 us of a backward at B32 T1024 C768)
+    dR[i] = dL[i] = dW2[i] = 0.f;
+    if (i < 4 * C) dbeta[i] = 0.f;
+    if (i < C) dalpha[i] = 0.f;
     {
         const int n = (int)(i / C), c = (int)(i % C);
         Rt[i] = R[((long long)(n / D) * C + c) * D + (n % D)];
@@ -653,6 +668,8 @@ __global__ void __launch_bounds__(g4::THREADS, 1) ddlerp_dpre_tc_kernel(const __
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
+    m = after_stream_order(m);
 
     if (warp == 8) {
         if (elect_one()) {
@@ -848,6 +865,9 @@ __global__ void __launch_bounds__(g5::THREADS, 1) ddlerp_main_tc_kernel(const __
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
+    dyp0 = after_stream_order(dyp0); dyp1 = after_stream_order(dyp1); dyp2 = after_stream_order(dyp2); dyp3 = after_stream_order(dyp3);
+    dpre = after_stream_order(dpre); mten = after_stream_order(mten); alpha = after_stream_order(alpha); beta = after_stream_order(beta);
     const uint32_t sb = smem_u32(sm);
 
     if (warp == EPI_WARPS) {
@@ -1198,8 +1218,7 @@ template <int D> static int launch_lerp(const CUtensorMap& mM, const CUtensorMap
     const long long tiles_per_seq = (p.T + BM - 1) / BM, units = tiles_per_seq * B * (p.C / g2::BN);
     if (units > 0x7fffffffLL) return kTooLarge;
     const unsigned grid = (unsigned)(units < sms ? units : sms);
-    kern<<<grid, g2::THREADS, smem, stream>>>(mM, mR, mX, mY, (const __nv_bfloat16*)p.beta, (int)p.C, (int)p.T, (int)tiles_per_seq, (int)units, status);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(kern, dim3(grid), g2::THREADS, smem, stream, mM, mR, mX, mY, (const __nv_bfloat16*)p.beta, (int)p.C, (int)p.T, (int)tiles_per_seq, (int)units, status) ? kOk : kLaunchFailed;
 }
 
 }  // namespace dtc
@@ -1234,10 +1253,9 @@ template <int D> static int launch_main_tc_t(const DdlerpBwdParams& p, void* ws,
     const long long tiles_per_seq = (T + BM - 1) / BM, tiles = tiles_per_seq * B, units = tiles * (C / 64);
     if (units > 0x7fffffffLL) return kTooLarge;
     const unsigned grid = (unsigned)(units < sms ? units : sms);
-    kern<<<grid, g5::THREADS, smem, stream>>>(mm, (const __nv_bfloat16*)p.dy[0], (const __nv_bfloat16*)p.dy[1], (const __nv_bfloat16*)p.dy[2],
+    return launch(kern, dim3(grid), g5::THREADS, smem, stream, mm, (const __nv_bfloat16*)p.dy[0], (const __nv_bfloat16*)p.dy[1], (const __nv_bfloat16*)p.dy[2],
                                              (const __nv_bfloat16*)p.dy[3], (const __nv_bfloat16*)p.dpre, (const __nv_bfloat16*)p.m, (const __nv_bfloat16*)p.alpha,
-                                             (const __nv_bfloat16*)p.beta, p.dR, p.dbeta, (int)C, (int)T, (int)tiles_per_seq, (int)tiles, (int)units, status);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+                                             (const __nv_bfloat16*)p.beta, p.dR, p.dbeta, (int)C, (int)T, (int)tiles_per_seq, (int)tiles, (int)units, status) ? kOk : kLaunchFailed;
 }
 // returns kBadShape for ranks this form does not cover (the caller then runs the mma.sync kernel)
 int launch_ddlerp_main_tc(const DdlerpBwdParams& p, void* ws, int* status, cudaStream_t stream) {
@@ -1246,14 +1264,14 @@ int launch_ddlerp_main_tc(const DdlerpBwdParams& p, void* ws, int* status, cudaS
     return kBadShape;
 }
 
-// the rearranged weights of the tcgen05 backward kernels into the scratch: R^T, L^T, R' behind dW2
+// the rearranged weights of the tcgen05 backward kernels into the scratch: R^T, L^T, R' behind dW2; dalpha, dbeta, dR, dL and dW2 zeroed
 int launch_ddlerp_prep_bwd(const DdlerpBwdParams& p, void* ws, cudaStream_t stream) {
     const long long C = p.C;
     const int n4 = 4 * p.D;
     __nv_bfloat16* Rt = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(ws) + (size_t)n4 * C * 4);
     const long long n = (long long)n4 * C;
-    dtc::ddlerp_prep_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)p.L, (const __nv_bfloat16*)p.R, Rt, Rt + n, Rt + 2 * n, (int)C, p.D);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(dtc::ddlerp_prep_bwd_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, (const __nv_bfloat16*)p.L, (const __nv_bfloat16*)p.R, Rt, Rt + n, Rt + 2 * n,
+                  p.dalpha, p.dbeta, p.dR, p.dL, (float*)ws, (int)C, p.D) ? kOk : kLaunchFailed;
 }
 
 // dpre (bf16 [rows, 4D]) from dy, x, R and m; ranks 16 and 32
@@ -1275,8 +1293,7 @@ template <int D> static int launch_dpre_tc_t(const DdlerpBwdParams& p, void* ws,
     static_assert(smem <= 232448, "two stages must fit one CTA");
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
     dim3 grid((unsigned)((T + BM - 1) / BM), (unsigned)B);
-    kern<<<grid, g4::THREADS, smem, stream>>>(mY, mX, mRt, mP, (const __nv_bfloat16*)p.m, (int)C, (int)T, status);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(kern, dim3(grid), g4::THREADS, smem, stream, mY, mX, mRt, mP, (const __nv_bfloat16*)p.m, (int)C, (int)T, status) ? kOk : kLaunchFailed;
 }
 // returns kBadShape for ranks this form does not cover (the caller then runs the mma.sync kernel)
 int launch_ddlerp_dpre_tc(const DdlerpBwdParams& p, void* ws, int* status, cudaStream_t stream) {
@@ -1291,7 +1308,7 @@ int launch_ddlerp_dL_tc(const DdlerpBwdParams& p, void* ws, int* status, cudaStr
     const long long B = p.rows / p.T, C = p.C, T = p.T;
     const int n4 = 4 * p.D;
     float* dW2 = (float*)ws;
-    if (cudaMemsetAsync(dW2, 0, sizeof(float) * n4 * C, stream) != cudaSuccess) return kLaunchFailed;
+    if (p.D != 16 && p.D != 32 && cudaMemsetAsync(dW2, 0, sizeof(float) * n4 * C, stream) != cudaSuccess) return kLaunchFailed;  // (otherwise: launch_ddlerp_prep_bwd)
     alignas(64) CUtensorMap mD, mX;
     const long long dd[3] = {n4, T, B}, sd[2] = {n4, T * n4}, dx[3] = {C, T, B}, sx[2] = {C, T * C};
     const int bx[3] = {64, BM, 1};
@@ -1310,11 +1327,9 @@ int launch_ddlerp_dL_tc(const DdlerpBwdParams& p, void* ws, int* status, cudaStr
     if (splits < 1) splits = 1;
     if (splits > total) splits = total;
     dim3 grid((unsigned)col_tiles, (unsigned)splits, (unsigned)row_tiles);
-    ddlerp_dw12_kernel<<<grid, g3::THREADS, smem, stream>>>(mD, mX, p.dL, dW2, (int)C, n4, (int)tiles_per_seq, (int)total, status);
-    if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
-    ddlerp_dl_finish_kernel<<<dim3((unsigned)((C + 127) / 128), (unsigned)((n4 + 7) / 8)), 128, 0, stream>>>(
-        p.dL, dW2, (const __nv_bfloat16*)p.alpha, (const __nv_bfloat16*)p.L, with_dalpha ? p.dalpha : nullptr, (int)C, n4);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    if (!launch(ddlerp_dw12_kernel, dim3(grid), g3::THREADS, smem, stream, mD, mX, p.dL, dW2, (int)C, n4, (int)tiles_per_seq, (int)total, status)) return kLaunchFailed;
+    return launch(ddlerp_dl_finish_kernel, dim3((unsigned)((C + 127) / 128), (unsigned)((n4 + 7) / 8)), 128, 0, stream, 
+        p.dL, dW2, (const __nv_bfloat16*)p.alpha, (const __nv_bfloat16*)p.L, with_dalpha ? p.dalpha : nullptr, (int)C, n4) ? kOk : kLaunchFailed;
 }
 
 size_t ddlerp_fwd_tc_workspace_bytes(long long C, int D) { return (size_t)(4 * D) * (size_t)(3 * C) * 2; }
@@ -1331,9 +1346,8 @@ int launch_ddlerp_fwd_tc(const DdlerpFwdParams& p, void* ws, int* status, cudaSt
     __nv_bfloat16* Rp = W12 + (long long)n4 * 2 * C;
     {
         const long long n = (long long)n4 * 3 * C;
-        ddlerp_prep_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)p.L, (const __nv_bfloat16*)p.alpha, (const __nv_bfloat16*)p.R,
-                                                                          W12, Rp, (int)C, D);
-        if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+        if (!launch(ddlerp_prep_kernel, dim3((unsigned)((n + 255) / 256)), 256, 0, stream, (const __nv_bfloat16*)p.L, (const __nv_bfloat16*)p.alpha, (const __nv_bfloat16*)p.R,
+                                                                          W12, Rp, (int)C, D)) return kLaunchFailed;
     }
     alignas(64) CUtensorMap mX, mXl, mW, mMs, mMl, mR, mY;
     {
@@ -1357,8 +1371,7 @@ int launch_ddlerp_fwd_tc(const DdlerpFwdParams& p, void* ws, int* status, cudaSt
         auto kern = alone ? ddlerp_gemm1_kernel<g1::MANY> : ddlerp_gemm1_kernel<g1::FEW>;
         const int smem = (alone ? g1::MANY : g1::FEW) * g1::STAGE_BYTES + (int)sizeof(g1::Ctrl) + 1024;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
-        kern<<<grid, g1::THREADS, smem, stream>>>(mX, mW, mMs, (int)C, n4, (int)T, status);
-        if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+        if (!launch(kern, dim3(grid), g1::THREADS, smem, stream, mX, mW, mMs, (int)C, n4, (int)T, status)) return kLaunchFailed;
     }
     return D == 16 ? launch_lerp<16>(mMl, mR, mXl, mY, p, B, status, stream) : launch_lerp<32>(mMl, mR, mXl, mY, p, B, status, stream);
 }

@@ -90,6 +90,7 @@ __device__ __forceinline__ void load_in_frags(uint32_t (&a)[D / 16][4], const bf
 
 template <int D>
 __global__ void __launch_bounds__(128, D == 16 ? 6 : 1) loras_fwd_kernel(LorasParams p) {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<LorasFwdSmem<D>*>(smem_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -227,6 +228,7 @@ template <int D> struct LorasBwdSmem {
 constexpr int BWD_THREADS = 256;
 template <int D>
 __global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel(LorasParams p) {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     auto& sm = *reinterpret_cast<LorasBwdSmem<D>*>(smem_raw);
     const int tid = threadIdx.x, warp = (tid >> 5) & 3, half = tid >> 7, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -490,6 +492,7 @@ __global__ void __launch_bounds__(BWD_THREADS, D <= 32 ? 2 : 1) loras_bwd_kernel
 
 // sums the per-head partials: out[l][row][d] = sum_h partial[l][row][h][d]; 8 values (16 bytes) per thread
 __global__ void loras_reduce_heads_kernel(LorasParams p, int H, int D) {
+    stream_order();
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;  // index over [rows, D / 8]
     const int l = blockIdx.y, per = D / 8;
     const long long row = i / per;
@@ -512,8 +515,7 @@ template <int D> static int launch_loras_fwd_t(const LorasParams& p, cudaStream_
     const int smem = (int)sizeof(LorasFwdSmem<D>);
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
     const long long tiles = (p.rows + 63) / 64, ny = tiles < 32768 ? tiles : 32768;  // y and z end at 65535
-    kern<<<dim3((unsigned)(p.C / HC), (unsigned)ny, (unsigned)((tiles + ny - 1) / ny)), 128, smem, stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(kern, dim3((unsigned)(p.C / HC), (unsigned)ny, (unsigned)((tiles + ny - 1) / ny)), 128, smem, stream, p) ? kOk : kLaunchFailed;
 }
 
 template <int D> static int launch_loras_bwd_t(const LorasParams& p, cudaStream_t stream) {
@@ -542,11 +544,9 @@ template <int D> static int launch_loras_bwd_t(const LorasParams& p, cudaStream_
     long long nseg = (long long)resident * sm_count() / H;
     if (nseg > tiles) nseg = tiles;
     if (nseg < 1) nseg = 1;
-    kern<<<dim3((unsigned)H, (unsigned)nseg), BWD_THREADS, smem, stream>>>(p);
-    if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+    if (!launch(kern, dim3((unsigned)H, (unsigned)nseg), BWD_THREADS, smem, stream, p)) return kLaunchFailed;
     const long long n = p.rows * (D / 8);
-    loras_reduce_heads_kernel<<<dim3((unsigned)((n + 255) / 256), 4), 256, 0, stream>>>(p, H, D);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(loras_reduce_heads_kernel, dim3((unsigned)((n + 255) / 256), 4), 256, 0, stream, p, H, D) ? kOk : kLaunchFailed;
 }
 
 int launch_loras_fwd(const LorasParams& p, cudaStream_t stream) {

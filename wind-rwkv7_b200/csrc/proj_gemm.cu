@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(THREADS) proj_gemm_kernel(const __grid_constan
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
 
     if (warp == 4) {
         if (elect_one()) {  // producer: one TMA request per operand block
@@ -235,8 +236,7 @@ int launch_proj_gemm(int count, const void* const* A, const void* const* W, void
     auto kern = alone ? proj_gemm_kernel<MANY> : proj_gemm_kernel<FEW>;
     const int smem = (alone ? MANY : FEW) * STAGE_BYTES + (int)sizeof(Ctrl) + 1024;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kLaunchFailed;
-    kern<<<grid, gemm::THREADS, smem, stream>>>(ps, status);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(kern, dim3(grid), gemm::THREADS, smem, stream, ps, status) ? kOk : kLaunchFailed;
 }
 
 }  // namespace wkv7

@@ -173,6 +173,7 @@ template <int PREC, bool SPLIT> __device__ __forceinline__ void mma2(float (&d)[
 // none of the row tests).
 template <int PREC, bool LN, bool TAIL, bool PAR>
 __global__ void __launch_bounds__(THREADS, PAR ? 2 : 1) wkv7_bwd_kernel(BwdParams p, Walked wk, const __grid_constant__ CkptMaps cmaps) {
+    stream_order();
     static_assert(!(PAR && LN), "attn_ln's state gradient needs the gradient of the recurrence output first");
     using Smem = BwdSmem<PREC, LN, PAR>;
     static_assert(!PAR || sizeof(Smem) + 1024 <= 116736, "two CTAs per SM");
@@ -953,6 +954,7 @@ static_assert(sizeof(Walk32Smem) <= 232448, "one CTA per SM");
 
 template <bool TAIL>
 __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk32_kernel(BwdParams p, float* tiles, int it0, int count) {
+    stream_order();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Walk32Smem& sm = *reinterpret_cast<Walk32Smem*>(smem_raw);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t4 = lane & 3, w = warp & 3;
@@ -1247,15 +1249,12 @@ template <int PREC, bool LN> static int launch_bwd_t(const BwdParams& p, cudaStr
         float* tiles = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.flags) + WORK_FLAG_BYTES);
         for (long long it0 = 0; it0 < chunks; it0 += walked) {
             const int n = (int)std::min<long long>(walked, chunks - it0), total = (int)chains * n, per = (total + slots - 1) / slots;
-            walk<<<(unsigned)chains, WALK_THREADS, sizeof(Walk32Smem), stream>>>(p, tiles, (int)it0, n);
-            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
-            kern<<<(unsigned)((total + per - 1) / per), THREADS, smem, stream>>>(p, Walked{tiles, (int)it0, n, per, total}, cmaps);
-            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+            if (!launch(walk, dim3((unsigned)chains), WALK_THREADS, sizeof(Walk32Smem), stream, p, tiles, (int)it0, n)) return kLaunchFailed;
+            if (!launch(kern, dim3((unsigned)((total + per - 1) / per)), THREADS, smem, stream, p, Walked{tiles, (int)it0, n, per, total}, cmaps)) return kLaunchFailed;
         }
         return kOk;
     }
-    kern<<<(unsigned)chains, THREADS, smem, stream>>>(p, Walked{}, cmaps);
-    if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+    if (!launch(kern, dim3((unsigned)chains), THREADS, smem, stream, p, Walked{}, cmaps)) return kLaunchFailed;
     return LN ? launch_reduce_dparams(p, stream) : kOk;
 }
 

@@ -168,6 +168,7 @@ constexpr int TILE_FLOATS = N * SS;  // layout of s0_at()
 
 template <bool TAIL, bool LN, bool PAR>
 __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p, WorkSplit ws, Tiles tiles, const __grid_constant__ BwdMaps maps) {
+    stream_order();
     extern __shared__ unsigned char smem_dyn[];
     using Smem = bf16bwd::Smem<LN>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u));
@@ -838,6 +839,7 @@ static_assert(sizeof(WalkSmem) + 1024 <= 232448, "one CTA per SM");
 
 template <bool TAIL>
 __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParams p, float* tiles, int it0, int count, const __grid_constant__ BwdMaps maps) {
+    stream_order();
     extern __shared__ unsigned char smem_dyn[];
     WalkSmem& sm = *reinterpret_cast<WalkSmem*>(smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t4 = lane & 3, w = warp & 3;
@@ -1037,17 +1039,14 @@ template <bool LN> static int launch_bwd_bf16_t(const BwdParams& p, cudaStream_t
         float* tiles = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.flags) + WORK_FLAG_BYTES);
         for (long long it0 = 0; it0 < chunks; it0 += walked) {
             const int n = (int)std::min<long long>(walked, chunks - it0), total = (int)chains * n, per = (total + slots - 1) / slots;
-            walk<<<(unsigned)chains, WALK_THREADS, wsmem, stream>>>(p, tiles, (int)it0, n, maps);
-            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
-            kern<<<(unsigned)((total + per - 1) / per), NTHREADS, smem, stream>>>(p, WorkSplit{0, per, n, total, nullptr}, Tiles{tiles, (int)it0}, maps);
-            if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+            if (!launch(walk, dim3((unsigned)chains), WALK_THREADS, wsmem, stream, p, tiles, (int)it0, n, maps)) return kLaunchFailed;
+            if (!launch(kern, dim3((unsigned)((total + per - 1) / per)), NTHREADS, smem, stream, p, WorkSplit{0, per, n, total, nullptr}, Tiles{tiles, (int)it0}, maps)) return kLaunchFailed;
         }
         return kOk;
     }
     const WorkSplit ws = plan_work(chains, chunks, 2, p.ds0 ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
-    kern<<<(unsigned)ws.ctas, NTHREADS, smem, stream>>>(p, ws, Tiles{}, maps);
-    if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
+    if (!launch(kern, dim3((unsigned)ws.ctas), NTHREADS, smem, stream, p, ws, Tiles{}, maps)) return kLaunchFailed;
     return LN ? launch_reduce_dparams(p, stream) : kOk;
 }
 

@@ -414,6 +414,21 @@ __device__ __forceinline__ void mbar_landed_uncounted(uint64_t* bar, volatile in
     mbar_wait_bounded<true>(bar, 1, never_set, status);
 }
 
+// Kernels are launched such that they may start before the one ahead of them in the stream has ended (launch() in wkv7_kernels.h), and
+// call this before they touch global memory: what stands before it - barriers, tensor memory - and the launch itself then overlap the
+// other kernel's end.  From here on the next kernel may start, which will in turn wait until this one has ended (a kernel that is not
+// launched so waits by itself); all of its CTAs are then running or have ended, so that none of them has to wait for a place that a CTA
+// of the next one holds.  For the same reason tensor memory is allocated before this call.
+__device__ __forceinline__ void stream_order() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// a pointer whose target is read through the read-only path: no load may be moved ahead of stream_order()
+template <typename T> __device__ __forceinline__ T* after_stream_order(T* p) {
+    asm volatile("" : "+l"(p) :: "memory");
+    return p;
+}
+
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t p;
     asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));

@@ -462,6 +462,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1) wkv7_fwd_tc_kernel(FwdParams p,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctrl->tmem_base;
+    stream_order();
 
     // Start state of a segment -> tensor memory and its checkpoint: warp wq of the group owns lanes 32 wq .. 32 wq + 31, of
     // which lanes 0-15 hold value rows 16 wq .. 16 wq + 15.  A chain's first chunk starts from s0 (or zeros); a chain that
@@ -1159,8 +1160,7 @@ template <int S, bool RND, bool LN, bool TAIL, bool AFF = false> static int laun
         if (ins[i] && !encode_bthn_map(ms[i], const_cast<void*>(ins[i]), p.B, p.T, p.H, p.st)) return kLaunchFailed;
     const WorkSplit ws = plan_work(p.B * p.H, (p.T + L - 1) / L, 1, p.sT ? p.flags : nullptr);
     if (ws.flags && cudaMemsetAsync(ws.flags, 0, ws.ctas * sizeof(unsigned), stream) != cudaSuccess) return kLaunchFailed;
-    kern<<<(unsigned)ws.ctas, THREADS_TC, smem, stream>>>(p, ws, maps);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch(kern, dim3((unsigned)ws.ctas), THREADS_TC, smem, stream, p, ws, maps) ? kOk : kLaunchFailed;
 }
 
 template <int S, bool RND, bool LN> static int launch_t(const FwdParams& p, cudaStream_t stream) {
