@@ -65,3 +65,23 @@ def test_calls_in_a_row(make, args):
             for a, b in zip(d0, d1):  # weight gradients are fp32 sums by atomics, in any order (and bf16 values behind them none)
                 assert th.isfinite(b).all()
                 assert float((a.float() - b.float()).norm()) <= 1e-5 * float(a.float().norm()) + 1e-12
+
+
+@pytest.mark.parametrize('B,H', [(1, 3), (30, 32), (38, 32)])  # a CTA per chain; the ring of several chains a CTA
+def test_decode_steps_in_a_row(B, H):
+    """Each step reads the state that the one before it leaves in place."""
+    from wind_rwkv.rwkv7 import attn_step, synthetic
+    ins = [[synthetic.wkv7_inputs(B, 1, H, N, seed=i, dtype=th.bfloat16, device='cuda')[n] for n in 'rwkvab'] for i in range(12)]
+
+    def run(sync):
+        th.manual_seed(1)
+        s, ys = th.randn(B, H, N, N, device='cuda') * .1, []
+        for x in ins:
+            ys.append(attn_step(*x, N, s, inplace=True)[0])
+            if sync:
+                th.cuda.synchronize()
+        th.cuda.synchronize()
+        return ys + [s]
+    apart = run(True)
+    for _ in range(5):
+        assert all(th.equal(a, b) for a, b in zip(apart, run(False)))

@@ -15,6 +15,8 @@
 // CTA, not by each of the 64 rows (8192 exponentials per chain).
 // What is left is the state traffic: 2 * 16 KB per chain and call, all loads of it in flight before the first barrier, six CTAs an
 // SM (40 registers; at 76 registers and three CTAs 1.2 times as long).  Many chains, up to eight steps: wkv7_step_ring_kernel below.
+// Both start while the kernel ahead of them drains (stream_order): steps in a row, T = 1, 6400 chains 37.3 -> 35.9 us, 3200 20.5 -> 18.1, 1280 10.3 ->
+// 8.9, 768 8.3 -> 6.5, and the smallest calls, whose time is the host's, 6.1 -> 5.5.  (The next but one state on its way, too: 10240 chains 56.3 -> 59.4.)
 #include "wkv7_kernels.h"
 
 namespace wkv7 {
@@ -47,6 +49,7 @@ __device__ __forceinline__ float step_row(float (&S)[16], const float (*u)[N], i
 
 template <typename IoT>
 __global__ void __launch_bounds__(256, 6) wkv7_step_kernel(StepParams p) {
+    stream_order();
     __shared__ __align__(16) float vec[2][6][N];  // decay, a, b, k, r, v of one step; two buffers: one barrier per step
     const int tid = threadIdx.x, i = tid >> 2, q = tid & 3;
     const long long bh = blockIdx.x;
@@ -114,8 +117,9 @@ __global__ void __launch_bounds__(256, RING_PER_SM) wkv7_step_ring_kernel(StepPa
         mbar_init(&full, 1);
         abort = zero = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (p.s0) { load(bh); ++loads; }
     }
+    stream_order();
+    if (tid == 0 && p.s0) { load(bh); ++loads; }
     long long base = offset(bh);
     IoT x0 = in0[base], x1 = x0;
     if (part < 2) x1 = in1[base];
@@ -172,9 +176,8 @@ template <typename IoT> static int launch_step_t(const StepParams& p, cudaStream
     const long long chains = p.B * p.H;
     // (the smallest calls, whose time is the host's, do not ask for the number of SMs)
     const long long resident = chains > 512 ? (long long)RING_PER_SM * sm_count() : chains;
-    if (chains > 2 * resident && chains <= 0x3fffffff && p.T <= RING_STEPS && p.status) wkv7_step_ring_kernel<IoT><<<(unsigned)resident, 256, 0, stream>>>(p, (int)chains);
-    else wkv7_step_kernel<IoT><<<(unsigned)chains, 256, 0, stream>>>(p);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    if (chains > 2 * resident && chains <= 0x3fffffff && p.T <= RING_STEPS && p.status) return launch(wkv7_step_ring_kernel<IoT>, dim3((unsigned)resident), 256, 0, stream, p, (int)chains) ? kOk : kLaunchFailed;
+    return launch(wkv7_step_kernel<IoT>, dim3((unsigned)chains), 256, 0, stream, p) ? kOk : kLaunchFailed;
 }
 int launch_step(const StepParams& p, int io_dtype, cudaStream_t stream) {
     return io_dtype == 0 ? launch_step_t<__nv_bfloat16>(p, stream) : launch_step_t<float>(p, stream);
