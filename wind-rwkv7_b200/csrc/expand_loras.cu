@@ -22,6 +22,11 @@ constexpr int HC = 64;  // channels per head
 // Seven special-function instructions an element (three tanh for the sigmoids, ex2 + lg2 for the softplus, ex2 for E), everything
 // else two elements an instruction: the op is bound by issue slots.
 struct Gates { F2 a, ma, mk, w, E; };
+__device__ __forceinline__ float lg2_approx(float x) {  // of 1 + e^.., at least 1: __log2f spends three instructions more on denormal arguments
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
 __device__ __forceinline__ F2 sigmoid2(F2 x) {
     x = mul2(x, f2(0.5f, 0.5f));
     return fma2(f2(tanh_f(x.x), tanh_f(x.y)), f2(0.5f, 0.5f), f2(0.5f, 0.5f));
@@ -40,7 +45,7 @@ template <bool SIG = true> __device__ __forceinline__ Gates lora_gates(F2 xa, F2
     o.mk = sigmoid2(xk);
     const F2 n = mul2(v, f2(-LOG2E, -LOG2E));
     const F2 e = add2(f2(ex2_approx(fminf(n.x, 115.f)), ex2_approx(fminf(n.y, 115.f))), f2(1.f, 1.f));
-    o.w = fma2(f2(__log2f(e.x), __log2f(e.y)), f2(-LN2, -LN2), f2(-0.5f, -0.5f));
+    o.w = fma2(f2(lg2_approx(e.x), lg2_approx(e.y)), f2(-LN2, -LN2), f2(-0.5f, -0.5f));
     const F2 x = mul2(mul2(o.w, o.mk), f2(LOG2E, LOG2E));
     o.E = f2(ex2_approx(x.x), ex2_approx(x.y));
     return o;
