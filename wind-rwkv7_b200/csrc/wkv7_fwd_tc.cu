@@ -27,8 +27,8 @@
 // some 500 to 800 cycles per stage, so that a stage shared with another one makes chunks wait): 16, 17 read the scores back from their quarter of
 // tensor memory, mask them and write AK, AB, QK, QB; 18, 23 invert (I - AB) and form QB AI (even and odd chunks); 20, 21 form AI^T bwf; 19
 // issues the two hops of the chain and 22, its helper, what does not stand behind the first hop.  The kernel's hot code has to stay
-// small: its warps run different parts of it at the same time, and where the compiler had unrolled the loops of the chain and its
-// helper (9 KB more) a chunk took 15 % longer, every wait of the chain 300 cycles instead of 200.
+// small: its warps run different parts of it at the same time, and while the compiler unrolled the loops of the chain and its
+// helper (9 KB more) and waits were twice as long, B64 T1024 H12 without checkpoints took 292 us where it took 273 afterwards.
 // (Not better: the scores by mma.sync in the preparation warps - every operand is read four times, 1.2 times slower; forming the
 // inverse's two 8x8 blocks in lanes 0-15 only, 1 % slower; waits with a time hint; the raw tiles' loads by the readers - a load takes its
 // thread some 300 cycles, and the readers became the longest loop; the loads after the next tiles instead of before them.)

@@ -17,7 +17,9 @@ template <typename... P, typename... A> inline bool launch(void (*kern)(P...), d
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     c.attrs = &attr; c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...) == cudaSuccess;
+    if (cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...) == cudaSuccess) return true;
+    cudaGetLastError();  // (reported by the status; not left for the caller's next check)
+    return false;
 }
 
 struct FwdParams {
