@@ -149,9 +149,8 @@ struct Ctrl {
 };
 
 // Bounded wait for the phase with the given parity.  Returns at once when the CTA has aborted.
-// SLEEP: the thread is suspended by the hardware (try_wait with a time hint) instead of polling, so
-// that the many warps that wait for the chain do not take issue slots from the warps that work; the
-// chain's own short waits poll.
+// SLEEP: 40 ns between polls, so that the many warps that wait for the chain do not take issue slots from the warps that work; the
+// chain's own short waits poll.  (0, 16 and 100 ns make no difference: try_wait itself suspends a warp for a while.)
 template <bool SLEEP>
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity, Ctrl* ctrl, int* status, long long limit = WAIT_LIMIT) {
     // Written out, since it stands at some twenty places of code that has to stay small; the status word is written when the CTA ends.
