@@ -17,6 +17,24 @@ def sms():
 @pytest.mark.parametrize('ckpt', [False, True])
 @pytest.mark.parametrize('extra,T', [(1, 16), (1, 80), (-1, 48), (70, 7), (70, 33), (149, 1000), (400, 65)])
 def test_forward(extra, T, ckpt, ln):
+    forward_both_ways(extra, T, ckpt, ln)
+
+
+@pytest.mark.parametrize('impl', [2, 3, 4, -4])
+@pytest.mark.parametrize('ln', [False, True])
+@pytest.mark.parametrize('T', [7, 16, 17, 33, 49, 64, 81, 96])
+def test_forward_many_short_chains(T, ln, impl):
+    """Some 17 chains of one to six chunks a CTA: a new start state every few chunks, written over the one before it when its last product has
+    read it; slots, descriptors and state buffers all go round several times, and the cut chains' pieces have all lengths."""
+    from wind_rwkv.rwkv7 import _lib
+    old = _lib.set_fwd_impl(impl)
+    try:
+        forward_both_ways(2400, T, impl != -4, ln)
+    finally:
+        _lib.set_fwd_impl(old)
+
+
+def forward_both_ways(extra, T, ckpt, ln):
     from wind_rwkv.rwkv7 import _lib, synthetic
     L = _lib.lib()
     B, H = 1, sms() + extra

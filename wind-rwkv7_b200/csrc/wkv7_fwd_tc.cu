@@ -470,7 +470,10 @@ __global__ void __launch_bounds__(THREADS_TC, 1) wkv7_fwd_tc_kernel(FwdParams p,
         if (__any_sync(0xffffffffu, ctrl->abort)) return;
         const int sbh = d.bh, sc = d.c;
         const uint32_t ta = tmem + C_INIT;
-        if (d.prev_first >= 0) mbar_wait<true>(&ctrl->done[d.prev_first % S], (d.prev_first / S) & 1, ctrl, p.status);  // its start state has been used
+        if (d.prev_first >= 0) {  // its start state has been used, by products that read it where this one is written
+            mbar_wait<true>(&ctrl->done[d.prev_first % S], (d.prev_first / S) & 1, ctrl, p.status);
+            tc_fence_after();
+        }
         const int row = AFF ? 32 * wq + lane : 16 * wq + (lane & 15), i = row & 63;
         if (sc > 0) wait_handoff(ws.flags + blockIdx.x - 1, &ctrl->abort, p.status);
         const float* src = sc > 0 ? p.sT : p.s0;
