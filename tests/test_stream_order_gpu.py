@@ -85,3 +85,48 @@ def test_decode_steps_in_a_row(B, H):
     apart = run(True)
     for _ in range(5):
         assert all(th.equal(a, b) for a, b in zip(apart, run(False)))
+
+
+def _queue(kind, dtype):
+    """What keeps a quarter (forward) or a twelfth (backward) of the SMs busy for milliseconds, as a call that issues it."""
+    from wind_rwkv.rwkv7 import attn, synthetic
+    sms = th.cuda.get_device_properties(0).multi_processor_count
+    H, T = (sms // 4, 8192) if kind == 'forward' else (sms // 12, 16384)
+    d = synthetic.wkv7_inputs(1, T, H, N, seed=0, dtype=dtype, device='cuda')
+    ins = [d[n] for n in 'rwkvab']
+    if kind == 'forward':
+        def call():
+            with th.no_grad():
+                return [attn(*ins, N) for _ in range(12)]
+        return call
+    for t in ins:
+        t.requires_grad_()
+    y = attn(*ins, N)
+    return lambda: th.autograd.grad(y, ins, d['dy'], retain_graph=True)
+
+
+@pytest.mark.parametrize('kind,dtype', [('forward', th.bfloat16), ('backward', th.bfloat16), ('backward', th.float32)])
+def test_waiting_kernels_leave_idle_sms_to_other_streams(kind, dtype):
+    """A few chains keep some SMs busy for long, with kernels queued behind them.  These must not take the idle SMs while they wait: a short
+    call on another stream, whose kernel needs whole SMs, is done long before the queue (alone it takes some 20 us; it may at most have to
+    wait for one and a half of the twelve forwards)."""
+    from wind_rwkv.rwkv7 import attn, synthetic
+    queue = _queue(kind, dtype)
+    d = synthetic.wkv7_inputs(1, 64, 64, N, seed=1, dtype=th.bfloat16, device='cuda')
+    ins = [d[n] for n in 'rwkvab']
+    other = th.cuda.Stream()
+
+    def once():
+        start, end, done = (th.cuda.Event(enable_timing=True) for _ in range(3))
+        start.record()
+        keep = [queue()]
+        end.record()
+        with th.cuda.stream(other), th.no_grad():
+            keep.append(attn(*ins, N))
+            done.record()
+        th.cuda.synchronize()
+        return start.elapsed_time(done), start.elapsed_time(end)
+    th.cuda.synchronize()
+    once()  # the allocator has its blocks, the kernels are loaded
+    short, whole = min(once() for _ in range(3))
+    assert short < whole / (8 if kind == 'forward' else 4), f'{short:.3f} ms of {whole:.3f}'

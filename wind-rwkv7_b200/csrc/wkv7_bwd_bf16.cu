@@ -168,7 +168,7 @@ constexpr int TILE_FLOATS = N * SS;  // layout of s0_at()
 
 template <bool TAIL, bool LN, bool PAR>
 __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p, WorkSplit ws, Tiles tiles, const __grid_constant__ BwdMaps maps) {
-    stream_order();
+    stream_wait();
     extern __shared__ unsigned char smem_dyn[];
     using Smem = bf16bwd::Smem<LN>;
     Smem& sm = *reinterpret_cast<Smem*>(smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u));
@@ -243,6 +243,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) wkv7_bwd_bf16_kernel(BwdParams p,
             load_record(0);
         }
         for (int n = 0; n < work.n; ++n) {
+            if (n + 1 == work.n) stream_release();
             const Desc d = sm.desc[n & 3];
             if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous chunk's output tiles have been read
             __syncthreads();  // (A)
@@ -839,7 +840,7 @@ static_assert(sizeof(WalkSmem) + 1024 <= 232448, "one CTA per SM");
 
 template <bool TAIL>
 __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParams p, float* tiles, int it0, int count, const __grid_constant__ BwdMaps maps) {
-    stream_order();
+    stream_wait();
     extern __shared__ unsigned char smem_dyn[];
     WalkSmem& sm = *reinterpret_cast<WalkSmem*>(smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t4 = lane & 3, w = warp & 3;
@@ -881,6 +882,7 @@ __global__ void __launch_bounds__(WALK_THREADS, 1) wkv7_bwd_walk_kernel(BwdParam
                          ::"r"(smem_u32(t.mats)), "l"(p.ckpt + ((long long)bh * nchunks + c) * CK_FLOATS + CK_AI), "r"((int)sizeof(t.mats)), "r"(smem_u32(&sm.raw_full[s]))
                          : "memory");
         }
+        stream_release();  // (at most SLOTS chunks before the end)
         // shared memory must outlive the loads, also where a wait has given up (n: the first of this warp's loads not issued)
         for (int i = max(warp & 1, n - SLOTS); i < n; i += 2) mbar_wait_bounded<true>(&sm.raw_full[i % SLOTS], (i / SLOTS) & 1, &sm.drain, p.status);
         return;

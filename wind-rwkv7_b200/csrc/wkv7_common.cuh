@@ -415,13 +415,21 @@ __device__ __forceinline__ void mbar_landed_uncounted(uint64_t* bar, volatile in
 }
 
 // Kernels are launched such that they may start before the one ahead of them in the stream has ended (launch() in wkv7_kernels.h), and
-// call this before they touch global memory: what stands before it - barriers, tensor memory - and the launch itself then overlap the
-// other kernel's end.  From here on the next kernel may start, which will in turn wait until this one has ended (a kernel that is not
-// launched so waits by itself); all of its CTAs are then running or have ended, so that none of them has to wait for a place that a CTA
-// of the next one holds.  For the same reason tensor memory is allocated before this call.
-__device__ __forceinline__ void stream_order() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+// call stream_wait() before they touch global memory: what stands before it - barriers, tensor memory - and the launch itself then overlap
+// the other kernel's end.  From stream_release() on, called by at least one thread of each CTA or left to the CTA's end, the next kernel
+// may start, which will in turn wait until this one has ended (a kernel that is not launched so waits by itself).  All CTAs of this kernel
+// are then running or have ended, so that none of them has to wait for a place that a CTA of the next one holds; for the same reason
+// tensor memory is allocated before stream_wait().
+// A kernel releases the next one only when it has waited itself, so that no more than one waits at a time; and kernels whose CTAs walk many
+// chunks release it with their last ones, a few us before they end.  Otherwise the next one's CTAs hold the shared memory of all SMs that
+// a few chains leave idle for as long as those take, and other streams stand still: beside the backward of 12 chains of 1024 chunks
+// (990 us) a forward of 64 chains on another stream is done after 180 to 200 us, with the release at the kernels' start it was after 990;
+// beside twelve forwards of 37 chains of 512 chunks (360 us each) after 195 us instead of 750.  One stream alone: no case slower.
+__device__ __forceinline__ void stream_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void stream_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void stream_order() {  // of a kernel with little to do in each CTA
+    stream_wait();
+    stream_release();
 }
 // a pointer whose target is read through the read-only path: no load may be moved ahead of stream_order()
 template <typename T> __device__ __forceinline__ T* after_stream_order(T* p) {

@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(THREADS_TC, 1) wkv7_fwd_tc_kernel(FwdParams p,
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctrl->tmem_base;
-    stream_order();
+    stream_wait();
 
     // Start state of a segment -> tensor memory and its checkpoint: warp wq of the group owns lanes 32 wq .. 32 wq + 31, of
     // which lanes 0-15 hold value rows 16 wq .. 16 wq + 15.  A chain's first chunk starts from s0 (or zeros); a chain that
@@ -556,10 +556,12 @@ __global__ void __launch_bounds__(THREADS_TC, 1) wkv7_fwd_tc_kernel(FwdParams p,
             if (elect_one()) {
                 const uint32_t sb = smem_u32(sm), dK = desc_kmajor(sb), dMN = desc_mnmajor(sb);
                 int seg_first = 0;
+                const int release_at = max(0, work.n - S);
                 Place<S> at{0, 0};
                 uint32_t Sa = tmem + C_S, Sn = Sa + 64, Sf = Sa + 128;
 #pragma unroll 1
                 for (int c = 0; c < work.n; ++c, at.advance(1)) {
+                    if (c == release_at) stream_release();
                     const uint32_t XY = tmem + C_XY + 32 * at.i, V = tmem + C_V + 16 * at.i, off = at.i * (G_BYTES >> 4), dSC = dK + off + (G_SC >> 4), dKWF = dMN + off + (G_KWF >> 4), dDF = dK + off + (G_DF >> 4);
                     uint32_t A = Sa;
                     if (c == seg_first) {
