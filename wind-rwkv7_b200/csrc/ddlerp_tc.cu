@@ -96,7 +96,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
 
 // ---- prep: W12 = [L (1 - alpha) | L alpha]  [4D, 2C],  R' [C, 4D] -------------------------------------------------------
 __global__ void ddlerp_prep_kernel(const __nv_bfloat16* __restrict__ L, const __nv_bfloat16* __restrict__ alpha, const __nv_bfloat16* __restrict__ R,
-                                   __nv_bfloat16* __restrict__ W12, __nv_bfloat16* __restrict__ Rp, int C, int D) {
+                                   __nv_bfloat16* W12, __nv_bfloat16* Rp, int C, int D) {
     stream_order();
     L = after_stream_order(L); alpha = after_stream_order(alpha); R = after_stream_order(R);
     const int n4 = 4 * D;
@@ -478,7 +478,7 @@ constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u
 // mapD: dpre as (column, time, batch), box 64 x 128 x 1;  mapX: x as (channel, time, batch), box 64 x 128 x 1.
 // grid: (column tiles of 256: first the x_t half, then the x_{t-1} half; token splits; row tiles of 128 of the 4D rows)
 __global__ void __launch_bounds__(g3::THREADS) ddlerp_dw12_kernel(const __grid_constant__ CUtensorMap mapD, const __grid_constant__ CUtensorMap mapX,
-                                                                 float* __restrict__ dW1, float* __restrict__ dW2, int C, int n4, int tiles_per_seq,
+                                                                 float* dW1, float* dW2, int C, int n4, int tiles_per_seq,
                                                                  int total_tiles, int* status) {
     using namespace g3;
     extern __shared__ unsigned char smem_dyn[];
@@ -568,8 +568,8 @@ __global__ void __launch_bounds__(g3::THREADS) ddlerp_dw12_kernel(const __grid_c
 
 // dL = dW1 (1 - alpha) + dW2 alpha, in place (dL holds dW1 on entry); a thread takes 8 rows of one channel.  With dalpha !=
 // nullptr (zero on entry) also dalpha[c] += sum_n L[n, c] (dW2 - dW1)[n, c]  ( = sum_t (dpre L)[t, c] (x_{t-1} - x_t)[c] ).
-__global__ void ddlerp_dl_finish_kernel(float* __restrict__ dL, const float* __restrict__ dW2, const __nv_bfloat16* __restrict__ alpha,
-                                        const __nv_bfloat16* __restrict__ L, float* __restrict__ dalpha, int C, int n4) {
+__global__ void ddlerp_dl_finish_kernel(float* dL, const float* __restrict__ dW2, const __nv_bfloat16* __restrict__ alpha,
+                                        const __nv_bfloat16* __restrict__ L, float* dalpha, int C, int n4) {
     stream_order();
     dW2 = after_stream_order(dW2); alpha = after_stream_order(alpha); L = after_stream_order(L);
     const int c = blockIdx.x * blockDim.x + threadIdx.x, n0 = blockIdx.y * 8;
@@ -612,9 +612,9 @@ __host__ __device__ constexpr int stage_bytes(int D) { return 4 * DY_BYTES + X_B
 
 // The backward's rearranged weights, one launch: R^T as [4D, C] (row k D + d = R[k][:, d]), L^T as [C, 4D], and R' as [C, 4D]
 // (column k D + d = R[k][c][d])
-__global__ void ddlerp_prep_bwd_kernel(const __nv_bfloat16* __restrict__ L, const __nv_bfloat16* __restrict__ R, __nv_bfloat16* __restrict__ Rt,
-                                       __nv_bfloat16* __restrict__ Lt, __nv_bfloat16* __restrict__ Rp, float* __restrict__ dalpha,
-                                       float* __restrict__ dbeta, float* __restrict__ dR, float* __restrict__ dL, float* __restrict__ dW2, int C, int D) {
+__global__ void ddlerp_prep_bwd_kernel(const __nv_bfloat16* __restrict__ L, const __nv_bfloat16* __restrict__ R, __nv_bfloat16* Rt,
+                                       __nv_bfloat16* Lt, __nv_bfloat16* Rp, float* dalpha,
+                                       float* dbeta, float* dR, float* dL, float* dW2, int C, int D) {
     stream_order();
     L = after_stream_order(L); R = after_stream_order(R);
     const int n4 = 4 * D;
@@ -833,8 +833,8 @@ __global__ void __launch_bounds__(g5::THREADS, 1) ddlerp_main_tc_kernel(const __
                                                                        const __nv_bfloat16* __restrict__ dyp1, const __nv_bfloat16* __restrict__ dyp2,
                                                                        const __nv_bfloat16* __restrict__ dyp3, const __nv_bfloat16* __restrict__ dpre,
                                                                        const __nv_bfloat16* __restrict__ mten, const __nv_bfloat16* __restrict__ alpha,
-                                                                       const __nv_bfloat16* __restrict__ beta, float* __restrict__ dR,
-                                                                       float* __restrict__ dbeta, int C, int T, int tiles_per_seq, int tiles, int units,
+                                                                       const __nv_bfloat16* __restrict__ beta, float* dR,
+                                                                       float* dbeta, int C, int T, int tiles_per_seq, int tiles, int units,
                                                                        int* status) {
     using namespace g5;
     constexpr int KB = 4 * D / 64, N4 = 4 * D;

@@ -431,7 +431,8 @@ __device__ __forceinline__ void stream_order() {  // of a kernel with little to 
     stream_wait();
     stream_release();
 }
-// a pointer whose target is read through the read-only path: no load may be moved ahead of stream_order()
+// A __restrict__ pointer of a kernel that waits: without this the compiler may move loads through it ahead of the wait, which it takes not to
+// touch what such a pointer alone leads to.  (Pointers that are not __restrict__ need nothing, and what is written is not.)
 template <typename T> __device__ __forceinline__ T* after_stream_order(T* p) {
     asm volatile("" : "+l"(p) :: "memory");
     return p;
