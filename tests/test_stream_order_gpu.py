@@ -130,3 +130,136 @@ def test_waiting_kernels_leave_idle_sms_to_other_streams(kind, dtype):
     once()  # the allocator has its blocks, the kernels are loaded
     short, whole = min(once() for _ in range(3))
     assert short < whole / (8 if kind == 'forward' else 4), f'{short:.3f} ms of {whole:.3f}'
+
+
+@pytest.mark.parametrize('D', [16, 32, 64])
+def test_ddlerp_sums_start_from_zero(D):
+    """The backward's outputs and its scratch hold NaN before the call.  The weight gradients are fp32 sums by atomics in any order: 1e-5 of
+    their norm between two calls; dx and the scratch's dpre have no such sums."""
+    from wind_rwkv.rwkv7 import _lib
+    lib = _lib.lib()
+    th.manual_seed(D)
+    B, T, C = 2, 130, 128
+    x, al, L, R, be = _bf(B, T, C), _bf(C, std=.5), _bf(4 * D, C, std=.1), _bf(4, C, D, std=.1), _bf(4, C, std=.5)
+    dys = [_bf(B, T, C) for _ in range(4)]
+    m, y = _bf(B, T, 4 * D), _bf(4, B, T, C)
+    assert lib.wkv7_ddlerp_fwd(*[t.data_ptr() for t in (x, al, L, R, be, m, y)], B, T, C, D, _lib.stream_of(x)) == 0
+
+    def call(fill):
+        def buf(*shape, dtype=th.float32):
+            return th.full(shape, fill, dtype=dtype, device='cuda')
+        outs = [buf(B, T, 4 * D, dtype=th.bfloat16), buf(B, T, C, dtype=th.bfloat16), buf(C), buf(4 * D, C), buf(4, C, D), buf(4, C)]
+        ws = buf(lib.wkv7_ddlerp_bwd_tc_workspace_bytes(C, D) // 4)
+        args = [x, al, L, R, be, m] + dys + outs + [ws]
+        assert lib.wkv7_ddlerp_bwd_tc(*[t.data_ptr() for t in args], B, T, C, D, _lib.stream_of(x)) == 0
+        th.cuda.synchronize()
+        assert _lib.device_status() == 0
+        return outs
+    zero, nan = call(0.), call(float('nan'))
+    assert th.equal(zero[0], nan[0]) and th.equal(zero[1], nan[1])
+    for a, b in zip(zero[2:], nan[2:]):
+        assert th.isfinite(b).all() and float((a - b).norm()) <= 1e-5 * float(a.norm())
+
+
+def _op(kind, seed):
+    """(f, outputs' gradients): f() is a whole forward and backward on inputs of its own, without torch kernels of its own between ours."""
+    from wind_rwkv.rwkv7 import attn, attn_ln, expand_loras, synthetic
+    th.manual_seed(seed)
+    if kind in ('ddlerp', 'mixer'):
+        f, ins, g = _ddlerp(2, 130, 128, 32) if kind == 'ddlerp' else _mixer(1, 65, 256)
+    elif kind == 'loras':
+        B, T, C, D = 2, 100, 128, 16
+        ins = ([_bf(B, T, C) for _ in range(2)] + [_bf(B, T, D) for _ in range(4)] + [th.randn(C, D, device='cuda') * .1 for _ in range(4)] +
+               [th.randn(C, device='cuda') * .5 for _ in range(4)])
+        f, g = lambda x: expand_loras(*x, N), [_bf(B, T, C) for _ in range(4)]
+    else:
+        dtype = th.float32 if kind == 'attn_f32' else th.bfloat16
+        B, T, H = (1, 64, 300) if kind == 'attn_cut' else (1, 512, 3) if kind == 'split' else (2, 203, 3)
+        d = synthetic.wkv7_inputs(B, T, H, N, seed=seed, dtype=dtype, device='cuda', s0_std=.1)
+        ins, g = [d[n] for n in 'rwkvab'], [d['dy'], th.randn(B, H, N, N, device='cuda')]
+        if kind == 'split':
+            def f(x):
+                with th.no_grad():
+                    return attn(*x, N, s0=d['s0'], return_state=True, time_split=4)
+            return lambda: list(f(ins))
+        if kind == 'attn_ln':
+            ins += list(synthetic.attn_ln_extras(B, T, H, N, seed=seed, dtype=dtype, device='cuda'))
+        ins.append(d['s0'])
+        f = lambda x: (attn_ln if kind == 'attn_ln' else attn)(*x[:-1], N, s0=x[-1], return_state=True)  # noqa: E731
+    for t in ins:
+        t.requires_grad_()
+
+    def run():
+        y = f(ins)
+        return [t.detach() for t in y] + list(th.autograd.grad(y, ins, g))
+    return run
+
+
+KINDS = ['ddlerp', 'loras', 'mixer', 'attn', 'attn_cut', 'attn_ln', 'attn_f32', 'split']
+
+
+def _same(want, got, kind):
+    for a, b in zip(want, got):
+        assert th.isfinite(b.float()).all()
+        if kind in ('attn', 'attn_cut', 'attn_f32', 'split'):
+            assert th.equal(a, b)
+        else:  # weight gradients are fp32 sums by atomics, in any order
+            assert float((a.float() - b.float()).norm()) <= 1e-5 * float(a.float().norm()) + 1e-12
+
+
+@pytest.mark.parametrize('kind', KINDS)
+def test_back_to_back(kind):
+    """Calls on inputs that were prepared beforehand, nothing else between them: one call's first kernel may start under the last one of the
+    call before, on the memory that the allocator has got back from that."""
+    ops = [_op(kind, i) for i in range(4)]
+    want = []
+    for op in ops:
+        want.append(op())
+        th.cuda.synchronize()
+    for _ in range(3):
+        got = [op() for op in ops]
+        th.cuda.synchronize()
+        for a, b in zip(want, got):
+            _same(a, b, kind)
+
+
+@pytest.mark.parametrize('kind', KINDS)
+def test_two_streams(kind):
+    """Two streams at once, with calls in a row on each."""
+    ops = [_op(kind, i) for i in range(2)]
+    want = [op() for op in ops]
+    th.cuda.synchronize()
+    streams = [th.cuda.Stream() for _ in ops]
+    got = [[], []]
+    for _ in range(4):
+        for i, (s, op) in enumerate(zip(streams, ops)):
+            with th.cuda.stream(s):
+                got[i].append(op())
+    th.cuda.synchronize()
+    for i in range(2):
+        for b in got[i]:
+            _same(want[i], b, kind)
+
+
+@pytest.mark.parametrize('kind', KINDS)
+def test_captured(kind):
+    """The launches recorded in a CUDA graph, twice in a row, and the graph replayed several times on new memory contents."""
+    op = _op(kind, 7)
+    side = th.cuda.Stream()
+    with th.cuda.stream(side):
+        for _ in range(2):
+            want = op()
+    th.cuda.synchronize()
+    want = [t.clone() for t in want]
+    graph = th.cuda.CUDAGraph()
+    with th.cuda.graph(graph):
+        got = [op(), op()]
+    for _ in range(3):
+        for outs in got:
+            for t in outs:
+                t.fill_(float('nan'))
+        graph.replay()
+        graph.replay()
+        th.cuda.synchronize()
+        for b in got:
+            _same(want, b, kind)
