@@ -88,7 +88,7 @@ int wkv7_selftest_bounded_wait(int64_t limit_cycles, int64_t* cycles_out, void* 
 /*
  * Which kernel wkv7_fwd and wkv7_attn_ln_fwd run for io_dtype WKV7_BF16 (no reference counterpart: the reference has one
  * forward kernel per dtype).  0: the warp-MMA kernel (mma.sync TF32, state in registers).  2, 3, 4: the
- * tcgen05 kernel (state in tensor memory) with one chunk more than that in flight per CTA (attn_ln: four chunks); negative values
+ * tcgen05 kernel (state in tensor memory) with 3, 4 or 5 chunks in flight per CTA (attn_ln: 4 with each of the three values); negative values
  * select the same kernel without the producer-side rounding of operands to TF32 (the tensor core then
  * truncates them: 0.4 % faster, about twice the state error).  The default is 4, or the value of the environment variable WKV7_FWD_TC when the library
  * is loaded.  Returns WKV7_ERR_SHAPE for any other value.  The fp32 dtypes always use the warp-MMA

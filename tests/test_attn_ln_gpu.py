@@ -152,3 +152,22 @@ def test_config2_dparams_slice():
     cut = lambda x: x.detach()[:, :, hs].double().cpu().numpy().reshape(B, T, 2, N)
     go = c_oracle.attn_ln_bwd(*[cut(x) for x in dev], cut(g), params.detach()[:, hs].double().cpu().numpy(), cut(d['dy']))
     assert maxabs_rms(pd.grad[:, hs], go[7]) <= 2e-2
+
+
+@pytest.mark.parametrize('sign', [1, -1])
+def test_sizes_of_the_forward_setting_are_one_kernel(sign):
+    """attn_ln has four chunks in flight a CTA whatever the size of the setting; its sign selects rounded or truncated operands."""
+    from wind_rwkv.rwkv7 import _lib, attn_ln, synthetic
+    B, T, H = 2, 203, 90
+    d = synthetic.wkv7_inputs(B, T, H, N, seed=0, dtype=th.bfloat16, device='cuda')
+    g, params = synthetic.attn_ln_extras(B, T, H, N, seed=0, dtype=th.bfloat16, device='cuda')
+
+    def run(impl):
+        _lib.set_fwd_impl(impl)
+        with th.no_grad():
+            return attn_ln(*[d[n] for n in NAMES], g, params, N, return_state=True)
+    y, sT = run(4 * sign)
+    for size in (2, 3):
+        y2, sT2 = run(size * sign)
+        assert th.equal(y, y2) and th.equal(sT, sT2)
+    assert not th.equal(sT, run(-4 * sign)[1])

@@ -50,7 +50,7 @@ float* static_scratch() {
 }
 
 // Forward implementation for bf16 attn (see wkv7_set_fwd_impl in the header): 0 = warp-MMA kernel,
-// +-2..4 = tcgen05 kernel with that many preparation groups.
+// +-2..4 = tcgen05 kernel with 3..5 slots (attn_ln: 4), negative: operands not rounded.
 bool valid_fwd_impl(int x) { return x == 0 || (x >= 2 && x <= 4) || (x <= -2 && x >= -4); }
 std::atomic<int>& fwd_impl() {
     static std::atomic<int> v([] {
@@ -203,8 +203,8 @@ static int fwd_common(const void* r, const void* w, const void* k, const void* v
     p.status = status_ptr();
     if (!p.status) return WKV7_ERR_LAUNCH;
     if (io_dtype == WKV7_BF16) {
-        const int groups = fwd_impl().load(std::memory_order_relaxed);
-        if (groups) return wkv7::launch_fwd_tc(p, groups, ln, (cudaStream_t)stream);
+        const int impl = fwd_impl().load(std::memory_order_relaxed);
+        if (impl) return wkv7::launch_fwd_tc(p, impl, ln, (cudaStream_t)stream);
     }
     return wkv7::launch_fwd(p, io_dtype, ln, (cudaStream_t)stream);
 }
@@ -249,7 +249,7 @@ int wkv7_fwd_time_split(const void* r, const void* w, const void* k, const void*
     for (const void* p : ptrs)
         if (p && !aligned16(p)) return WKV7_ERR_ALIGN;
     if (B * nseg * H > 0x7fffffff) return WKV7_ERR_TOO_LARGE;
-    const int groups = fwd_impl().load(std::memory_order_relaxed);
+    const int impl = fwd_impl().load(std::memory_order_relaxed);
     wkv7::FwdParams p{};
     p.r = r; p.w = w; p.k = k; p.v = v; p.a = a; p.b = b; p.s0 = s0; p.y = y; p.sT = sT;
     p.B = B; p.T = T; p.H = H;
@@ -257,7 +257,7 @@ int wkv7_fwd_time_split(const void* r, const void* w, const void* k, const void*
     p.flags = (unsigned*)workspace;
     p.status = status_ptr();
     if (!p.status) return WKV7_ERR_LAUNCH;
-    return wkv7::launch_fwd_time_split(p, (int)nseg, groups ? groups : 4, (cudaStream_t)stream);
+    return wkv7::launch_fwd_time_split(p, (int)nseg, impl ? impl : 4, (cudaStream_t)stream);
 }
 
 int wkv7_step(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* s0,

@@ -1204,21 +1204,21 @@ int launch_bounded_wait_selftest(long long limit_cycles, int* status, long long*
     return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
 }
 
-template <bool LN> static int launch_ln(const FwdParams& p, int groups, cudaStream_t stream) {
-    switch (groups) {
-        case 2: return tc::launch_t<LN ? 4 : 3, true, LN>(p, stream);
-        case 3: return tc::launch_t<LN ? 4 : 4, true, LN>(p, stream);
-        case 4: return tc::launch_t<LN ? 4 : 5, true, LN>(p, stream);
-        case -2: return tc::launch_t<LN ? 4 : 3, false, LN>(p, stream);
-        case -3: return tc::launch_t<LN ? 4 : 4, false, LN>(p, stream);
-        case -4: return tc::launch_t<LN ? 4 : 5, false, LN>(p, stream);
+// impl as wkv7_set_fwd_impl has it: its size selects attn's slots, its sign whether operands are rounded.  Five slots are the default because
+// they are faster at every size: with three / four / five, L2 flushed, B64 T1024 H12 340 / 301 / 283 us, with checkpoints 387 / 371 / 369;
+// B8 T8192 H40 1002 / 868 / 809; B3 T1003 H16 72 / 64 / 61.  attn_ln has room for four beside its epilogue's tiles.
+int launch_fwd_tc(const FwdParams& p, int impl, bool ln, cudaStream_t stream) {
+    if (p.sM) return p.T % L ? tc::launch_tt<5, true, false, true, true>(p, stream) : tc::launch_tt<5, true, false, false, true>(p, stream);
+    if (ln) return impl > 0 ? tc::launch_t<4, true, true>(p, stream) : tc::launch_t<4, false, true>(p, stream);
+    switch (impl) {
+        case 2: return tc::launch_t<3, true, false>(p, stream);
+        case 3: return tc::launch_t<4, true, false>(p, stream);
+        case 4: return tc::launch_t<5, true, false>(p, stream);
+        case -2: return tc::launch_t<3, false, false>(p, stream);
+        case -3: return tc::launch_t<4, false, false>(p, stream);
+        case -4: return tc::launch_t<5, false, false>(p, stream);
         default: return kBadShape;
     }
-}
-
-int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream) {
-    if (p.sM) return p.T % L ? tc::launch_tt<5, true, false, true, true>(p, stream) : tc::launch_tt<5, true, false, false, true>(p, stream);
-    return ln ? launch_ln<true>(p, groups, stream) : launch_ln<false>(p, groups, stream);
 }
 
 }  // namespace wkv7

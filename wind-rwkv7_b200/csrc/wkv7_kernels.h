@@ -90,12 +90,12 @@ size_t bwd_workspace_bytes(long long B, long long T, long long H, bool ln);  // 
 size_t bwd32_workspace_bytes(long long B, long long T, long long H);         // and for fp32 ones, attn
 int launch_reduce_dparams(const BwdParams& p, cudaStream_t stream);  // dparams = sum over the batch of dparams_ws
 int launch_bwd(const BwdParams& p, int io_dtype, bool ln, cudaStream_t stream);
-// tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true); |groups| + 1 = chunks in flight per CTA (2..4; attn_ln: always four chunks); negative: operands are
-// not rounded to TF32 by their producer (the tensor core truncates them)
-int launch_fwd_tc(const FwdParams& p, int groups, bool ln, cudaStream_t stream);
+// tcgen05 forward (bf16 IO; attn, or attn_ln with ln = true).  impl 2, 3, 4: a CTA has 3, 4 or 5 slots, i.e. chunks in flight (attn_ln: always 4); negative:
+// the same with operands not rounded to TF32 by their producer (the tensor core truncates them)
+int launch_fwd_tc(const FwdParams& p, int impl, bool ln, cudaStream_t stream);
 // bf16 forward with the sequences cut into nseg segments each (wkv7_time_split.cu)
 size_t time_split_workspace_bytes(long long B, long long H, int nseg);
-int launch_fwd_time_split(const FwdParams& p, int nseg, int groups, cudaStream_t stream);
+int launch_fwd_time_split(const FwdParams& p, int nseg, int impl, cudaStream_t stream);
 // for each of `count` products C[M,N] = act(A[M,K] W[N,K]^T), bf16, A's rows lda apart, tanh on columns [tanh_from, tanh_to); tcgen05 + TMA (proj_gemm.cu)
 constexpr int PROJ_MAX = 6;
 int launch_proj_gemm(int count, const void* const* A, const void* const* W, void* const* C, const int64_t* N, const int64_t* K, const int64_t* lda,

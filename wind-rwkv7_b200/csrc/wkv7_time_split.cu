@@ -73,7 +73,7 @@ static_assert(ROWS == 8 && N == 64, "thread mapping");
 size_t time_split_workspace_bytes(long long B, long long H, int nseg) { return WORK_FLAG_BYTES + 3 * (size_t)(B * nseg * H) * NN * sizeof(float); }
 
 // p: the whole sequences, p.st.b == p.T * p.st.t, p.T % nseg == 0, p.flags: the workspace
-int launch_fwd_time_split(const FwdParams& p, int nseg, int groups, cudaStream_t stream) {
+int launch_fwd_time_split(const FwdParams& p, int nseg, int impl, cudaStream_t stream) {
     const long long chains = p.B * nseg * p.H;
     float* start = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(p.flags) + WORK_FLAG_BYTES);
     float *R = start + chains * NN, *M = R + chains * NN;
@@ -81,13 +81,13 @@ int launch_fwd_time_split(const FwdParams& p, int nseg, int groups, cudaStream_t
     q.T = p.T / nseg; q.st.b = q.T * p.st.t;
     q.B = p.B == 1 ? nseg - 1 : p.B * nseg;
     q.sT = R; q.sM = M; q.nseg = nseg;
-    int rc = launch_fwd_tc(q, groups, false, stream);
+    int rc = launch_fwd_tc(q, impl, false, stream);
     if (rc != kOk) return rc;
     split_starts_kernel<<<dim3((unsigned)(p.B * p.H), N / ROWS), 128, 0, stream>>>(p.s0, R, M, start, nseg, p.H);
     if (cudaGetLastError() != cudaSuccess) return kLaunchFailed;
     q.B = p.B * nseg;
     q.s0 = start; q.sM = nullptr;
-    if ((rc = launch_fwd_tc(q, groups, false, stream)) != kOk) return rc;
+    if ((rc = launch_fwd_tc(q, impl, false, stream)) != kOk) return rc;
     for (long long b = 0; b < p.B; ++b)
         if (p.sT && cudaMemcpyAsync(p.sT + b * p.H * NN, R + (b * nseg + nseg - 1) * p.H * NN, p.H * NN * sizeof(float), cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
             return kLaunchFailed;

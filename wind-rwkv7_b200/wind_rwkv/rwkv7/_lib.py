@@ -194,8 +194,8 @@ def device_status():
 
 
 def set_fwd_impl(impl):
-    """Selects the bf16 attn forward kernel: 0 = warp-MMA, 2..4 = tcgen05 with that many preparation
-    groups (negative: operands truncated, not rounded, to TF32).  Returns the previous value."""
+    """Selects the bf16 forward kernel of attn and attn_ln: 0 = warp-MMA, 2..4 = tcgen05 with 3..5 chunks in flight a CTA
+    (attn_ln: always 4; negative: operands truncated, not rounded, to TF32).  Returns the previous value."""
     old = lib().wkv7_get_fwd_impl()
     check(lib().wkv7_set_fwd_impl(int(impl)), 'wkv7_set_fwd_impl')
     return old
