@@ -620,7 +620,7 @@ __global__ void ddlerp_prep_bwd_kernel(const __nv_bfloat16* __restrict__ L, cons
     const int n4 = 4 * D;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)C * n4) return;
-    // the sums that the following kernels add to start from zero (as five memsets they were 18 us of a backward at B32 T1024 C768)
+    // the sums that the following kernels add to start from zero (five memsets took 11 us of 318 more, forward and backward, B32 T1024 C768)
     dR[i] = dL[i] = dW2[i] = 0.f;
     if (i < 4 * C) dbeta[i] = 0.f;
     if (i < C) dalpha[i] = 0.f;

@@ -22,7 +22,7 @@ constexpr int HC = 64;  // channels per head
 // Seven special-function instructions an element (three tanh for the sigmoids, ex2 + lg2 for the softplus, ex2 for E), everything
 // else two elements an instruction: the op is bound by issue slots.
 struct Gates { F2 a, ma, mk, w, E; };
-__device__ __forceinline__ float lg2_approx(float x) {  // of 1 + e^.., at least 1: __log2f spends three instructions more on denormal arguments
+__device__ __forceinline__ float lg2_approx(float x) {  // of 1 + e^.., at least 1; with __log2f B32 T1024 C768, forward and backward, took 276 us, with this 271
     float y;
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;

@@ -355,11 +355,12 @@ template <int PREC, int X = 0> __device__ __forceinline__ void tri_inverse_colum
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// Bounded wait for the phase of an mbarrier with the given parity; the one wait every kernel of this library uses.
+// Bounded wait for the phase of an mbarrier with the given parity, of all kernels but the tcgen05 forward, which has one of its own
+// (mbar_wait in wkv7_fwd_tc.cu: the same limits, a poll interval of 40 ns, the status word written when the CTA ends).
 // Returns at once, false, when the CTA has aborted.  When `limit` clocks pass without the phase completing it raises the
 // CTA's abort flag (every later wait then falls through), records kDeviceTimeout in the device status word and
 // returns: a lost copy or a missing arrival ends with an error code, never with a hung GPU.
-// SLEEP: the thread is suspended by the hardware (try_wait with a time hint) instead of polling.
+// SLEEP: 100 ns between polls, for warps that wait for long beside others that work.
 constexpr long long MBAR_WAIT_LIMIT = 1LL << 28;  // clocks (~0.14 s): far beyond any legitimate wait within a CTA
 // The wait for another CTA's half of a cut chain (wait_handoff below) may legitimately take longer: the CTAs of one launch run at
 // different speeds when other work shares the GPU with them, and a range of work can be 0.1 s long.  The waits of the same CTA that
@@ -378,10 +379,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     const uint32_t addr = smem_u32(bar);
     const uint32_t start = clock(), most = (uint32_t)limit;
     uint32_t spin = 0;
-    // Polling variant: the abort flag is read after every failed probe.  A tighter loop that looked at it only every
-    // 32nd probe made the tcgen05 forward 1.3 % slower: the chain's polls take issue slots from the working warps.
-    // The loop is kept as small as it can be: it is inlined at some fifteen places, and the tcgen05 forward's warps run
-    // different code at the same time out of one instruction cache (the clock64 form of this loop was 1 KB a place).
+    // (The loop is kept as small as it can be: it is inlined at many places of kernels whose loops fill the instruction cache; with
+    // 64-bit clocks it was 1 KB a place.)
     for (;;) {
         uint32_t ok;
         asm volatile("{\n.reg .pred P;\nmbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\nselp.u32 %0, 1, 0, P;\n}\n"
@@ -420,7 +419,7 @@ __device__ __forceinline__ void mbar_landed_uncounted(uint64_t* bar, volatile in
 // may start, which will in turn wait until this one has ended (a kernel that is not launched so waits by itself).  All CTAs of this kernel
 // are then running or have ended, so that none of them has to wait for a place that a CTA of the next one holds; for the same reason
 // tensor memory is allocated before stream_wait().
-// A kernel releases the next one only when it has waited itself, so that no more than one waits at a time; and kernels whose CTAs walk many
+// A kernel releases the next one only when it has waited itself, so that no more than one of a stream waits; and kernels whose CTAs walk many
 // chunks release it with their last ones, a few us before they end.  Otherwise the next one's CTAs hold the shared memory of all SMs that
 // a few chains leave idle for as long as those take, and other streams stand still: beside the backward of 12 chains of 1024 chunks
 // (990 us) a forward of 64 chains on another stream is done after 180 to 200 us, with the release at the kernels' start it was after 990;

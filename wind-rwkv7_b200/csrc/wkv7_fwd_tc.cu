@@ -17,7 +17,9 @@
 // What bounds it: the instructions of its 24 warps, 3500 a chunk, at 60 % of the issue slots, with some 1000 shared-memory wavefronts of loads
 // and stores and 360 of operand reads beside them; a group's loop (scan, loads, operand tiles, the scores' product) is 4400 cycles for every
 // third chunk, the chain itself some 1000.  1400 cycles a chunk without checkpoints (B8 T8192 H40: 795 us, 881 before the slots, the
-// readers and the helper below), 1850 with (B64 T1024 H12: 332 us, 3.3 TB/s of it written, which is what bounds that).
+// readers and the helper below), 1850 with (B64 T1024 H12: 332 us, 3.3 TB/s of it written).  With them, 7 % more instructions at 52 % of the
+// issue slots, and the raw tiles come late out of a DRAM that is at 4.8 TB/s: 4.6 warps per issue wait for loads instead of 2.9.  It is not the
+// writes alone: of 369 us with the L2 flushed, the records' matrices left out (a fifth of 1 GB) save 16, the states 57, both 86.
 //
 // Warp roles (768 threads).  A chunk's operand tiles, scores and results lie in one of S slots of shared and tensor memory, a place
 // apart from the warps that fill it: chunk c has slot c % S from its tiles until its results have been read.  (With a slot per preparation

@@ -7,9 +7,9 @@
 namespace wkv7 {
 
 // Launches a kernel that calls stream_wait(): it may start while the one ahead of it in the stream drains.  For kernels that follow others
-// closely: B32 T1024 C768, ddlerp forward and backward 315 -> 289 us (with five memsets less), expand_loras 284 -> 276, time mixer 2081 ->
-// 2028; layer of 515 rows, C = 2048, forward 151 -> 136; B3 T1003 H16, attn forward and backward 178 -> 171.  (Not so launched, since
-// it did not pay: the fp32 forward, B8 T512 H12 287 -> 293 us, and the sums between the two walks of time_split, 497 -> 521.)
+// closely.  Without / with this alone, us: B32 T1024 C768, ddlerp forward and backward 307 / 288, expand_loras 277 / 269, time mixer 2104 /
+// 2073; layer of 515 rows, C = 2048, forward 149 / 134; attn forward and backward, B3 T1003 H16 170 / 163, fp32 B8 T512 H12 289 / 285.  (Not so
+// launched, since it did not pay: the fp32 forward, B8 T512 H12 287 -> 293 us, and the sums between the two walks of time_split, 497 -> 521.)
 template <typename... P, typename... A> inline bool launch(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t c{};
     c.gridDim = grid; c.blockDim = dim3(threads); c.dynamicSmemBytes = smem; c.stream = stream;

@@ -15,8 +15,8 @@
 // CTA, not by each of the 64 rows (8192 exponentials per chain).
 // What is left is the state traffic: 2 * 16 KB per chain and call, all loads of it in flight before the first barrier, six CTAs an
 // SM (40 registers; at 76 registers and three CTAs 1.2 times as long).  Many chains, up to eight steps: wkv7_step_ring_kernel below.
-// Both start while the kernel ahead of them drains (stream_order): steps in a row, T = 1, 6400 chains 37.3 -> 35.9 us, 3200 20.5 -> 18.1, 1280 10.3 ->
-// 8.9, 768 8.3 -> 6.5, and the smallest calls, whose time is the host's, 6.1 -> 5.5.  (The next but one state on its way, too: 10240 chains 56.3 -> 59.4.)
+// Both start while the kernel ahead of them drains (stream_order): steps in a row, T = 1, 6400 chains 37.0 -> 35.8 us, 3200 20.5 -> 18.0, 1280 10.3 ->
+// 8.9, 768 8.2 -> 6.4, and the smallest calls, whose time is the host's, 6.1 -> 5.6.  (The next but one state on its way, too: 10240 chains 56.3 -> 59.4.)
 #include "wkv7_kernels.h"
 
 namespace wkv7 {
