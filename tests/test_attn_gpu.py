@@ -134,6 +134,18 @@ def test_tcgen05_variants(impl):
         _lib.set_fwd_impl(old)
 
 
+@pytest.mark.parametrize('impl', [2, 3, 4, -2, -3, -4])
+@pytest.mark.parametrize('T', [9, 90, 203])
+def test_tcgen05_variants_partial_last_chunk(T, impl):
+    """Three, four and five chunks in flight with sequences that end within a chunk (builds of their own), against the oracle."""
+    from wind_rwkv.rwkv7 import _lib
+    old = _lib.set_fwd_impl(impl)
+    try:
+        run_case(2, T, 3, th.bfloat16, s0=True, dsT=True, seed=T)
+    finally:
+        _lib.set_fwd_impl(old)
+
+
 @pytest.mark.parametrize('dtype', [th.float32, th.bfloat16])
 def test_upstream_test_distribution(dtype):
     """Value distributions of tests/test_attn.py:25-30 at its check shape (B2 T1024 C64), 4 of 12 heads."""
